@@ -332,76 +332,102 @@ template <> __device__ __forceinline__ float rg_gate_act<bf16>(float z) {
 }
 
 // spans [n_seq, 3] = {slot, first row, rows}, or null: every row is a sequence of its own with the slot of tok_slot.
-#define RG_SUB 4             // tokens to a group of the scan's ring of inputs
-#define RG_DEPTH 8           // groups in the ring: 32 tokens' inputs under way
-#define RG_SCAN_THREADS 32    // one warp to a block: one long prompt of a few thousand channels then reaches every SM
+//
+// A block of one warp walks 32 channels of a sequence (one long prompt of a few thousand channels then reaches every SM);
+// the inputs of the next 60 tokens are under way into shared memory by asynchronous copies, in groups of four tokens (three
+// copies of 16 bytes a lane).  What bounds a walk is a trip to memory divided by the tokens under way.  Loads into
+// registers could not keep 32 tokens under way however they were written: a warp has six counters for loads under way, and
+// waiting for one group's waits for every later load on the same counter.  Measured with 2,494 rows of 5,120 channels in four
+// prompts of up to 900 tokens (153 MB): 144 us with the ring in registers, 63 us so.
+#define RG_SUB 4             // tokens to a group
+#define RG_DEPTH 16          // groups in the ring
+#define RG_SCAN_THREADS 32
 template <typename T>
 __global__ void __launch_bounds__(RG_SCAN_THREADS)
 rglru_scan_kernel(const float* __restrict__ a, const float* __restrict__ b, const T* __restrict__ y, long long ldy,
                   const void* __restrict__ y_bias, int bias_dtype, float* __restrict__ state, long long state_stride,
                   const int* __restrict__ spans, const int* __restrict__ tok_slot, T* __restrict__ out, long long ldo,
-                  int width) {
+                  int width, int wide) {
     gi_pdl_start();
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    if (c >= width) return;
+    const int lane = threadIdx.x, cw = blockIdx.y * RG_SCAN_THREADS, c = cw + lane;
+    const bool live = c < width;
     int slot, start, len;
     if (spans) { slot = spans[3 * blockIdx.x]; start = spans[3 * blockIdx.x + 1]; len = spans[3 * blockIdx.x + 2]; }
     else { slot = tok_slot[blockIdx.x]; start = blockIdx.x; len = 1; }
     if (slot < 0) {
-        for (int t = 0; t < len; ++t) out[(size_t)(start + t) * ldo + c] = from_f32<T>(0.f);
+        for (int t = 0; t < len && live; ++t) out[(size_t)(start + t) * ldo + c] = from_f32<T>(0.f);
         return;
     }
-    const float yb = y_bias ? load_w(y_bias, bias_dtype, c) : 0.f;
-    float S = state[(size_t)slot * state_stride + c];
+    const float yb = y_bias && live ? load_w(y_bias, bias_dtype, c) : 0.f;
+    float S = live ? state[(size_t)slot * state_stride + c] : 0.f;
     if (len == 1) {                                          // a decode step's row: nothing to run ahead of
+        if (!live) return;
         const size_t r = (size_t)start;
         S = fmaf(a[r * width + c], S, b[r * width + c]);
         out[r * ldo + c] = from_f32<T>(S * rg_gate_act<T>(to_f32(y[r * ldy + c]) + yb));
         state[(size_t)slot * state_stride + c] = S;
         return;
     }
-    // The inputs of the next 32 tokens are on their way while a token is walked: a ring of eight groups of four
-    // tokens in registers, each refilled right after it was used; beyond that the lines of the 32 tokens after
-    // those are asked into L2 (a hint: lane j names token j of them).  A group is walked in two passes: the chain of
-    // dependent multiply-adds alone, then the gate branch's activation and the products, which wait for nothing.
-    const int lane = threadIdx.x & 31;
-    const size_t cw = (size_t)(c - lane);                    // the warp's first channel
-    float ra[RG_DEPTH][RG_SUB], rb[RG_DEPTH][RG_SUB], ry[RG_DEPTH][RG_SUB];
-    auto fetch = [&](int t0, float (&fa)[RG_SUB], float (&fb)[RG_SUB], float (&fy)[RG_SUB]) {
+    __shared__ __align__(16) float a_s[RG_DEPTH][RG_SUB][32], b_s[RG_DEPTH][RG_SUB][32];
+    __shared__ __align__(16) T y_s[RG_DEPTH][RG_SUB][32];
+    const int groups = (len + RG_SUB - 1) / RG_SUB;
+    // lane l copies 16 bytes of token l / 8 of a group (bytes beyond the last channel are zero-filled); a group's last
+    // tokens beyond the sequence are its last row again, and not walked
+    auto fetch = [&](int grp) {
+        if (grp < groups) {
+            const int s = grp % RG_DEPTH;
+            if (wide) {
+                const int j = lane >> 3, o = (lane & 7) * 4, n = min(16, max(0, (width - cw - o) * 4));
+                const size_t at = (size_t)(start + min(grp * RG_SUB + j, len - 1)) * width + (n ? cw + o : 0);
+                rg_cp_async_16(&a_s[s][j][o], a + at, n);
+                rg_cp_async_16(&b_s[s][j][o], b + at, n);
+                constexpr int PER = 16 / (int)sizeof(T), LPR = 32 / PER;       // elements to a copy, lanes to a row
+                if (lane < RG_SUB * LPR) {
+                    const int jy = lane / LPR, oy = lane % LPR * PER, ny = min(16, max(0, (width - cw - oy) * (int)sizeof(T)));
+                    rg_cp_async_16(&y_s[s][jy][oy], y + (size_t)(start + min(grp * RG_SUB + jy, len - 1)) * ldy + (ny ? cw + oy : 0), ny);
+                }
+            } else {
+                for (int j = 0; j < RG_SUB; ++j) {           // rows that do not start on 16 bytes
+                    const size_t r = (size_t)(start + min(grp * RG_SUB + j, len - 1));
+                    a_s[s][j][lane] = live ? a[r * width + c] : 0.f;
+                    b_s[s][j][lane] = live ? b[r * width + c] : 0.f;
+                    y_s[s][j][lane] = live ? y[r * ldy + c] : from_f32<T>(0.f);
+                }
+            }
+        }
+        rg_cp_async_commit();
+    };
+    for (int g = 0; g < RG_DEPTH - 1; ++g) fetch(g);
+    T* dst = out + (size_t)start * ldo + c;
+    for (int grp = 0; grp < groups; ++grp) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(RG_DEPTH - 2));
+        __syncwarp();                                        // every lane's copies of this group, and the last group's reads
+        fetch(grp + RG_DEPTH - 1);
+        // The chain of dependent multiply-adds alone, then what waits for nothing, all four tokens of it side by side and
+        // outside any branch: a warp has its scheduler nearly to itself, so a serial step costs its whole latency.
+        const int s = grp % RG_DEPTH, left = len - grp * RG_SUB;
+        float ga[RG_SUB], gb[RG_SUB], gy[RG_SUB];
 #pragma unroll
         for (int j = 0; j < RG_SUB; ++j) {
-            const bool in = t0 + j < len;
-            const size_t r = (size_t)(start + (in ? t0 + j : 0));
-            fa[j] = in ? a[r * width + c] : 1.f;             // beyond the sequence: S stays as it is
-            fb[j] = in ? b[r * width + c] : 0.f;
-            fy[j] = in ? to_f32(y[r * ldy + c]) : 0.f;
-        }
-    };
-#pragma unroll
-    for (int d = 0; d < RG_DEPTH; ++d) fetch(d * RG_SUB, ra[d], rb[d], ry[d]);
-    for (int t0 = 0; t0 < len; t0 += RG_DEPTH * RG_SUB) {
-        if (t0 + 2 * RG_DEPTH * RG_SUB + lane < len) {
-            const size_t r = (size_t)(start + t0 + 2 * RG_DEPTH * RG_SUB + lane);
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(a + r * width + cw));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(b + r * width + cw));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(y + r * ldy + cw));
+            ga[j] = a_s[s][j][lane];
+            gb[j] = b_s[s][j][lane];
+            gy[j] = rg_gate_act<T>(to_f32(y_s[s][j][lane]) + yb);
         }
 #pragma unroll
-        for (int d = 0; d < RG_DEPTH; ++d) {
-            const int t1 = t0 + d * RG_SUB;
-            float sv[RG_SUB];
-#pragma unroll
-            for (int j = 0; j < RG_SUB; ++j) {
-                S = fmaf(ra[d][j], S, rb[d][j]);
-                sv[j] = S;
-            }
-#pragma unroll
-            for (int j = 0; j < RG_SUB; ++j)
-                if (t1 + j < len) out[(size_t)(start + t1 + j) * ldo + c] = from_f32<T>(sv[j] * rg_gate_act<T>(ry[d][j] + yb));
-            fetch(t1 + RG_DEPTH * RG_SUB, ra[d], rb[d], ry[d]);
+        for (int j = 0; j < RG_SUB; ++j) {
+            S = fmaf(j < left ? ga[j] : 1.f, S, j < left ? gb[j] : 0.f);      // beyond the sequence: S stays as it is
+            gy[j] *= S;
         }
+        T v[RG_SUB];
+#pragma unroll
+        for (int j = 0; j < RG_SUB; ++j) v[j] = from_f32<T>(gy[j]);
+#pragma unroll
+        for (int j = 0; j < RG_SUB; ++j)
+            if (j < left && live) dst[(size_t)j * ldo] = v[j];
+        dst += (size_t)RG_SUB * ldo;
     }
-    state[(size_t)slot * state_stride + c] = S;
+    rg_cp_async_wait_0();
+    if (live) state[(size_t)slot * state_stride + c] = S;
 }
 
 extern "C" int gi_rglru_scan(const float* a, const float* b, const void* y, long long ldy, int act_dtype, const void* y_bias,
@@ -411,13 +437,15 @@ extern "C" int gi_rglru_scan(const float* a, const float* b, const void* y, long
     GI_REQUIRE((width + RG_SCAN_THREADS - 1) / RG_SCAN_THREADS <= 65535, "gi_rglru_scan: %d channels", width);
     if (n_seqs == 0) return 0;
     dim3 grid(n_seqs, (width + RG_SCAN_THREADS - 1) / RG_SCAN_THREADS);
+    const int item = act_dtype == GI_DTYPE_F32 ? 4 : 2;
+    const int wide = width % 4 == 0 && ldy * item % 16 == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) % 16 == 0;
     cudaStream_t s = (cudaStream_t)stream;
     if (act_dtype == GI_DTYPE_F32)
         gi_launch(rglru_scan_kernel<float>, grid, dim3(RG_SCAN_THREADS), 0, s, a, b, (const float*)y, ldy, y_bias, bias_dtype, state,
-                  state_stride, spans, tok_slot, (float*)out, ldo, width);
+                  state_stride, spans, tok_slot, (float*)out, ldo, width, wide);
     else if (act_dtype == GI_DTYPE_BF16)
         gi_launch(rglru_scan_kernel<bf16>, grid, dim3(RG_SCAN_THREADS), 0, s, a, b, (const bf16*)y, ldy, y_bias, bias_dtype, state,
-                  state_stride, spans, tok_slot, (bf16*)out, ldo, width);
+                  state_stride, spans, tok_slot, (bf16*)out, ldo, width, wide);
     else
         GI_REQUIRE(false, "gi_rglru_scan: activation dtype %d", act_dtype);
     return gi_check_launch("gi_rglru_scan");

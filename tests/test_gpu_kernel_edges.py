@@ -45,3 +45,33 @@ def test_causal_convolution_over_runs_of_rows(dtype, K, C, pad, lens):
             want_state[s, :(K - 1) * C] = seen[m:].reshape(-1)
         at += m
     assert (state.double() - want_state).abs().max() <= 2.0 ** -23 * 8
+
+
+# ---- scan of the recurrent unit --------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width, pad", [(32, 8), (100, 0), (66, 2), (35, 0), (324, 4)])
+@pytest.mark.parametrize("lens", [[1, 2], [3, 4, 5], [59, 60, 61], [64, 130, 1]])
+def test_recurrent_scan_at_the_ends_of_its_ring(dtype, width, pad, lens):
+    """Sequences around the number of tokens that are under way, channels that are and are not whole warps and whole
+    16-byte words, and a portion of padding rows."""
+    from garlic_inference_b200.ops import kernels
+    n = sum(lens) + 3
+    a, b = torch.rand(n, width, generator=torch.Generator().manual_seed(1)).to(DEV), rnd(n, width, seed=2)
+    y, yb, state = rnd(n, width + pad, seed=3, dtype=dtype)[:, :width], rnd(width, seed=4), rnd(len(lens) + 1, width + 4, seed=5)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    spans = torch.tensor([[i, s, m] for i, (s, m) in enumerate(zip(starts, lens))] + [[-1, n - 3, 3]], dtype=torch.int32, device=DEV)
+    before, slots = state.clone(), torch.zeros(n, dtype=torch.int32, device=DEV)
+    got = kernels.rglru_scan(a, b, y, yb, state, spans, slots)
+    act = torch.nn.functional.gelu(y.double() + yb.double(), approximate="tanh")
+    for i, (s, m) in enumerate(zip(starts, lens)):
+        S, low = before[i, :width].double(), torch.zeros(width, dtype=torch.float64, device=DEV)
+        for t in range(s, s + m):
+            S = a[t].double() * S + b[t].double()
+            low = a[t].double() * low + 2.0 ** -23 * S.abs()               # a rounding a token, carried along
+            tol = (low + 1e-6) * act[t].abs() + (2.0 ** -20 if dtype == torch.float32 else 2.0 ** -7) * (S * act[t]).abs() + 1e-6
+            if dtype == torch.bfloat16:                                    # the hardware's tanh: 2^-10.9 of 1
+                tol = tol + 0.5 * 2.0 ** -10 * (S * (y[t].double() + yb.double())).abs()
+            assert ((got[t].double() - S * act[t]).abs() <= tol).all()
+        assert ((state[i, :width].double() - S).abs() <= low + 1e-6).all()
+    assert float(got[n - 3:].abs().max()) == 0.0 and torch.equal(state[len(lens)], before[len(lens)])
+    assert torch.equal(state[:, width:], before[:, width:])
