@@ -47,6 +47,39 @@ def test_causal_convolution_over_runs_of_rows(dtype, K, C, pad, lens):
     assert (state.double() - want_state).abs().max() <= 2.0 ** -23 * 8
 
 
+# ---- gates of the recurrent unit -------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("blocks, bw", [(3, 8), (2, 64), (3, 72), (2, 320), (2, 20)])
+@pytest.mark.parametrize("n", [1, 17, 128, 129, 300])
+def test_recurrent_gates_with_bfloat16_matrices(blocks, bw, n):
+    """Blocks narrower than a tile of outputs, whole and part tiles of outputs, inputs and rows; an infinite input; the
+    same bits for a row alone and among others."""
+    from garlic_inference_b200.ops import kernels
+    W = blocks * bw
+    u = rnd(n, W, seed=1, scale=2.0)
+    u[n - 1, 1] = math.inf
+    wa, wi = (rnd(blocks, bw, bw, seed=s, scale=bw ** -0.5, dtype=torch.bfloat16) for s in (2, 3))
+    ba, bi, lam = rnd(W, seed=4), rnd(W, seed=5), rnd(W, seed=6, scale=2.0)
+    a, b = kernels.rglru_gates(u, wa, wi, ba, bi, lam, 8.0)
+    ud = u.double().view(n, blocks, bw)
+    z = [torch.einsum("nbi,bio->nbo", ud, w.double()).reshape(n, W) + v.double() for w, v in ((wa, ba), (wi, bi))]
+    # every addition of a partial sum may lose one unit of the largest partial sum's last place
+    dz = [(3 * bw / 16 + 3) * 2.0 ** -23 * (torch.einsum("nbi,bio->nbo", ud.abs(), w.double().abs()).reshape(n, W) + v.double().abs())
+          for w, v in ((wa, ba), (wi, bi))]
+    log_a = -8.0 * torch.sigmoid(z[0]) * torch.nn.functional.softplus(lam.double())
+    want_a = torch.exp(log_a)
+    want_b = torch.sqrt(-torch.expm1(2 * log_a)) * torch.sigmoid(z[1]) * u.double()
+    fine = torch.ones(n, W, dtype=torch.bool, device=DEV)
+    fine[n - 1, :bw] = False                                               # the block that holds the infinite input
+    tol_a = want_a * (log_a.abs() * (dz[0] + 2.0 ** -20) + 2.0 ** -21)
+    tol_b = want_b.abs() * (dz[0] + dz[1] + 2.0 ** -19)
+    assert ((a.double() - want_a).abs() <= tol_a + 1e-30)[fine].all()
+    assert ((b.double() - want_b).abs() <= tol_b + 1e-30)[fine].all()
+    torch.testing.assert_close(a[n - 1, :bw].double(), want_a[n - 1, :bw], rtol=1e-5, atol=1e-30)
+    assert torch.equal(b[n - 1, :bw].isfinite(), want_b[n - 1, :bw].isfinite())
+    alone = kernels.rglru_gates(u[n // 2:n // 2 + 1].contiguous(), wa, wi, ba, bi, lam, 8.0)
+    assert torch.equal(alone[0][0], a[n // 2]) or bool(alone[0][0].isnan().any())
+
+
 # ---- scan of the recurrent unit --------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width, pad", [(32, 8), (100, 0), (66, 2), (35, 0), (324, 4)])
