@@ -108,3 +108,23 @@ def test_recurrent_scan_at_the_ends_of_its_ring(dtype, width, pad, lens):
         assert ((state[i, :width].double() - S).abs() <= low + 1e-6).all()
     assert float(got[n - 3:].abs().max()) == 0.0 and torch.equal(state[len(lens)], before[len(lens)])
     assert torch.equal(state[:, width:], before[:, width:])
+
+
+# ---- float32 product -------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("N, K", [(1, 4), (17, 7), (64, 128), (200, 130), (1100, 260), (4800, 36)])
+def test_float32_product_has_the_same_bits_by_every_kernel(N, K):
+    """Row counts on both sides of every choice of kernel and tile, sizes that are and are not whole tiles, slices and
+    16-byte words, rows that lie apart: all against 64 bits, and every row with the bits of its product alone."""
+    from garlic_inference_b200.ops import kernels
+    w, full = rnd(N, K, seed=1), rnd(700, K + 5, seed=2)
+    alone = {}
+    for M in (1, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 129, 300, 700):
+        for a in (full[:M, :K].contiguous(), full[:M, :K]):
+            out = torch.full((M, N + 3), 7.0, device=DEV)
+            kernels.sgemm_nt_strided(a, w, out[:, :N])
+            want = a.double() @ w.double().T
+            tol = (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)       # a rounding an addition
+            assert ((out[:, :N].double() - want).abs() <= tol).all() and bool((out[:, N:] == 7.0).all())
+            for r in {0, M // 2, M - 1}:
+                one = alone.setdefault(r, kernels.sgemm_nt(full[r:r + 1, :K].contiguous(), w)[0])
+                assert torch.equal(out[r, :N], one), f"{M} rows, row {r}"
