@@ -1470,42 +1470,60 @@ def attention_decode_masked_bf16(q: torch.Tensor, k_pool: torch.Tensor, v_pool: 
     return out
 
 
-def tcgen05_attention_takes(dtype: torch.dtype, head_dim: int, page_size: int) -> bool:
-    """Whether the tcgen05 prefill attention takes this element type, head size and page size."""
-    return dtype == torch.bfloat16 and head_dim == 128 and page_size % 64 == 0
+def tcgen05_attention_takes(dtype: torch.dtype, head_dim: int, page_size: int, value_dim: Optional[int] = None,
+                            n_dist: int = 0, means: bool = False, column_gate: bool = False) -> bool:
+    """Whether the tcgen05 prefill attention takes this element type, head size (and size of the values, where it is
+    another) and page size, with a table of `n_dist` biases by distance, rows for blocks (`means`) or a gate per
+    output column.  The table lies in shared memory beside the tiles, two blocks to an SM."""
+    d, dv = head_dim, value_dim or head_dim
+    if dtype != torch.bfloat16 or page_size % 64 or d not in (64, 128) or dv not in (64, 128):
+        return False
+    if means and (d, dv) != (128, 128) or (column_gate or n_dist) and (d, dv) == (64, 128):
+        return False
+    tiles = 256 * d + 2 * 128 * (d + dv)                      # the query tile and two stages of keys and of values
+    return n_dist == 0 or (not means and not column_gate and tiles + 1536 + 4 * (n_dist + 384) <= 113 << 10)
 
 
 def attention_prefill_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor,
                               q_tiles128: torch.Tensor, scale: float, window: int, rows_covered: bool = False,
                               chunk: int = 0, sinks: Optional[torch.Tensor] = None, means=None, keep_first: int = 0,
-                              gate: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Flash attention of q [n, n_q, 128] over the paged cache on tcgen05 tensor cores (TMA-fed, S, P and
-    P V in tensor memory).  `q_tiles128` int32 [n_tiles, 4] cuts the rows into runs of at most 128
-    consecutive tokens of one sequence: {slot, first row, rows, position of the first row}.  `chunk` > 0: a query
+                              gate: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, maps: int = 1,
+                              dist_bias: Optional[torch.Tensor] = None, rot: Optional[tuple] = None) -> torch.Tensor:
+    """Flash attention of q [n, n_q * maps, d] over the paged cache on tcgen05 tensor cores (TMA-fed, S, P and
+    P V in tensor memory), d and the values' dv 64 or 128.  `q_tiles128` int32 [n_tiles, 4] cuts the rows into runs of at
+    most 128 consecutive tokens of one sequence: {slot, first row, rows, position of the first row}.  `chunk` > 0: a query
     sees only the keys of its own chunk of positions.  `sinks` float32 [n_q]: a score per head that joins the
-    softmax's denominator without a value.  `means`, `keep_first`: as `attention_masked`.  `gate` [n, n_q * 128] (rows
-    that start on 16 bytes) or [n, n_q]: logits whose sigmoid multiplies the result.  `out` [n, n_q * 128]: written
-    there, rows in no tile stay as they are."""
+    softmax's denominator without a value.  `means`, `keep_first`, `dist_bias`: as `attention_masked`; `maps`: as
+    `attention_prefill_masked_bf16`.  `gate` [n, n_q * dv] (rows that start on 16 bytes) or [n, n_q]: logits whose sigmoid
+    multiplies the result.  `out` [n, n_q * maps * dv] (rows may lie apart): written there, rows in no tile stay as they
+    are.  `rot` = (rows [positions, columns], first column): the last 64 of q's 192 dimensions meet these 64 columns of a
+    row per position, the same for all heads (paged as the pools are), and k_pool holds the first 128."""
     l = require_gpu()
     _dense(q, "q", torch.bfloat16), _dense(k_pool, "k_pool", torch.bfloat16), _dense(v_pool, "v_pool", torch.bfloat16)
     _dense(block_table, "block_table", torch.int32), _dense(q_tiles128, "q_tiles128", torch.int32)
-    n, n_q, d = q.shape
-    n_pages, n_kv, page_size, pool_d = k_pool.shape
-    if pool_d != d or v_pool.shape != k_pool.shape:
-        raise KernelError(f"cache pools {tuple(k_pool.shape)} do not fit head_dim {d}")
+    n, rows, d, dv, n_pages, n_kv, page_size = _masked_shapes(q if rot is None else q[:, :, :q.shape[2] - 64], k_pool, v_pool, maps)
+    rot_args = (None, 0, 0)
+    if rot is not None:
+        shared, first = rot
+        _rows(shared, "rot", torch.bfloat16)
+        if shared.shape[0] < n_pages * page_size or not 0 <= first <= shared.shape[1] - 64:
+            raise KernelError(f"a shared key part in columns {first} .. of {tuple(shared.shape)} for {n_pages * page_size} positions")
+        d, rot_args = d + 64, (_ptr(shared), shared.stride(0), int(first))
     if q_tiles128.dim() != 2 or q_tiles128.shape[1] != 4 or q_tiles128.data_ptr() % 16:
         raise KernelError("q_tiles128 must be int32 [n_tiles, 4] starting on 16 bytes")
     # rows in no tile (padding) stay zero; when the caller says that every row lies in a tile, nothing is filled
-    _check_sinks_bias(sinks, None, n_q)
+    n_dist = _check_sinks_bias(sinks, dist_bias, rows)
     if out is None:
-        out = (torch.empty if rows_covered else torch.zeros)((n, n_q * d), dtype=q.dtype, device=q.device)
-    elif _dense(out, "out", q.dtype).shape != (n, n_q * d):
-        raise KernelError(f"out {tuple(out.shape)} for a result of {(n, n_q * d)}")
+        out = (torch.empty if rows_covered else torch.zeros)((n, rows * dv), dtype=q.dtype, device=q.device)
+    elif _rows(out, "out", q.dtype).shape != (n, rows * dv):
+        raise KernelError(f"out {tuple(out.shape)} for a result of {(n, rows * dv)}")
     check(l.gi_attention_prefill_tcgen05(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(block_table), _ptr(q_tiles128),
-                                         q_tiles128.shape[0], _ptr(out), n, n_q, n_kv, d, page_size,
+                                         q_tiles128.shape[0], _ptr(out), out.stride(0) if n > 1 else rows * dv, n, rows // maps,
+                                         n_kv, d, dv, int(maps), page_size,
                                          block_table.shape[1], n_pages, int(window or 0), int(chunk or 0), float(scale),
                                          _ptr(tcgen05_error_flag(q.device)), _ptr(sinks), *_means_args(means, k_pool, v_pool),
-                                         int(keep_first), *_gate_args(gate, n, n_q, d), _stream()), l)
+                                         int(keep_first), *_gate_args(gate, n, rows, dv), *rot_args, _ptr(dist_bias), n_dist,
+                                         _stream()), l)
     return out
 
 

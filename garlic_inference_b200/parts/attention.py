@@ -110,8 +110,8 @@ class GQAAttention(Mixer):
         """Attention of q [n, n_q, d] over the cache; returns [n, n_q * d].
 
         bfloat16 with heads of 128 and pages that are a multiple of 64 tokens: the tcgen05 kernels (flash
-        attention for runs of tokens, split-KV when every sequence brings one token and the group is at most
-        16).  Otherwise bfloat16 with a head size the mma.sync kernels take: the split-KV kernel for single
+        attention for runs of tokens, for heads of 64 too; split-KV when every sequence brings one token and the group
+        is at most 16).  Otherwise bfloat16 with a head size the mma.sync kernels take: the split-KV kernel for single
         tokens, the flash kernel for runs.  Everything else (float32, other head sizes, larger groups in
         decode) goes to the exact-order kernel."""
         covered = (not ctx.all_single) and ctx.n_tokens == sum(ctx.seq_lens)

@@ -41,8 +41,8 @@ value tensors: the schedule points it at another layer's cache entry, whose keys
 them: after convolution and rotation) it reads with its own queries, mask and everything else.
 
 All projections that read x are one packed product.  Which attention runs: in bfloat16, with key and value
-sizes that the tensor-core kernels take (multiples of 16 up to 128, equal or one twice the other; one map with
-keys and values of 128 and pages of a multiple of 64 tokens: the tcgen05 prompt kernel): the flash
+sizes that the tensor-core kernels take (multiples of 16 up to 128, equal or one twice the other; keys and values
+of 64 or 128 and pages of a multiple of 64 tokens: the tcgen05 prompt kernel, every map in one launch): the flash
 kernel for steps that bring several tokens of a sequence and the split-KV kernel for decode steps, once per map,
 with the chunk mask in them (float32 scores, softmax and sums; the weights rounded to bfloat16 as the second
 product's operand).  Everything else (float32, other sizes): the exact-order kernel, whose result at a position does not depend on how the tokens were cut into steps.  What
@@ -214,10 +214,12 @@ class MaskedAttention(Mixer):
         return kernels.mma_attention_takes(self.rt.dtype, self.d, self.dv)
 
     def _run_rows(self, kv) -> int:
-        """Height of the query runs of the prompt kernel that takes this mixer: 128 (tcgen05: one map, keys and
-        values of 128, pages of a multiple of 64), 64 (mma.sync), 0 (the exact-order kernel, which needs none)."""
-        if self.maps == 1 and self.d == self.dv and self.dist_bias is None and \
-                kernels.tcgen05_attention_takes(self.rt.dtype, self.d, kv.page_size):
+        """Height of the query runs of the prompt kernel that takes this mixer: 128 (tcgen05: keys and values of 64 or
+        128, pages of a multiple of 64, and what `tcgen05_attention_takes` says of the rest), 64 (mma.sync), 0 (the
+        exact-order kernel, which needs none)."""
+        if kernels.tcgen05_attention_takes(self.rt.dtype, self.d, kv.page_size, self.dv,
+                                           n_dist=0 if self.dist_bias is None else self.dist_bias.shape[0],
+                                           means=bool(self.pool), column_gate=self.output_gate):
             return 128
         return 64 if self._tensor_cores() else 0
 
@@ -286,8 +288,7 @@ class MaskedAttention(Mixer):
             if rows == 128:
                 att = kernels.attention_prefill_tcgen05(q, kv.k_pool, kv.v_pool, kv.block_table, runs, self.scale,
                                                         self.window, rows_covered=covered, chunk=self.chunk,
-                                                        sinks=self.sinks, means=kv.means, keep_first=self.keep_first,
-                                                        gate=inside)
+                                                        maps=self.maps, gate=inside, **extras)
             else:
                 att = kernels.attention_prefill_masked_bf16(q, kv.k_pool, kv.v_pool, kv.block_table, runs, self.scale,
                                                             window=self.window, chunk=self.chunk, maps=self.maps,

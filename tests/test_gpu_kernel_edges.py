@@ -128,3 +128,103 @@ def test_float32_product_has_the_same_bits_by_every_kernel(N, K):
             for r in {0, M // 2, M - 1}:
                 one = alone.setdefault(r, kernels.sgemm_nt(full[r:r + 1, :K].contiguous(), w)[0])
                 assert torch.equal(out[r, :N], one), f"{M} rows, row {r}"
+
+
+# ---- tcgen05 prompt attention at sizes other than heads of 128 -------------------------------------------------------------
+def _pools(lens, heads, d, page, seed, extra_pages=3):
+    """(dense [len, heads, d] per sequence, pool, block table) with pages handed out in a mixed order."""
+    need = [-(-n // page) for n in lens]
+    order = torch.randperm(sum(need) + extra_pages, generator=torch.Generator().manual_seed(3)).tolist()
+    pool = rnd(len(order), heads, page, d, seed=seed + 1, dtype=torch.bfloat16)
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    dense = []
+    for s, n in enumerate(lens):
+        x = rnd(n, heads, d, seed=seed + 10 + s, dtype=torch.bfloat16)
+        for lp in range(need[s]):
+            table[s, lp] = order.pop()
+            part = x[lp * page:(lp + 1) * page]
+            pool[int(table[s, lp]), :, :len(part)] = part.transpose(0, 1)
+        dense.append(x)
+    return dense, pool, table.to(DEV)
+
+
+def _runs128(lens, new):
+    from garlic_inference_b200.parts import StepShape
+    from garlic_inference_b200.parts.attention import query_runs
+    starts = [sum(new[:i]) for i in range(len(new))]
+    shape = StepShape(list(range(len(lens))), starts, new, [n - m for n, m in zip(lens, new)], False)
+    return torch.from_numpy(query_runs(shape, 128)).to(DEV), starts
+
+
+def _attend64(q, k, v, pos0, scale, window=0, chunk=0, keep=0, sink=None, bias=None):
+    """q [m, d] of one head at positions pos0 .., k [n, d], v [n, dv] in 64 bits."""
+    i = pos0 + torch.arange(q.shape[0], device=DEV)[:, None]
+    j = torch.arange(k.shape[0], device=DEV)[None]
+    seen = (j <= i) & ((i - j < window) | (j < keep) if window else True) & ((i // chunk == j // chunk) if chunk else True)
+    s = q.double() @ k.double().T * scale
+    if bias is not None:
+        s = s + bias.double()[(i - j).clamp(0, len(bias) - 1)]
+    s = s.masked_fill(~seen, -math.inf)
+    top = s.max(-1, keepdim=True).values if sink is None else torch.maximum(s.max(-1, keepdim=True).values, sink.double())
+    e = torch.exp(s - top)
+    return e @ v.double() / (e.sum(-1, keepdim=True) + (0.0 if sink is None else torch.exp(sink.double() - top)))
+
+
+# the probabilities' rounding to 8 bits (2^-8 of a weighted mean of values of size 1, up to 4 here), their exponent's and the
+# result's own: one part in 100 of the largest value
+ATT_TOL = dict(rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("d, dv, maps, n_dist, page", [(64, 64, 1, 0, 64), (64, 128, 2, 0, 64), (64, 128, 1, 0, 128), (128, 64, 1, 0, 64),
+                                                       (128, 64, 1, 90, 64), (64, 64, 1, 700, 128), (128, 128, 1, 1, 64), (64, 64, 2, 0, 64)])
+@pytest.mark.parametrize("mask", [{}, {"window": 70}, {"window": 33, "keep_first": 70}, {"chunk": 100}])
+def test_prompt_attention_on_tensor_memory_at_other_sizes(d, dv, maps, n_dist, page, mask):
+    """Tiles that are and are not whole, portions behind cached tokens, every mask, several maps per head, tables of biases
+    shorter and longer than the sequences, sinks and gates where they are taken."""
+    from garlic_inference_b200.ops import kernels
+    H, G = 6, 2
+    lens, new = [1, 37, 300, 64, 65, 513], [1, 37, 250, 64, 3, 513]
+    assert kernels.tcgen05_attention_takes(torch.bfloat16, d, page, dv, n_dist=n_dist)
+    ks, k_pool, table = _pools(lens, G * maps, d, page, 20)
+    vs, v_pool, _ = _pools(lens, G, dv, page, 60)
+    runs, starts = _runs128(lens, new)
+    n, scale = sum(new) + 2, d ** -0.5                                     # two rows in no tile
+    q = rnd(n, H * maps, d, seed=5, dtype=torch.bfloat16)
+    bias = rnd(n_dist, H, seed=6) if n_dist else None
+    for sinks, gate in [(None, None)] + ([(rnd(H, seed=7), None)] if maps == 1 else []) + \
+            ([(None, rnd(n, H, seed=8, dtype=torch.bfloat16)), (None, rnd(n, H * dv, seed=9, dtype=torch.bfloat16))]
+             if maps == 1 and not n_dist and (d, dv) != (64, 128) else []):
+        kw = dict(sinks=sinks, gate=gate, maps=maps, dist_bias=bias, chunk=mask.get("chunk", 0), keep_first=mask.get("keep_first", 0))
+        got = kernels.attention_prefill_tcgen05(q, k_pool, v_pool, table, runs, scale, mask.get("window", 0), **kw).view(n, H * maps, dv)
+        assert float(got[-2:].abs().max()) == 0.0
+        wide = torch.full((n, H * maps * dv + 8), 3.0, dtype=torch.bfloat16, device=DEV)      # into columns of a wider matrix
+        kernels.attention_prefill_tcgen05(q, k_pool, v_pool, table, runs, scale, mask.get("window", 0), out=wide[:, 8:], **kw)
+        assert torch.equal(wide[:-2, 8:].reshape(-1), got[:-2].reshape(-1)) and bool((wide[:, :8] == 3.0).all()) and bool((wide[-2:] == 3.0).all())
+        for s, (at, m) in enumerate(zip(starts, new)):
+            for hh in range(H * maps):
+                h, g = hh // maps, hh // maps // (H // G)
+                want = _attend64(q[at:at + m, hh], ks[s][:, g * maps + hh % maps], vs[s][:, g], lens[s] - m, scale,
+                                 mask.get("window", 0), mask.get("chunk", 0), mask.get("keep_first", 0),
+                                 None if sinks is None else sinks[h], None if bias is None else bias[:, h])
+                if gate is not None:
+                    want = want * torch.sigmoid((gate if gate.shape[1] == H * dv else gate.repeat_interleave(dv, 1))[at:at + m, h * dv:(h + 1) * dv].double())
+                torch.testing.assert_close(got[at:at + m, hh].double(), want, **ATT_TOL)
+    kernels.check_bounded_waits(torch.device("cuda", 0))
+
+
+@pytest.mark.parametrize("past, m", [(0, 1), (0, 129), (63, 70), (300, 40)])
+@pytest.mark.parametrize("window", [0, 90])
+def test_prompt_attention_with_a_key_part_that_all_heads_share(past, m, window):
+    """Keys of 128 and a shared part of 64 in columns of rows of their own, with a sink and a gate per head."""
+    from garlic_inference_b200.ops import kernels
+    H, T, scale = 3, past + m, 192 ** -0.5
+    pad = -(-T // 64) * 64
+    k, v, rows = (rnd(*shape, seed=i, dtype=torch.bfloat16) for i, shape in enumerate([(1, H, pad, 128), (1, H, pad, 128), (pad, 88)]))
+    q, gate, sinks = rnd(m, H, 192, seed=4, dtype=torch.bfloat16), rnd(m, H, seed=5, dtype=torch.bfloat16), rnd(H, seed=6)
+    table = torch.zeros((1, 1), dtype=torch.int32, device=DEV)
+    runs, _ = _runs128([T], [m])
+    got = kernels.attention_prefill_tcgen05(q, k, v, table, runs, scale, window, rot=(rows, 16), gate=gate, sinks=sinks).view(m, H, 128)
+    for h in range(H):
+        want = _attend64(q[:, h], torch.cat([k[0, h, :T], rows[:T, 16:80]], -1), v[0, h, :T], past, scale, window, sink=sinks[h])
+        torch.testing.assert_close(got[:, h].double(), want * torch.sigmoid(gate[:, h:h + 1].double()), **ATT_TOL)
+    kernels.check_bounded_waits(torch.device("cuda", 0))
