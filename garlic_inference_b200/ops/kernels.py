@@ -1060,7 +1060,7 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor
     return out
 
 
-def latent_prepare(q_src: torch.Tensor, q_off: int, kv_src: Optional[torch.Tensor], c_off: int, q_lat: torch.Tensor,
+def latent_prepare(q_src: torch.Tensor, q_off: int, kv_src: Optional[torch.Tensor], c_off: int, q_lat: Optional[torch.Tensor],
                    norm_w: Optional[torch.Tensor], eps: float, freq: torch.Tensor, magnitude: float, n_rot: int,
                    tok_pos: torch.Tensor, tok_slot: torch.Tensor, block_table: torch.Tensor, pool: torch.Tensor,
                    n_heads: int, plain_dim: int, rot_dim: int, rank: int, status: torch.Tensor, append: bool = True,
@@ -1069,11 +1069,14 @@ def latent_prepare(q_src: torch.Tensor, q_off: int, kv_src: Optional[torch.Tenso
     shared key part | zeros] into `pool` [pages, 1, page_size, row] from columns c_off .. of `kv_src` (None for a
     layer that reads rows another layer cached) and returns the queries [n, heads, row] = [q' | rotated part |
     zeros], q' = `q_lat` [n, heads, rank], the rotated part from `q_src`'s columns (heads of plain_dim + rot_dim from
-    q_off on).  `half_layout`: dimension i turns with i + n_rot/2 instead of 2i with 2i + 1."""
+    q_off on).  With `q_lat` None the queries keep their own unrotated columns: [n, heads, plain_dim + rot_dim].
+    `half_layout`: dimension i turns with i + n_rot/2 instead of 2i with 2i + 1."""
     l = require_gpu()
     act = q_src.dtype
-    _rows(q_src, "q_src"), _dense(q_lat, "q_lat", act), _dense(freq, "freq", torch.float32)
+    _rows(q_src, "q_src"), _dense(freq, "freq", torch.float32)
     _dense(pool, "pool", act)
+    if q_lat is not None:
+        _dense(q_lat, "q_lat", act)
     if kv_src is not None:
         _rows(kv_src, "kv_src", act), _dense(norm_w, "norm_w")
     elif append:
@@ -1082,10 +1085,10 @@ def latent_prepare(q_src: torch.Tensor, q_off: int, kv_src: Optional[torch.Tenso
         _dense(t, name, torch.int32)
     n = q_src.shape[0]
     n_pages, one, page_size, row_w = pool.shape
-    if one != 1 or q_lat.shape != (n, n_heads, rank) or freq.numel() * 2 != n_rot or \
+    if one != 1 or (q_lat is not None and q_lat.shape != (n, n_heads, rank)) or freq.numel() * 2 != n_rot or \
             (kv_src is not None and norm_w.numel() != rank):
         raise KernelError("latent_prepare: the pool, q_lat, the norm weight or the frequencies do not fit the sizes")
-    q_out = torch.empty((n, n_heads, row_w), dtype=act, device=q_src.device)
+    q_out = torch.empty((n, n_heads, row_w if q_lat is not None else plain_dim + rot_dim), dtype=act, device=q_src.device)
     check(l.gi_latent_prepare(_ptr(q_src), q_src.stride(0), q_off, _ptr(kv_src), kv_src.stride(0) if kv_src is not None else 0,
                               c_off, int(half_layout), _ptr(q_lat), code(act), _ptr(norm_w),
                               code(norm_w.dtype) if norm_w is not None else F32, float(eps), _ptr(freq), float(magnitude),

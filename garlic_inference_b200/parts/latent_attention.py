@@ -30,11 +30,13 @@ float32) is this package's kernel, and the weighted sum is a second product [tok
 kv_rank]; the sequence's rows are gathered from its pages once per step and the tokens are cut into blocks
 whose scores fit `SCORE_BYTES`.  Tensor cores do both products; the weights are rounded to bfloat16 only as
 the second product's operand.
-Without a rotated part, portions of plain_dim + value_dim tokens and more in bfloat16 (sizes that the flash kernels take)
-expand the keys and values they see, [heads, keys, plain_dim] and [heads, keys, value_dim] by two batched products of the
+Long portions in bfloat16 (from plain_dim + value_dim tokens on without a rotated part, at sizes that the flash kernels
+take; from `ROT_MIN_ROWS` on, at a sequence's start from PRODUCT_MIN_ROWS on, with a rotated part of 64 beside 128 plain dimensions and values of 128) expand the keys and
+values they see, [heads, keys, plain_dim] and [heads, keys, value_dim] by two batched products of the
 gathered rows, and run the flash kernel for prompts over them as one large page (tcgen05 for sizes of 128, mma.sync
-otherwise; window, sink and gate inside it): an expanded key costs kv_rank (plain_dim + value_dim) once and saves about
-kv_rank per new token, and no scores are written to memory.
+otherwise; window, sink and gate inside it; a rotated part is read from the gathered rows, the same for all heads): an
+expanded key costs kv_rank (plain_dim + value_dim) once and saves about kv_rank per new token, and no scores are written
+to memory.
 The rotation is the position part's (its frequencies, magnitude and layout: pairs (2i, 2i+1), or halves (i,
 i + n/2)).  Upstream has grouped-query attention only (src/models/qwen3/qwen3.cpp:140-179).
 """
@@ -54,6 +56,12 @@ from .linear_attention import pack_rows
 PRODUCT_MIN_ROWS = 32
 SCORE_BYTES = 256 << 20        # float32 scores of one block of tokens (all heads, all keys)
 WINDOW_BLOCK = 256             # tokens of a block when a window cuts the keys
+# From how many new tokens of a sequence behind cached ones on its keys and values are expanded when they have a rotated
+# part (a sequence's first tokens: from PRODUCT_MIN_ROWS on).  Everything before the output product of a layer of 4,096 with
+# 32 heads over a latent of 512, by products with the latent rows / expanded, in us: 32 tokens alone 47 / 38, 256 alone
+# 101 / 54, 2,048 alone 836 / 193; behind 2,000: 64 81 / 97, 128 112 / 102, 256 175 / 107; behind 6,000: 128 206 / 213,
+# 512 669 / 236.
+ROT_MIN_ROWS = 128
 EXPAND_BYTES = 2 << 30         # keys and values of one sequence expanded for a portion
 
 
@@ -131,9 +139,12 @@ class LatentAttention(Mixer):
 
     def _expands(self, n_new: int, past: int, page: int) -> bool:
         keys = (-(-(past + n_new) // page) - self._first_page(past, page)) * page
-        return (self.rt.dtype == torch.bfloat16 and self.dr == 0 and n_new >= max(PRODUCT_MIN_ROWS, self.d + self.dv)
+        if self.dr == 0:
+            least, taken = max(PRODUCT_MIN_ROWS, self.d + self.dv), kernels.mma_attention_takes(self.rt.dtype, self.d, self.dv)
+        else:
+            least, taken = ROT_MIN_ROWS if past else PRODUCT_MIN_ROWS, (self.d, self.dr, self.dv) == (128, 64, 128) and self.rank % 8 == 0 and keys % 64 == 0
+        return (self.rt.dtype == torch.bfloat16 and n_new >= least and taken
                 and self.w_uv.dtype == torch.bfloat16 and self.w_uk_t.dtype == torch.bfloat16
-                and kernels.mma_attention_takes(self.rt.dtype, self.d, self.dv)
                 and self.H * keys * (self.d + self.dv) * 2 <= EXPAND_BYTES)
 
     def _run_rows(self, keys: int) -> int:
@@ -155,7 +166,7 @@ class LatentAttention(Mixer):
         return which, np.concatenate(runs) if runs else np.zeros((0, 4), dtype=np.int32)
 
     def _runs_name(self, page: int) -> str:
-        return f"latent_runs_{self.window}_{page}_{self.d}_{self.dv}_{self.H}"
+        return f"latent_runs_{self.window}_{page}_{self.d}_{self.dr}_{self.dv}_{self.rank}_{self.H}"
 
     def step_arrays(self, shape, cache):
         page = cache.kv.page_size
@@ -164,7 +175,8 @@ class LatentAttention(Mixer):
         return {self._runs_name(page): lambda: self._runs_of(shape, page)[1]}
 
     def _attend_expanded(self, q, kv, ctx, which, gate, out):
-        """Attention of the expanded portions of q [n, H, plain_dim], gated, into their rows of `out` [n, H * value_dim]."""
+        """Attention of the expanded portions of q [n, H, plain_dim + rot_dim] (its rotated part turned), gated, into their
+        rows of `out` [n, H * value_dim]."""
         page = kv.page_size
         pool = kv.k_pool.view(kv.k_pool.shape[0], page, self.row)
         runs = ctx.arrays.get(self._runs_name(page))
@@ -176,11 +188,12 @@ class LatentAttention(Mixer):
         for i, p0, keys, rows in which:
             n_runs = -(-ctx.seq_lens[i] // rows)
             c = pool.index_select(0, kv.block_table[ctx.seq_slots[i], p0:p0 + keys // page].long()).view(1, keys, self.row)
+            rot = {"rot": (c[0], self.rank)} if self.dr else {}
             c = c[:, :, :self.rank].expand(self.H, keys, self.rank)
             k, v = torch.bmm(c, self.w_uk_t), torch.bmm(c, self.w_uv.transpose(1, 2))
             args = (q, k.unsqueeze(0), v.unsqueeze(0), self._one_page, runs[at:at + n_runs], self.scale)
             if rows == 128:
-                kernels.attention_prefill_tcgen05(*args, self.window, sinks=self.sink_f32, gate=gate, out=out)
+                kernels.attention_prefill_tcgen05(*args, self.window, sinks=self.sink_f32, gate=gate, out=out, **rot)
             else:
                 kernels.attention_prefill_masked_bf16(*args, window=self.window, sinks=self.sink_f32, gate=gate, out=out)
             at += n_runs
@@ -211,19 +224,27 @@ class LatentAttention(Mixer):
         q = q_src[:, q_off:q_off + self.H * (self.d + self.dr)].view(n, self.H, self.d + self.dr)
         plain = not self.head_gate and out is None and out_mul == 1.0
         gate = proj[:, self.g_off:self.g_off + self.H] if self.head_gate else None
-        # portions whose keys and values are expanded (the latents above are in the cache by now)
+        prepared = (self.c_norm, self.eps, freq, magnitude, n_rot, ctx.tok_pos, ctx.tok_slot, kv.block_table, kv.k_pool, self.H,
+                    self.d, self.dr, self.rank, ctx.status)
+        # portions whose keys and values are expanded
         which = []
-        if both and out is None and out_mul == 1.0 and not ctx.all_single and not ctx.captured and ctx.seq_lens:
+        if (both or self.dr) and out_mul == 1.0 and not ctx.all_single and not ctx.captured and ctx.seq_lens:
             which, _ = self._runs_of(ctx, kv.page_size)
-        if len(which) == len(ctx.seq_lens) > 0 and n == sum(ctx.seq_lens):
-            done = torch.empty((n, self.H * self.dv), dtype=self.rt.dtype, device=x.device)
-            self._attend_expanded(q.contiguous(), kv, ctx, which, gate, done)
+            # columns to write into: rows that start on 16 bytes, and not by the mma.sync kernel
+            if out is not None and (any(rows != 128 for *_, rows in which) or out.data_ptr() % 16 or out.stride(0) % 8):
+                which = []
+        whole = len(which) == len(ctx.seq_lens) > 0 and n == sum(ctx.seq_lens)
+        if which:
+            q_own = q.contiguous() if not self.dr else \
+                kernels.latent_prepare(q_src, q_off, proj if self.own_kv else None, self.c_off or 0, None, *prepared,
+                                       append=writes_cache and whole, half_layout=half)
+        if whole:                                    # the latents are in the cache by now
+            done = torch.empty((n, self.H * self.dv), dtype=self.rt.dtype, device=x.device) if out is None else out
+            self._attend_expanded(q_own, kv, ctx, which, gate, done)
             return done
         q_lat = per_head_linear(q[:, :, :self.d], self.w_uk_t)                       # [n, H, rank]
         q_rows = q_lat if both and self.row == self.rank else \
-            kernels.latent_prepare(q_src, q_off, proj if self.own_kv and not both else None, self.c_off or 0, q_lat,
-                                   self.c_norm, self.eps, freq, magnitude, n_rot, ctx.tok_pos, ctx.tok_slot, kv.block_table,
-                                   kv.k_pool, self.H, self.d, self.dr, self.rank, ctx.status,
+            kernels.latent_prepare(q_src, q_off, proj if self.own_kv and not both else None, self.c_off or 0, q_lat, *prepared,
                                    append=writes_cache and not both, half_layout=half)
         o_lat = self.attend(q_rows, kv, ctx, skip={w[0] for w in which})
         # with a gate (or a factor, or columns to write into) the values leave their product in float32 and are
@@ -234,7 +255,7 @@ class LatentAttention(Mixer):
         if not plain:
             done = kernels.attn_finish(done, self.H, 1, None, None, out_mul, gate, self.rt.dtype, out=out)
         if which:
-            self._attend_expanded(q.contiguous(), kv, ctx, which, gate, done)
+            self._attend_expanded(q_own, kv, ctx, which, gate, done)
         return done
 
     def attend(self, q_rows, kv, ctx, skip=frozenset()):

@@ -228,3 +228,81 @@ def test_prompt_attention_with_a_key_part_that_all_heads_share(past, m, window):
         want = _attend64(q[:, h], torch.cat([k[0, h, :T], rows[:T, 16:80]], -1), v[0, h, :T], past, scale, window, sink=sinks[h])
         torch.testing.assert_close(got[:, h].double(), want * torch.sigmoid(gate[:, h:h + 1].double()), **ATT_TOL)
     kernels.check_bounded_waits(torch.device("cuda", 0))
+
+
+# ---- latent attention: portions whose keys and values are expanded beside a rotated part -----------------------------------
+@pytest.mark.parametrize("layout, q_rank, gate, sink, pad", [("half", 24, True, False, 0), ("interleaved", 0, False, True, 8),
+                                                             ("half", 24, True, True, 3)])
+@pytest.mark.parametrize("lens, past", [([130], [0]), ([200, 3, 64, 129], [70, 10, 0, 300]), ([127, 128], [0, 1])])
+def test_latent_portions_with_a_rotated_part(layout, q_rank, gate, sink, pad, lens, past):
+    """Portions on both sides of the length from which keys and values are expanded, alone and in one step, whole and behind
+    cached tokens; into columns of a wider matrix that do and do not start on 16 bytes (`pad`); against 64 bits."""
+    from garlic_inference_b200.cache import PagedCache
+    from garlic_inference_b200.parts import RotaryPositions, Runtime, StepContext
+    from garlic_inference_b200.parts.latent_attention import LatentAttention
+    H, hid, r, d, dr, dv = 3, 64, 40, 128, 64, 128
+    params = dict(hidden_size=hid, n_heads=H, plain_dim=d, rot_dim=dr, value_dim=dv, kv_rank=r, q_rank=q_rank,
+                  softmax_scale=0.07, eps=1e-6, head_gate=gate, sink=sink, own_kv=True)
+    w = {n: rnd(*t.shape, seed=i, scale=t.shape[-1] ** -0.5 if len(t.shape) > 1 else 1.0, dtype=torch.bfloat16)
+         for i, (n, t) in enumerate(sorted(LatentAttention.wanted(params).items()))}
+
+    class Load:
+        def dtype(self, *names):
+            return torch.bfloat16
+
+        def __call__(self, n, out=None):
+            return w[n] if out is None else out.copy_(w[n])
+
+    rt = Runtime(torch.bfloat16, torch.device("cuda", 0))
+    part = LatentAttention(params, Load(), rt)
+    rot = RotaryPositions(dict(head_dim=dr, rotary_dim=dr, theta=1e4, max_positions=1024, layout=layout, tables=False), None, rt)
+    cache = PagedCache([part.cache_requirement()], max_tokens=2048, max_positions=1024, dtype=torch.bfloat16, device="cuda")
+    xs = [rnd(p + m, hid, seed=90 + i, dtype=torch.bfloat16) for i, (m, p) in enumerate(zip(lens, past))]
+    slots = [cache.alloc_slot() for _ in lens]
+
+    def run(ns, befores, **kw):
+        which = [i for i, m in enumerate(ns) if m]
+        s, ns, befores = [slots[i] for i in which], [ns[i] for i in which], [befores[i] for i in which]
+        cache.prepare(s, ns)
+        cat = lambda f: torch.cat([torch.as_tensor(f(i), dtype=torch.int32) for i in range(len(s))]).to(DEV)
+        n = sum(ns)
+        ctx = StepContext(n, torch.zeros(n, dtype=torch.int32, device=DEV), cat(lambda i: torch.arange(befores[i], befores[i] + ns[i])),
+                          cat(lambda i: torch.full((ns[i],), s[i])), s, [sum(ns[:i]) for i in range(len(s))], ns, befores, False,
+                          1024, status=cache.status)
+        x = torch.cat([xs[i][befores[j]:befores[j] + ns[j]] for j, i in enumerate(which)])
+        y = part.pre_output(x, ctx, cache.view(0), rot, True, **kw)
+        cache.commit(s, ns)
+        return y
+
+    if any(past):
+        run(past, [0] * len(past))
+    n = sum(lens)
+    wide = torch.zeros((n, H * dv + 16), dtype=torch.bfloat16, device=DEV)
+    got = run(lens, past) if pad == 0 else run(lens, past, out=wide[:, pad:pad + H * dv])
+    f = 1e4 ** (-2.0 * torch.arange(dr // 2, dtype=torch.float64, device=DEV) / dr)
+
+    def turn(x):
+        a = torch.arange(x.shape[0], dtype=torch.float64, device=DEV)[:, None, None] * f
+        u, v = (x[..., :dr // 2], x[..., dr // 2:]) if layout == "half" else (x[..., ::2], x[..., 1::2])
+        u, v = u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin()
+        return torch.cat([u, v], -1) if layout == "half" else torch.stack([u, v], -1).flatten(-2)
+
+    W = {k: v.double() for k, v in w.items()}
+    rms = lambda x, g: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * g
+    at = 0
+    for x, m, p in zip(xs, lens, past):
+        x, T = x.double(), len(x)
+        q = ((rms(x @ W["dq"].T, W["dq.norm"]) @ W["uq"].T) if q_rank else x @ W["q"].T).view(T, H, d + dr)
+        c = x @ W["dkv"].T
+        c, kr = rms(c[:, :r], W["dkv.norm"]), turn(c[:, None, r:])[:, 0]
+        k, v = (c @ W["uk"].T).view(T, H, d), (c @ W["uv"].T).view(T, H, dv)
+        q = torch.cat([q[..., :d], turn(q[..., d:])], -1)
+        for h in range(H):
+            want = _attend64(q[p:, h], torch.cat([k[:, h], kr], -1), v[:, h], p, 0.07, sink=W["sink"][h] if sink else None)
+            if gate:
+                want = want * torch.sigmoid(x[p:] @ W["g"][h])[:, None]
+            # beside the attention's own roundings those of q, k, v and the latents (2^-9 each of values of size 1 to 4)
+            torch.testing.assert_close(got[at:at + m].view(m, H, dv)[:, h].double() if pad == 0 else
+                                       got[at:at + m, h * dv:(h + 1) * dv].double(), want, rtol=4e-2, atol=4e-2)
+        at += m
+    cache.check_status()
