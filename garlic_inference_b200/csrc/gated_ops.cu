@@ -239,6 +239,58 @@ __global__ void gated_group_rmsnorm_kernel(const float* __restrict__ o, const T*
     }
 }
 
+// Groups of up to 512 columns in words of four: a warp per (row, group), each lane's words read once and kept, the sum in
+// five exchanges.  Which kernel runs follows from the group's size and the operands' alignment alone.  2,048 rows of 16 groups
+// of 128: 36 us with a block per group (three barriers for one element a thread), 16 us so (32 MB).
+#define GG_WARPS 8
+template <typename T>
+__global__ void __launch_bounds__(GG_WARPS * 32)
+gated_group_rmsnorm_warp_kernel(const float* __restrict__ o, const T* __restrict__ g, long long ldg,
+                                const void* __restrict__ weight, int w_dtype, int w_len,
+                                T* __restrict__ out, long long n_groups, int groups, int gs, float eps, int gate_kind,
+                                float mul, long long ld_out) {
+    gi_pdl_start();
+    const long long at = (long long)blockIdx.x * GG_WARPS + (threadIdx.x >> 5);
+    if (at >= n_groups) return;
+    const long long r = at / groups;
+    const int grp = (int)(at - r * groups), lane = threadIdx.x & 31;
+    const float* orow = o + at * gs;
+    float4 x[4], z[4];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = (i * 32 + lane) * 4;
+        if (c < gs) {
+            x[i] = load4_f32(orow + c);
+            z[i] = load4_act(g + r * ldg + grp * gs + c);
+            ss += x[i].x * x[i].x; ss += x[i].y * x[i].y; ss += x[i].z * x[i].z; ss += x[i].w * x[i].w;
+        }
+    }
+    const float inv = 1.f / sqrtf(warp_sum(ss) / (float)gs + eps);
+    auto one = [&](float v, float w, float t) { return v * inv * w * (gate_kind == 0 ? sigmoid_f(t) : t * sigmoid_f(t)) * mul; };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = (i * 32 + lane) * 4, col = grp * gs + c;
+        if (c < gs) {
+            const float4 w = load4_w(weight, w_dtype, col % w_len);
+            store4_act(out + r * ld_out + col, make_float4(one(x[i].x, w.x, z[i].x), one(x[i].y, w.y, z[i].y),
+                                                           one(x[i].z, w.z, z[i].z), one(x[i].w, w.w, z[i].w)));
+        }
+    }
+}
+template <typename T>
+static bool launch_group_norm_warps(const float* o, const T* g, long long ldg, const void* weight, int w_dtype, int w_len, T* out,
+                                    int n_rows, int groups, int gs, float eps, int gate_kind, float mul, long long ld_out, cudaStream_t s) {
+    const size_t word = 4 * sizeof(T);
+    if (gs > 512 || gs % 4 || ldg % 4 || ld_out % 4 || (uintptr_t)o % 16 || (uintptr_t)g % word || (uintptr_t)out % word ||
+        (uintptr_t)weight % (w_dtype == GI_DTYPE_F32 ? 16 : 8)) return false;
+    const long long n = (long long)n_rows * groups, blocks = (n + GG_WARPS - 1) / GG_WARPS;
+    if (blocks > 0x7fffffff) return false;
+    gi_launch(gated_group_rmsnorm_warp_kernel<T>, dim3((unsigned)blocks), dim3(GG_WARPS * 32), 0, s, o, g, ldg, weight, w_dtype, w_len, out,
+              n, groups, gs, eps, gate_kind, mul, ld_out);
+    return true;
+}
+
 extern "C" int gi_gated_group_rmsnorm(const float* o, const void* g, long long ldg, const void* weight, int w_dtype,
                                       int w_len, void* out, int act_dtype, int n_rows, int groups, int gs, float eps,
                                       int gate_kind, float mul, long long ld_out, void* stream) {
@@ -250,6 +302,9 @@ extern "C" int gi_gated_group_rmsnorm(const float* o, const void* g, long long l
     if (n_rows == 0) return 0;
     const int threads = gs >= 4096 ? 512 : (gs >= 1024 ? 256 : (gs >= 128 ? 128 : (gs > 32 ? 64 : 32)));
     cudaStream_t s = (cudaStream_t)stream;
+    if (act_dtype == GI_DTYPE_F32 ? launch_group_norm_warps<float>(o, (const float*)g, ldg, weight, w_dtype, w_len, (float*)out, n_rows, groups, gs, eps, gate_kind, mul, ld_out, s)
+                                  : act_dtype == GI_DTYPE_BF16 && launch_group_norm_warps<bf16>(o, (const bf16*)g, ldg, weight, w_dtype, w_len, (bf16*)out, n_rows, groups, gs, eps, gate_kind, mul, ld_out, s))
+        return gi_check_launch("gi_gated_group_rmsnorm");
     if (act_dtype == GI_DTYPE_F32)
         gi_launch(gated_group_rmsnorm_kernel<float>, dim3(n_rows, groups), dim3(threads), 0, s, o, (const float*)g, ldg,
                   weight, w_dtype, w_len, (float*)out, groups, gs, eps, gate_kind, mul, ld_out);

@@ -306,3 +306,46 @@ def test_latent_portions_with_a_rotated_part(layout, q_rank, gate, sink, pad, le
                                        got[at:at + m, h * dv:(h + 1) * dv].double(), want, rtol=4e-2, atol=4e-2)
         at += m
     cache.check_status()
+
+
+# ---- row-wise kernels that move words of four ----------------------------------------------------------------------------------
+@pytest.mark.parametrize("hidden", [4, 100, 1024, 4100, 9000, 6])
+@pytest.mark.parametrize("n", [1, 300])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_embedding_rows(hidden, n, dtype):
+    from garlic_inference_b200.ops import kernels
+    table = rnd(50, hidden, seed=1, dtype=dtype)
+    ids = torch.randint(0, 50, (n,), generator=torch.Generator().manual_seed(2)).to(torch.int32).to(DEV)
+    ids[0] = 50                                                            # outside the vocabulary: zeros
+    want = table.float()[ids.clamp(max=49).long()] * 0.5
+    want[0] = 0.0
+    assert torch.equal(kernels.embedding(ids, table, scale=0.5), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("groups, gs, pad", [(3, 4, 0), (5, 132, 4), (2, 512, 0), (1, 516, 0), (3, 10, 2), (4, 128, 1)])
+@pytest.mark.parametrize("n", [1, 37])
+def test_norms_of_groups_and_heads_with_gates(dtype, groups, gs, pad, n):
+    """The read-out's norm per group and the attention's finish per head, sizes on both sides of a warp's words and rows that
+    do and do not start on them."""
+    from garlic_inference_b200.ops import kernels
+    tol = dict(rtol=2e-5, atol=1e-5) if dtype == torch.float32 else dict(rtol=2.0 ** -7, atol=1e-3)      # one rounding of the result
+    W = groups * gs
+    o, g = rnd(n, W, seed=1), rnd(n, W + pad, seed=2, dtype=dtype)[:, :W]
+    w = rnd(gs, seed=3, dtype=dtype)
+    out = torch.full((n, W + pad), 5.0, dtype=dtype, device=DEV)
+    kernels.gated_group_rmsnorm(o, g, w, 1e-5, groups=groups, gate_kind="silu", mul=0.7, out=out[:, pad:])
+    x = o.double().view(n, groups, gs)
+    x = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * w.double()).view(n, W) * torch.nn.functional.silu(g.double()) * 0.7
+    torch.testing.assert_close(out[:, pad:].double(), x, **tol)
+    assert bool((out[:, :pad] == 5.0).all())
+    lam = torch.tensor([0.3], device=DEV)
+    for maps, gate in ((2, rnd(n, groups + 1, seed=4, dtype=dtype)[:, 1:]), (1, g), (2, None)):
+        att = rnd(n, groups * maps * gs, seed=5, dtype=dtype)
+        got = kernels.attn_finish(att, groups, maps, lam if maps == 2 else None, 1e-5, 0.4, gate, dtype, out=out[:, pad:])
+        a = att.double().view(n, groups, maps, gs)
+        a = a[:, :, 0] - lam.double() * a[:, :, 1] if maps == 2 else a[:, :, 0]
+        a = a / torch.sqrt((a * a).mean(-1, keepdim=True) + 1e-5) * 0.4
+        if gate is not None:
+            a = a * torch.sigmoid(gate.double().view(n, groups, -1))
+        torch.testing.assert_close(got.double(), a.view(n, W), **tol)
