@@ -560,6 +560,224 @@ delta_scan_kernel(const float* __restrict__ qkv, long long ldq, int q_off, int k
     if (live) scan_store_state<R, P>(S, st, part);
 }
 
+// ---- the gated delta rule over prompts
+// The same recurrence in two kernels.  The first makes what a token needs once for all slices of value columns: q and k as
+// unit vectors, the decays and beta (in the kernel above every block makes them again, 128 softpluses and exponentials a
+// token, and a chunk's walk waits for its staging).  The second walks, a ring of asynchronous copies ahead, 8 tokens to a
+// group; the read-outs of a group meet in one exchange.  Sums, products and their order are the kernel's above, and so are
+// the bits.  What bounds it is the chain from one token's state to the next (decay, a sum of four, three exchanges, the
+// write) in a scheduler that has one warp.
+// Measured, 2,048 tokens, 16 heads of 128 x 128 on 8 key heads, a decay per channel: 1,015 us in one kernel, 374 us in two
+// (the first 18).
+#define DS_GROUP 8           // tokens to a group of the ring, the lanes of a column
+#define DS_STAGES 4
+#define DS_COLS 16           // value columns to a block
+
+// qk [n, Hk, 2, d]: q (unit, times q_scale) and k (unit).  gb [n, H, d + 4] (CH) or [n, H, 4]: decays, then beta.  A warp per
+// (token, key head) and per (token, head).
+template <int CH>
+__global__ void __launch_bounds__(256)
+delta_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_off, int k_off, const float* __restrict__ ab,
+                     long long ldab, int b_off, int a_off, const float* __restrict__ al, long long ldal,
+                     const void* __restrict__ A_log, const void* __restrict__ dt_bias, int p_dtype, float* __restrict__ qk,
+                     float* __restrict__ gb, long long n_items, int H, int Hk, int d, float unit_eps, float q_scale) {
+    gi_pdl_start();
+    const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= n_items) return;
+    const int lane = threadIdx.x & 31, c = lane * 4;
+    const long long t = item / (H + Hk);
+    const int part = (int)(item - t * (H + Hk));
+    if (part < Hk) {
+        const float* row = qkv + t * ldq + (size_t)part * d;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+        float sq = 0.f, sk = 0.f;
+        if (c < d) {
+            q = *reinterpret_cast<const float4*>(row + q_off + c);
+            k = *reinterpret_cast<const float4*>(row + k_off + c);
+        }
+        sq = fmaf(q.x, q.x, sq); sq = fmaf(q.y, q.y, sq); sq = fmaf(q.z, q.z, sq); sq = fmaf(q.w, q.w, sq);
+        sk = fmaf(k.x, k.x, sk); sk = fmaf(k.y, k.y, sk); sk = fmaf(k.z, k.z, sk); sk = fmaf(k.w, k.w, sk);
+        const float iq = q_scale / sqrtf(warp_sum(sq) + unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + unit_eps);
+        if (c < d) {
+            float* dst = qk + (t * Hk + part) * (2LL * d) + c;
+            *reinterpret_cast<float4*>(dst) = make_float4(q.x * iq, q.y * iq, q.z * iq, q.w * iq);
+            *reinterpret_cast<float4*>(dst + d) = make_float4(k.x * ik, k.y * ik, k.z * ik, k.w * ik);
+        }
+        return;
+    }
+    const int h = part - Hk;
+    const float rate = expf(load_w(A_log, p_dtype, h));
+    const float* a = al + t * ldal + a_off;
+    float* dst = gb + (t * H + h) * (CH ? d + 4LL : 4LL);
+    if (CH && c < d) {
+        float4 g;
+        g.x = expf(-rate * rc_softplus(a[h * d + c] + load_w(dt_bias, p_dtype, h * d + c)));
+        g.y = expf(-rate * rc_softplus(a[h * d + c + 1] + load_w(dt_bias, p_dtype, h * d + c + 1)));
+        g.z = expf(-rate * rc_softplus(a[h * d + c + 2] + load_w(dt_bias, p_dtype, h * d + c + 2)));
+        g.w = expf(-rate * rc_softplus(a[h * d + c + 3] + load_w(dt_bias, p_dtype, h * d + c + 3)));
+        *reinterpret_cast<float4*>(dst + c) = g;
+    }
+    if (lane == 0) {
+        const float g = CH ? 0.f : expf(-rate * rc_softplus(a[h] + load_w(dt_bias, p_dtype, h)));
+        *reinterpret_cast<float4*>(dst + (CH ? d : 0)) = make_float4(rc_sigmoid(ab[t * ldab + b_off + h]), g, 0.f, 0.f);
+    }
+}
+
+// Keys of D = 8 R, W value columns to a thread.  spans [n_seq, 3]; out float32 [n, H dv].
+template <int R, int CH, int W>
+__global__ void __launch_bounds__(DS_COLS / W * 8, 1)
+delta_walk_kernel(const float* __restrict__ qk, const float* __restrict__ gb, const float* __restrict__ qkv, long long ldq, int v_off,
+                  float* __restrict__ state, long long state_stride, const int* __restrict__ spans, float* __restrict__ out, int H,
+                  int Hk, int dv) {
+    gi_pdl_start();
+    constexpr int P = 8, D = R * P, DS_THREADS = DS_COLS / W * P, GB = CH ? D + 4 : 4;       // floats of a row of decays and beta
+    constexpr int TOKEN = 2 * D + GB + DS_COLS, QK_COPIES = 2 * D / 4, G_COPIES = CH ? D / 4 : 0;      // a token's floats, its 16-byte copies
+    extern __shared__ __align__(16) float ds_smem[];                   // [stage][token][q | k | decays, beta | v]
+    const int slot = spans[3 * blockIdx.x], start = spans[3 * blockIdx.x + 1], len = spans[3 * blockIdx.x + 2];
+    const int h = blockIdx.y, v0 = blockIdx.z * DS_COLS, kh = h / (H / Hk), tid = threadIdx.x;
+    const int part = tid % P, col = tid / P * W;                       // this thread's columns: v0 + col (and the next)
+    if (slot < 0) {
+        for (int t = 0; t < len; ++t)
+            if (part < W) out[(size_t)(start + t) * H * dv + h * dv + v0 + col + part] = 0.f;
+        return;
+    }
+    const int groups = (len + DS_GROUP - 1) / DS_GROUP;
+    const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(ds_smem);
+    auto copy = [&](uint32_t dst, const float* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src)); };
+    // a group's tokens beyond the sequence's end are its last token again, and not walked
+    auto fetch = [&](int grp) {
+        if (grp < groups) {
+            const uint32_t base = smem0 + (uint32_t)(grp % DS_STAGES) * (DS_GROUP * TOKEN * 4);
+            const int t0 = grp * DS_GROUP, last = len - 1;
+#pragma unroll
+            for (int i = 0; i < DS_GROUP * QK_COPIES / DS_THREADS; ++i) {
+                const int id = tid + DS_THREADS * i, j = id / QK_COPIES, c = id % QK_COPIES;
+                copy(base + (j * TOKEN + 4 * c) * 4, qk + ((size_t)(start + min(t0 + j, last)) * Hk + kh) * (2 * D) + 4 * c);
+            }
+#pragma unroll
+            for (int i = 0; i < DS_GROUP * G_COPIES / DS_THREADS; ++i) {
+                const int id = tid + DS_THREADS * i, j = id / (G_COPIES ? G_COPIES : 1), c = id % (G_COPIES ? G_COPIES : 1);
+                copy(base + (j * TOKEN + 2 * D + 4 * c) * 4, gb + ((size_t)(start + min(t0 + j, last)) * H + h) * GB + 4 * c);
+            }
+            if (tid < 32) {
+                const int j = tid / 4, c = tid % 4;
+                copy(base + (j * TOKEN + 2 * D + GB + 4 * c) * 4, qkv + (size_t)(start + min(t0 + j, last)) * ldq + v_off + h * dv + v0 + 4 * c);
+            } else if (tid < 40) {
+                const int j = tid - 32;
+                copy(base + (j * TOKEN + 2 * D + GB - 4) * 4, gb + ((size_t)(start + min(t0 + j, last)) * H + h) * GB + GB - 4);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::);
+    };
+    for (int g = 0; g < DS_STAGES - 1; ++g) fetch(g);
+    float* st = state + (size_t)slot * state_stride + ((size_t)h * dv + v0 + col) * D;
+    f32x2 S[W][R / 2];
+#pragma unroll
+    for (int w = 0; w < W; ++w) scan_load_pairs<R, P>(S[w], st + w * D, part, true);
+    float* dst = out + (size_t)start * H * dv + h * dv + v0 + col;
+    for (int grp = 0; grp < groups; ++grp) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(DS_STAGES - 2));
+        __syncthreads();                                               // the group is there, and the one before it is done with
+        fetch(grp + DS_STAGES - 1);
+        const int left = len - grp * DS_GROUP;
+        float o[W][P];
+        // Token j: its operands come out of shared memory while the token before is walked, and what is read of the state
+        // with that token's q is summed beside the decay and the sum with this one's k, so that neither lies in the chain.
+        struct Operands { f32x2 k[R / 2], g[CH ? R / 2 : 1], q[R / 2]; float beta, v[W]; };
+        // (volatile, so that they stay ahead of the exchanges of the token that is walked)
+        const uint32_t tok_addr = smem0 + (uint32_t)(grp % DS_STAGES) * (DS_GROUP * TOKEN * 4);
+        auto pair = [](uint32_t at, f32x2& x, f32x2& y) { asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(at)); };
+        auto operands = [&](Operands& a, int j) {
+            const uint32_t x = tok_addr + j * (TOKEN * 4);
+#pragma unroll
+            for (int i = 0; i < R / 4; ++i) {
+                pair(x + (D + KEY_OF(i, part)) * 4, a.k[2 * i], a.k[2 * i + 1]);
+                if (CH) pair(x + (2 * D + KEY_OF(i, part)) * 4, a.g[CH ? 2 * i : 0], a.g[CH ? 2 * i + 1 : 0]);
+            }
+            float decay;                                               // of the whole head
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a.beta), "=f"(decay) : "r"(x + (2 * D + GB - 4) * 4));
+            if (!CH) a.g[0] = both2(decay);
+#pragma unroll
+            for (int w = 0; w < W; ++w) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(a.v[w]) : "r"(x + (2 * D + GB + col + w) * 4));
+#pragma unroll
+            for (int i = 0; i < R / 4; ++i) pair(x + KEY_OF(i, part) * 4, a.q[2 * i], a.q[2 * i + 1]);
+        };
+        auto read = [&](const Operands& a, int j) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                f32x2 oa = 0ull, ob = 0ull;
+#pragma unroll
+                for (int i = 0; i < R / 4; ++i) {
+                    oa = fma2(S[w][2 * i], a.q[2 * i], oa);
+                    ob = fma2(S[w][2 * i + 1], a.q[2 * i + 1], ob);
+                }
+                o[w][j] = sum2(oa, ob);
+            }
+        };
+        auto write = [&](const Operands& a) {
+            f32x2 ra[W], rb[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                ra[w] = rb[w] = 0ull;
+#pragma unroll
+                for (int i = 0; i < R / 4; ++i) {
+                    S[w][2 * i] = mul2(S[w][2 * i], a.g[CH ? 2 * i : 0]);
+                    S[w][2 * i + 1] = mul2(S[w][2 * i + 1], a.g[CH ? 2 * i + 1 : 0]);
+                    ra[w] = fma2(S[w][2 * i], a.k[2 * i], ra[w]);
+                    rb[w] = fma2(S[w][2 * i + 1], a.k[2 * i + 1], rb[w]);
+                }
+            }
+            float r[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) r[w] = sum2(ra[w], rb[w]);
+#pragma unroll
+            for (int off = 1; off < P; off <<= 1)                      // part_sum of every column, side by side
+#pragma unroll
+                for (int w = 0; w < W; ++w) r[w] += __shfl_xor_sync(0xffffffffu, r[w], off);
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const f32x2 u = both2(a.beta * (a.v[w] - r[w]));
+#pragma unroll
+                for (int i = 0; i < R / 2; ++i) S[w][i] = fma2(a.k[i], u, S[w][i]);
+            }
+        };
+        Operands a[2];
+        if (left >= DS_GROUP) {                                        // no branch between tokens
+            operands(a[0], 0);
+#pragma unroll
+            for (int j = 0; j < DS_GROUP; ++j) {
+                if (j) read(a[(j + 1) & 1], j - 1);
+                if (j + 1 < DS_GROUP) operands(a[(j + 1) & 1], j + 1);
+                write(a[j & 1]);
+            }
+            read(a[(DS_GROUP - 1) & 1], DS_GROUP - 1);
+        } else {
+#pragma unroll
+            for (int j = 0; j < DS_GROUP; ++j) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) o[w][j] = 0.f;
+                if (j < left) {                                        // the same for the whole block
+                    operands(a[0], j);
+                    write(a[0]);
+                    read(a[0], j);
+                }
+            }
+        }
+        // token `part` of the group ends in lane `part`
+        float y[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) y[w] = part_sum_tokens<P>(o[w], part);
+        if (part < left) {
+            float* at = dst + (size_t)(grp * DS_GROUP + part) * H * dv;
+            if (W == 2) *reinterpret_cast<float2*>(at) = make_float2(y[0], y[W - 1]);
+            else *at = y[0];
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+#pragma unroll
+    for (int w = 0; w < W; ++w) scan_store_pairs<R, P>(S[w], st + w * D, part);
+}
+
 // Floats of one head's state for key dimension d and value dimension dv, as the scans lay it out.
 extern "C" long long gi_scan_state_floats(int d, int dv) {
     const int dp = scan_padded(d);
@@ -614,4 +832,42 @@ extern "C" int gi_delta_scan(const float* qkv, long long ldq, int q_off, int k_o
         SCAN_DISPATCH_X(delta_scan_kernel, float, SCAN_COMMA(0), qkv, ldq, q_off, k_off, v_off, ab, ldab, b_off, a_off, al, ldal, A_log, dt_bias, p_dtype, state, state_stride, spans, tok_slot, out, H, Hk, d, dv, unit_eps, q_scale, vec)
     }
     return gi_check_launch("gi_delta_scan");
+}
+
+// gi_delta_scan over prompts by the two kernels above: keys of 64 or 128, values in whole blocks of columns, rows of qkv and of
+// the state that start on 16 bytes.  `scratch`: n_rows (2 Hk d + H (d + 4 or 4)) floats, on 16 bytes.
+extern "C" int gi_delta_scan_prompt(const float* qkv, long long ldq, int q_off, int k_off, int v_off, const float* ab,
+                                    long long ldab, int b_off, int a_off, const float* a_sep, long long lda_sep,
+                                    const void* A_log, const void* dt_bias, int p_dtype, float* state, long long state_stride,
+                                    const int* spans, float* out, float* scratch, int n_rows, int n_seq, int H, int Hk, int d,
+                                    int dv, float unit_eps, float q_scale, int channel_decay, void* stream) {
+    GI_REQUIRE(n_seq >= 0 && n_rows >= 0 && H > 0 && Hk > 0 && H % Hk == 0 && (d == 64 || d == 128) && dv > 0 && dv % DS_COLS == 0,
+               "gi_delta_scan_prompt: %d heads on %d key heads, keys of %d, values of %d", H, Hk, d, dv);
+    GI_REQUIRE(H <= 65535 && dv / DS_COLS <= 65535, "gi_delta_scan_prompt: %d heads of %d values", H, dv);
+    GI_REQUIRE(state_stride >= (long long)H * dv * d && state_stride % 4 == 0 && (uintptr_t)state % 16 == 0,
+               "gi_delta_scan_prompt: state rows of %lld floats", state_stride);
+    GI_REQUIRE(ldq % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && ((uintptr_t)qkv | (uintptr_t)scratch) % 16 == 0 &&
+               (uintptr_t)out % 8 == 0, "gi_delta_scan_prompt: rows start on 16 bytes");
+    if (n_seq == 0 || n_rows == 0) return 0;
+    cudaStream_t s = (cudaStream_t)stream;
+    const float* al = a_sep ? a_sep : ab;
+    const long long ldal = a_sep ? lda_sep : ldab;
+    float *qk = scratch, *gb = scratch + (size_t)n_rows * Hk * 2 * d;
+    const long long items = (long long)n_rows * (H + Hk);
+    GI_REQUIRE((items + 7) / 8 <= 0x7fffffff, "gi_delta_scan_prompt: %d rows", n_rows);
+    const auto prepare = channel_decay ? delta_prepare_kernel<1> : delta_prepare_kernel<0>;
+    gi_launch(prepare, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, qkv, ldq, q_off, k_off, ab, ldab, b_off, a_off, al, ldal, A_log,
+              dt_bias, p_dtype, qk, gb, items, H, Hk, d, unit_eps, q_scale);
+    if (int rc = gi_check_launch("gi_delta_scan_prompt")) return rc;
+    const size_t smem = (size_t)DS_STAGES * DS_GROUP * (2 * d + (channel_decay ? d + 4 : 4) + DS_COLS) * sizeof(float);
+    // One column to a thread where the blocks fit the SMs side by side: four warps to an SM, one to a scheduler.  Two columns
+    // beyond: half the reads of shared memory, which then are what several blocks to an SM wait for.
+    const bool few = (long long)n_seq * H * (dv / DS_COLS) <= 148;
+#define DS_WALK(R, CH) (few ? delta_walk_kernel<R, CH, 1> : delta_walk_kernel<R, CH, 2>)
+    const auto walk = d == 128 ? (channel_decay ? DS_WALK(16, 1) : DS_WALK(16, 0)) : (channel_decay ? DS_WALK(8, 1) : DS_WALK(8, 0));
+#undef DS_WALK
+    if (int rc = gi_reserve_smem((const void*)walk, smem, "gi_delta_scan_prompt")) return rc;
+    gi_launch(walk, dim3(n_seq, H, dv / DS_COLS), dim3(few ? DS_COLS * 8 : DS_COLS * 4), smem, s, (const float*)qk, (const float*)gb, qkv,
+              ldq, v_off, state, state_stride, spans, out, H, Hk, dv);
+    return gi_check_launch("gi_delta_scan_prompt");
 }

@@ -910,6 +910,9 @@ def decay_scan(qkv: torch.Tensor, offsets: tuple, decay: torch.Tensor, state: to
     return out
 
 
+DELTA_PAIR_TOKENS = 8
+
+
 def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: tuple, A_log: torch.Tensor,
                dt_bias: torch.Tensor, state: torch.Tensor, spans: Optional[torch.Tensor], tok_slot: torch.Tensor,
                n_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, unit_eps: float,
@@ -927,6 +930,20 @@ def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: 
     out = torch.empty((n, n_heads * value_dim), dtype=torch.float32, device=qkv.device)
     if decay_logits is not None:
         _rows(decay_logits, "decay_logits", torch.float32)
+    # Prompts at sizes that the pair of kernels takes: from a few tokens a sequence on (a decode step's rows and shorter
+    # portions stay with the one kernel: a launch less, and no tokens to run ahead of).  The bits are the same.
+    if spans is not None and n >= DELTA_PAIR_TOKENS * n_seq and key_dim in (64, 128) and value_dim % 16 == 0 and \
+            all(v % 4 == 0 for v in (qkv.stride(0), state.stride(0), *offsets)) and \
+            qkv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
+        width = 2 * n_kv_heads * key_dim + n_heads * (key_dim + 4 if channel_decay else 4)
+        scratch = torch.empty((n, width), dtype=torch.float32, device=qkv.device)
+        check(l.gi_delta_scan_prompt(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0), *map(int, ab_offsets),
+                                     _ptr(decay_logits), decay_logits.stride(0) if decay_logits is not None else 0, _ptr(A_log),
+                                     _ptr(dt_bias), code(A_log.dtype), _ptr(state), state.stride(0), _ptr(spans), _ptr(out),
+                                     _ptr(scratch), n, n_seq, n_heads, n_kv_heads, key_dim, value_dim, float(unit_eps),
+                                     float(key_dim) ** -0.5, int(channel_decay), _stream()), l)
+        counters.launches += 1                               # two kernels behind one entry point
+        return out
     check(l.gi_delta_scan(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0),
                           *map(int, ab_offsets), _ptr(decay_logits),
                           decay_logits.stride(0) if decay_logits is not None else 0, _ptr(A_log), _ptr(dt_bias), code(A_log.dtype), _ptr(state),

@@ -349,3 +349,42 @@ def test_norms_of_groups_and_heads_with_gates(dtype, groups, gs, pad, n):
         if gate is not None:
             a = a * torch.sigmoid(gate.double().view(n, groups, -1))
         torch.testing.assert_close(got.double(), a.view(n, W), **tol)
+
+
+# ---- delta rule over prompts ------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("d, dv, H, Hk", [(128, 128, 16, 8), (64, 128, 20, 20), (64, 16, 3, 3), (128, 48, 2, 1)])
+@pytest.mark.parametrize("lens", [[8], [1, 7, 9, 64], [33, 100, 2, 16]])
+def test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, d, dv, H, Hk, lens, monkeypatch):
+    """Sequences of whole and part groups of tokens, shorter than the ring, a padding portion; against the kernel that decode
+    steps run (bits) and against 64 bits."""
+    from garlic_inference_b200.ops import kernels
+    n, n_dec = sum(lens) + 2, H * d if channel else H
+    qkv, ab, al = rnd(n, 2 * Hk * d + H * dv, seed=1), rnd(n, 2 * H, seed=2), rnd(n, n_dec, seed=3)
+    A_log, dt = rnd(H, seed=4, scale=0.3), rnd(n_dec, seed=5)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    spans = torch.tensor([[i, s, m] for i, (s, m) in enumerate(zip(starts, lens))] + [[-1, n - 2, 2]], dtype=torch.int32, device=DEV)
+    slots = torch.zeros(n, dtype=torch.int32, device=DEV)
+    first = rnd(len(lens) + 1, H * dv * d + 8, seed=6, scale=0.1)
+
+    def run(pair):
+        monkeypatch.setattr(kernels, "DELTA_PAIR_TOKENS", 0 if pair else 1 << 30)
+        state = first.clone()
+        out = kernels.delta_scan(qkv, (0, Hk * d, 2 * Hk * d), ab, (H, 0), A_log, dt, state, spans, slots, H, Hk, d, dv, 1e-6,
+                                 channel_decay=channel, decay_logits=al)
+        return out, state
+
+    (got, state), (one, state1) = run(True), run(False)
+    assert torch.equal(got, one) and torch.equal(state, state1)
+    assert float(got[n - 2:].abs().max()) == 0.0
+    q, k, v = (qkv[:, a:b].double() for a, b in ((0, Hk * d), (Hk * d, 2 * Hk * d), (2 * Hk * d, 2 * Hk * d + H * dv)))
+    unit = lambda x: (x.view(n, Hk, d) / torch.sqrt((x.view(n, Hk, d) ** 2).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // Hk, 1)
+    q, k, v, beta = unit(q) * d ** -0.5, unit(k), v.view(n, H, dv), torch.sigmoid(ab[:, H:].double())
+    g = torch.exp(-torch.exp(A_log.double())[:, None] * torch.nn.functional.softplus(al.double() + dt.double()).view(n, H, -1))
+    for i, (s, m) in enumerate(zip(starts, lens)):
+        S = first[i, :H * dv * d].double().view(H, dv, d)
+        for t in range(s, s + m):
+            S = S * g[t][:, None, :]
+            u = beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0])
+            S = S + u[:, :, None] * k[t][:, None, :]
+            torch.testing.assert_close(got[t].view(H, dv).double(), (S @ q[t][:, :, None])[..., 0], rtol=1e-4, atol=1e-5)
