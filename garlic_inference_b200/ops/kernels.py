@@ -702,6 +702,29 @@ def moe_group(idx: torch.Tensor, x: torch.Tensor, n_experts: int):
     return where, ends, rows
 
 
+def moe_products_takes(n_experts: int, n_out: int, inner: int) -> bool:
+    """Whether the experts' tcgen05 product takes these sizes."""
+    return 0 < n_experts <= 256 and inner % 8 == 0 and 2 * n_experts * n_out < 1 << 31
+
+
+def moe_products(rows: torch.Tensor, ends: torch.Tensor, w: torch.Tensor, unit=None) -> torch.Tensor:
+    """Every expert's rows (bfloat16 [pairs, inner] in the order of the experts, `ends` int32 [experts] each one's last row
+    + 1) times its matrix of w [experts, out, inner] transposed: [pairs, out] with `unit` None, relu(.)^2 of it with
+    "relu_squared", and with a `glu_shape` tuple unit(gate, up) of w's gate rows and the up rows behind them,
+    [pairs, out / 2].  float32 sums and activation, one rounding."""
+    l = require_gpu()
+    _dense(rows, "rows", torch.bfloat16), _dense(ends, "ends", torch.int32), _dense(w, "w", torch.bfloat16)
+    n, k = rows.shape
+    if w.dim() != 3 or w.shape[2] != k or ends.numel() != w.shape[0] or (isinstance(unit, tuple) and w.shape[1] % 2):
+        raise KernelError(f"rows {tuple(rows.shape)} and ends {tuple(ends.shape)} do not fit experts {tuple(w.shape)}")
+    kind = 1 if isinstance(unit, tuple) else {None: 0, "relu_squared": 2}[unit]
+    n_out = w.shape[1] // 2 if kind == 1 else w.shape[1]
+    out = torch.empty((n, n_out), dtype=torch.bfloat16, device=rows.device)
+    check(l.gi_moe_grouped(_ptr(rows), _ptr(w), _ptr(ends), _ptr(out), w.shape[0], n, n_out, k, kind,
+                           *(unit if kind == 1 else (0, 1.0, 0.0, 0.0, 0.0)), _ptr(tcgen05_error_flag(rows.device)), _stream()), l)
+    return out
+
+
 def moe_combine(buf: torch.Tensor, where: Optional[torch.Tensor], wt: torch.Tensor,
                 add: Optional[torch.Tensor] = None, add_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[t] = (add[t] +) sum_j wt[t, j] buf[where[t, j]] (float32 sums in the order of j); without `where`: row

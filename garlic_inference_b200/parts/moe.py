@@ -28,8 +28,9 @@ run them.  A step of a few rows (a decode step; such a step may be recorded, so 
 host): kernels that read the chosen experts' matrices only, a warp per matrix row, the experts taken from
 device memory.  More rows: the (token, choice) pairs are put in the order of their experts by a counting sort on
 the device (which also gathers the tokens' vectors into that order), the experts run two matrix products over
-their own rows, and one kernel sums each token's `top` results with its weights in the router's order.  In bfloat16 the two products are the library's grouped product (`torch._grouped_mm`: the rows
-of every expert in one launch, the groups' ends read from device memory, nothing comes to the host); in float32,
+their own rows, and one kernel sums each token's `top` results with its weights in the router's order.  In bfloat16 the two products are this package's tcgen05 kernel, the activation inside the first, as long as
+an expert has few rows on average (`OWN_PRODUCT_MAX_MEAN`), and the library's grouped product beyond (`torch._grouped_mm`); either
+takes the rows of every expert in one launch, the groups' ends read from device memory, nothing comes to the host; in float32,
 or where the library has no grouped product, the counts come to the host once and every chosen expert runs this
 package's products over its rows.  Either way a token's result does not depend on the other tokens of the step
 beyond the rounding of the products.
@@ -47,6 +48,12 @@ from .base import FeedForward, register_part
 # The row-by-row kernels read an expert's matrices once per (token, choice) pair, the grouped product once per
 # expert: from a few tokens on, pairs share experts.
 ROWWISE_MAX_ROWS = 8
+# Up to how many rows an expert has on average the two products are this package's own kernel, which is bound by reading
+# the chosen experts' matrices once (the activation runs inside the first); beyond, the products themselves weigh and the
+# library's grouped product, with rows on the wide side of the tensor cores, is faster.  The whole part with 16 gated experts
+# of 9,216 on 4,096, 2 chosen, library / own in us: 16 tokens 677 / 497, 64 841 / 608, 256 843 / 627, 512 915 / 857,
+# 1,024 941 / 1,133; 64 experts of 1,024 on 2,048, 6 chosen: 64 tokens 211 / 171, 512 252 / 214, 1,024 301 / 297.
+OWN_PRODUCT_MAX_MEAN = 64
 
 
 class RoutedExperts(FeedForward):
@@ -163,7 +170,11 @@ class RoutedExperts(FeedForward):
             return kernels.moe_rowwise(x, self.w_up, self.w_down, idx, wt, self.act, add=add, add_gate=gate)
         # expert by expert: the pairs (token, choice) in the order of their experts; `where` is each pair's row
         where, ends, rows = kernels.moe_group(idx, x, self.E)
-        if grouped:
+        if grouped and n * self.top <= OWN_PRODUCT_MAX_MEAN * self.E and kernels.moe_products_takes(self.E, self.ff, self.hidden) and \
+                kernels.moe_products_takes(self.E, self.hidden, self.ff):
+            a = kernels.moe_products(rows, ends, self.w_up, self.act)
+            buf = kernels.moe_products(a, ends, self.w_down)
+        elif grouped:
             a = self._activate(torch._grouped_mm(rows, self.w_up.transpose(1, 2), offs=ends))
             buf = torch._grouped_mm(a, self.w_down.transpose(1, 2), offs=ends)
         else:

@@ -388,3 +388,31 @@ def test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, d, dv, H, Hk, le
             u = beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0])
             S = S + u[:, :, None] * k[t][:, None, :]
             torch.testing.assert_close(got[t].view(H, dv).double(), (S @ q[t][:, :, None])[..., 0], rtol=1e-4, atol=1e-5)
+
+
+# ---- experts' products ------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("E, K, n_out", [(4, 64, 128), (3, 72, 200), (40, 128, 96), (16, 1032, 264)])
+@pytest.mark.parametrize("counts", ["even", "one", "none_first", "many"])
+@pytest.mark.parametrize("unit", [None, "relu_squared", "glu"])
+def test_products_of_the_experts_rows(E, K, n_out, counts, unit):
+    """Experts without rows, one with all of them, parts of tiles on every side, row counts on both sides of an item's 32 and
+    64 rows, against 64 bits."""
+    from garlic_inference_b200.ops import kernels
+    n = {"even": [3] * E, "one": [0] * (E - 1) + [70], "none_first": [0, 33, 0] + [1] * (E - 3),
+         "many": [65 + 7 * (e % 3) for e in range(E)]}[counts]
+    ends = torch.tensor([sum(n[:e + 1]) for e in range(E)], dtype=torch.int32, device=DEV)
+    glu = kernels.glu_shape("swish", 1.7, 1.5, 1.0, 1.0) if unit == "glu" else unit
+    rows = rnd(sum(n), K, seed=1, dtype=torch.bfloat16)
+    w = rnd(E, n_out * (2 if unit == "glu" else 1), K, seed=2, scale=K ** -0.5, dtype=torch.bfloat16)
+    got = kernels.moe_products(rows, ends, w, glu)
+    at = 0
+    for e in range(E):
+        z = rows[at:at + n[e]].double() @ w[e].double().T
+        if unit == "relu_squared":
+            z = z.clamp(min=0) ** 2
+        elif unit == "glu":
+            g, u = z[:, :n_out].clamp(max=1.5), z[:, n_out:].clamp(-1.0, 1.0)
+            z = g * torch.sigmoid(1.7 * g) * (u + 1.0)
+        torch.testing.assert_close(got[at:at + n[e]].double(), z, rtol=2.0 ** -8, atol=1e-4)      # one rounding, float32 sums
+        at += n[e]
+    kernels.check_bounded_waits(torch.device("cuda", 0))
