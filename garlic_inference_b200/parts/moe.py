@@ -48,6 +48,12 @@ from .base import FeedForward, register_part
 # The row-by-row kernels read an expert's matrices once per (token, choice) pair, the grouped product once per
 # expert: from a few tokens on, pairs share experts.
 ROWWISE_MAX_ROWS = 8
+# ... and where the tcgen05 product could run instead, only while the pairs' matrices are this many bytes: that product reads
+# an expert chosen twice once and streams faster, but starts 25 us later (the pairs have to be put in order first).  The whole
+# part row by row / by products in us: 16 experts of 9,216 on 4,096, 2 chosen (453 MB a token): 1 token 153 / 134, 4 332 / 297,
+# 8 538 / 434; 4,224 on 2,048: 2 tokens (208 MB) 73 / 75, 4 104 / 94; 64 of 1,024 on 2,048, 6 chosen: 4 tokens (302 MB)
+# 82 / 93, 6 100 / 100; 8 of 2,816 on 1,024, 1 chosen: 6 tokens (104 MB) 38 / 48.
+ROWWISE_MAX_BYTES = 400 << 20
 # Up to how many rows an expert has on average the two products are this package's own kernel, which is bound by reading
 # the chosen experts' matrices once (the activation runs inside the first); beyond, the products themselves weigh and the
 # library's grouped product, with rows on the wide side of the tensor cores, is faster.  The whole part with 16 gated experts
@@ -166,12 +172,15 @@ class RoutedExperts(FeedForward):
         add = linear(glu_product(x, self.shared, self.shared_unit), self.shared_down) if self.shared is not None else None
         grouped = self._grouped(x)
         products = self.gated or self.activation == "relu_squared"     # what the expert-by-expert path computes
-        if n <= ROWWISE_MAX_ROWS or not products or (ctx.captured and not grouped):
+        own = grouped and n * self.top <= OWN_PRODUCT_MAX_MEAN * self.E and \
+            kernels.moe_products_takes(self.E, self.ff, self.hidden) and kernels.moe_products_takes(self.E, self.hidden, self.ff)
+        pair_bytes = (self.w_up[0].numel() + self.w_down[0].numel()) * self.w_up.element_size()
+        few = n <= ROWWISE_MAX_ROWS and not (own and n * self.top * pair_bytes >= ROWWISE_MAX_BYTES)
+        if few or not products or (ctx.captured and not grouped):
             return kernels.moe_rowwise(x, self.w_up, self.w_down, idx, wt, self.act, add=add, add_gate=gate)
         # expert by expert: the pairs (token, choice) in the order of their experts; `where` is each pair's row
         where, ends, rows = kernels.moe_group(idx, x, self.E)
-        if grouped and n * self.top <= OWN_PRODUCT_MAX_MEAN * self.E and kernels.moe_products_takes(self.E, self.ff, self.hidden) and \
-                kernels.moe_products_takes(self.E, self.hidden, self.ff):
+        if own:
             a = kernels.moe_products(rows, ends, self.w_up, self.act)
             buf = kernels.moe_products(a, ends, self.w_down)
         elif grouped:

@@ -416,3 +416,28 @@ def test_products_of_the_experts_rows(E, K, n_out, counts, unit):
         torch.testing.assert_close(got[at:at + n[e]].double(), z, rtol=2.0 ** -8, atol=1e-4)      # one rounding, float32 sums
         at += n[e]
     kernels.check_bounded_waits(torch.device("cuda", 0))
+
+
+@pytest.mark.parametrize("unit", ["glu", "relu_squared"])
+@pytest.mark.parametrize("n", [1, 2, 8, 9])
+def test_routed_experts_of_few_rows_by_rows_and_by_products(unit, n, monkeypatch):
+    """The part's two ways for a decode step's rows, chosen by the bytes of the pairs' matrices."""
+    import garlic_inference_b200.parts.moe as moe
+    from garlic_inference_b200.parts import Runtime, StepContext
+    params = dict(hidden_size=64, expert_size=136, n_experts=6, top=2, expert="glu" if unit == "glu" else "two_matrix")
+    w = {k: rnd(*t.shape, seed=i, scale=t.shape[-1] ** -0.5, dtype=torch.bfloat16) for i, (k, t) in enumerate(moe.RoutedExperts.wanted(params).items())}
+
+    class Load:
+        def dtype(self, *names):
+            return torch.bfloat16
+
+        def __call__(self, name, out=None):
+            return w[name] if out is None else out.copy_(w[name])
+
+    part = moe.RoutedExperts(params, Load(), Runtime(torch.bfloat16, torch.device("cuda", 0)))
+    x, z = rnd(n, 64, seed=50, dtype=torch.bfloat16), torch.zeros(n, dtype=torch.int32, device=DEV)
+    got = []
+    for limit in (0, 1 << 40):
+        monkeypatch.setattr(moe, "ROWWISE_MAX_BYTES", limit)
+        got.append(part.step(x, StepContext(n, z, z, z)).double())
+    torch.testing.assert_close(got[0], got[1], rtol=2e-2, atol=1e-2)       # roundings of the activation and of the pairs' results
