@@ -1085,11 +1085,12 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor
     if one != 1 or pool_row != row:
         raise KernelError(f"a pool {tuple(pool.shape)} does not hold rows of {row} shared by all heads")
     if n_splits is None:
-        # Slices of the keys: about 256 blocks in all, at most 16 slices.  Measured at 32 heads over rows of 576 with
-        # 2,048 cached tokens (us at 4 / 8 / 16 / 32 slices): 1 sequence 108 / 69 / 52 / 52, 8 sequences
-        # 108 / 69 / 54 / 73, 64 sequences 210 / 228 / 245 / 329.
+        # Slices of the keys: about 384 blocks in all (two to an SM and some to even out sequences of different lengths), 256
+        # from 33 sequences on, at most 16 slices.  Measured at 32 heads over rows of 576 (us at 4 / 8 / 16 / 32 slices): 1 sequence of 2,048 tokens
+        # 70 / 47 / 37 / 39, 8 sequences 71 / 47 / 39 / 49, 32 sequences 80 / 71 / 83 / 113, 20 sequences of 200 to 4,000 tokens
+        # (in a step of 32 rows) 122 / 93 / 78 / 107, 64 sequences 115 / 135 / 146 / 208; 12 slices of 32: 85 and 79.
         groups = -(-heads // 32)
-        n_splits = max(1, min(16, 256 // max(1, n * groups)))
+        n_splits = max(1, min(16, (384 if n * groups <= 32 else 256) // max(1, n * groups)))
     part = torch.empty((n, n_splits, heads, rank + 2), dtype=torch.float32, device=q.device)
     out = torch.empty((n, heads * rank), dtype=torch.bfloat16, device=q.device)
     check(l.gi_latent_decode(_ptr(q), _ptr(pool), _ptr(block_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(part),
