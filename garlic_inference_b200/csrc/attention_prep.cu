@@ -15,8 +15,9 @@
 //                     grows with the position p, 1 + temp_coef ln(floor((p + 1) / temp_every) + 1).  All float32.
 //                     Cosine and sine may both be multiplied by a `magnitude`.  After the rotation, optionally
 //                     (`head_eps` > 0): every query and key head is divided by its own root mean square over its d
-//                     dimensions (eps inside the root, no weight).  With that option and the half layout (or no rotation)
-//                     and widths that fit, a second kernel runs: a group of lanes per head, four elements per access.
+//                     dimensions (eps inside the root, no weight).  Without the norms over all heads, the queries' factor
+//                     and block means, and with widths that fit, a second kernel runs: a group of lanes per head, four
+//                     elements per access.
 //                     Optionally (`pool_block` P > 0): a token that completes a block of P positions also leaves the
 //                     mean of the block's P keys, and of its P values, as the cache holds them (float32 sum, one
 //                     rounding), as one row of the pools of block means.  For steps that bring one token of a
@@ -111,6 +112,13 @@ __device__ __forceinline__ void pool_block(const T* k_pool, const T* v_pool, con
     }
 }
 
+// A pair of elements after its turn, with the roundings spelled out: both kernels below give the same bits, whichever a step's
+// options choose.
+__device__ __forceinline__ void turn_pair(float u, float v, float c, float s, float& a, float& b) {
+    a = __fmaf_rn(u, c, -__fmul_rn(v, s));
+    b = __fmaf_rn(v, c, __fmul_rn(u, s));
+}
+
 template <typename TI, typename T, bool MEANS>
 __global__ void attn_prepare_kernel(const TI* __restrict__ src, long long ld, int q_off, int k_off, int v_off,
                                     const float* __restrict__ freq, int n_rot, int half_layout,
@@ -167,7 +175,8 @@ __global__ void attn_prepare_kernel(const TI* __restrict__ src, long long ld, in
             for (int r = lane; r < pairs; r += 32) {
                 const int a = half_layout ? r : 2 * r, b = half_layout ? r + pairs : 2 * r + 1;
                 const float u = val(h * d + a), v = val(h * d + b), c = cs[r], s = cs[pairs + r];
-                const float ua = u * c - v * s, vb = v * c + u * s;
+                float ua, vb;
+                turn_pair(u, v, c, s, ua, vb);
                 sum += ua * ua + vb * vb;
             }
             for (int i = lane; i < rest; i += 32) { const float x = val(h * d + n_rot + i); sum += x * x; }
@@ -197,7 +206,8 @@ __global__ void attn_prepare_kernel(const TI* __restrict__ src, long long ld, in
         const bool is_q = h < n_qh;
         const float u = val(h * d + a), v = val(h * d + b);
         const float c = cs[r], s = cs[pairs + r];
-        float ua = u * c - v * s, vb = v * c + u * s;
+        float ua, vb;
+        turn_pair(u, v, c, s, ua, vb);
         if (head_eps > 0.f) { ua *= hm[h]; vb *= hm[h]; }
         if (is_q) {
             T* o = q_out + ((size_t)t * n_qh + h) * d;
@@ -233,8 +243,8 @@ __global__ void attn_prepare_kernel(const TI* __restrict__ src, long long ld, in
     }
 }
 
-// The same for heads that are divided by their root mean square: a group of LPH lanes per head, every access four
-// neighbouring elements.  A query's or key's words are its rotated pairs of words (4 dimensions and their 4 partners, half
+// The same where nothing ties a token's heads together: a group of LPH lanes per head, every access four neighbouring
+// elements; heads may be divided by their root mean square.  A query's or key's words are its rotated pairs of words (4 dimensions and their 4 partners, half
 // layout) and then the words that pass; lane i of the group owns pair or word i.  A value's words are the lanes' in pairs
 // too (v_second: how far the second lies behind the first, 0 for widths that are no multiple of 8).  A block takes TOK tokens (their angles made once, before
 // the wait) and walks the heads (queries, keys, values) that its place on the grid's second axis gives it; a head's bias
@@ -251,7 +261,8 @@ attn_prepare_heads_kernel(const TI* __restrict__ src, long long ld, int q_off, i
                           const int* __restrict__ tok_slot, const int* __restrict__ block_table, T* __restrict__ k_pool,
                           T* __restrict__ v_pool, T* __restrict__ q_out, int n_tokens, int n_qh, int n_kh, int n_vh, int d,
                           int dv, int page_size, int max_pages, int n_pool_pages, int append, int* __restrict__ status,
-                          const void* __restrict__ bias, int bias_dtype, float magnitude, float head_eps, int lph_, int v_second) {
+                          const void* __restrict__ bias, int bias_dtype, float magnitude, float head_eps, int lph_, int v_second,
+                          int inter) {
     gi_pdl_launch_dependents();
     extern __shared__ __align__(16) float cs[];   // per token cos [n_rot/2], sin [n_rot/2]
     __shared__ int page_of[TOK], row_of[TOK];     // where each token's key and value go; page -1: nowhere
@@ -287,7 +298,8 @@ attn_prepare_heads_kernel(const TI* __restrict__ src, long long ld, int q_off, i
     gi_pdl_wait();
     const int lph = LPH > 0 ? LPH : lph_;
     const int groups = APH_THREADS / lph, group = threadIdx.x / lph, lane = threadIdx.x - group * lph;
-    const int pair_words = pairs / 4, words = pair_words + (d - n_rot) / 4;
+    // interleaved pairs lie in one word, the others (r, r + n_rot/2) in two that a lane holds both of
+    const int pair_words = inter ? 0 : pairs / 4, words = inter ? d / 4 : pair_words + (d - n_rot) / 4, passed = inter ? 0 : n_rot;
     const int qk = n_qh + (k_off >= 0 ? n_kh : 0), heads = qk + (k_off >= 0 ? n_vh : 0);
     const float share = 1.f / (float)d;
     const int n_here = min(TOK, n_tokens - t0);
@@ -295,10 +307,10 @@ attn_prepare_heads_kernel(const TI* __restrict__ src, long long ld, int q_off, i
         const int h = h0 + group;                 // a group past the last head walks along for the shuffles
         const bool is_v = h >= qk;
         // the lane's word inside its head, and how far its second word lies behind it (0: there is none)
-        const int at = is_v || lane < pair_words ? 4 * lane : n_rot + 4 * (lane - pair_words);
+        const int at = is_v || lane < pair_words ? 4 * lane : passed + 4 * (lane - pair_words);
         const int second = is_v ? v_second : (lane < pair_words ? pairs : 0);
         const bool mine = h < heads && lane < (is_v ? (v_second ? dv / 8 : dv / 4) : words), two = mine && second > 0;
-        const bool turns = two && !is_v;
+        const bool turns = two && !is_v, turns_inside = inter && mine && !is_v && at < n_rot;
         const int col = is_v ? v_off + (h - qk) * dv : (h < n_qh ? q_off + h * d : k_off + (h - n_qh) * d);
         float4 ba = make_float4(0.f, 0.f, 0.f, 0.f), bb = ba;
         if (bias && mine) {
@@ -327,17 +339,26 @@ attn_prepare_heads_kernel(const TI* __restrict__ src, long long ld, int q_off, i
                 const float4 c = *reinterpret_cast<const float4*>(cs + k * n_rot + at);
                 const float4 s = *reinterpret_cast<const float4*>(cs + k * n_rot + pairs + at);
                 const float4 u = a, v = b;
-                a = make_float4(u.x * c.x - v.x * s.x, u.y * c.y - v.y * s.y, u.z * c.z - v.z * s.z, u.w * c.w - v.w * s.w);
-                b = make_float4(v.x * c.x + u.x * s.x, v.y * c.y + u.y * s.y, v.z * c.z + u.z * s.z, v.w * c.w + u.w * s.w);
+                turn_pair(u.x, v.x, c.x, s.x, a.x, b.x); turn_pair(u.y, v.y, c.y, s.y, a.y, b.y);
+                turn_pair(u.z, v.z, c.z, s.z, a.z, b.z); turn_pair(u.w, v.w, c.w, s.w, a.w, b.w);
             }
-            float sum = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;      // words that are not the lane's are zeros
-            sum += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
+            if (turns_inside) {
+                const float2 c = *reinterpret_cast<const float2*>(cs + k * n_rot + at / 2);
+                const float2 s = *reinterpret_cast<const float2*>(cs + k * n_rot + pairs + at / 2);
+                const float4 u = a;
+                turn_pair(u.x, u.y, c.x, s.x, a.x, a.y);
+                turn_pair(u.z, u.w, c.y, s.y, a.z, a.w);
+            }
+            if (head_eps > 0.f) {                     // the same for the whole launch
+                float sum = a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;  // words that are not the lane's are zeros
+                sum += b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w;
 #pragma unroll
-            for (int o = LPH > 0 ? LPH / 2 : 16; o > 0; o >>= 1)
-                if (LPH > 0 || o < lph) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            const float m = is_v ? 1.f : aph_inv_root<T>(sum * share + head_eps);
-            a.x *= m; a.y *= m; a.z *= m; a.w *= m;
-            b.x *= m; b.y *= m; b.z *= m; b.w *= m;
+                for (int o = LPH > 0 ? LPH / 2 : 16; o > 0; o >>= 1)
+                    if (LPH > 0 || o < lph) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                const float m = is_v ? 1.f : aph_inv_root<T>(sum * share + head_eps);
+                a.x *= m; a.y *= m; a.z *= m; a.w *= m;
+                b.x *= m; b.y *= m; b.z *= m; b.w *= m;
+            }
             if (mine && k < n_here) {
                 T* dst = base + (size_t)k * n_qh * d + at;
                 bool there = true;
@@ -407,25 +428,29 @@ extern "C" int gi_attn_prepare(const void* src, int src_dtype, long long ld, int
     const BlockMeans means = {mean_k, mean_v, mean_table, mean_block, mean_rows, mean_max_pages, mean_pages};
     if (n_tokens == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
-    // heads divided by their root mean square: a group of lanes per head, when every word of four elements falls into place
-    if (head_eps > 0.f && (half_layout || n_rot == 0) && !norm_w && temp_every == 0 && mean_block == 0 && n_rot % 8 == 0 &&
-        d % 4 == 0 && dv % 4 == 0) {
+    // nothing that ties a token's heads together (a norm over all of them, the queries' factor, block means): a group of lanes
+    // per head, when every word of four elements falls into place.  2,048 tokens, 32 rows of queries and 8 of keys of 64 and
+    // 4 heads of values of 128 out of float32 columns: 23.6 us with a block per token, element by element, 11 us so.  (Heads
+    // divided by their root mean square with interleaved pairs stay with the block per token, whose sums run in their order.)
+    const bool inter = !half_layout && n_rot > 0;
+    if (!norm_w && temp_every == 0 && mean_block == 0 && n_rot % (inter ? 4 : 8) == 0 && d % 4 == 0 && dv % 4 == 0 &&
+        (head_eps == 0.f || !inter)) {
         const int esz = src_dtype == GI_DTYPE_F32 ? 4 : 2, ez = act_dtype == GI_DTYPE_F32 ? 4 : 2;
-        const int words = n_rot / 8 + (d - n_rot) / 4, v_second = dv % 8 == 0 ? dv / 2 : 0;
+        const int words = inter ? d / 4 : n_rot / 8 + (d - n_rot) / 4, v_second = dv % 8 == 0 ? dv / 2 : 0;
         const int v_words = v_second ? dv / 8 : dv / 4, most = k_off >= 0 && v_words > words ? v_words : words;
         int lph = 1;
         while (lph < most) lph *= 2;
         const bool on_words = ld % 4 == 0 && q_off % 4 == 0 && (k_off < 0 || (k_off % 4 == 0 && v_off % 4 == 0)) &&
                               (uintptr_t)src % (4 * esz) == 0 && (uintptr_t)q_out % (4 * ez) == 0 && (uintptr_t)k_pool % (4 * ez) == 0 &&
                               (uintptr_t)v_pool % (4 * ez) == 0 && (uintptr_t)bias % 16 == 0;
-        if (lph <= 32 && on_words) {
+        if (lph <= 32 && on_words && (size_t)n_rot * 4 * sizeof(float) <= 40 * 1024) {
             const int heads = n_qh + (k_off >= 0 ? n_kh + n_vh : 0), groups = APH_THREADS / lph;
             const int rounds = (heads + groups - 1) / groups;
 #define APH_LAUNCH(TI, T, TOK)                                                                                       \
             gi_launch(lph == 16 ? attn_prepare_heads_kernel<TI, T, TOK, 16> : attn_prepare_heads_kernel<TI, T, TOK, 0>, dim3((n_tokens + TOK - 1) / TOK, TOK > 1 ? (rounds + 1) / 2 : rounds),  \
                       dim3(APH_THREADS), (size_t)TOK * n_rot * sizeof(float), s, (const TI*)src, ld, q_off, k_off, v_off, freq,  \
                       n_rot, tok_pos, tok_slot, block_table, (T*)k_pool, (T*)v_pool, (T*)q_out, n_tokens, n_qh, n_kh, n_vh, d,  \
-                      dv, page_size, max_pages, n_pool_pages, append, status, bias, bias_dtype, magnitude, head_eps, lph, v_second)
+                      dv, page_size, max_pages, n_pool_pages, append, status, bias, bias_dtype, magnitude, head_eps, lph, v_second, inter)
 #define APH_TOK(TI, T) if (n_tokens >= 256) APH_LAUNCH(TI, T, 4); else APH_LAUNCH(TI, T, 1)
             if (src_dtype == GI_DTYPE_F32 && act_dtype == GI_DTYPE_F32) { APH_TOK(float, float); }
             else if (src_dtype == GI_DTYPE_F32 && act_dtype == GI_DTYPE_BF16) { APH_TOK(float, bf16); }

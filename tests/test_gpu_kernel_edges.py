@@ -441,3 +441,56 @@ def test_routed_experts_of_few_rows_by_rows_and_by_products(unit, n, monkeypatch
         monkeypatch.setattr(moe, "ROWWISE_MAX_BYTES", limit)
         got.append(part.step(x, StepContext(n, z, z, z)).double())
     torch.testing.assert_close(got[0], got[1], rtol=2e-2, atol=1e-2)       # roundings of the activation and of the pairs' results
+
+
+# ---- between projections and attention ----------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("src_dtype, dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("d, dv, n_rot, half", [(64, 128, 0, False), (128, 64, 128, False), (128, 128, 64, True), (24, 20, 12, False),
+                                                (80, 80, 72, True), (24, 20, 6, False)])
+@pytest.mark.parametrize("n, bias, own", [(1, True, True), (5, False, True), (301, True, True), (7, False, False)])
+def test_queries_keys_and_values_by_words_and_by_elements(src_dtype, dtype, d, dv, n_rot, half, n, bias, own):
+    """The kernel that gives a head a group of lanes against the one that takes a token element by element (columns that do not
+    start on words): the same bits, rotations of both layouts, sizes that are not whole groups, padding rows; and 64 bits."""
+    from garlic_inference_b200.ops import kernels
+    H, G, page = 5, 2, 16
+    cols = H * d + (G * d + G * dv if own else 0)
+    src = rnd(n, cols, seed=1, dtype=src_dtype)
+    pos = (torch.arange(n, dtype=torch.int32) * 3 % 400).to(DEV)
+    slots = torch.zeros(n, dtype=torch.int32, device=DEV)
+    table = torch.arange(400 // page, dtype=torch.int32, device=DEV).flip(0).contiguous().view(1, -1)
+    if n > 1:
+        slots[n // 2] = -1
+        pos[:] = torch.randperm(400, generator=torch.Generator().manual_seed(2))[:n].to(DEV)       # every token a place of its own
+    freq = torch.tensor([1e4 ** (-2.0 * i / max(n_rot, 1)) for i in range(n_rot // 2)], device=DEV)
+    b = rnd(cols, seed=3) if bias else None
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(shift):
+        wide = torch.zeros((n, -(-(cols + shift) // 4) * 4 + shift), dtype=src_dtype, device=DEV)
+        wide[:, shift:shift + cols] = src
+        kp = torch.zeros((400 // page, G, page, d), dtype=dtype, device=DEV)
+        vp = torch.zeros((400 // page, G, page, dv), dtype=dtype, device=DEV)
+        k_off, v_off = (shift + H * d, shift + H * d + G * d) if own else (-1, 0)
+        q = kernels.attn_prepare(wide, shift, k_off, v_off, freq, n_rot, half, pos, slots, table if own else None, kp if own else None,
+                                 vp if own else None, H, d, dtype, status, append=own, bias=b, magnitude=1.25)
+        return q, kp, vp
+
+    words, elements = run(0), run(1)
+    assert all(torch.equal(x, y) for x, y in zip(words, elements)) and int(status.item()) == 0
+    x = src.double() + (b.double() if bias else 0.0)
+    q = x[:, :H * d].view(n, H, d)
+    a = pos.double()[:, None] * freq.double()
+    c, s = a.cos()[:, None] * 1.25, a.sin()[:, None] * 1.25
+    u, v = (q[..., :n_rot // 2], q[..., n_rot // 2:n_rot]) if half else (q[..., 0:n_rot:2], q[..., 1:n_rot:2])
+    turned = [u * c - v * s, v * c + u * s]
+    want = q.clone()
+    if n_rot:
+        want[..., :n_rot] = torch.cat(turned, -1) if half else torch.stack(turned, -1).flatten(-2)
+    tol = dict(rtol=2.0 ** -8, atol=2e-4) if dtype == torch.bfloat16 else dict(rtol=1e-5, atol=2e-4)      # float32 angles up to 400
+    torch.testing.assert_close(words[0].double(), want, **tol)
+    if own:
+        for t in range(0, n, 11):
+            if int(slots[t]) >= 0:
+                at = int(pos[t])
+                got = words[2][int(table[0, at // page]), :, at % page].double()
+                torch.testing.assert_close(got, x[t, H * d + G * d:].view(G, dv), **tol)
