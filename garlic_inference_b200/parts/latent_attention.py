@@ -151,19 +151,23 @@ class LatentAttention(Mixer):
         """Rows of a run of the flash kernel that takes a page of `keys` expanded keys."""
         return 128 if self.d == self.dv and kernels.tcgen05_attention_takes(self.rt.dtype, self.d, keys) else 64
 
+    def _portions(self, shape, page: int) -> list:
+        """[(sequence, first page, keys, rows of a run)] of the step's portions that are expanded."""
+        which = []
+        for i, (n_new, past) in enumerate(zip(shape.seq_lens, shape.seq_past)):
+            if self._expands(n_new, past, page):
+                p0 = self._first_page(past, page)
+                keys = (-(-(past + n_new) // page) - p0) * page
+                which.append((i, p0, keys, self._run_rows(keys)))
+        return which
+
     def _runs_of(self, shape, page: int):
-        """[(sequence, first page, keys, rows of a run)] of the step's portions that are expanded, and all their runs one
-        after the other; slot 0 and positions counted from the first page, as the expanded page holds them."""
+        """All runs of those portions one after the other; slot 0 and positions counted from the first page, as the expanded
+        page holds them."""
         import numpy as np
-        which, runs = [], []
-        for i, (start, n_new, past) in enumerate(zip(shape.seq_starts, shape.seq_lens, shape.seq_past)):
-            if not self._expands(n_new, past, page):
-                continue
-            p0 = self._first_page(past, page)
-            keys = (-(-(past + n_new) // page) - p0) * page
-            which.append((i, p0, keys, self._run_rows(keys)))
-            runs.append(query_runs(StepShape([0], [start], [n_new], [past - p0 * page], False), which[-1][3]))
-        return which, np.concatenate(runs) if runs else np.zeros((0, 4), dtype=np.int32)
+        runs = [query_runs(StepShape([0], [shape.seq_starts[i]], [shape.seq_lens[i]], [shape.seq_past[i] - p0 * page], False), rows)
+                for i, p0, _, rows in self._portions(shape, page)]
+        return np.concatenate(runs) if runs else np.zeros((0, 4), dtype=np.int32)
 
     def _runs_name(self, page: int) -> str:
         return f"latent_runs_{self.window}_{page}_{self.d}_{self.dr}_{self.dv}_{self.rank}_{self.H}"
@@ -172,7 +176,7 @@ class LatentAttention(Mixer):
         page = cache.kv.page_size
         if shape.all_single or not any(self._expands(m, p, page) for m, p in zip(shape.seq_lens, shape.seq_past)):
             return {}
-        return {self._runs_name(page): lambda: self._runs_of(shape, page)[1]}
+        return {self._runs_name(page): lambda: self._runs_of(shape, page)}
 
     def _attend_expanded(self, q, kv, ctx, which, gate, out):
         """Attention of the expanded portions of q [n, H, plain_dim + rot_dim] (its rotated part turned), gated, into their
@@ -181,7 +185,7 @@ class LatentAttention(Mixer):
         pool = kv.k_pool.view(kv.k_pool.shape[0], page, self.row)
         runs = ctx.arrays.get(self._runs_name(page))
         if runs is None:                           # a context put together by hand: cut and copy here
-            runs = ctx.arrays[self._runs_name(page)] = torch.from_numpy(self._runs_of(ctx, page)[1]).to(q.device)
+            runs = ctx.arrays[self._runs_name(page)] = torch.from_numpy(self._runs_of(ctx, page)).to(q.device)
         if self._one_page is None:
             self._one_page = torch.zeros((1, 1), dtype=torch.int32, device=q.device)
         at = 0
@@ -229,7 +233,7 @@ class LatentAttention(Mixer):
         # portions whose keys and values are expanded
         which = []
         if (both or self.dr) and out_mul == 1.0 and not ctx.all_single and not ctx.captured and ctx.seq_lens:
-            which, _ = self._runs_of(ctx, kv.page_size)
+            which = self._portions(ctx, kv.page_size)
             # columns to write into: rows that start on 16 bytes, and not by the mma.sync kernel
             if out is not None and (any(rows != 128 for *_, rows in which) or out.data_ptr() % 16 or out.stride(0) % 8):
                 which = []
