@@ -414,16 +414,21 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
     const int per = (n_chunks + n_splits - 1) / n_splits;
     const int c0 = first_chunk + split * per, c1 = min(first_chunk + n_chunks, c0 + per);
     if (dead && slot >= 0 && threadIdx.x == 0) atomicExch(status, 4);
+    if (c0 >= c1) {
+        // No keys in this slice: the merge reads its maximum alone, so the heads' columns of zeros are not written.  A decode
+        // step of 19 sequences of up to 24 tokens, 32 heads, 11 of 12 slices empty: 234 -> 223 us.
+        if (threadIdx.x < HG && h0 + (int)threadIdx.x < H) my[(size_t)(h0 + threadIdx.x) * stride] = -INFINITY;
+        return;
+    }
     const int vec_per_row = dk / 8, words = dk / 2;
 
-    if (c0 < c1)
-        for (int idx = threadIdx.x; idx < HG * (kw / 4); idx += blockDim.x) {
-            const int hh = idx / (kw / 4), v = idx - hh * (kw / 4);
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (h0 + hh < H && v < vec_per_row)
-                val = *reinterpret_cast<const uint4*>(q + ((size_t)t * H + h0 + hh) * dk + v * 8);
-            *reinterpret_cast<uint4*>(q_b + hh * kw + v * 4) = val;
-        }
+    for (int idx = threadIdx.x; idx < HG * (kw / 4); idx += blockDim.x) {
+        const int hh = idx / (kw / 4), v = idx - hh * (kw / 4);
+        uint4 val = make_uint4(0u, 0u, 0u, 0u);
+        if (h0 + hh < H && v < vec_per_row)
+            val = *reinterpret_cast<const uint4*>(q + ((size_t)t * H + h0 + hh) * dk + v * 8);
+        *reinterpret_cast<uint4*>(q_b + hh * kw + v * 4) = val;
+    }
     float m[4], l[4];
 #pragma unroll
     for (int hh = 0; hh < 4; ++hh) { m[hh] = -INFINITY; l[hh] = 0.f; }

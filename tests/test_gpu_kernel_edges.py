@@ -494,3 +494,30 @@ def test_queries_keys_and_values_by_words_and_by_elements(src_dtype, dtype, d, d
                 at = int(pos[t])
                 got = words[2][int(table[0, at // page]), :, at % page].double()
                 torch.testing.assert_close(got, x[t, H * d + G * d:].view(G, dv), **tol)
+
+
+# ---- one token per sequence over latent rows ---------------------------------------------------------------------------
+@pytest.mark.parametrize("heads", [17, 33])
+@pytest.mark.parametrize("n_splits, window", [(1, 0), (2, 0), (16, 0), (16, 40)])
+def test_latent_decode_with_slices_that_hold_no_keys(heads, n_splits, window):
+    """Fewer chunks of 32 rows than slices, down to a row without a sequence; the slices' buffer is left full of NaN first,
+    as the allocator may hand it out."""
+    from garlic_inference_b200.ops import kernels
+    row, rank, page, scale = 72, 64, 16, 0.2
+    pos = [0, 31, 32, 70, 200, 0]
+    n, per = len(pos), 13
+    table = torch.arange(n * per, dtype=torch.int32, device=DEV).view(n, per).flip(0).contiguous()
+    q, pool = rnd(n, heads, row, seed=1, dtype=torch.bfloat16), rnd(n * per, 1, page, row, seed=2, dtype=torch.bfloat16)
+    slot = torch.tensor(list(range(n - 1)) + [-1], dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    buffer = torch.full((n, n_splits, heads, rank + 2), float("nan"), device=DEV)
+    del buffer
+    got = kernels.latent_decode(q, pool, table, torch.tensor(pos, dtype=torch.int32, device=DEV), slot, scale, None, rank, status,
+                                n_splits=n_splits, window=window).view(n, heads, rank).double()
+    assert status.item() == 0 and not got[-1].any()
+    for t, p in enumerate(pos[:-1]):
+        keys = pool[table[t].long()].reshape(per * page, row)[max(0, p - window + 1) if window else 0:p + 1].double()
+        w = torch.softmax(q[t].double() @ keys.T * scale, -1)
+        # the weights and the result are rounded to bfloat16, 2^-9 of each; the rest is float32
+        bound = 1.1 * 2 ** -8 * (w @ keys[:, :rank].abs()) + 1e-5
+        assert ((got[t] - w @ keys[:, :rank]).abs() <= bound).all()
