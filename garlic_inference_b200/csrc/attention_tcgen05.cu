@@ -78,6 +78,7 @@ struct FtControl {
     unsigned long long s_full[2];
     unsigned long long p_ready[2];
     unsigned long long o_done;
+    unsigned long long bias_free, bias_ready;
     unsigned int tmem_base;
     int abort;
 };
@@ -247,6 +248,8 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
         }
         for (int b = 0; b < 2; ++b) { ft_mbar_init(&ctl->s_full[b], 1); ft_mbar_init(&ctl->p_ready[b], 4); }
         ft_mbar_init(&ctl->o_done, 1);
+        ft_mbar_init(&ctl->bias_free, 4);
+        ft_mbar_init(&ctl->bias_ready, 4);
         ctl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -410,18 +413,24 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const bool w = ft_mbar_wait(bar, parity, abort);
             return __all_sync(0xffffffffu, w);
         };
-        int g0 = 0;
+        int qn = 0, g0 = 0;                              // qn: items whose biases were put down
         FtItem im;
         for (int round = 0; ok; ++round) {
             const int have = item_at(round, im);
             if (have < 0) break;
             if (have == 0) continue;
             const int pos = im.pos0 + r;
-            if (BIAS) {                                  // the head's biases; every warp is done with those of the item before
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (BIAS) {                                  // the head's biases, by all four warps once each is done with the item's before
+                auto meet = [&](void* bar) {             // a warp that gave up never arrives, so the others' waits have to be bounded too
+                    __syncwarp();
+                    if (lane == 0) ft_mbar_arrive(bar);
+                    return wait_warp(bar, qn & 1);
+                };
+                if (!meet(&ctl->bias_free)) { ok = false; break; }
                 for (int i = (int)threadIdx.x - 64 - FT_BIAS_PAD; i < n_dist + FT_BIAS_PAD; i += 128)
                     bias_s[i] = dist_bias[(size_t)min(max(i, 0), n_dist - 1) * n_q + im.h] * 1.4426950408889634f;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!meet(&ctl->bias_ready)) { ok = false; break; }
+                ++qn;
             }
             float ref = -INFINITY, l = 0.f;              // exponentials are taken against `ref`; l is the sum of them
             for (int it = 0; it < im.n_tiles; ++it) {

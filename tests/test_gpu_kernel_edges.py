@@ -212,6 +212,26 @@ def test_prompt_attention_on_tensor_memory_at_other_sizes(d, dv, maps, n_dist, p
     kernels.check_bounded_waits(torch.device("cuda", 0))
 
 
+@pytest.mark.parametrize("n_dist", [40, 500])
+def test_distance_biases_where_a_block_walks_many_items(n_dist):
+    """More than six items of different heads to every persistent block, each with a table of its own in the same place."""
+    from garlic_inference_b200.ops import kernels
+    H, G, d, dv, page = 40, 8, 128, 64, 64
+    new = [1 + (37 * i) % 131 for i in range(44)]
+    lens = [m + (29 * i) % 90 for i, m in enumerate(new)]
+    ks, k_pool, table = _pools(lens, G, d, page, 20)
+    vs, v_pool, _ = _pools(lens, G, dv, page, 90)
+    runs, starts = _runs128(lens, new)
+    assert runs.shape[0] * H > 6 * 2 * 148
+    q, bias = rnd(sum(new), H, d, seed=5, dtype=torch.bfloat16), rnd(n_dist, H, seed=6)
+    got = kernels.attention_prefill_tcgen05(q, k_pool, v_pool, table, runs, d ** -0.5, 0, dist_bias=bias).view(-1, H, dv)
+    for s, (at, m) in enumerate(zip(starts, new)):
+        for h in range(H):
+            want = _attend64(q[at:at + m, h], ks[s][:, h * G // H], vs[s][:, h * G // H], lens[s] - m, d ** -0.5, bias=bias[:, h])
+            torch.testing.assert_close(got[at:at + m, h].double(), want, **ATT_TOL)
+    kernels.check_bounded_waits(torch.device("cuda", 0))
+
+
 @pytest.mark.parametrize("past, m", [(0, 1), (0, 129), (63, 70), (300, 40)])
 @pytest.mark.parametrize("window", [0, 90])
 def test_prompt_attention_with_a_key_part_that_all_heads_share(past, m, window):
