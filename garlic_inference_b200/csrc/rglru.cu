@@ -263,13 +263,16 @@ rglru_gates_wide_kernel(const float* __restrict__ u, const TW* __restrict__ wa_t
 
 // The same gates on tensor cores, for bfloat16 matrices.  A float32 input is the exact sum of three bfloat16 numbers
 // (its 24 bits of mantissa cut into 8 + 8 + 8), every product of one of them with a bfloat16 weight is exact in float32,
-// and the tensor core sums in float32: three `mma.sync` in place of one chain of float32 multiply-adds, at the same
-// precision (against 64 bits, in the block of 2,494 rows below: the layer's result is as far off as before).  A block of
+// and three `mma.sync` sum 16 inputs' products from zero.  The sums of all inputs are made of those by adds that round to
+// nearest: the tensor core cuts its sums off, and carried through all inputs that put b four to six times as far from 64
+// bits as the kernels above with float32 multiply-adds.  Relative errors of b (2-norm) against 64 bits in units of 1e-8, those
+// kernels / sums carried through / so, inputs of size 1: blocks of 64 7.6 / 10.8 / 7.5, 128 8.0 / 17.1 / 7.6, 320 8.8 / 38.9 / 8.0,
+// 1,280 25 / 156 / 9.6; a's 3.2 / 3.2 to 5.4 / 3.2.  A block of
 // 8 warps takes 128 rows x 64 outputs of both gates, a warp 16 rows of it (the split of its inputs then serves 128
 // columns); inputs and weights come through a ring of three chunks of 32 inputs.  A row's sums do not depend on the
 // other rows, and prompts and decode steps run the same kernel, so its bits still depend on the block width alone.
 // Bound by the tensor pipe's legacy path and by the exponentials of the last step.  Measured with blocks of 320
-// channels, 16 of them: 2,494 rows 945 -> 191 us, 8 rows 24 -> 16 us.
+// channels, 16 of them: 2,494 rows 945 -> 210 us (191 with the sums carried through), 8 rows 24 -> 19 us.
 #define RM_ROWS 128
 #define RM_OUT 64
 #define RM_KC 32
@@ -291,10 +294,11 @@ __device__ __forceinline__ void rm_split(float2 v, uint32_t& hi, uint32_t& mid, 
     lo = __byte_perm(__float_as_uint(rx - __uint_as_float(mx & 0xffff0000u)),
                      __float_as_uint(ry - __uint_as_float(my & 0xffff0000u)), 0x7632);
 }
-__device__ __forceinline__ void rm_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// d = a b + c
+__device__ __forceinline__ void rm_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&c)[4]) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
 
 __global__ void __launch_bounds__(256, 2)
@@ -348,6 +352,7 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
     const bool works = row0 + warp * 16 < n_rows;            // a warp whose rows lie beyond the last only copies
+    const float zero[4] = {0.f, 0.f, 0.f, 0.f};
     for (int chunk = 0; chunk < chunks; ++chunk) {
         rg_cp_async_wait_1();
         __syncthreads();                                     // this chunk is there, and the one before it is done with
@@ -361,6 +366,14 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
 #pragma unroll
             for (int e = 0; e < 4; ++e)                      // rows g, g + 8; inputs 2 t, 2 t + 1 and 8 further
                 rm_split(*reinterpret_cast<const float2*>(us + (e & 1) * 8 * RM_ULD + kk + (e >> 1) * 8), hi[e], mid[e], lo[e]);
+            auto products = [&](float (&sum)[4], uint32_t b0, uint32_t b1) {
+                float d[4];
+                rm_mma(d, lo, b0, b1, zero);
+                rm_mma(d, mid, b0, b1, d);
+                rm_mma(d, hi, b0, b1, d);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[e] += d[e];
+            };
 #pragma unroll
             for (int gate = 0; gate < 2; ++gate)
 #pragma unroll
@@ -369,12 +382,8 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
                     const bf16* at = ws + (gate * RM_KC + kk + (lane & 15)) * RM_WLD + j * 8 + (lane >> 4) * 8;
                     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                                  : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"((uint32_t)__cvta_generic_to_shared(at)));
-                    rm_mma(acc[gate][j], lo, b[0], b[1]);
-                    rm_mma(acc[gate][j + 1], lo, b[2], b[3]);
-                    rm_mma(acc[gate][j], mid, b[0], b[1]);
-                    rm_mma(acc[gate][j + 1], mid, b[2], b[3]);
-                    rm_mma(acc[gate][j], hi, b[0], b[1]);
-                    rm_mma(acc[gate][j + 1], hi, b[2], b[3]);
+                    products(acc[gate][j], b[0], b[1]);
+                    products(acc[gate][j + 1], b[2], b[3]);
                 }
         }
     }
