@@ -282,13 +282,13 @@ rglru_gates_wide_kernel(const float* __restrict__ u, const TW* __restrict__ wa_t
 #define RM_STAGE_BYTES (RM_ROWS * RM_ULD * 4 + 2 * RM_KC * RM_WLD * 2)
 
 // {x, y} as three pairs of bfloat16 that sum to them exactly: the upper 16 bits, the upper 16 bits of what is left, and the
-// rest.  An infinity or NaN stays in the first (its remainder would be a NaN).
+// rest.  An infinity stays in the first (its remainder would be a NaN); a NaN's remainder is one, whatever its upper bits say.
 __device__ __forceinline__ void rm_split(float2 v, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
     hi = __byte_perm(x, y, 0x7632);
     float rx = v.x - __uint_as_float(x & 0xffff0000u), ry = v.y - __uint_as_float(y & 0xffff0000u);
-    if ((x & 0x7f800000u) == 0x7f800000u) rx = 0.f;
-    if ((y & 0x7f800000u) == 0x7f800000u) ry = 0.f;
+    if ((x & 0x7fffffffu) == 0x7f800000u) rx = 0.f;
+    if ((y & 0x7fffffffu) == 0x7f800000u) ry = 0.f;
     const uint32_t mx = __float_as_uint(rx), my = __float_as_uint(ry);
     mid = __byte_perm(mx, my, 0x7632);
     lo = __byte_perm(__float_as_uint(rx - __uint_as_float(mx & 0xffff0000u)),
@@ -299,6 +299,13 @@ __device__ __forceinline__ void rm_mma(float (&d)[4], const uint32_t (&a)[4], ui
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+// One output's sum by float32 multiply-adds of the whole inputs: what the three parts of a finite input times an infinite
+// weight are not (a part that is zero makes a NaN of it).
+__device__ __noinline__ float rm_plain(const float* u, const bf16* w, int bw) {
+    float s = 0.f;
+    for (int k = 0; k < bw; ++k) s = fmaf(to_f32(w[(size_t)k * bw]), u[k], s);
+    return s;
 }
 
 __global__ void __launch_bounds__(256, 2)
@@ -402,7 +409,12 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
             float2 ra, rb;
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float r = rg_sigmoid(acc[0][j][half * 2 + e] + vecs[0][oo + e]), i = rg_sigmoid(acc[1][j][half * 2 + e] + vecs[1][oo + e]);
+                float za = acc[0][j][half * 2 + e], zi = acc[1][j][half * 2 + e];
+                if (za != za || zi != zi) {
+                    za = rm_plain(u + at - o, wa_t + (size_t)blk * bw * bw + o + e, bw);
+                    zi = rm_plain(u + at - o, wi_t + (size_t)blk * bw * bw + o + e, bw);
+                }
+                const float r = rg_sigmoid(za + vecs[0][oo + e]), i = rg_sigmoid(zi + vecs[1][oo + e]);
                 const float log_a = -decay_scale * r * vecs[2][oo + e];
                 const float keep = sqrtf(fmaxf(-expm1f(2.f * log_a), 0.f));
                 (e ? ra.y : ra.x) = expf(log_a);

@@ -102,6 +102,27 @@ def test_recurrent_gates_on_tensor_cores_are_as_close_as_by_multiply_adds(blocks
         assert (got.double() - w).norm() <= 1.01 * (other.double() - w).norm()
 
 
+@pytest.mark.parametrize("n", [1, 17, 200])
+def test_recurrent_gates_beyond_the_finite_are_those_of_multiply_adds(n):
+    """Infinite weights times inputs whose second and third parts are zero, infinite inputs times weights that are and are not
+    zero, a NaN whose upper 16 bits are an infinity's: infinities and NaN where the multiply-adds have them."""
+    from garlic_inference_b200.ops import kernels
+    blocks, bw = 2, 72
+    u = rnd(n, blocks * bw, seed=1)
+    u[:, 3] = 1.5                                                          # one part
+    u[0, 4] = math.inf
+    u[n - 1, 80:81].view(torch.int32)[0] = 0x7f800001
+    wa, wi = (rnd(blocks, bw, bw, seed=s, scale=bw ** -0.5, dtype=torch.bfloat16) for s in (2, 3))
+    wa[0, 3, 5], wa[0, 3, 6], wi[0, 3, 7], wi[0, 4, 8], wa[1, 9, 1] = math.inf, -math.inf, math.inf, 0.0, math.nan
+    ba, bi, lam = rnd(blocks * bw, seed=4), rnd(blocks * bw, seed=5), rnd(blocks * bw, seed=6)
+    tensor, plain = (kernels.rglru_gates(u, wa.to(t), wi.to(t), ba, bi, lam, 8.0) for t in (torch.bfloat16, torch.float32))
+    for got, want in zip(tensor, plain):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        ok = want.isfinite()
+        torch.testing.assert_close(got[ok], want[ok], rtol=1e-5, atol=1e-5)
+    assert float(tensor[0][n - 1, 6]) == 1.0 or n == 1                     # a gate shut by minus infinity keeps the state
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width, pad", [(32, 8), (100, 0), (66, 2), (35, 0), (324, 4)])
 @pytest.mark.parametrize("lens", [[1, 2], [3, 4, 5], [59, 60, 61], [64, 130, 1]])
