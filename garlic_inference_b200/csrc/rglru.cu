@@ -267,19 +267,20 @@ rglru_gates_wide_kernel(const float* __restrict__ u, const TW* __restrict__ wa_t
 // nearest: the tensor core cuts its sums off, and carried through all inputs that put b four to six times as far from 64
 // bits as the kernels above with float32 multiply-adds.  Relative errors of b (2-norm) against 64 bits in units of 1e-8, those
 // kernels / sums carried through / so, inputs of size 1: blocks of 64 7.6 / 10.8 / 7.5, 128 8.0 / 17.1 / 7.6, 320 8.8 / 38.9 / 8.0,
-// 1,280 25 / 156 / 9.6; a's 3.2 / 3.2 to 5.4 / 3.2.  A block of
-// 8 warps takes 128 rows x 64 outputs of both gates, a warp 16 rows of it (the split of its inputs then serves 128
-// columns); inputs and weights come through a ring of three chunks of 32 inputs.  A row's sums do not depend on the
-// other rows, and prompts and decode steps run the same kernel, so its bits still depend on the block width alone.
-// Bound by the tensor pipe's legacy path and by the exponentials of the last step.  Measured with blocks of 320
-// channels, 16 of them: 2,494 rows 945 -> 210 us (191 with the sums carried through), 8 rows 24 -> 19 us.
-#define RM_ROWS 128
+// 1,280 25 / 156 / 9.6; a's 3.2 / 3.2 to 5.4 / 3.2.
+// A block of 8 warps takes 16 MW rows x 64 outputs of both gates; inputs and weights come through a ring of three chunks of
+// 32 inputs.  Many rows: a warp has 16 rows and all 64 outputs, so that the split of its inputs serves 128 columns (MW 8).
+// Few rows: the warps share the outputs of the same rows (MW 1: 8 outputs of both gates each), since one warp with all of
+// them would have the products of a chunk to itself.  A row's sums are the same in every form and do not depend on the
+// other rows, so its bits depend on the block width alone.
+// Bound by the tensor pipe's legacy path and by the exponentials of the last step.  Measured in us, multiply-adds / always
+// MW 8 / so: 16 blocks of 320, 2,494 rows 945 / 210 / 210, 64 rows 38 / 24 / 17, 8 rows 25 / 19 / 8; 64 blocks of 64, 8 rows
+// 8.4 / 10.7 / 4.0, 64 rows 10.5 / 15 / 6.0; 16 blocks of 128, 64 rows 9.9 / 17 / 5.9, 512 rows 42 / 19 / 16.
 #define RM_OUT 64
 #define RM_KC 32
 #define RM_STAGES 3
 #define RM_ULD (RM_KC + 8)           // row length of the staged inputs: pairs of floats without bank conflicts
 #define RM_WLD (RM_OUT + 8)          // of the staged weights: the rows that ldmatrix reads start 4 banks apart
-#define RM_STAGE_BYTES (RM_ROWS * RM_ULD * 4 + 2 * RM_KC * RM_WLD * 2)
 
 // {x, y} as three pairs of bfloat16 that sum to them exactly: the upper 16 bits, the upper 16 bits of what is left, and the
 // rest.  An infinity stays in the first (its remainder would be a NaN); a NaN's remainder is one, whatever its upper bits say.
@@ -308,19 +309,23 @@ __device__ __noinline__ float rm_plain(const float* u, const bf16* w, int bw) {
     return s;
 }
 
+// MW: warps along the rows, 16 rows each; the 8 / MW warps of the same rows share the 64 outputs, 8 MW each.
+template <int MW>
 __global__ void __launch_bounds__(256, 2)
 rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_t, const bf16* __restrict__ wi_t,
                        const void* __restrict__ ba, const void* __restrict__ bi, const void* __restrict__ lam, int vec_dtype,
                        float decay_scale, float* __restrict__ a_out, float* __restrict__ b_out, int n_rows, int width, int bw) {
+    constexpr int ROWS = 16 * MW, STAGE_BYTES = ROWS * RM_ULD * 4 + 2 * RM_KC * RM_WLD * 2;
     gi_pdl_start();
     extern __shared__ __align__(16) unsigned char rg_smem[];
     __shared__ float vecs[3][RM_OUT];                        // both biases and softplus(lam) of this block's outputs
     const int slices = (bw + RM_OUT - 1) / RM_OUT;           // neighbouring blocks share their rows' inputs
-    const int o0 = (int)(blockIdx.x % slices) * RM_OUT, row0 = (int)(blockIdx.x / slices) * RM_ROWS, blk = blockIdx.y;
+    const int o0 = (int)(blockIdx.x % slices) * RM_OUT, row0 = (int)(blockIdx.x / slices) * ROWS, blk = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int wr = warp % MW * 16, wc = warp / MW * (8 * MW);          // the warp's first row and output of the block
     const int chunks = (bw + RM_KC - 1) / RM_KC;
-    auto stage_u = [&](int s) { return reinterpret_cast<float*>(rg_smem + (size_t)s * RM_STAGE_BYTES); };
-    auto stage_w = [&](int s) { return reinterpret_cast<bf16*>(rg_smem + (size_t)s * RM_STAGE_BYTES + RM_ROWS * RM_ULD * 4); };
+    auto stage_u = [&](int s) { return reinterpret_cast<float*>(rg_smem + (size_t)s * STAGE_BYTES); };
+    auto stage_w = [&](int s) { return reinterpret_cast<bf16*>(rg_smem + (size_t)s * STAGE_BYTES + ROWS * RM_ULD * 4); };
     // A chunk's inputs and weights, 16 bytes at a time; what lies outside (rows, inputs or outputs beyond the last) is
     // zero-filled and its address is that of something inside.
     auto fetch = [&](int chunk) {
@@ -329,10 +334,10 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
             float* us = stage_u(s);
             bf16* ws = stage_w(s);
 #pragma unroll
-            for (int i = 0; i < RM_ROWS * (RM_KC / 4) / 256; ++i) {
+            for (int i = 0; i < (ROWS * (RM_KC / 4) + 255) / 256; ++i) {
                 const int id = threadIdx.x + 256 * i, r = id / (RM_KC / 4), c = id % (RM_KC / 4) * 4;
                 const bool in = row0 + r < n_rows && k0 + c < bw;
-                rg_cp_async_16(us + r * RM_ULD + c, u + (in ? (size_t)(row0 + r) * width + blk * bw + k0 + c : 0), in ? 16 : 0);
+                if (r < ROWS) rg_cp_async_16(us + r * RM_ULD + c, u + (in ? (size_t)(row0 + r) * width + blk * bw + k0 + c : 0), in ? 16 : 0);
             }
 #pragma unroll
             for (int i = 0; i < 2 * RM_KC * (RM_OUT / 8) / 256; ++i) {
@@ -351,22 +356,22 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
         vecs[1][threadIdx.x] = load_w(bi, vec_dtype, c);
         vecs[2][threadIdx.x] = rg_softplus(load_w(lam, vec_dtype, c));
     }
-    float acc[2][RM_OUT / 8][4];
+    float acc[2][MW][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < RM_OUT / 8; ++j)
+        for (int j = 0; j < MW; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-    const bool works = row0 + warp * 16 < n_rows;            // a warp whose rows lie beyond the last only copies
+    const bool works = row0 + wr < n_rows && o0 + wc < bw;   // a warp whose rows or outputs lie beyond the last only copies
     const float zero[4] = {0.f, 0.f, 0.f, 0.f};
     for (int chunk = 0; chunk < chunks; ++chunk) {
         rg_cp_async_wait_1();
         __syncthreads();                                     // this chunk is there, and the one before it is done with
         fetch(chunk + RM_STAGES - 1);
         if (!works) continue;
-        const float* us = stage_u(chunk % RM_STAGES) + (warp * 16 + g) * RM_ULD + 2 * t;
-        const bf16* ws = stage_w(chunk % RM_STAGES);
+        const float* us = stage_u(chunk % RM_STAGES) + (wr + g) * RM_ULD + 2 * t;
+        const bf16* ws = stage_w(chunk % RM_STAGES) + wc;
 #pragma unroll
         for (int kk = 0; kk < RM_KC; kk += 16) {
             uint32_t hi[4], mid[4], lo[4];
@@ -383,26 +388,34 @@ rglru_gates_mma_kernel(const float* __restrict__ u, const bf16* __restrict__ wa_
             };
 #pragma unroll
             for (int gate = 0; gate < 2; ++gate)
+                if (MW == 1) {
+                    uint32_t b[2];
+                    const bf16* at = ws + (gate * RM_KC + kk + (lane & 15)) * RM_WLD;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                                 : "=r"(b[0]), "=r"(b[1]) : "r"((uint32_t)__cvta_generic_to_shared(at)));
+                    products(acc[gate][0], b[0], b[1]);
+                } else {
 #pragma unroll
-                for (int j = 0; j < RM_OUT / 8; j += 2) {
-                    uint32_t b[4];
-                    const bf16* at = ws + (gate * RM_KC + kk + (lane & 15)) * RM_WLD + j * 8 + (lane >> 4) * 8;
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"((uint32_t)__cvta_generic_to_shared(at)));
-                    products(acc[gate][j], b[0], b[1]);
-                    products(acc[gate][j + 1], b[2], b[3]);
+                    for (int j = 0; j + 1 < MW; j += 2) {
+                        uint32_t b[4];
+                        const bf16* at = ws + (gate * RM_KC + kk + (lane & 15)) * RM_WLD + j * 8 + (lane >> 4) * 8;
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                     : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"((uint32_t)__cvta_generic_to_shared(at)));
+                        products(acc[gate][j], b[0], b[1]);
+                        products(acc[gate][j + 1], b[2], b[3]);
+                    }
                 }
         }
     }
     rg_cp_async_wait_0();
     if (!works) return;
 #pragma unroll
-    for (int j = 0; j < RM_OUT / 8; ++j) {
-        const int oo = j * 8 + 2 * t, o = o0 + oo;
+    for (int j = 0; j < MW; ++j) {
+        const int oo = wc + j * 8 + 2 * t, o = o0 + oo;
         if (o >= bw) continue;                               // a multiple of 8: the pair's other output is in as well
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            const int row = row0 + warp * 16 + g + half * 8;
+            const int row = row0 + wr + g + half * 8;
             if (row >= n_rows) continue;
             const size_t at = (size_t)row * width + blk * bw + o;
             const float2 x = *reinterpret_cast<const float2*>(u + at);
@@ -439,11 +452,22 @@ extern "C" int gi_rglru_gates(const float* u, const void* wa_t, const void* wi_t
     // well, and nine products.)
     if (w_dtype == GI_DTYPE_BF16 && bw % 8 == 0 && ((uintptr_t)u | (uintptr_t)wa_t | (uintptr_t)wi_t) % 16 == 0 &&
         ((uintptr_t)a_out | (uintptr_t)b_out) % 8 == 0) {
-        const size_t smem = (size_t)RM_STAGES * RM_STAGE_BYTES;
-        if (int rc = gi_reserve_smem((const void*)rglru_gates_mma_kernel, smem, "gi_rglru_gates")) return rc;
-        dim3 grid((unsigned)((bw + RM_OUT - 1) / RM_OUT) * (unsigned)((n_rows + RM_ROWS - 1) / RM_ROWS), blocks);
-        gi_launch(rglru_gates_mma_kernel, grid, dim3(256), smem, (cudaStream_t)stream, u, (const bf16*)wa_t, (const bf16*)wi_t,
-                  ba, bi, lam, vec_dtype, decay_scale, a_out, b_out, n_rows, width, bw);
+        // the tallest tile that rows fill by more than a half and that leaves an SM each a block of threads
+        const long long across = (long long)((bw + RM_OUT - 1) / RM_OUT) * blocks;
+        int mw = 8;
+        while (mw > 1 && (n_rows <= 8 * mw || across * ((n_rows + 16 * mw - 1) / (16 * mw)) < 148)) mw /= 2;
+#define RM_LAUNCH(MW) do {                                                                                                     \
+            const size_t smem = (size_t)RM_STAGES * (16 * MW * RM_ULD * 4 + 2 * RM_KC * RM_WLD * 2);                           \
+            if (int rc = gi_reserve_smem((const void*)rglru_gates_mma_kernel<MW>, smem, "gi_rglru_gates")) return rc;          \
+            dim3 grid((unsigned)((bw + RM_OUT - 1) / RM_OUT) * (unsigned)((n_rows + 16 * MW - 1) / (16 * MW)), blocks);        \
+            gi_launch(rglru_gates_mma_kernel<MW>, grid, dim3(256), smem, (cudaStream_t)stream, u, (const bf16*)wa_t,           \
+                      (const bf16*)wi_t, ba, bi, lam, vec_dtype, decay_scale, a_out, b_out, n_rows, width, bw);                \
+        } while (0)
+        if (mw == 1) RM_LAUNCH(1);
+        else if (mw == 2) RM_LAUNCH(2);
+        else if (mw == 4) RM_LAUNCH(4);
+        else RM_LAUNCH(8);
+#undef RM_LAUNCH
         return gi_check_launch("gi_rglru_gates");
     }
     // outputs per block of threads and tokens per tile: as many as shared memory takes (the sizes depend on the

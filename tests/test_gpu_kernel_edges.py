@@ -123,6 +123,26 @@ def test_recurrent_gates_beyond_the_finite_are_those_of_multiply_adds(n):
     assert float(tensor[0][n - 1, 6]) == 1.0 or n == 1                     # a gate shut by minus infinity keeps the state
 
 
+@pytest.mark.parametrize("blocks, bw", [(80, 72), (40, 136), (160, 8)])
+def test_recurrent_gates_have_the_same_bits_in_tiles_of_every_height(blocks, bw):
+    """Steps whose tiles are 16, 32, 64 and 128 rows high (`blocks` of channels enough for each), whole and part tiles."""
+    from garlic_inference_b200.ops import kernels
+    W = blocks * bw
+    u = rnd(300, W, seed=1, scale=2.0)
+    wa, wi = (rnd(blocks, bw, bw, seed=s, scale=bw ** -0.5, dtype=torch.bfloat16) for s in (2, 3))
+    rest = wa, wi, rnd(W, seed=4), rnd(W, seed=5), rnd(W, seed=6), 8.0
+    whole = kernels.rglru_gates(u, *rest)
+    z = [torch.einsum("nbi,bio->nbo", u.double().view(300, blocks, bw), w.double()).reshape(300, W) + b.double()
+         for w, b in ((wa, rest[2]), (wi, rest[3]))]
+    log_a = -8.0 * torch.sigmoid(z[0]) * torch.nn.functional.softplus(rest[4].double())
+    want = torch.exp(log_a), torch.sqrt(-torch.expm1(2 * log_a)) * torch.sigmoid(z[1]) * u.double()
+    for got, w in zip(whole, want):
+        assert (got.double() - w).norm() <= 1e-6 * w.norm()
+    for at, n in ((0, 1), (3, 16), (17, 17), (20, 40), (100, 64), (64, 65), (0, 128), (170, 129)):
+        for got, w in zip(kernels.rglru_gates(u[at:at + n].contiguous(), *rest), whole):
+            assert torch.equal(got, w[at:at + n]), n
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width, pad", [(32, 8), (100, 0), (66, 2), (35, 0), (324, 4)])
 @pytest.mark.parametrize("lens", [[1, 2], [3, 4, 5], [59, 60, 61], [64, 130, 1]])
