@@ -34,6 +34,10 @@ __device__ __forceinline__ void rg_cp_async_4(float* smem, const float* gmem) {
 __device__ __forceinline__ void rg_cp_async_16(void* smem, const void* gmem, int bytes) {      // the rest of the 16 is zero-filled
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(bytes));
 }
+// 4 bytes, the first n of them copied and the others zero
+__device__ __forceinline__ void rg_cp_async_4n(void* dst, const void* src, int n) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n));
+}
 __device__ __forceinline__ void rg_cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void rg_cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::); }
 __device__ __forceinline__ void rg_cp_async_wait_0() { asm volatile("cp.async.wait_group 0;\n" ::); }
@@ -538,10 +542,13 @@ template <> __device__ __forceinline__ float rg_gate_act<bf16>(float z) {
 // copies of 16 bytes a lane).  What bounds a walk is a trip to memory divided by the tokens under way.  Loads into
 // registers could not keep 32 tokens under way however they were written: a warp has six counters for loads under way, and
 // waiting for one group's waits for every later load on the same counter.  Measured with 2,494 rows of 5,120 channels in four
-// prompts of up to 900 tokens (153 MB): 144 us with the ring in registers, 63 us so.
+// prompts of up to 900 tokens (153 MB): 144 us with the ring in registers, 63 us so.  Rows that do not start on 16 bytes
+// are copied 4 bytes a lane (a, b and y each by its own alignment): 129 us with y in columns from the fourth on, 83 us in
+// float32 from the first; loads that a group waited for took 205 and 221 us.
 #define RG_SUB 4             // tokens to a group
 #define RG_DEPTH 16          // groups in the ring
 #define RG_SCAN_THREADS 32
+#define RG_YLD 40            // row length of the staged y: 32 elements, one more where a row starts inside a word, rows on 16 bytes
 template <typename T>
 __global__ void __launch_bounds__(RG_SCAN_THREADS)
 rglru_scan_kernel(const float* __restrict__ a, const float* __restrict__ b, const T* __restrict__ y, long long ldy,
@@ -569,29 +576,44 @@ rglru_scan_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
         return;
     }
     __shared__ __align__(16) float a_s[RG_DEPTH][RG_SUB][32], b_s[RG_DEPTH][RG_SUB][32];
-    __shared__ __align__(16) T y_s[RG_DEPTH][RG_SUB][32];
+    __shared__ __align__(16) T y_s[RG_DEPTH][RG_SUB][RG_YLD];
     const int groups = (len + RG_SUB - 1) / RG_SUB;
+    // 1 for a row of bfloat16 y that starts in the middle of a 4-byte word: its elements lie one place further in y_s
+    auto y_row = [&](int t) { return y + (size_t)(start + min(t, len - 1)) * ldy + cw; };
+    auto y_shift = [&](const T* row) { return sizeof(T) == 2 ? (int)((uintptr_t)row >> 1 & 1) : 0; };
     // lane l copies 16 bytes of token l / 8 of a group (bytes beyond the last channel are zero-filled); a group's last
     // tokens beyond the sequence are its last row again, and not walked
     auto fetch = [&](int grp) {
         if (grp < groups) {
             const int s = grp % RG_DEPTH;
-            if (wide) {
+            if (wide & 1) {
                 const int j = lane >> 3, o = (lane & 7) * 4, n = min(16, max(0, (width - cw - o) * 4));
                 const size_t at = (size_t)(start + min(grp * RG_SUB + j, len - 1)) * width + (n ? cw + o : 0);
                 rg_cp_async_16(&a_s[s][j][o], a + at, n);
                 rg_cp_async_16(&b_s[s][j][o], b + at, n);
+            } else {
+#pragma unroll
+                for (int j = 0; j < RG_SUB; ++j) {           // rows that do not start on 16 bytes: a float a lane
+                    const size_t at = (size_t)(start + min(grp * RG_SUB + j, len - 1)) * width + (live ? c : 0);
+                    rg_cp_async_4n(&a_s[s][j][lane], a + at, live ? 4 : 0);
+                    rg_cp_async_4n(&b_s[s][j][lane], b + at, live ? 4 : 0);
+                }
+            }
+            if (wide & 2) {
                 constexpr int PER = 16 / (int)sizeof(T), LPR = 32 / PER;       // elements to a copy, lanes to a row
                 if (lane < RG_SUB * LPR) {
                     const int jy = lane / LPR, oy = lane % LPR * PER, ny = min(16, max(0, (width - cw - oy) * (int)sizeof(T)));
-                    rg_cp_async_16(&y_s[s][jy][oy], y + (size_t)(start + min(grp * RG_SUB + jy, len - 1)) * ldy + (ny ? cw + oy : 0), ny);
+                    rg_cp_async_16(&y_s[s][jy][oy], y_row(grp * RG_SUB + jy) + (ny ? oy : -cw), ny);
                 }
             } else {
-                for (int j = 0; j < RG_SUB; ++j) {           // rows that do not start on 16 bytes
-                    const size_t r = (size_t)(start + min(grp * RG_SUB + j, len - 1));
-                    a_s[s][j][lane] = live ? a[r * width + c] : 0.f;
-                    b_s[s][j][lane] = live ? b[r * width + c] : 0.f;
-                    y_s[s][j][lane] = live ? y[r * ldy + c] : from_f32<T>(0.f);
+                // A row's elements by whole 4-byte words of memory, a word a lane: the first may hold the element in front of
+                // the row (a part of the same aligned word, so of the same allocation), the last is cut off at the row's end.
+                constexpr int PER = 4 / (int)sizeof(T), WORDS = 32 / PER + (PER > 1);
+#pragma unroll
+                for (int j = 0; j < RG_SUB; ++j) {
+                    const T* row = y_row(grp * RG_SUB + j);
+                    const int sh = y_shift(row), ny = min(4, max(0, (min(32, width - cw) + sh - lane * PER) * (int)sizeof(T)));
+                    if (lane < WORDS) rg_cp_async_4n(&y_s[s][j][lane * PER], row - sh + (ny ? lane * PER : 0), ny);
                 }
             }
         }
@@ -611,7 +633,7 @@ rglru_scan_kernel(const float* __restrict__ a, const float* __restrict__ b, cons
         for (int j = 0; j < RG_SUB; ++j) {
             ga[j] = a_s[s][j][lane];
             gb[j] = b_s[s][j][lane];
-            gy[j] = rg_gate_act<T>(to_f32(y_s[s][j][lane]) + yb);
+            gy[j] = rg_gate_act<T>(to_f32(y_s[s][j][lane + (wide & 2 ? 0 : y_shift(y_row(grp * RG_SUB + j)))]) + yb);
         }
 #pragma unroll
         for (int j = 0; j < RG_SUB; ++j) {
@@ -638,7 +660,8 @@ extern "C" int gi_rglru_scan(const float* a, const float* b, const void* y, long
     if (n_seqs == 0) return 0;
     dim3 grid(n_seqs, (width + RG_SCAN_THREADS - 1) / RG_SCAN_THREADS);
     const int item = act_dtype == GI_DTYPE_F32 ? 4 : 2;
-    const int wide = width % 4 == 0 && ldy * item % 16 == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) % 16 == 0;
+    // 1: rows of a and b start on 16 bytes, 2: rows of y do
+    const int wide = (width % 4 == 0 && ((uintptr_t)a | (uintptr_t)b) % 16 == 0 ? 1 : 0) | (ldy * item % 16 == 0 && (uintptr_t)y % 16 == 0 ? 2 : 0);
     cudaStream_t s = (cudaStream_t)stream;
     if (act_dtype == GI_DTYPE_F32)
         gi_launch(rglru_scan_kernel<float>, grid, dim3(RG_SCAN_THREADS), 0, s, a, b, (const float*)y, ldy, y_bias, bias_dtype, state,

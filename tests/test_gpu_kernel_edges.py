@@ -172,6 +172,29 @@ def test_recurrent_scan_at_the_ends_of_its_ring(dtype, width, pad, lens):
     assert torch.equal(state[:, width:], before[:, width:])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width", [40, 65, 130])
+@pytest.mark.parametrize("first, row", [(0, 136), (8, 144), (4, 148), (2, 146), (1, 137), (3, 138), (0, 137)])
+def test_recurrent_scan_over_columns_at_every_alignment(dtype, width, first, row):
+    """y in columns whose rows start on 16, 8, 4 and 2 bytes, the same or another for every row: the bits of dense rows."""
+    from garlic_inference_b200.ops import kernels
+    lens = [70, 1, 6]
+    n = sum(lens)
+    a, b = torch.rand(n, width, generator=torch.Generator().manual_seed(1)).to(DEV), rnd(n, width, seed=2)
+    wide = rnd(n, row, seed=3, dtype=dtype)
+    y = wide[:, first:first + width]
+    spans = torch.tensor([[i, sum(lens[:i]), m] for i, m in enumerate(lens)], dtype=torch.int32, device=DEV)
+    slots, states = torch.zeros(n, dtype=torch.int32, device=DEV), [rnd(len(lens), width, seed=5) for _ in range(2)]
+    padded = torch.zeros(n, -(-width // 8) * 8, dtype=dtype, device=DEV)
+    padded[:, :width] = y                                                  # rows on 16 bytes
+    want, got = (kernels.rglru_scan(a, b, v, None, s, spans, slots) for v, s in ((padded[:, :width], states[0]), (y, states[1])))
+    assert torch.equal(got, want) and torch.equal(*states)
+    one = torch.empty_like(wide)                                           # (a and b off 16 bytes as well)
+    shifted = [torch.empty(n * width + 1, device=DEV)[1:].view(n, width).copy_(v) for v in (a, b)]
+    out = kernels.rglru_scan(*shifted, y, None, rnd(len(lens), width, seed=5), spans, slots, out=one[:, first:first + width])
+    assert torch.equal(out, want)
+
+
 # ---- float32 product -------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("N, K", [(1, 4), (17, 7), (64, 128), (200, 130), (1100, 260), (4800, 36)])
 def test_float32_product_has_the_same_bits_by_every_kernel(N, K):
