@@ -74,8 +74,10 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ x, long long ldx, 
 // neighbour) instead of K times one element at a time.  Bound by memory: it reads 2 and writes 4 bytes an element.
 // Measured at 2,048 rows of 4,096 bfloat16 channels and 4 taps: 73 us with a thread per element, 21 us so.  The
 // order of a sum is the other kernel's, oldest input first, and so are the bits.  Taken for up to 4 taps (beyond, the
-// window's registers pass what a vector of channels gains) of at least CONV_ROWS rows whose channels come in whole
-// aligned vectors.
+// window's registers pass what a vector of channels gains) where channels come in whole aligned vectors and the step has
+// enough elements that its threads fill the chip (a thread has 32): per element / in rows in us at 4,096 channels 34 rows 3.8 / 8.3,
+// 64 rows 4.1 / 5.7, 256 rows 10.6 / 6.9; 512 channels 1,024 rows 6.4 / 7.2.
+#define CONV_MIN_ELEMENTS (3LL << 18)
 #define CONV_ROWS 8
 #define CONV_V 4
 template <typename T, int K>
@@ -138,38 +140,57 @@ causal_conv_rows_kernel(const T* __restrict__ x, long long ldx, int C, const voi
     }
 }
 
-// A block looks through CONV_SPAN rows for the last ones of sequences and renews their slots' states, CONV_STATE_C channels
-// of each.  (A block per row and 128 channels, nearly all of which found their row not to be a last one and ended, took
-// 69 us at 2,048 rows of 4,096 channels: the launching of 65,536 blocks.  This takes 6 us.)
-#define CONV_SPAN 32
-#define CONV_STATE_C 512
-template <typename T>
-__global__ void __launch_bounds__(128)
-conv_state_update_kernel(const T* __restrict__ x, long long ldx, int C, int K,
+// A block looks through `span` rows (at most 32) for the last ones of sequences; its eight warps take them in turn and renew
+// CONV_STATE_C channels of their slots' states.  KK: the taps, 0: as many as are asked for.  What is read is asked for before
+// any of it is looked at: a warp's time is two trips to memory (the slots, then the inputs).  4,096 channels in us, a block per
+// row and 128 channels / a block that renewed one last row of 32 after the other / so: one prompt of 2,048 68 / 4.5 / 3.5 (the
+// first is the launching of 65,536 blocks), 512 sequences of 2 tokens 35 / 57 / 9, 33 of 1 and one of 20 3.2 / 90 / 2.9.
+#define CONV_STATE_C 256
+template <typename T, int KK>
+__global__ void __launch_bounds__(256)
+conv_state_update_kernel(const T* __restrict__ x, long long ldx, int C, int K_,
                          float* __restrict__ state, long long state_stride,
-                         const int* __restrict__ tok_slot, int n_rows,
+                         const int* __restrict__ tok_slot, int n_rows, int span,
                          const void* __restrict__ in_bias, int bias_dtype) {
     gi_pdl_start();
-    const int r0 = blockIdx.x * CONV_SPAN, lane = threadIdx.x & 31;
-    const int row = r0 + lane;                       // every warp looks at all CONV_SPAN rows
-    const int own = row < n_rows ? tok_slot[row] : -1;
-    const int next = row + 1 < n_rows ? tok_slot[row + 1] : -1;
+    constexpr int PER = CONV_STATE_C / 32, KEEP = (KK ? KK : CONV_MAX_TAPS) - 1, AT_ONCE = KK ? PER : 1;
+    const int K = KK ? KK : K_, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * span + lane;
+    const bool in = lane < span && row < n_rows;
+    const int own = in ? tok_slot[row] : -1, next = in && row + 1 < n_rows ? tok_slot[row + 1] : -1;
     unsigned last = __ballot_sync(0xffffffffu, own >= 0 && own != next);
-    const int c_end = min(C, (int)(blockIdx.y + 1) * CONV_STATE_C);
-    while (last) {
-        const int r = r0 + __ffs(last) - 1;
-        last &= last - 1;
-        const int slot = tok_slot[r];
+    const int c0 = blockIdx.y * CONV_STATE_C + lane;
+    for (int nth = 0; last; ++nth, last &= last - 1) {
+        if ((nth & 7) != warp) continue;
+        const int at = __ffs(last) - 1, r = blockIdx.x * span + at, slot = __shfl_sync(0xffffffffu, own, at);
         const int have = rows_before(tok_slot, r, slot, K - 1);
         float* st = state + (size_t)slot * state_stride;
-        for (int c = blockIdx.y * CONV_STATE_C + threadIdx.x; c < c_end; c += 128) {
-            const float bin = in_bias ? load_w(in_bias, bias_dtype, c) : 0.f;
-            float vals[CONV_MAX_TAPS];
-            for (int m = 0; m < K - 1; ++m) {
-                const int j = K - 2 - m;             // how far before the last row
-                vals[m] = j <= have ? to_f32(x[(size_t)(r - j) * ldx + c]) + bin : st[(size_t)(K - 1 + have - j) * C + c];
+        for (int i0 = 0; i0 < PER; i0 += AT_ONCE) {          // channels whose inputs are under way together
+            float vals[AT_ONCE][KEEP];
+            T xs[AT_ONCE][KEEP];
+#pragma unroll
+            for (int m = 0; m < KEEP; ++m) {                 // a place takes the row K - 2 - m before the last one, or what the state
+                if (m >= K - 1) break;                       // held of that age
+                const int j = K - 2 - m;
+#pragma unroll
+                for (int i = 0; i < AT_ONCE; ++i) {
+                    const int c = c0 + 32 * (i0 + i);
+                    if (c < C) xs[i][m] = x[(size_t)(r - min(j, have)) * ldx + c];
+                    if (c < C && have < K - 2) vals[i][m] = st[(size_t)min(K - 1 + have - j, K - 2) * C + c];
+                }
             }
-            for (int m = 0; m < K - 1; ++m) st[(size_t)m * C + c] = vals[m];
+#pragma unroll
+            for (int i = 0; i < AT_ONCE; ++i) {
+                const int c = c0 + 32 * (i0 + i);
+                const float bin = in_bias && c < C ? load_w(in_bias, bias_dtype, c) : 0.f;
+#pragma unroll
+                for (int m = 0; m < KEEP; ++m) {
+                    if (m >= K - 1) break;
+                    if (K - 2 - m <= have) vals[i][m] = to_f32(xs[i][m]) + bin;
+                }
+#pragma unroll
+                for (int m = 0; m < KEEP; ++m)
+                    if (m < K - 1 && c < C) st[(size_t)m * C + c] = vals[i][m];
+            }
         }
     }
 }
@@ -178,7 +199,7 @@ template <typename T>
 static bool launch_conv_rows(const T* x, long long ldx, int C, const void* taps, int taps_dtype, int K, const float* state,
                              long long state_stride, const int* tok_slot, float* out, int n_rows, int act,
                              const void* in_bias, const void* out_bias, int bias_dtype, cudaStream_t s) {
-    if (K > 4 || n_rows < CONV_ROWS || C % CONV_V || ldx % CONV_V || (uintptr_t)x % (CONV_V * sizeof(T)) || (uintptr_t)out % 16)
+    if (K > 4 || (long long)n_rows * C < CONV_MIN_ELEMENTS || C % CONV_V || ldx % CONV_V || (uintptr_t)x % (CONV_V * sizeof(T)) || (uintptr_t)out % 16)
         return false;
     dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C + 128 * CONV_V - 1) / (128 * CONV_V));
 #define CONV_LAUNCH(KK)                                                                                                       \
@@ -194,8 +215,12 @@ static void launch_conv(const T* x, long long ldx, int C, const void* taps, int 
                         long long state_stride, const int* tok_slot, float* out, int n_rows, int update_state, int act,
                         const void* in_bias, const void* out_bias, int bias_dtype, cudaStream_t s) {
     if (update_state == 1) {
-        dim3 grid((n_rows + CONV_SPAN - 1) / CONV_SPAN, (C + CONV_STATE_C - 1) / CONV_STATE_C);
-        if (K > 1) gi_launch(conv_state_update_kernel<T>, grid, dim3(128), 0, s, x, ldx, C, K, state, state_stride, tok_slot, n_rows, in_bias, bias_dtype);
+        if (K <= 1) return;
+        const auto kernel = K == 2 ? conv_state_update_kernel<T, 2> : K == 3 ? conv_state_update_kernel<T, 3> : K == 4 ? conv_state_update_kernel<T, 4> : conv_state_update_kernel<T, 0>;
+        // few rows: a warp for each, should they all be last ones; many: fewer blocks (what costs is launching them)
+        const int span = n_rows <= 512 ? 8 : 32;
+        gi_launch(kernel, dim3((n_rows + span - 1) / span, (C + CONV_STATE_C - 1) / CONV_STATE_C), dim3(256), 0, s, x, ldx, C, K, state,
+                  state_stride, tok_slot, n_rows, span, in_bias, bias_dtype);
         return;
     }
     // (a step whose rows are all sequences of their own renews the state in the launch of a thread per element)

@@ -47,6 +47,47 @@ def test_causal_convolution_over_runs_of_rows(dtype, K, C, pad, lens):
     assert (state.double() - want_state).abs().max() <= 2.0 ** -23 * 8
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+def test_causal_convolution_of_many_elements_has_the_bits_of_few(dtype, K):
+    """Rows by the kernel that keeps runs of them, the same columns a few at a time by the kernel of a thread per element."""
+    from garlic_inference_b200.ops import kernels
+    C, lens = 6152, [7, 1, 24, 33, 64]
+    n = sum(lens) + 1
+    assert n * C > 3 << 18 > n * 1024
+    x, taps, bin_, bout = rnd(n, C, seed=1, dtype=dtype), rnd(C, K, seed=2, dtype=dtype), rnd(C, seed=3), rnd(C, seed=4)
+    state = rnd(len(lens), max(1, K - 1) * C, seed=5)
+    slots = torch.tensor(sum(([i] * m for i, m in enumerate(lens)), []) + [-1], dtype=torch.int32, device=DEV)
+    got = kernels.causal_conv_silu(x, taps, state, slots, in_bias=bin_, out_bias=bout)
+    for at in range(0, C, 1024):
+        cut = slice(at, min(C, at + 1024))
+        w = min(C, at + 1024) - at
+        part = state[:, :(K - 1) * C].view(len(lens), K - 1, C)[:, :, cut].reshape(len(lens), -1) if K > 1 else state[:, :w]
+        want = kernels.causal_conv_silu(x[:, cut], taps[cut].contiguous(), part.contiguous(), slots, in_bias=bin_[cut].contiguous(),
+                                        out_bias=bout[cut].contiguous())
+        assert torch.equal(got[:, cut], want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K", [2, 3, 4, 6])
+@pytest.mark.parametrize("lens", [[1] * 33 + [20], [2] * 300, [1, 2, 3, 4, 5] * 9 + [1] * 500])
+def test_convolution_states_of_many_sequences(dtype, K, lens):
+    """Steps in which many of neighbouring rows are the last of their sequences, few and many rows, with padding between."""
+    from garlic_inference_b200.ops import kernels
+    C, rows = 300, []
+    order = torch.randperm(len(lens), generator=torch.Generator().manual_seed(1)).tolist()
+    for i, m in zip(order, lens):
+        rows += [i] * m + ([-1] if i % 7 == 0 else [])
+    x, bias, state = rnd(len(rows), C, seed=2, dtype=dtype), rnd(C, seed=3), rnd(len(lens) + 1, (K - 1) * C + 4, seed=4)
+    want = state.clone()
+    for i in order:
+        mine = [r for r, s in enumerate(rows) if s == i]
+        seen = torch.cat([state[i, :(K - 1) * C].view(K - 1, C), x[mine].float() + bias])
+        want[i, :(K - 1) * C] = seen[len(mine):].reshape(-1)
+    kernels.conv_state_update(x, K, state, torch.tensor(rows, dtype=torch.int32, device=DEV), in_bias=bias)
+    assert torch.equal(state, want)
+
+
 # ---- gates of the recurrent unit -------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("blocks, bw", [(3, 8), (2, 64), (3, 72), (2, 320), (2, 20)])
 @pytest.mark.parametrize("n", [1, 17, 128, 129, 300])
