@@ -432,9 +432,13 @@ extern "C" int gi_attn_prepare(const void* src, int src_dtype, long long ld, int
     // per head, when every word of four elements falls into place.  2,048 tokens, 32 rows of queries and 8 of keys of 64 and
     // 4 heads of values of 128 out of float32 columns: 23.6 us with a block per token, element by element, 11 us so.  (Heads
     // divided by their root mean square with interleaved pairs stay with the block per token, whose sums run in their order.)
+    // Narrow tokens of long prompts stay with the block per token, whose threads have one or two pairs each.  Per element / by
+    // groups in us: 16 + 4 + 4 heads of 48 255 tokens 4.4 / 3.9, 700 5.1 / 6.2, 2,048 9.5 / 11.5; 2 + 1 + 1 of 128 700 3.9 / 4.2,
+    // 2,048 6.5 / 7.8; 16 + 16 + 16 of 40 (1,920 elements) 2,048 12.8 / 11.6.
     const bool inter = !half_layout && n_rot > 0;
+    const bool narrow = n_tokens >= 384 && (long long)n_qh * d + (k_off >= 0 ? (long long)n_kh * d + (long long)n_vh * dv : 0) < 1280;
     if (!norm_w && temp_every == 0 && mean_block == 0 && n_rot % (inter ? 4 : 8) == 0 && d % 4 == 0 && dv % 4 == 0 &&
-        (head_eps == 0.f || !inter)) {
+        (head_eps == 0.f ? !narrow : !inter)) {
         const int esz = src_dtype == GI_DTYPE_F32 ? 4 : 2, ez = act_dtype == GI_DTYPE_F32 ? 4 : 2;
         const int words = inter ? d / 4 : n_rot / 8 + (d - n_rot) / 4, v_second = dv % 8 == 0 ? dv / 2 : 0;
         const int v_words = v_second ? dv / 8 : dv / 4, most = k_off >= 0 && v_words > words ? v_words : words;
@@ -451,7 +455,10 @@ extern "C" int gi_attn_prepare(const void* src, int src_dtype, long long ld, int
                       dim3(APH_THREADS), (size_t)TOK * n_rot * sizeof(float), s, (const TI*)src, ld, q_off, k_off, v_off, freq,  \
                       n_rot, tok_pos, tok_slot, block_table, (T*)k_pool, (T*)v_pool, (T*)q_out, n_tokens, n_qh, n_kh, n_vh, d,  \
                       dv, page_size, max_pages, n_pool_pages, append, status, bias, bias_dtype, magnitude, head_eps, lph, v_second, inter)
-#define APH_TOK(TI, T) if (n_tokens >= 256) APH_LAUNCH(TI, T, 4); else APH_LAUNCH(TI, T, 1)
+            // four tokens to a block (angles and biases read once for them) where that leaves blocks enough; one / four in us: 256 tokens
+            // of 48 heads of 64 (512 blocks of one) 4.1 / 6.0, of 128 (768) 4.5 / 5.9, of 128 in interleaved pairs (1,536) 7.4 / 6.5;
+            // 700 of 64 (1,400) 7.0 / 6.6
+#define APH_TOK(TI, T) if (n_tokens >= 256 && (long long)n_tokens * rounds >= 1100) APH_LAUNCH(TI, T, 4); else APH_LAUNCH(TI, T, 1)
             if (src_dtype == GI_DTYPE_F32 && act_dtype == GI_DTYPE_F32) { APH_TOK(float, float); }
             else if (src_dtype == GI_DTYPE_F32 && act_dtype == GI_DTYPE_BF16) { APH_TOK(float, bf16); }
             else if (src_dtype == GI_DTYPE_BF16 && act_dtype == GI_DTYPE_BF16) { APH_TOK(bf16, bf16); }

@@ -642,6 +642,31 @@ def test_queries_keys_and_values_by_words_and_by_elements(src_dtype, dtype, d, d
                 torch.testing.assert_close(got, x[t, H * d + G * d:].view(G, dv), **tol)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("d, dv, n_rot, H, G", [(128, 128, 128, 10, 2), (48, 64, 32, 16, 4), (64, 32, 64, 40, 8)])
+def test_queries_keys_and_values_of_long_steps_have_the_bits_of_short_ones(dtype, half, d, dv, n_rot, H, G):
+    """Steps that take four tokens to a block, or narrow tokens element by element, against their rows in steps of a few tokens."""
+    from garlic_inference_b200.ops import kernels
+    n, page, cols = 1201, 64, (H + G) * d + G * dv
+    src = rnd(n, cols, seed=1, dtype=dtype)
+    freq = torch.tensor([1e4 ** (-2.0 * i / n_rot) for i in range(n_rot // 2)], device=DEV)
+    table = torch.arange(-(-n // page), dtype=torch.int32, device=DEV).flip(0).contiguous().view(1, -1)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(cuts):
+        kp, vp = (torch.zeros((table.numel(), G, page, w), dtype=dtype, device=DEV) for w in (d, dv))
+        q = [kernels.attn_prepare(src[a:b], 0, H * d, (H + G) * d, freq, n_rot, half, torch.arange(a, b, dtype=torch.int32, device=DEV),
+                                  torch.zeros(b - a, dtype=torch.int32, device=DEV), table, kp, vp, H, d, dtype, status)
+             for a, b in zip(cuts, cuts[1:])]
+        return torch.cat(q), kp, vp
+
+    want = run(list(range(0, n, 200)) + [n])
+    for cuts in ([0, n], [0, 383, 767, n], [0, 255, 511, n]):
+        assert all(torch.equal(x, y) for x, y in zip(run(cuts), want))
+    assert int(status.item()) == 0
+
+
 # ---- one token per sequence over latent rows ---------------------------------------------------------------------------
 @pytest.mark.parametrize("heads", [17, 33])
 @pytest.mark.parametrize("n_splits, window", [(1, 0), (2, 0), (16, 0), (16, 40)])
