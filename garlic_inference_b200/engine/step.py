@@ -162,7 +162,7 @@ class Engine:
             arrays={name: dev.view(a.shape) for (name, a), dev in zip(extra.items(), uploaded[:n_extra])},
             seq_slots=slots, seq_starts=starts, seq_lens=lens, seq_past=past, all_single=shape.all_single,
             max_kv_len=max(p + n for p, n in zip(past, lens)),
-            status=self.cache.status)
+            status=self.cache.status, notes=shape.notes)
         logits = self.model.forward(ctx, self.cache, d_want if want_rows.size else None)
         self.cache.commit(slots, lens)
         return logits

@@ -33,6 +33,33 @@ def query_runs(shape, rows: int) -> np.ndarray:
     return np.asarray(runs, dtype=np.int32).reshape(-1, 4)
 
 
+def _key_tiles(shape, window: int, chunk: int, keep: int) -> tuple:
+    """(tiles of 64 keys that a run of 128 query rows walks on average, runs), worked out once per step."""
+    key = ("key_tiles", window, chunk, keep)
+    if key not in shape.notes:
+        new, past = np.asarray(shape.seq_lens, dtype=np.int64), np.asarray(shape.seq_past, dtype=np.int64)
+        n = -(-new // 128)
+        first = np.repeat(past, n) + 128 * (np.arange(n.sum()) - np.repeat(np.cumsum(n) - n, n))
+        last = np.minimum(first + 128, np.repeat(past + new, n)) - 1
+        begin = np.maximum(first - window + 1, 0) if window else np.zeros_like(first)
+        if chunk:
+            begin = np.maximum(begin, first // chunk * chunk)
+        tiles = last // 64 - begin // 64 + 1 + np.minimum(-(-keep // 64), begin // 64)
+        shape.notes[key] = (float(tiles.mean()) if len(tiles) else 0.0, len(tiles))
+    return shape.notes[key]
+
+
+def short_walks(shape, d: int, dv: int, heads: int, window: int = 0, chunk: int = 0, keep: int = 0) -> bool:
+    """Whether the queries of a step see so few keys that the mma.sync prompt kernel is faster than the tcgen05 one at sizes
+    other than one map of 128: a block of the latter takes 128 queries of a head, and what it sets up for them (the copies, the
+    first scores, the first probabilities) costs it 2 us more than it gains on one tile of 64 keys.  mma.sync / tcgen05 in us, 32
+    heads of 64: 1 x 16 tokens 5.8 / 7.4, 300 x 3 behind 30 cached 113 / 180, 32 x 20 behind 20 17 / 23 (one tile); 1 x 100
+    8.7 / 10.9, 256 x 16 behind 112 102 / 106 (two); 16 x 64 behind 128 1.4 times as fast (three); 1 x 64 behind 2,000
+    101 / 35.  16 heads with two maps of 64 over 128, two tiles: 1 x 128 11.3 / 12.3, 16 x 128 1.5 times as fast."""
+    tiles, runs = _key_tiles(shape, window, chunk, keep)
+    return tiles <= 1 or (tiles <= 2 and ((d, dv) == (64, 64) or runs * heads <= 148))
+
+
 class GQAAttention(Mixer):
     kind = "gqa_attention"
     graph_safe = True
@@ -88,15 +115,16 @@ class GQAAttention(Mixer):
         o = self.attend(q, kv, ctx)
         return linear(o, self.w_o)
 
-    def _run_rows(self, kv) -> int:
-        """Height of the query runs the prompt kernel for this head size, type and page size takes (0: the
+    def _run_rows(self, kv, shape=None) -> int:
+        """Height of the query runs the prompt kernel for this head size, type, page size and step takes (0: the
         exact-order kernel, which needs none)."""
-        if kernels.tcgen05_attention_takes(self.rt.dtype, self.d, kv.page_size):
+        if kernels.tcgen05_attention_takes(self.rt.dtype, self.d, kv.page_size) and \
+                (self.d == 128 or shape is None or not short_walks(shape, self.d, self.d, self.n_q, self.window or 0)):
             return 128
         return 64 if kernels.mma_attention_takes(self.rt.dtype, self.d) else 0
 
     def step_arrays(self, shape, cache):
-        rows = 0 if shape.all_single else self._run_rows(cache.kv)
+        rows = 0 if shape.all_single else self._run_rows(cache.kv, shape)
         return {f"query_runs_{rows}": lambda: query_runs(shape, rows)} if rows else {}
 
     def _runs(self, ctx, rows: int) -> torch.Tensor:
@@ -110,8 +138,8 @@ class GQAAttention(Mixer):
         """Attention of q [n, n_q, d] over the cache; returns [n, n_q * d].
 
         bfloat16 with heads of 128 and pages that are a multiple of 64 tokens: the tcgen05 kernels (flash
-        attention for runs of tokens, for heads of 64 too; split-KV when every sequence brings one token and the group
-        is at most 16).  Otherwise bfloat16 with a head size the mma.sync kernels take: the split-KV kernel for single
+        attention for runs of tokens, for heads of 64 too unless they see few keys; split-KV when every sequence brings
+        one token and the group is at most 16).  Otherwise bfloat16 with a head size the mma.sync kernels take: the split-KV kernel for single
         tokens, the flash kernel for runs.  Everything else (float32, other head sizes, larger groups in
         decode) goes to the exact-order kernel."""
         covered = (not ctx.all_single) and ctx.n_tokens == sum(ctx.seq_lens)
@@ -123,7 +151,7 @@ class GQAAttention(Mixer):
                 return kernels.attention_decode_bf16(q, kv.k_pool, kv.v_pool, kv.block_table, ctx.tok_pos,
                                                      ctx.tok_slot, self.scale, self.window or 0)
         elif ctx.seq_lens:
-            rows = self._run_rows(kv) if q.dtype == self.rt.dtype else 0
+            rows = self._run_rows(kv, ctx) if q.dtype == self.rt.dtype else 0
             if rows == 128:
                 return kernels.attention_prefill_tcgen05(q, kv.k_pool, kv.v_pool, kv.block_table, self._runs(ctx, 128),
                                                          self.scale, self.window or 0, rows_covered=covered)

@@ -84,6 +84,7 @@ class StepShape:
     seq_lens: list                      # new tokens of each sequence
     seq_past: list                      # positions already in the cache
     all_single: bool                    # every sequence brings exactly one token
+    notes: dict = field(default_factory=dict)      # what parts worked out about the step, once for all layers
 
 
 @dataclass
@@ -122,6 +123,8 @@ class StepContext:
     # A vector [hidden] that joins every row of the stream before the next block reads it (set by the model for
     # a scheduled run that has one); a block hands it to its first norm or adds it itself, and clears it.
     stream_offset: Optional[torch.Tensor] = None
+
+    notes: dict = field(default_factory=dict)      # the shape's (`StepShape.notes`)
 
     def seq_spans(self) -> Optional[torch.Tensor]:
         """int32 [n_seq, 3] = {slot, first row, rows} on the device for kernels that walk each sequence's rows

@@ -58,7 +58,7 @@ import torch
 from ..cache import EntryRequirement, KVRequirement, StateRequirement
 from ..ops import kernels, linear
 from ..weights.loader import TensorWant
-from .attention import query_runs
+from .attention import query_runs, short_walks
 from .base import Mixer, register_part
 from .linear_attention import pack_rows
 
@@ -213,18 +213,21 @@ class MaskedAttention(Mixer):
     def _tensor_cores(self) -> bool:
         return kernels.mma_attention_takes(self.rt.dtype, self.d, self.dv)
 
-    def _run_rows(self, kv) -> int:
-        """Height of the query runs of the prompt kernel that takes this mixer: 128 (tcgen05: keys and values of 64 or
-        128, pages of a multiple of 64, and what `tcgen05_attention_takes` says of the rest), 64 (mma.sync), 0 (the
-        exact-order kernel, which needs none)."""
+    def _run_rows(self, kv, shape=None) -> int:
+        """Height of the query runs of the prompt kernel that takes this mixer's step: 128 (tcgen05: keys and values of 64
+        or 128, pages of a multiple of 64, what `tcgen05_attention_takes` says of the rest, and at sizes other than one map
+        of 128 without biases queries that see more than a few keys, as they do without a step), 64 (mma.sync), 0 (the exact-order kernel, which needs
+        none)."""
         if kernels.tcgen05_attention_takes(self.rt.dtype, self.d, kv.page_size, self.dv,
                                            n_dist=0 if self.dist_bias is None else self.dist_bias.shape[0],
-                                           means=bool(self.pool), column_gate=self.output_gate):
+                                           means=bool(self.pool), column_gate=self.output_gate) and \
+                ((self.d, self.dv, self.maps) == (128, 128, 1) and self.dist_bias is None or
+                 shape is None or not short_walks(shape, self.d, self.dv, self.H * self.maps, self.window, self.chunk, self.keep_first)):
             return 128
         return 64 if self._tensor_cores() else 0
 
     def step_arrays(self, shape, cache):
-        rows = 0 if shape.all_single else self._run_rows(cache.kv)
+        rows = 0 if shape.all_single else self._run_rows(cache.kv, shape)
         return {f"query_runs_{rows}": lambda: query_runs(shape, rows)} if rows else {}
 
     def _rotation(self, position):
@@ -279,8 +282,8 @@ class MaskedAttention(Mixer):
             att = kernels.attention_decode_masked_bf16(q, kv.k_pool, kv.v_pool, kv.block_table, ctx.tok_pos, ctx.tok_slot,
                                                        self.scale, window=self.window, chunk=self.chunk, maps=self.maps,
                                                        gate=inside, **extras)
-        elif not ctx.all_single and ctx.seq_lens and self._run_rows(kv):
-            rows = self._run_rows(kv)
+        elif not ctx.all_single and ctx.seq_lens and self._run_rows(kv, ctx):
+            rows = self._run_rows(kv, ctx)
             runs = ctx.arrays.get(f"query_runs_{rows}")
             if runs is None:                      # a context put together by hand: cut and copy here
                 runs = ctx.arrays[f"query_runs_{rows}"] = torch.from_numpy(query_runs(ctx, rows)).to(x.device)
