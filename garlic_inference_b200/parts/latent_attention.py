@@ -62,6 +62,12 @@ WINDOW_BLOCK = 256             # tokens of a block when a window cuts the keys
 # 101 / 54, 2,048 alone 836 / 193; behind 2,000: 64 81 / 97, 128 112 / 102, 256 175 / 107; behind 6,000: 128 206 / 213,
 # 512 669 / 236.
 ROT_MIN_ROWS = 128
+# ... and in a step of which other portions are not expanded, from how many scores (all heads, every key by every new token) on:
+# both ways' preparations run then, 55 us more on the host and 10 to 30 on the device.  The layer of 16 heads on 2,048 beside 40
+# new tokens behind 1,500, by products / expanded in us of the host's clock: 256 alone (1 M scores) 458 / 522, 256 behind 2,000
+# (9 M) 468 / 517, 2,000 behind 2,000 (128 M) 917 / 543; 32 heads on 4,096 beside 20 new tokens: 256 alone (2 M) 538 / 537, 256
+# behind 2,000 (18 M) 610 / 566, 700 behind 2,000 (60 M) 899 / 641.
+MIXED_MIN_SCORES = 1 << 24
 EXPAND_BYTES = 2 << 30         # keys and values of one sequence expanded for a portion
 
 
@@ -161,6 +167,8 @@ class LatentAttention(Mixer):
                 p0 = self._first_page(past, page)
                 keys = (-(-(past + n_new) // page) - p0) * page
                 which.append((i, p0, keys, self._run_rows(keys)))
+        if self.dr and len(which) < len(shape.seq_lens):
+            which = [w for w in which if self.H * shape.seq_lens[w[0]] * w[2] >= MIXED_MIN_SCORES]
         return which
 
     def _runs_of(self, shape, page: int):
@@ -176,7 +184,7 @@ class LatentAttention(Mixer):
 
     def step_arrays(self, shape, cache):
         page = cache.kv.page_size
-        if shape.all_single or not any(self._expands(m, p, page) for m, p in zip(shape.seq_lens, shape.seq_past)):
+        if shape.all_single or not self._portions(shape, page):
             return {}
         return {self._runs_name(page): lambda: self._runs_of(shape, page)}
 

@@ -455,6 +455,26 @@ def test_latent_portions_with_a_rotated_part(layout, q_rank, gate, sink, pad, le
 
 
 # ---- row-wise kernels that move words of four ----------------------------------------------------------------------------------
+@pytest.mark.parametrize("layout, q_rank, gate, sink, pad", [("half", 24, True, False, 0), ("interleaved", 0, False, True, 8)])
+def test_latent_portions_expanded_beside_others_that_are_not(layout, q_rank, gate, sink, pad, monkeypatch):
+    """The step of four portions above with every portion that may be expanded so, whatever it gains: two are, two are not.  And
+    the choice itself: beside other portions only those of many scores, alone all of them."""
+    from types import SimpleNamespace
+    from garlic_inference_b200.parts import StepShape
+    from garlic_inference_b200.parts import latent_attention
+    from garlic_inference_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(latent_attention, "MIXED_MIN_SCORES", 0)
+    test_latent_portions_with_a_rotated_part(layout, q_rank, gate, sink, pad, [200, 3, 64, 129], [70, 10, 0, 300])
+    monkeypatch.undo()
+    part = SimpleNamespace(dr=64, d=128, dv=128, rank=512, H=32, window=0, rt=SimpleNamespace(dtype=torch.bfloat16),
+                           w_uv=torch.zeros(1, dtype=torch.bfloat16), w_uk_t=torch.zeros(1, dtype=torch.bfloat16))
+    for name in ("_expands", "_first_page", "_first_seen", "_run_rows"):
+        setattr(part, name, getattr(LatentAttention, name).__get__(part))
+    chosen = lambda lens, past: [w[0] for w in LatentAttention._portions(part, StepShape([], [], lens, past, False), 64)]
+    assert chosen([200], [70]) == [0] and chosen([200, 40], [70, 0]) == [0, 1]
+    assert chosen([200, 3], [70, 10]) == [] and chosen([3, 200, 512], [10, 70, 512]) == [2]      # 32 x 512 x 1,024 scores: the line
+
+
 @pytest.mark.parametrize("hidden", [4, 100, 1024, 4100, 9000, 6])
 @pytest.mark.parametrize("n", [1, 300])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
