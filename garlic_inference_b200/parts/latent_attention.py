@@ -68,7 +68,10 @@ ROT_MIN_ROWS = 128
 # (9 M) 468 / 517, 2,000 behind 2,000 (128 M) 917 / 543; 32 heads on 4,096 beside 20 new tokens: 256 alone (2 M) 538 / 537, 256
 # behind 2,000 (18 M) 610 / 566, 700 behind 2,000 (60 M) 899 / 641.
 MIXED_MIN_SCORES = 1 << 24
-EXPAND_BYTES = 2 << 30         # keys and values of one sequence expanded for a portion
+EXPAND_BYTES = 2 << 30         # keys and values of one sequence: more are not expanded
+# Of these so many at a time are, some heads after the other, so that a portion needs no more memory than its scores in blocks
+# of SCORE_BYTES did (without a bound 100,000 keys of 32 heads of 128 + 128 took 1.6 GB).
+EXPAND_RUN_BYTES = 256 << 20
 
 
 class LatentAttention(Mixer):
@@ -203,13 +206,23 @@ class LatentAttention(Mixer):
             n_runs = -(-ctx.seq_lens[i] // rows)
             c = pool.index_select(0, kv.block_table[ctx.seq_slots[i], p0:p0 + keys // page].long()).view(1, keys, self.row)
             rot = {"rot": (c[0], self.rank)} if self.dr else {}
-            c = c[:, :, :self.rank].expand(self.H, keys, self.rank)
-            k, v = torch.bmm(c, self.w_uk_t), torch.bmm(c, self.w_uv.transpose(1, 2))
-            args = (q, k.unsqueeze(0), v.unsqueeze(0), self._one_page, runs[at:at + n_runs], self.scale)
-            if rows == 128:
-                kernels.attention_prefill_tcgen05(*args, self.window, sinks=self.sink_f32, gate=gate, out=out, **rot)
-            else:
-                kernels.attention_prefill_masked_bf16(*args, window=self.window, sinks=self.sink_f32, gate=gate, out=out)
+            # as many heads at a time as EXPAND_RUN_BYTES takes (the mma.sync kernel writes whole rows: all of them)
+            step = self.H if rows != 128 else max(1, min(self.H, EXPAND_RUN_BYTES // (2 * keys * (self.d + self.dv))))
+            for h in range(0, self.H, step):
+                some = slice(h, min(self.H, h + step))
+                latents = c[:, :, :self.rank].expand(some.stop - h, keys, self.rank)
+                k, v = torch.bmm(latents, self.w_uk_t[some]), torch.bmm(latents, self.w_uv[some].transpose(1, 2))
+                sinks, own_gate, own_out = self.sink_f32, gate, out
+                if step < self.H:
+                    sinks, own_gate = (t if t is None else t[..., some] for t in (sinks, gate))
+                    own_out = out[:, some.start * self.dv:some.stop * self.dv]
+                args = (q if step == self.H else q[:, some].contiguous(), k.unsqueeze(0), v.unsqueeze(0), self._one_page,
+                        runs[at:at + n_runs], self.scale)
+                if rows == 128:
+                    kernels.attention_prefill_tcgen05(*args, self.window, sinks=sinks, gate=own_gate, out=own_out, **rot)
+                else:
+                    kernels.attention_prefill_masked_bf16(*args, window=self.window, sinks=sinks, gate=own_gate, out=own_out)
+                del k, v, args                     # freed before the next heads' are made
             at += n_runs
 
     def step(self, x, ctx, cache, position, writes_cache=True):

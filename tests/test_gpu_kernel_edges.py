@@ -475,6 +475,48 @@ def test_latent_portions_expanded_beside_others_that_are_not(layout, q_rank, gat
     assert chosen([200, 3], [70, 10]) == [] and chosen([3, 200, 512], [10, 70, 512]) == [2]      # 32 x 512 x 1,024 scores: the line
 
 
+@pytest.mark.parametrize("bytes_, pad", [(1, 0), (2 * 2 * 512 * 256, 8)])
+def test_latent_portions_expanded_some_heads_at_a_time(bytes_, pad, monkeypatch):
+    """One head at a time and, with 512 keys, two and then one of three, with gates and sinks; whole rows and columns."""
+    from garlic_inference_b200.parts import latent_attention
+    monkeypatch.setattr(latent_attention, "EXPAND_RUN_BYTES", bytes_)
+    test_latent_portions_with_a_rotated_part("half", 24, True, True, pad, [130, 200], [0, 300])
+
+
+def test_latent_portions_need_no_more_memory_than_their_scores_did():
+    """A portion behind 60,000 cached tokens, 32 heads: 1 GB of keys and values in all, at most 256 MB of them at a time."""
+    from garlic_inference_b200.parts import Runtime, StepContext, latent_attention
+    from garlic_inference_b200.parts.latent_attention import LatentAttention
+    H, hid, r, past, new, page = 32, 64, 64, 60000, 128, 64
+    params = dict(hidden_size=hid, n_heads=H, plain_dim=128, rot_dim=64, value_dim=128, kv_rank=r, q_rank=0, softmax_scale=0.07,
+                  eps=1e-6, head_gate=False, own_kv=True)
+
+    class Load:
+        def dtype(self, *names):
+            return torch.bfloat16
+
+        def __call__(self, n, out=None):
+            t = rnd(*LatentAttention.wanted(params)[n].shape, seed=len(n), scale=0.1, dtype=torch.bfloat16)
+            return t if out is None else out.copy_(t)
+
+    part = LatentAttention(params, Load(), Runtime(torch.bfloat16, torch.device("cuda", 0)))
+    pages = -(-(past + new) // page)
+    from types import SimpleNamespace
+    kv = SimpleNamespace(page_size=page, k_pool=rnd(pages, 1, page, part.row, seed=1, dtype=torch.bfloat16),
+                         block_table=torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1))
+    ctx = StepContext(new, *(torch.zeros(new, dtype=torch.int32, device=DEV) for _ in range(3)), [0], [0], [new], [past], False, past + new)
+    which = part._portions(ctx, page)
+    assert len(which) == 1
+    q, out = rnd(new, H, 192, seed=2, dtype=torch.bfloat16), torch.zeros(new, H * 128, dtype=torch.bfloat16, device=DEV)
+    part._attend_expanded(q, kv, ctx, which, None, out)                     # (the library's workspace is made)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    part._attend_expanded(q, kv, ctx, which, None, out)
+    gathered = pages * page * part.row * 2
+    assert torch.cuda.max_memory_allocated() - before <= (256 << 20) + 2 * gathered + (4 << 20)
+
+
 @pytest.mark.parametrize("hidden", [4, 100, 1024, 4100, 9000, 6])
 @pytest.mark.parametrize("n", [1, 300])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
