@@ -648,17 +648,20 @@ delta_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_off, in
     }
 }
 
-// Keys of D = 8 R, W value columns to a thread.  spans [n_seq, 3]; out float32 [n, H dv].
+// Keys of D = 8 R, W value columns to a thread.  spans [n_seq, 3]; out float32 [n, H dv].  qk and gb hold rows row0 .. row1 - 1
+// of the step; the rows before were walked by earlier launches, whose state this one goes on from.
 template <int R, int CH, int W>
 __global__ void __launch_bounds__(DS_COLS / W * 8, 1)
 delta_walk_kernel(const float* __restrict__ qk, const float* __restrict__ gb, const float* __restrict__ qkv, long long ldq, int v_off,
                   float* __restrict__ state, long long state_stride, const int* __restrict__ spans, float* __restrict__ out, int H,
-                  int Hk, int dv) {
+                  int Hk, int dv, int row0, int row1) {
     gi_pdl_start();
     constexpr int P = 8, D = R * P, DS_THREADS = DS_COLS / W * P, GB = CH ? D + 4 : 4;       // floats of a row of decays and beta
     constexpr int TOKEN = 2 * D + GB + DS_COLS, QK_COPIES = 2 * D / 4, G_COPIES = CH ? D / 4 : 0;      // a token's floats, its 16-byte copies
     extern __shared__ __align__(16) float ds_smem[];                   // [stage][token][q | k | decays, beta | v]
-    const int slot = spans[3 * blockIdx.x], start = spans[3 * blockIdx.x + 1], len = spans[3 * blockIdx.x + 2];
+    const int slot = spans[3 * blockIdx.x], start = max(spans[3 * blockIdx.x + 1], row0);
+    const int len = min(spans[3 * blockIdx.x + 1] + spans[3 * blockIdx.x + 2], row1) - start;      // the span's rows of this launch
+    if (len <= 0) return;
     const int h = blockIdx.y, v0 = blockIdx.z * DS_COLS, kh = h / (H / Hk), tid = threadIdx.x;
     const int part = tid % P, col = tid / P * W;                       // this thread's columns: v0 + col (and the next)
     if (slot < 0) {
@@ -677,19 +680,19 @@ delta_walk_kernel(const float* __restrict__ qk, const float* __restrict__ gb, co
 #pragma unroll
             for (int i = 0; i < DS_GROUP * QK_COPIES / DS_THREADS; ++i) {
                 const int id = tid + DS_THREADS * i, j = id / QK_COPIES, c = id % QK_COPIES;
-                copy(base + (j * TOKEN + 4 * c) * 4, qk + ((size_t)(start + min(t0 + j, last)) * Hk + kh) * (2 * D) + 4 * c);
+                copy(base + (j * TOKEN + 4 * c) * 4, qk + ((size_t)(start - row0 + min(t0 + j, last)) * Hk + kh) * (2 * D) + 4 * c);
             }
 #pragma unroll
             for (int i = 0; i < DS_GROUP * G_COPIES / DS_THREADS; ++i) {
                 const int id = tid + DS_THREADS * i, j = id / (G_COPIES ? G_COPIES : 1), c = id % (G_COPIES ? G_COPIES : 1);
-                copy(base + (j * TOKEN + 2 * D + 4 * c) * 4, gb + ((size_t)(start + min(t0 + j, last)) * H + h) * GB + 4 * c);
+                copy(base + (j * TOKEN + 2 * D + 4 * c) * 4, gb + ((size_t)(start - row0 + min(t0 + j, last)) * H + h) * GB + 4 * c);
             }
             if (tid < 32) {
                 const int j = tid / 4, c = tid % 4;
                 copy(base + (j * TOKEN + 2 * D + GB + 4 * c) * 4, qkv + (size_t)(start + min(t0 + j, last)) * ldq + v_off + h * dv + v0 + 4 * c);
             } else if (tid < 40) {
                 const int j = tid - 32;
-                copy(base + (j * TOKEN + 2 * D + GB - 4) * 4, gb + ((size_t)(start + min(t0 + j, last)) * H + h) * GB + GB - 4);
+                copy(base + (j * TOKEN + 2 * D + GB - 4) * 4, gb + ((size_t)(start - row0 + min(t0 + j, last)) * H + h) * GB + GB - 4);
             }
         }
         asm volatile("cp.async.commit_group;\n" ::);
@@ -860,11 +863,12 @@ extern "C" int gi_delta_scan(const float* qkv, long long ldq, int q_off, int k_o
 }
 
 // gi_delta_scan over prompts by the two kernels above: keys of 64 or 128, values in whole blocks of columns, rows of qkv and of
-// the state that start on 16 bytes.  `scratch`: n_rows (2 Hk d + H (d + 4 or 4)) floats, on 16 bytes.
+// the state that start on 16 bytes.  `scratch`: scratch_rows (2 Hk d + H (d + 4 or 4)) floats, on 16 bytes; a step of more rows is
+// walked that many at a time, each from the state that the one before left.
 extern "C" int gi_delta_scan_prompt(const float* qkv, long long ldq, int q_off, int k_off, int v_off, const float* ab,
                                     long long ldab, int b_off, int a_off, const float* a_sep, long long lda_sep,
                                     const void* A_log, const void* dt_bias, int p_dtype, float* state, long long state_stride,
-                                    const int* spans, float* out, float* scratch, int n_rows, int n_seq, int H, int Hk, int d,
+                                    const int* spans, float* out, float* scratch, int scratch_rows, int n_rows, int n_seq, int H, int Hk, int d,
                                     int dv, float unit_eps, float q_scale, int channel_decay, void* stream) {
     GI_REQUIRE(n_seq >= 0 && n_rows >= 0 && H > 0 && Hk > 0 && H % Hk == 0 && (d == 64 || d == 128) && dv > 0 && dv % DS_COLS == 0,
                "gi_delta_scan_prompt: %d heads on %d key heads, keys of %d, values of %d", H, Hk, d, dv);
@@ -877,13 +881,11 @@ extern "C" int gi_delta_scan_prompt(const float* qkv, long long ldq, int q_off, 
     cudaStream_t s = (cudaStream_t)stream;
     const float* al = a_sep ? a_sep : ab;
     const long long ldal = a_sep ? lda_sep : ldab;
-    float *qk = scratch, *gb = scratch + (size_t)n_rows * Hk * 2 * d;
-    const long long items = (long long)n_rows * (H + Hk);
-    GI_REQUIRE((items + 7) / 8 <= 0x7fffffff, "gi_delta_scan_prompt: %d rows", n_rows);
+    GI_REQUIRE(scratch_rows > 0, "gi_delta_scan_prompt: room for %d rows", scratch_rows);
+    if (scratch_rows > n_rows) scratch_rows = n_rows;
+    float *qk = scratch, *gb = scratch + (size_t)scratch_rows * Hk * 2 * d;
+    GI_REQUIRE(((long long)scratch_rows * (H + Hk) + 7) / 8 <= 0x7fffffff, "gi_delta_scan_prompt: %d rows", scratch_rows);
     const auto prepare = channel_decay ? delta_prepare_kernel<1> : delta_prepare_kernel<0>;
-    gi_launch(prepare, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, qkv, ldq, q_off, k_off, ab, ldab, b_off, a_off, al, ldal, A_log,
-              dt_bias, p_dtype, qk, gb, items, H, Hk, d, unit_eps, q_scale);
-    if (int rc = gi_check_launch("gi_delta_scan_prompt")) return rc;
     const size_t smem = (size_t)DS_STAGES * DS_GROUP * (2 * d + (channel_decay ? d + 4 : 4) + DS_COLS) * sizeof(float);
     // One column to a thread where the blocks fit the SMs side by side: four warps to an SM, one to a scheduler.  Two columns
     // beyond: half the reads of shared memory, which then are what several blocks to an SM wait for.
@@ -892,7 +894,15 @@ extern "C" int gi_delta_scan_prompt(const float* qkv, long long ldq, int q_off, 
     const auto walk = d == 128 ? (channel_decay ? DS_WALK(16, 1) : DS_WALK(16, 0)) : (channel_decay ? DS_WALK(8, 1) : DS_WALK(8, 0));
 #undef DS_WALK
     if (int rc = gi_reserve_smem((const void*)walk, smem, "gi_delta_scan_prompt")) return rc;
-    gi_launch(walk, dim3(n_seq, H, dv / DS_COLS), dim3(few ? DS_COLS * 8 : DS_COLS * 4), smem, s, (const float*)qk, (const float*)gb, qkv,
-              ldq, v_off, state, state_stride, spans, out, H, Hk, dv);
-    return gi_check_launch("gi_delta_scan_prompt");
+    for (long long row0 = 0; row0 < n_rows; row0 += scratch_rows) {
+        const int rows = (int)(n_rows - row0 < scratch_rows ? n_rows - row0 : scratch_rows);
+        const long long items = (long long)rows * (H + Hk);
+        gi_launch(prepare, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, qkv + row0 * ldq, ldq, q_off, k_off, ab + row0 * ldab, ldab,
+                  b_off, a_off, al + row0 * ldal, ldal, A_log, dt_bias, p_dtype, qk, gb, items, H, Hk, d, unit_eps, q_scale);
+        if (int rc = gi_check_launch("gi_delta_scan_prompt")) return rc;
+        gi_launch(walk, dim3(n_seq, H, dv / DS_COLS), dim3(few ? DS_COLS * 8 : DS_COLS * 4), smem, s, (const float*)qk, (const float*)gb, qkv,
+                  ldq, v_off, state, state_stride, spans, out, H, Hk, dv, (int)row0, (int)row0 + rows);
+        if (int rc = gi_check_launch("gi_delta_scan_prompt")) return rc;
+    }
+    return 0;
 }

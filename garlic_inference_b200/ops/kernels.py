@@ -934,6 +934,7 @@ def decay_scan(qkv: torch.Tensor, offsets: tuple, decay: torch.Tensor, state: to
 
 
 DELTA_PAIR_TOKENS = 8
+DELTA_SCRATCH_BYTES = 256 << 20    # what the pair keeps of a step's tokens at a time (15,000 of 16 heads of 128 on 8 key heads)
 
 
 def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: tuple, A_log: torch.Tensor,
@@ -959,13 +960,14 @@ def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: 
             all(v % 4 == 0 for v in (qkv.stride(0), state.stride(0), *offsets)) and \
             qkv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
         width = 2 * n_kv_heads * key_dim + n_heads * (key_dim + 4 if channel_decay else 4)
-        scratch = torch.empty((n, width), dtype=torch.float32, device=qkv.device)
+        at_a_time = min(n, max(64, DELTA_SCRATCH_BYTES // (4 * width)))
+        scratch = torch.empty((at_a_time, width), dtype=torch.float32, device=qkv.device)
         check(l.gi_delta_scan_prompt(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0), *map(int, ab_offsets),
                                      _ptr(decay_logits), decay_logits.stride(0) if decay_logits is not None else 0, _ptr(A_log),
                                      _ptr(dt_bias), code(A_log.dtype), _ptr(state), state.stride(0), _ptr(spans), _ptr(out),
-                                     _ptr(scratch), n, n_seq, n_heads, n_kv_heads, key_dim, value_dim, float(unit_eps),
+                                     _ptr(scratch), at_a_time, n, n_seq, n_heads, n_kv_heads, key_dim, value_dim, float(unit_eps),
                                      float(key_dim) ** -0.5, int(channel_decay), _stream()), l)
-        counters.launches += 1                               # two kernels behind one entry point
+        counters.launches += 2 * -(-n // at_a_time) - 1      # two kernels for every so many tokens behind one entry point
         return out
     check(l.gi_delta_scan(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0),
                           *map(int, ab_offsets), _ptr(decay_logits),

@@ -598,6 +598,35 @@ def test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, d, dv, H, Hk, le
             torch.testing.assert_close(got[t].view(H, dv).double(), (S @ q[t][:, :, None])[..., 0], rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("lens", [[200], [33, 100, 2, 16], [64, 64, 9]])
+def test_delta_rule_by_two_kernels_some_rows_at_a_time(channel, lens, monkeypatch):
+    """The same bits where the step's rows pass what is kept of them at a time (64 here): sequences cut in one and in two places,
+    at a cut's edge, and wholly behind it."""
+    from garlic_inference_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_SCRATCH_BYTES", 1)
+    test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, 64, 16, 3, 3, lens, monkeypatch)
+    test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, 128, 48, 2, 1, lens, monkeypatch)
+
+
+def test_delta_rule_over_many_tokens_keeps_a_bounded_scratch(monkeypatch):
+    """40,000 tokens of 16 heads of 128 would keep 680 MB: the room taken is the bound's, and the launches are counted."""
+    from garlic_inference_b200.ops import counters, kernels
+    H, Hk, d, dv, n = 16, 8, 128, 16, 40000
+    qkv, ab, al = rnd(n, 2 * Hk * d + H * dv, seed=1), rnd(n, 2 * H, seed=2), rnd(n, H * d, seed=3)
+    spans = torch.tensor([[0, 0, n]], dtype=torch.int32, device=DEV)
+    args = (qkv, (0, Hk * d, 2 * Hk * d), ab, (H, 0), rnd(H, seed=4), rnd(H * d, seed=5), torch.zeros(1, H * dv * d, device=DEV), spans,
+            torch.zeros(n, dtype=torch.int32, device=DEV), H, Hk, d, dv, 1e-6)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before, launched = torch.cuda.memory_allocated(), counters.launches
+    out = kernels.delta_scan(*args, channel_decay=True, decay_logits=al)
+    assert torch.cuda.max_memory_allocated() - before <= out.numel() * 4 + (256 << 20) + (4 << 20)
+    assert counters.launches - launched == 2 * 3
+    del out
+
+
 # ---- experts' products ------------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("E, K, n_out", [(4, 64, 128), (3, 72, 200), (40, 128, 96), (16, 1032, 264)])
 @pytest.mark.parametrize("counts", ["even", "one", "none_first", "many"])
