@@ -1306,8 +1306,10 @@ def check_bounded_waits(device) -> None:
         key = torch.device(device).index or 0
         if key in _streamk_space:
             _streamk_space[key][1].zero_()
-        raise WaitRanOut(f"a tcgen05 kernel gave up a bounded wait (code {code}: 11-13 product, 21-23 attention, "
-                         "24 unmapped page, 31-33 stream-K product, 34 a partial sum that was never announced)")
+        raise WaitRanOut(f"a tcgen05 kernel gave up a bounded wait or what it was asked for (code {code}: 11-13 product, 21-23 "
+                         "prompt attention, 24 unmapped page, 25 shared memory that does not start on 1,024 bytes and nothing "
+                         "written, 31-33 stream-K product, 34 a partial sum that was never announced, 41-43 decode attention, "
+                         "44 unmapped page, 61-63 experts' product)")
 
 
 def streamk_test_unanswered_flags(limit: int) -> None:

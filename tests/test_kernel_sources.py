@@ -31,3 +31,21 @@ def test_no_barrier_without_a_limit_between_bounded_waits(name):
         between = re.sub(r"//[^\n]*", "", body[waits[0]:waits[-1]])
         assert not re.search(r"\bbar\.(cta\.)?(sync|red)|\bbarrier\.(cta\.)?(sync|red)|__syncthreads|__syncthreads_", between), kernel
     assert found, f"{name}: no kernel with bounded waits was recognised"
+
+
+def test_every_code_of_a_kernel_that_gave_up_is_explained(monkeypatch):
+    """The message names each code that the sources can put into the error flag, alone or in a range."""
+    import torch
+    from garlic_inference_b200.ops import kernels
+    codes = {int(c) for p in CSRC.glob("*.cu") for c in re.findall(r"#define \w+_ERR_\w+ (\d+)", p.read_text())}
+    assert len(codes) > 15
+    flag = torch.zeros(1, dtype=torch.int32)
+    monkeypatch.setattr(kernels, "tcgen05_error_flag", lambda device: flag)
+    for code in sorted(codes):
+        flag[0] = code
+        with pytest.raises(kernels.WaitRanOut) as e:
+            kernels.check_bounded_waits("cpu")
+        said = str(e.value).split(":", 1)[1]
+        ranges = [(int(a), int(b or a)) for a, b in re.findall(r"(?:^|, | )(\d\d)(?:-(\d\d))? [a-z]", said)]
+        assert any(a <= code <= b for a, b in ranges), (code, ranges)
+        assert int(flag) == 0
