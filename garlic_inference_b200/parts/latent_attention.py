@@ -163,7 +163,10 @@ class LatentAttention(Mixer):
             kernels.tcgen05_attention_takes(self.rt.dtype, self.d, keys) else 64
 
     def _portions(self, shape, page: int) -> list:
-        """[(sequence, first page, keys, rows of a run)] of the step's portions that are expanded."""
+        """[(sequence, first page, keys, rows of a run)] of the step's portions that are expanded, worked out once per step."""
+        name = self._runs_name(page)
+        if name in shape.notes:
+            return shape.notes[name]
         which = []
         for i, (n_new, past) in enumerate(zip(shape.seq_lens, shape.seq_past)):
             if self._expands(n_new, past, page):
@@ -172,6 +175,7 @@ class LatentAttention(Mixer):
                 which.append((i, p0, keys, self._run_rows(keys)))
         if self.dr and len(which) < len(shape.seq_lens):
             which = [w for w in which if self.H * shape.seq_lens[w[0]] * w[2] >= MIXED_MIN_SCORES]
+        shape.notes[name] = which
         return which
 
     def _runs_of(self, shape, page: int):

@@ -468,7 +468,7 @@ def test_latent_portions_expanded_beside_others_that_are_not(layout, q_rank, gat
     monkeypatch.undo()
     part = SimpleNamespace(dr=64, d=128, dv=128, rank=512, H=32, window=0, rt=SimpleNamespace(dtype=torch.bfloat16),
                            w_uv=torch.zeros(1, dtype=torch.bfloat16), w_uk_t=torch.zeros(1, dtype=torch.bfloat16))
-    for name in ("_expands", "_first_page", "_first_seen", "_run_rows"):
+    for name in ("_expands", "_first_page", "_first_seen", "_run_rows", "_runs_name"):
         setattr(part, name, getattr(LatentAttention, name).__get__(part))
     chosen = lambda lens, past: [w[0] for w in LatentAttention._portions(part, StepShape([], [], lens, past, False), 64)]
     assert chosen([200], [70]) == [0] and chosen([200, 40], [70, 0]) == [0, 1]
