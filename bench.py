@@ -1473,7 +1473,7 @@ def study_netolorn(args, pk) -> int:
             note(f"latent_attend_{tag}_{n_rows}", ms, flops=2.0 * H * seen * (2 * 512 + rot) if many else 0.0,
                  bytes_=0.0 if many else seen * part.row * 2)
             if many and not rot:                   # what a prompt runs instead: keys and values expanded, then the flash kernel
-                which, _ = part._runs_of(ctx, page)
+                which = part._portions(ctx, page)
                 q_exp, g_exp, o_exp = bf(T, H, 128), bf(T, H), bf(T, H * 128)
                 ms = timed(lambda: part._attend_expanded(q_exp, view.kv, ctx, which, g_exp, o_exp))
                 note(f"latent_attend_expanded_{tag}_{n_rows}", ms, flops=2.0 * H * (seen * 256 + T * 512 * 256))
