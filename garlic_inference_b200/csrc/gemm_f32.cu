@@ -236,7 +236,7 @@ extern "C" int gi_sgemm_nt(const float* A, const float* W, float* C, int M, int 
     GI_REQUIRE(M >= 0 && N > 0 && K > 0, "gi_sgemm_nt: sizes must be positive");
     GI_REQUIRE(lda >= K && ldc >= N, "gi_sgemm_nt: row strides shorter than the rows");
     if (M == 0) return 0;
-    GI_REQUIRE((M + 63) / 64 <= 65535, "gi_sgemm_nt: %d rows in one product is beyond %d", M, 65535 * 64);
+    GI_REQUIRE(((long long)M + 63) / 64 <= 65535, "gi_sgemm_nt: %d rows in one product is beyond %d", M, 65535 * 64);
     const int vec = K % 4 == 0 && lda % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
     cudaStream_t s = (cudaStream_t)stream;
     // Every kernel and tile gives the same bits, so the choice is by time alone: the least of what each was measured to take
@@ -260,10 +260,12 @@ extern "C" int gi_sgemm_nt(const float* A, const float* W, float* C, int M, int 
     const double t32 = c32 <= 1 ? 32.0 : c32 <= 2 ? 48.0 : 20.0 * c32;
     const double t64 = c64 <= 2 ? 62.0 : 51.0 * ((long long)(c64 + 1) / 2);             // two warps: every second block shares their schedulers
     const double t_b = c_b <= 1 ? 68.0 : 51.0 * c_b, t_w = c_w <= 1 ? 100.0 : 89.0 * c_w;
-    const double least = fmin(fmin(t_rows, t32), fmin(t64, fmin(t_b, t_w)));
-    if (least == t_rows) {
+    // (tiles of 32 rows take half as many rows in one launch as the check above lets through)
+    const bool tall = ((long long)M + 31) / 32 > 65535;
+    const double least = fmin(tall ? t64 : fmin(t_rows, t32), fmin(t64, fmin(t_b, t_w)));
+    if (!tall && least == t_rows) {
         if (int rc = launch_rows<32, 4>(A, W, C, M, N, K, lda, ldc, vec, s)) return rc;
-    } else if (least == t32) launch_tiles<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldc, vec, s);
+    } else if (!tall && least == t32) launch_tiles<32, 64, 4, 4>(A, W, C, M, N, K, lda, ldc, vec, s);
     else if (least == t64) launch_tiles<64, 64, 8, 8>(A, W, C, M, N, K, lda, ldc, vec, s);
     else if (least == t_b) launch_tiles<64, 128, 8, 8>(A, W, C, M, N, K, lda, ldc, vec, s);
     else launch_tiles<128, 128, 8, 16>(A, W, C, M, N, K, lda, ldc, vec, s);

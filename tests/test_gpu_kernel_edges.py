@@ -256,6 +256,21 @@ def test_float32_product_has_the_same_bits_by_every_kernel(N, K):
                 assert torch.equal(out[r, :N], one), f"{M} rows, row {r}"
 
 
+@pytest.mark.parametrize("M", [2097120, 2097121, 4194240])
+@pytest.mark.parametrize("N", [3, 16])
+def test_float32_product_of_millions_of_rows(M, N):
+    """Around the rows that tiles of 32 take in one launch, and the most that are taken at all: the bits of a few rows."""
+    from garlic_inference_b200.ops import KernelError, kernels
+    K = 4
+    a, w = torch.randn(M, K, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV), rnd(N, K, seed=2)
+    out = kernels.sgemm_nt(a, w)
+    for at in (0, M // 2, M - 200):
+        assert torch.equal(out[at:at + 200], kernels.sgemm_nt(a[at:at + 200].contiguous(), w))
+    if M == 4194240:
+        with pytest.raises(KernelError, match="rows"):
+            kernels.sgemm_nt(torch.zeros(M + 1, 1, device=DEV), torch.zeros(1, 1, device=DEV))
+
+
 # ---- tcgen05 prompt attention at sizes other than heads of 128 -------------------------------------------------------------
 def _pools(lens, heads, d, page, seed, extra_pages=3):
     """(dense [len, heads, d] per sequence, pool, block table) with pages handed out in a mixed order."""
