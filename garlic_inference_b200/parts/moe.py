@@ -149,6 +149,9 @@ class RoutedExperts(FeedForward):
                 load(f"e{e}.gate", out=self.w_up[e, :self.ff])
             load(f"e{e}.up", out=self.w_up[e, rows - self.ff:])
             load(f"e{e}.down", out=self.w_down[e])
+        self.pair_bytes = (rows + self.ff) * self.hidden * self.w_up.element_size()       # one expert's matrices
+        self.own_takes = dtype == torch.bfloat16 and kernels.moe_products_takes(self.E, self.ff, self.hidden) and \
+            kernels.moe_products_takes(self.E, self.hidden, self.ff)
 
     def route(self, x):
         """(chosen experts int32 [n, top], their weights float32 [n, top], the logit of the shared expert's gate float32
@@ -172,11 +175,9 @@ class RoutedExperts(FeedForward):
         add = linear(glu_product(x, self.shared, self.shared_unit), self.shared_down) if self.shared is not None else None
         grouped = self._grouped(x)
         products = self.gated or self.activation == "relu_squared"     # what the expert-by-expert path computes
-        own = grouped and n * self.top <= OWN_PRODUCT_MAX_MEAN * self.E and \
-            kernels.moe_products_takes(self.E, self.ff, self.hidden) and kernels.moe_products_takes(self.E, self.hidden, self.ff)
-        pair_bytes = (self.w_up[0].numel() + self.w_down[0].numel()) * self.w_up.element_size()
-        few = n <= ROWWISE_MAX_ROWS and not (own and n * self.top * pair_bytes >= ROWWISE_MAX_BYTES)
-        if few or not products or (ctx.captured and not grouped):
+        own = self.own_takes and x.dtype == torch.bfloat16 and n * self.top <= OWN_PRODUCT_MAX_MEAN * self.E
+        few = n <= ROWWISE_MAX_ROWS and not (own and n * self.top * self.pair_bytes >= ROWWISE_MAX_BYTES)
+        if few or not products or (ctx.captured and not (own or grouped)):
             return kernels.moe_rowwise(x, self.w_up, self.w_down, idx, wt, self.act, add=add, add_gate=gate)
         # expert by expert: the pairs (token, choice) in the order of their experts; `where` is each pair's row
         where, ends, rows = kernels.moe_group(idx, x, self.E)

@@ -695,6 +695,37 @@ def test_routed_experts_of_few_rows_by_rows_and_by_products(unit, n, monkeypatch
     torch.testing.assert_close(got[0], got[1], rtol=2e-2, atol=1e-2)       # roundings of the activation and of the pairs' results
 
 
+@pytest.mark.parametrize("E, n, library, own", [(4, 128, True, True), (4, 129, True, False), (4, 128, False, True), (4, 129, False, False),
+                                                (256, 20, True, True), (257, 20, True, False), (257, 20, False, False)])
+def test_which_products_the_experts_run(E, n, library, own, monkeypatch):
+    """Up to 64 rows an expert on average and 256 experts the package's own, also where the library has no grouped product; the
+    row-by-row kernels' results either way."""
+    import garlic_inference_b200.parts.moe as moe
+    from garlic_inference_b200.parts import Runtime, StepContext
+    params = dict(hidden_size=64, expert_size=136, n_experts=E, top=2, expert="glu")
+    w = {k: rnd(*t.shape, seed=i, scale=t.shape[-1] ** -0.5, dtype=torch.bfloat16) for i, (k, t) in enumerate(moe.RoutedExperts.wanted(params).items())}
+
+    class Load:
+        def dtype(self, *names):
+            return torch.bfloat16
+
+        def __call__(self, name, out=None):
+            return w[name] if out is None else out.copy_(w[name])
+
+    part = moe.RoutedExperts(params, Load(), Runtime(torch.bfloat16, torch.device("cuda", 0)))
+    if not library:
+        monkeypatch.delattr(torch, "_grouped_mm")
+    calls, real = [], moe.kernels.moe_products
+    monkeypatch.setattr(moe.kernels, "moe_products", lambda *a: calls.append(1) or real(*a))
+    x, z = rnd(n, 64, seed=50, dtype=torch.bfloat16), torch.zeros(n, dtype=torch.int32, device=DEV)
+    got = part.step(x, StepContext(n, z, z, z)).double()
+    assert len(calls) == (2 if own else 0)
+    monkeypatch.setattr(moe, "ROWWISE_MAX_ROWS", 1 << 30)
+    monkeypatch.setattr(moe, "ROWWISE_MAX_BYTES", 1 << 60)
+    rowwise = part.step(x, StepContext(n, z, z, z)).double()                # a warp per matrix row, float32 sums
+    torch.testing.assert_close(got, rowwise, rtol=2e-2, atol=1e-2)         # roundings of the activation and of the pairs' results
+
+
 # ---- between projections and attention ----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("src_dtype, dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
 @pytest.mark.parametrize("d, dv, n_rot, half", [(64, 128, 0, False), (128, 64, 128, False), (128, 128, 64, True), (24, 20, 12, False),
