@@ -1072,6 +1072,17 @@ def latent_decode_takes(dtype: torch.dtype, row: int, rank: int, heads: int) -> 
             and group * row * 4 + 32 * (row // 2 + 1) * 4 <= 220 * 1024)
 
 
+def latent_decode_slices(n: int, heads: int) -> int:
+    """Slices of the keys for a step of n rows: about 320 blocks in all (two to an SM and some to even out sequences of
+    different lengths), 256 from 33 blocks of queries on, at most 16 slices.  A recorded step's rows are a power of two, so at up
+    to 32 heads the first number matters at 32 rows, where sequences number 17 to 32.  Measured there at 32 heads over rows of
+    576, us at 8 / 10 / 12 slices: 17 sequences of 2,048 tokens 68 / 61 / 57, 24 69 / 62 / 58, 28 69 / 63 / 79, 32 72 / 74 / 86,
+    32 of 500 33 / 36 / 36; of 200 to 4,000 tokens 17 93 / 79 / 76, 20 93 / 79 / 76, 32 98 / 89 / 97.  1 sequence of 2,048 tokens
+    at 4 / 8 / 16 slices 70 / 46 / 37, 8 sequences 71 / 47 / 39; 64 115 / 135 / 143, of 200 to 4,000 174 / 156 / 163."""
+    blocks = n * -(-heads // 32)
+    return max(1, min(16, (320 if blocks <= 32 else 256) // max(1, blocks)))
+
+
 def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor, tok_pos: torch.Tensor,
                   tok_slot: torch.Tensor, scale: float, sinks: Optional[torch.Tensor], rank: int,
                   status: torch.Tensor, n_splits: Optional[int] = None, window: int = 0) -> torch.Tensor:
@@ -1087,12 +1098,7 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor
     if one != 1 or pool_row != row:
         raise KernelError(f"a pool {tuple(pool.shape)} does not hold rows of {row} shared by all heads")
     if n_splits is None:
-        # Slices of the keys: about 384 blocks in all (two to an SM and some to even out sequences of different lengths), 256
-        # from 33 sequences on, at most 16 slices.  Measured at 32 heads over rows of 576 (us at 4 / 8 / 16 / 32 slices): 1 sequence of 2,048 tokens
-        # 70 / 47 / 37 / 39, 8 sequences 71 / 47 / 39 / 49, 32 sequences 80 / 71 / 83 / 113, 20 sequences of 200 to 4,000 tokens
-        # (in a step of 32 rows) 122 / 93 / 78 / 107, 64 sequences 115 / 135 / 146 / 208; 12 slices of 32: 85 and 79.
-        groups = -(-heads // 32)
-        n_splits = max(1, min(16, (384 if n * groups <= 32 else 256) // max(1, n * groups)))
+        n_splits = latent_decode_slices(n, heads)
     part = torch.empty((n, n_splits, heads, rank + 2), dtype=torch.float32, device=q.device)
     out = torch.empty((n, heads * rank), dtype=torch.bfloat16, device=q.device)
     check(l.gi_latent_decode(_ptr(q), _ptr(pool), _ptr(block_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(part),

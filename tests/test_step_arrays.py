@@ -95,3 +95,9 @@ def test_queries_that_see_few_keys_keep_the_mma_sync_prompt_kernel():
     windowed = SimpleNamespace(**{**vars(gqa(64)), "window": 40})
     assert GQAAttention._run_rows(windowed, kv, far) == 128   # positions 1,961 to 2,063: tiles 30 to 32
     assert GQAAttention._run_rows(windowed, kv, _shape([20], [2000])) == 64      # up to 2,019: two tiles of a long sequence
+
+
+def test_slices_of_a_latent_decode_step():
+    from garlic_inference_b200.ops.kernels import latent_decode_slices
+    assert [latent_decode_slices(n, 32) for n in (1, 16, 32, 33, 64, 256, 1000)] == [16, 16, 10, 7, 4, 1, 1]
+    assert [latent_decode_slices(n, 128) for n in (1, 4, 8, 16)] == [16, 16, 10, 4] and latent_decode_slices(0, 8) == 16
