@@ -515,6 +515,18 @@ flash_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __
                     pk[j >> 1] = *reinterpret_cast<uint32_t*>(&v);
                 }
                 l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                // Rows of values behind the last one that the item sees hold what the page's owner before left there: a probability
+                // of zero times an infinity or NaN would be a NaN, so they are made zeros.
+                const int valid = of_blocks ? ft_blocks_seen(im.pos0 + im.n_rows - 1, window, means.block) - key0 : im.pos0 + im.n_rows - key0;
+                if (valid < FT_BN) {                     // the last tile, the same for all four warps
+                    const int sv = g % V_STAGES;
+                    if (!wait_warp(&ctl->v_full[sv], (g / V_STAGES) & 1)) { ok = false; break; }
+                    for (int i = (int)threadIdx.x - 64; i < (FT_BN - valid) * DV / 8; i += 128) {     // (the swizzle stays inside a row)
+                        const int row = valid + i / (DV / 8), word = i % (DV / 8);
+                        *reinterpret_cast<uint4*>(v_tiles + sv * V_BYTES + word / 8 * FT_KV_PART + row * 128 + word % 8 * 16) = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
                 ft_st32(lane_base + FT_COL_S + b * FT_BN, pk);
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();

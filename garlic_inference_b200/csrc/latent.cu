@@ -6,7 +6,8 @@
 // shared rotated part and its value is W_uv,h c, so with q'_h = W_uk,h^T q_h (made by a per-head product
 // before this kernel) the score is  q'_h . c + rot(q_rot,h) . rot(k_rot),  attention over the cache rows
 // themselves gives sum_j p_j c_j, and W_uv,h is applied to that afterwards: the cache is read once for all
-// heads and keys and values are never expanded.
+// heads and keys and values are not expanded.  (For long portions of prompts they are, outside this file; the queries are
+// then their own unrotated columns beside the rotated part.)
 //
 // Rotation: pair (2i, 2i+1) of the rotated part (or, in the half layout, pair (i, i + n_rot/2)), i < n_rot / 2,
 // turns by the float32 product position * freq[i]; cosine and sine are multiplied by `magnitude`; dimensions from
@@ -380,12 +381,11 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-//
 // Two blocks fit an SM: one's copies and barriers run under the other's products, so a block stages one chunk at a time.  A
 // chunk costs its block a serial chain (copy, scores, softmax, weighted rows); the scores' steps therefore go in two
 // sums of half the width each, their fragments four steps ahead.  Measured with 20 sequences of 200 to 4,000 tokens, 32 heads,
-// rows of 576 (a recorded step has 32 rows), in 8 slices: 112 us before
-// both and before the look-ups were a warp's, 93 us so; 64 sequences of 2,048 in 4 slices 214 -> 115 us.
+// rows of 576 (a recorded step has 32 rows), in 8 slices: 112 us before both and before the look-ups were a warp's, 93 us so;
+// 64 sequences of 2,048 in 4 slices 214 -> 115 us.
 template <int NTW>
 __global__ void __launch_bounds__(LD_WARPS * 32, 2)
 latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,

@@ -353,6 +353,39 @@ def test_prompt_attention_on_tensor_memory_at_other_sizes(d, dv, maps, n_dist, p
     kernels.check_bounded_waits(torch.device("cuda", 0))
 
 
+@pytest.mark.parametrize("d, dv, maps, n_dist, rot", [(64, 64, 1, 0, False), (64, 128, 2, 0, False), (128, 64, 1, 0, False),
+                                                      (128, 128, 1, 0, False), (128, 128, 1, 0, True), (64, 64, 1, 90, False)])
+@pytest.mark.parametrize("window", [0, 50])
+def test_prompt_attention_beside_what_a_page_held_before(d, dv, maps, n_dist, rot, window):
+    """Infinities and NaN behind a sequence's last token (left in its page by the page's owner before) reach no result."""
+    from garlic_inference_b200.ops import kernels
+    H, G, page = (3, 3, 128) if rot else (4, 2, 128)
+    lens, new = ([300], [70]) if rot else ([1, 37, 300, 64, 65, 513, 128], [1, 37, 70, 64, 3, 513, 100])
+    if rot:
+        page = 320
+    ks, k_pool, table = _pools(lens, G * maps, d, page, 20, extra_pages=0)
+    vs, v_pool, _ = _pools(lens, G, dv, page, 60, extra_pages=0)
+    shared = rnd(page, 64, seed=4, dtype=torch.bfloat16) if rot else None
+    runs, starts = _runs128(lens, new)
+    q = rnd(sum(new), H * maps, d + 64 * rot, seed=5, dtype=torch.bfloat16)
+    bias = rnd(n_dist, H, seed=6) if n_dist else None
+    run = lambda: kernels.attention_prefill_tcgen05(q, k_pool, v_pool, table, runs, d ** -0.5, window, maps=maps, dist_bias=bias,
+                                                    rows_covered=True, **({"rot": (shared, 0)} if rot else {}))
+    for pool in (k_pool, v_pool):                                          # zeros behind the ends, then anything
+        for s, n in enumerate(lens):
+            if n % page:
+                pool[int(table[s, n // page]), :, n % page:] = 0.0
+    want = run()
+    for pool, bad in ((k_pool, (math.nan, math.inf)), (v_pool, (math.inf, math.nan))):
+        for s, n in enumerate(lens):
+            if n % page:
+                pool[int(table[s, n // page]), :, n % page:, ::2], pool[int(table[s, n // page]), :, n % page:, 1::2] = bad
+    if rot:
+        shared[lens[0]:] = math.nan
+    assert torch.isfinite(want).all() and torch.equal(run(), want)
+    kernels.check_bounded_waits(torch.device("cuda", 0))
+
+
 @pytest.mark.parametrize("n_dist", [40, 500])
 def test_distance_biases_where_a_block_walks_many_items(n_dist):
     """More than six items of different heads to every persistent block, each with a table of its own in the same place."""

@@ -511,3 +511,17 @@ def test_biased_router_and_an_addend_with_a_gate():
             got = kernels.moe_combine(buf, None, wt, add, z[:, E:])
             want = (buf.view(n, top, 72).double() * wt[:, :, None].double()).sum(1) + torch.sigmoid(z[:, E:].double()) * add.double()
             torch.testing.assert_close(got.double(), want, rtol=tol, atol=tol)
+
+
+def test_the_benchmarks_study_runs():
+    """`bench.py --study netolorn` calls the parts beside their public steps; it has to follow them."""
+    import json
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parent.parent
+    done = subprocess.run([sys.executable, "bench.py", "--study", "netolorn", "--steps", "1", "--warmup", "3"], cwd=root,
+                          capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+    out = json.loads(done.stdout.strip().splitlines()[-1])
+    assert any("latent_attend_expanded" in k for k in json.dumps(out).split('"'))
