@@ -31,12 +31,13 @@ kv_rank]; the sequence's rows are gathered from its pages once per step and the 
 whose scores fit `SCORE_BYTES`.  Tensor cores do both products; the weights are rounded to bfloat16 only as
 the second product's operand.
 Long portions in bfloat16 (from plain_dim + value_dim tokens on without a rotated part, at sizes that the flash kernels
-take; from `ROT_MIN_ROWS` on, at a sequence's start from PRODUCT_MIN_ROWS on, with a rotated part of 64 beside 128 plain dimensions and values of 128) expand the keys and
-values they see, [heads, keys, plain_dim] and [heads, keys, value_dim] by two batched products of the
-gathered rows, and run the flash kernel for prompts over them as one large page (tcgen05 for sizes of 128, mma.sync
-otherwise; window, sink and gate inside it; a rotated part is read from the gathered rows, the same for all heads): an
-expanded key costs kv_rank (plain_dim + value_dim) once and saves about kv_rank per new token, and no scores are written
-to memory.
+take; from `ROT_MIN_ROWS` on, at a sequence's start from PRODUCT_MIN_ROWS on, with a rotated part of 64 beside 128 plain
+dimensions and values of 128, and beside portions that are not expanded only from `MIXED_MIN_SCORES` scores on) expand the
+keys and values they see, as many heads at a time as `EXPAND_RUN_BYTES` takes, [heads, keys, plain_dim] and [heads,
+keys, value_dim] by two batched products of the gathered rows, and run the flash kernel for prompts over them as one
+large page (tcgen05 for sizes of 128 and, beyond two tiles of keys, of 64; mma.sync otherwise; window, sink and gate
+inside it; a rotated part is read from the gathered rows, the same for all heads): an expanded key costs kv_rank
+(plain_dim + value_dim) once and saves about kv_rank per new token, and no scores are written to memory.
 The rotation is the position part's (its frequencies, magnitude and layout: pairs (2i, 2i+1), or halves (i,
 i + n/2)).  Upstream has grouped-query attention only (src/models/qwen3/qwen3.cpp:140-179).
 """
