@@ -1,6 +1,6 @@
 // True float32 matrix product for the 32-bit engine: C[M,N] = A[M,K] . W[N,K]^T
-// with float32 FMA on the CUDA cores, never a tensor-core or reduced-precision
-// mode.  Each output element is one accumulator summed over k in ascending
+// with float32 FMA on the CUDA cores, for weights that gemm_f32_tcgen05.cu does
+// not take (small ones, and rows that do not start on 16 bytes).  Each output element is one accumulator summed over k in ascending
 // order, so a row's result is the same bits whatever M is: whole prompts,
 // single tokens and batches agree exactly, and so do the two kernels here.
 //

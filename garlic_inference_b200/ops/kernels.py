@@ -1169,6 +1169,30 @@ def latent_norms(src: torch.Tensor, q_off: int, c_off: int, q_norm: torch.Tensor
     return q_out
 
 
+# float32 weights with at least this many elements (and inputs) run on tensor cores, in three exact parts: from there on a row alone
+# takes as long as by FMAs (9.6 us against 9.0 at 1,024 x 1,024, 14 against 17 at 2,048 x 2,048) and many rows a third
+SPLIT_MIN_ELEMENTS = 1 << 20
+SPLIT_MIN_INPUTS = 512
+SPLIT_SPACE = 1 << 27          # bytes of the parts of A at a time
+
+
+def _sgemm(l, a: torch.Tensor, lda: int, w: torch.Tensor, out: torch.Tensor, ldc: int) -> None:
+    """Which of the two float32 products runs follows from the weight alone, so that a row's bits do not depend on the step."""
+    (m, k), n = a.shape, w.shape[0]
+    if n * k < SPLIT_MIN_ELEMENTS or k < SPLIT_MIN_INPUTS or k % 4 or w.data_ptr() % 16 or m == 0:
+        check(l.gi_sgemm_nt(_ptr(a), _ptr(w), _ptr(out), m, n, k, lda, ldc, _stream()), l)
+        return
+    row_bytes = 6 * ((k + 7) // 8 * 8)
+    rows = min(m, max(128, SPLIT_SPACE // row_bytes // 128 * 128))
+    flag = _ptr(tcgen05_error_flag(a.device))
+    for r in range(0, m, rows):
+        part = min(rows, m - r)
+        size = l.gi_sgemm_split_space(part, n, k)
+        space = torch.empty(size, dtype=torch.uint8, device=a.device)
+        check(l.gi_sgemm_split_nt(_ptr(a[r:]), _ptr(w), _ptr(out[r:]), _ptr(space), size, part, n, k, lda, ldc, 0, 0, flag, _stream()), l)
+        counters.launches += l.gi_sgemm_split_launches(part, n, k) - 1
+
+
 def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a [M,K] . w[N,K]^T in true float32."""
     l = require_gpu()
@@ -1179,7 +1203,7 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = Non
     if out is None:
         out = torch.empty((m, n), dtype=torch.float32, device=a.device)
     _dense(out, "out", torch.float32)
-    check(l.gi_sgemm_nt(_ptr(a), _ptr(w), _ptr(out), m, n, k, k, n, _stream()), l)
+    _sgemm(l, a, k, w, out, n)
     return out
 
 
@@ -1190,8 +1214,7 @@ def sgemm_nt_strided(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> tor
     (m, k), (n, k2) = a.shape, w.shape
     if k != k2 or out.shape != (m, n):
         raise KernelError(f"a {tuple(a.shape)}, w {tuple(w.shape)} and out {tuple(out.shape)} do not fit")
-    check(l.gi_sgemm_nt(_ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0) if m > 1 else k,
-                        out.stride(0) if m > 1 else n, _stream()), l)
+    _sgemm(l, a, a.stride(0) if m > 1 else k, w, out, out.stride(0) if m > 1 else n)
     return out
 
 
@@ -1315,7 +1338,7 @@ def check_bounded_waits(device) -> None:
         raise WaitRanOut(f"a tcgen05 kernel gave up a bounded wait or what it was asked for (code {code}: 11-13 product, 21-23 "
                          "prompt attention, 24 unmapped page, 25 shared memory that does not start on 1,024 bytes and nothing "
                          "written, 31-33 stream-K product, 34 a partial sum that was never announced, 41-43 decode attention, "
-                         "44 unmapped page, 61-63 experts' product)")
+                         "44 unmapped page, 61-63 experts' product, 71-74 float32 product)")
 
 
 def streamk_test_unanswered_flags(limit: int) -> None:

@@ -90,6 +90,9 @@ _SIGNATURES = {
     "gi_attention_decode_tcgen05": ([P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P], I),
     "gi_attention_decode_combine": ([P, P, P, I, I, I, P], I),
     "gi_sgemm_nt": ([P, P, P, I, I, I, L, L, P], I),
+    "gi_sgemm_split_nt": ([P, P, P, P, L, I, I, I, L, L, I, I, P, P], I),
+    "gi_sgemm_split_space": ([I, I, I], L),
+    "gi_sgemm_split_launches": ([I, I, I], I),
     "gi_gemv_bf16": ([P, P, P, I, I, I, I, P], I),
     "gi_gemm_skinny_bf16": ([P, P, P, I, I, I, I, I, I, P], I),
     "gi_gemv_swiglu_bf16": ([P, P, P, I, I, P], I),

@@ -1,9 +1,10 @@
 """y = x W^T for a weight stored [out, in], the way every projection here is.
 
 Which product runs:
-  * float32 weight: this package's own float32 FMA kernel (no tensor-core or
-    reduced-precision mode); bfloat16 activations are widened first and the
-    result narrowed again.
+  * float32 weight: this package's own float32 products (FMAs, or for weights
+    of a million elements and more tensor cores on three exact parts of every
+    number; no reduced precision); bfloat16 activations are widened first and
+    the result narrowed again.
   * bfloat16 weight of 256 MB and more (the head), 1 to 64 rows, and of 90 MB
     and more (the feed-forward's) at 9 to 32 rows: this package's stream-K
     tcgen05 kernel, which cuts the weight evenly over the SMs.

@@ -256,6 +256,56 @@ def test_float32_product_has_the_same_bits_by_every_kernel(N, K):
                 assert torch.equal(out[r, :N], one), f"{M} rows, row {r}"
 
 
+@pytest.mark.parametrize("N, K", [(1030, 1024), (2048, 516), (300, 3500)])
+def test_float32_product_on_tensor_cores(N, K):
+    """Weights of a million elements: rows on both sides of every tile height, inputs that are no whole slices, rows that lie
+    apart and rows that do not start on 16 bytes: within the error of float32 sums, every row with the bits of its product alone."""
+    from garlic_inference_b200.ops import kernels
+    assert N * K >= kernels.SPLIT_MIN_ELEMENTS and K >= kernels.SPLIT_MIN_INPUTS
+    w, full = rnd(N, K, seed=1), rnd(400, K + 5, seed=2)
+    alone = {}
+    for M in (1, 2, 15, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129, 400):
+        for a in (full[:M, :K].contiguous(), full[:M, :K]):
+            out = torch.full((M, N + 3), 7.0, device=DEV)
+            kernels.sgemm_nt_strided(a, w, out[:, :N])
+            want = a.double() @ w.double().T
+            tol = (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)       # a rounding an addition
+            assert ((out[:, :N].double() - want).abs() <= tol).all() and bool((out[:, N:] == 7.0).all())
+            for r in {0, M // 2, M - 1}:
+                one = alone.setdefault(r, kernels.sgemm_nt(full[r:r + 1, :K].contiguous(), w)[0])
+                assert torch.equal(out[r, :N], one), f"{M} rows, row {r}"
+    kernels.check_bounded_waits(DEV)
+
+
+@pytest.mark.parametrize("M, N, K", [(1, 130, 64), (16, 128, 68), (70, 257, 640), (200, 128, 1000)])
+def test_every_form_of_the_float32_product_gives_the_same_bits(M, N, K):
+    """All tile heights, with the inputs of a tile in one block and shared out; infinities, NaN and numbers that round up to an
+    infinity come out as by multiply-adds."""
+    from garlic_inference_b200.ops import kernels
+    from garlic_inference_b200.ops.library import check, require_gpu
+    l, flag = require_gpu(), kernels.tcgen05_error_flag(torch.device(DEV, 0))
+    a, w = rnd(M, K, seed=3), rnd(N, K, seed=4)
+    a[0, 5], a[M // 2, 9], a[M - 1, K - 1] = math.inf, math.nan, 3.4e38
+    w[N - 1, 3], w[7, 11], w[9] = -math.inf, 3.4028234e38, 0.0
+    want = torch.empty(M, N, device=DEV)
+    check(l.gi_sgemm_nt(a.data_ptr(), w.data_ptr(), want.data_ptr(), M, N, K, K, N, 0), l)
+    space = torch.empty(6 * M * (K + 8) + 4 * M * N * (K // 64 + 1) + 512, dtype=torch.uint8, device=DEV)
+    first = None
+    for tile in (16, 32, 64, 96, 128):
+        for shares in (1, 3, 100):
+            out = torch.full((M, N), 7.0, device=DEV)
+            check(l.gi_sgemm_split_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), space.data_ptr(), space.numel(), M, N, K, K, N, tile, shares,
+                                      flag.data_ptr(), 0), l)
+            first = out if first is None else first
+            assert torch.equal(out.view(torch.int32), first.view(torch.int32)), (tile, shares)
+    odd = ~want.isfinite()
+    assert torch.equal(first.isfinite(), want.isfinite()) and torch.equal(first[odd].isnan(), want[odd].isnan())
+    assert torch.equal(first[odd & ~want.isnan()], want[odd & ~want.isnan()])
+    with pytest.raises(Exception, match="work space"):
+        check(l.gi_sgemm_split_nt(a.data_ptr(), w.data_ptr(), want.data_ptr(), space.data_ptr(), 16, M, N, K, K, N, 32, 1, flag.data_ptr(), 0), l)
+    kernels.check_bounded_waits(DEV)
+
+
 @pytest.mark.parametrize("M", [2097120, 2097121, 4194240])
 @pytest.mark.parametrize("N", [3, 16])
 def test_float32_product_of_millions_of_rows(M, N):
