@@ -148,6 +148,11 @@ __device__ __forceinline__ t5_f2 t5_add2(t5_f2 a, t5_f2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ t5_f2 t5_mul2(t5_f2 a, t5_f2 b) {
+    t5_f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ t5_f2 t5_fma2(t5_f2 a, t5_f2 b, t5_f2 c) {
     t5_f2 d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));

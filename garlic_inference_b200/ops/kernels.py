@@ -935,17 +935,25 @@ def decay_scan(qkv: torch.Tensor, offsets: tuple, decay: torch.Tensor, state: to
 
 DELTA_PAIR_TOKENS = 8
 DELTA_SCRATCH_BYTES = 256 << 20    # what the pair keeps of a step's tokens at a time (15,000 of 16 heads of 128 on 8 key heads)
+# Tokens a sequence from which on a prompt is taken in chunks, where the caller lets it: a chunk's preparation costs the same however few
+# blocks (16 value columns of a head of a sequence) there are, and token by token is a chain that many blocks hide.  In us, token by token /
+# so, heads of 128 x 128: 1 x 64 tokens of 8 heads 15.9 / 15.5, 1 x 128 27.5 / 18.8, 1 x 2,048 373 / 140; 16 heads: 2 x 100 28.3 / 28.5,
+# 4 x 128 54.5 / 51.9, 8 x 100 82 / 86, 8 x 256 193 / 174, 16 x 128 177 / 192, 64 x 32 182 / 325.
+DELTA_CHUNK_TOKENS = 64
+DELTA_CHUNK_BLOCKS = 512           # as many more tokens for every so many blocks
+DELTA_CHUNK_ROWS = 1024            # and room for so many rows at a time
 
 
 def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: tuple, A_log: torch.Tensor,
                dt_bias: torch.Tensor, state: torch.Tensor, spans: Optional[torch.Tensor], tok_slot: torch.Tensor,
                n_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, unit_eps: float,
-               channel_decay: bool = False, decay_logits: Optional[torch.Tensor] = None) -> torch.Tensor:
+               channel_decay: bool = False, decay_logits: Optional[torch.Tensor] = None, chunks: bool = False) -> torch.Tensor:
     """The gated delta rule over the step's rows, from and to `state`.  `qkv` float32 [n, C] holds q, k (per key
     head) and v (per head) at `offsets`; `ab` float32 holds the logits of beta and of the decay at `ab_offsets`
     (one column per head; with `channel_decay` the decay has one column per head and key channel, and dt_bias as
     many elements).  `decay_logits`: the decay's logits as a float32 matrix of their own (its column
-    ab_offsets[1] is the first).  Returns float32 [n, n_heads * value_dim]."""
+    ab_offsets[1] is the first).  `chunks`: prompts may be taken 16 tokens at a time, as precise but with sums in another
+    order, so that a token's bits depend on where its portion begins.  Returns float32 [n, n_heads * value_dim]."""
     l = require_gpu()
     _rows(qkv, "qkv", torch.float32), _rows(ab, "ab", torch.float32), _rows(state, "state", torch.float32)
     _dense(A_log, "A_log"), _dense(dt_bias, "dt_bias", A_log.dtype)
@@ -959,6 +967,18 @@ def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: 
     if spans is not None and n >= DELTA_PAIR_TOKENS * n_seq and key_dim in (64, 128) and value_dim % 16 == 0 and \
             all(v % 4 == 0 for v in (qkv.stride(0), state.stride(0), *offsets)) and \
             qkv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
+        each = l.gi_delta_chunk_bytes(n_heads, key_dim, value_dim)
+        at_a_time = min(n, (DELTA_SCRATCH_BYTES // each - n_seq) * 16)
+        blocks = n_seq * n_heads * value_dim // 16
+        if chunks and n * DELTA_CHUNK_BLOCKS >= DELTA_CHUNK_TOKENS * n_seq * (DELTA_CHUNK_BLOCKS + blocks) and at_a_time >= min(n, DELTA_CHUNK_ROWS):
+            space = torch.empty((at_a_time // 16 + n_seq) * each, dtype=torch.uint8, device=qkv.device)
+            check(l.gi_delta_chunk_scan(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0), *map(int, ab_offsets),
+                                        _ptr(decay_logits), decay_logits.stride(0) if decay_logits is not None else 0, _ptr(A_log),
+                                        _ptr(dt_bias), code(A_log.dtype), _ptr(state), state.stride(0), _ptr(spans), _ptr(out),
+                                        _ptr(space), at_a_time, n, n_seq, n_heads, n_kv_heads, key_dim, value_dim, float(unit_eps),
+                                        float(key_dim) ** -0.5, int(channel_decay), _ptr(tcgen05_error_flag(qkv.device)), _stream()), l)
+            counters.launches += 2 * -(-n // at_a_time) - 1
+            return out
         width = 2 * n_kv_heads * key_dim + n_heads * (key_dim + 4 if channel_decay else 4)
         at_a_time = min(n, max(64, DELTA_SCRATCH_BYTES // (4 * width)))
         scratch = torch.empty((at_a_time, width), dtype=torch.float32, device=qkv.device)
@@ -1338,7 +1358,7 @@ def check_bounded_waits(device) -> None:
         raise WaitRanOut(f"a tcgen05 kernel gave up a bounded wait or what it was asked for (code {code}: 11-13 product, 21-23 "
                          "prompt attention, 24 unmapped page, 25 shared memory that does not start on 1,024 bytes and nothing "
                          "written, 31-33 stream-K product, 34 a partial sum that was never announced, 41-43 decode attention, "
-                         "44 unmapped page, 61-63 experts' product, 71-74 float32 product)")
+                         "44 unmapped page, 61-63 experts' product, 71-74 float32 product, 81 delta rule)")
 
 
 def streamk_test_unanswered_flags(limit: int) -> None:

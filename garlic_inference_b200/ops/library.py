@@ -69,6 +69,8 @@ _SIGNATURES = {
     "gi_decay_scan": ([P, L, I, I, I, I, P, P, L, P, P, P, I, I, I, I, P], I),
     "gi_moe_grouped": ([P, P, P, P, I, I, I, I, I, I, F, F, F, F, P, P], I),
     "gi_delta_scan_prompt": ([P, L, I, I, I, P, L, I, I, P, L, P, P, I, P, L, P, P, P, I, I, I, I, I, I, I, F, F, I, P], I),
+    "gi_delta_chunk_bytes": ([I, I, I], L),
+    "gi_delta_chunk_scan": ([P, L, I, I, I, P, L, I, I, P, L, P, P, I, P, L, P, P, P, I, I, I, I, I, I, I, F, F, I, P, P], I),
     "gi_delta_scan": ([P, L, I, I, I, P, L, I, I, P, L, P, P, I, P, L, P, P, P, I, I, I, I, I, F, F, I, P], I),
     "gi_matrix_memory_state_floats": ([I, I], L),
     "gi_matrix_memory_scan": ([P, L, I, I, I, I, P, L, I, I, P, P, F, F, P, L, P, P, P, I, I, I, I, P], I),

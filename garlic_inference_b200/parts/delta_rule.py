@@ -115,7 +115,8 @@ class GatedDeltaRule(Mixer):
                            out_dtype=torch.float32)
         o = kernels.delta_scan(qkv, (self.q_off, self.k_off, self.v_off), ba, (self.b_off, self.a_off), self.A_log,
                                self.dt_bias, cache.state, ctx.seq_spans(), ctx.tok_slot, self.H, self.Hk, self.d,
-                               self.dv, self.unit_eps, channel_decay=self.channel_decay, decay_logits=decay)
+                               self.dv, self.unit_eps, channel_decay=self.channel_decay, decay_logits=decay,
+                               chunks=x.dtype == torch.bfloat16)          # (the 32-bit engine's bits do not depend on the cut)
         if self.gate_rank:
             gate = linear(proj[:, self.g_off:self.g_off + self.gate_rank].contiguous(), self.w_g2)
         else:

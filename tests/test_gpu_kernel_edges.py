@@ -707,6 +707,57 @@ def test_delta_rule_by_two_kernels_some_rows_at_a_time(channel, lens, monkeypatc
     test_delta_rule_by_two_kernels_has_the_bits_of_one(channel, 128, 48, 2, 1, lens, monkeypatch)
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("d, dv, H, Hk", [(128, 128, 4, 2), (64, 16, 3, 3), (128, 144, 2, 1)])
+@pytest.mark.parametrize("lens, at_a_time", [([1, 15, 16, 17, 33], None), ([100], None), ([70, 3, 64], 40)])
+def test_delta_rule_in_chunks(channel, d, dv, H, Hk, lens, at_a_time, monkeypatch):
+    """Part chunks, a padding portion, decays of zero and of one, a step cut into rows that are taken at a time: against 64 bits, as
+    close as token by token."""
+    from garlic_inference_b200.ops import kernels
+    from garlic_inference_b200.ops.library import require_gpu
+    n, n_dec = sum(lens) + 2, H * d if channel else H
+    qkv, ab, al = rnd(n, 2 * Hk * d + H * dv, seed=1), rnd(n, 2 * H, seed=2), rnd(n, n_dec, seed=3, scale=2.0)
+    al[1], al[2, 0] = 1e4, -1e4                                  # a decay of zero, one of one
+    A_log, dt = rnd(H, seed=4, scale=0.3), rnd(n_dec, seed=5) - 2.0
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    spans = torch.tensor([[i, s, m] for i, (s, m) in enumerate(zip(starts, lens))] + [[-1, n - 2, 2]], dtype=torch.int32, device=DEV)
+    slots = torch.zeros(n, dtype=torch.int32, device=DEV)
+    first = rnd(len(lens) + 1, H * dv * d + 8, seed=6, scale=0.1)
+    if at_a_time:
+        monkeypatch.setattr(kernels, "DELTA_SCRATCH_BYTES", require_gpu().gi_delta_chunk_bytes(H, d, dv) * (len(lens) + 1 + at_a_time // 16))
+        monkeypatch.setattr(kernels, "DELTA_CHUNK_ROWS", 16)
+
+    def run(chunks):
+        monkeypatch.setattr(kernels, "DELTA_CHUNK_TOKENS", 0)
+        state, launched = first.clone(), kernels.counters.launches
+        out = kernels.delta_scan(qkv, (0, Hk * d, 2 * Hk * d), ab, (H, 0), A_log, dt, state, spans, slots, H, Hk, d, dv, 1e-6,
+                                 channel_decay=channel, decay_logits=al, chunks=chunks)
+        return out, state, kernels.counters.launches - launched
+
+    got, state, launched = run(True)
+    one, state1, _ = run(False)
+    assert launched == 2 * (-(-n // (at_a_time // 16 * 16)) if at_a_time else 1)
+    assert not torch.equal(got, one) and float(got[n - 2:].abs().max()) == 0.0 and torch.equal(state[:, H * dv * d:], first[:, H * dv * d:])
+    q, k, v = (qkv[:, a:b].double() for a, b in ((0, Hk * d), (Hk * d, 2 * Hk * d), (2 * Hk * d, 2 * Hk * d + H * dv)))
+    unit = lambda x: (x.view(n, Hk, d) / torch.sqrt((x.view(n, Hk, d) ** 2).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // Hk, 1)
+    q, k, v, beta = unit(q) * d ** -0.5, unit(k), v.view(n, H, dv), torch.sigmoid(ab[:, H:].double())
+    g = torch.exp(-torch.exp(A_log.double())[:, None] * torch.nn.functional.softplus(al.double() + dt.double()).view(n, H, -1))
+    want, last = torch.zeros(n, H, dv, dtype=torch.float64, device=DEV), first.double()
+    for i, (s, m) in enumerate(zip(starts, lens)):
+        S = first[i, :H * dv * d].double().view(H, dv, d)
+        for t in range(s, s + m):
+            S = S * g[t][:, None, :]
+            u = beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0])
+            S = S + u[:, :, None] * k[t][:, None, :]
+            want[t] = (S @ q[t][:, :, None])[..., 0]
+        last[i, :H * dv * d] = S.reshape(-1)
+    far = lambda x, y: float((x.double() - y).norm() / y.norm())
+    # some eight roundings to 2^-24 of a number between unit vectors and a result; token by token they are as many
+    for x, x1, y in ((got, one, want.view(n, -1)), (state, state1, last)):
+        assert far(x, y) < 8 * 2.0 ** -24 and far(x, y) < 2.0 * far(x1, y) + 2.0 ** -24
+    kernels.check_bounded_waits(DEV)
+
+
 def test_delta_rule_over_many_tokens_keeps_a_bounded_scratch(monkeypatch):
     """40,000 tokens of 16 heads of 128 would keep 680 MB: the room taken is the bound's, and the launches are counted."""
     from garlic_inference_b200.ops import counters, kernels
