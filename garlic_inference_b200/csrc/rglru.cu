@@ -14,16 +14,13 @@
 // both matrices in shared memory and streams tiles of tokens past them.  Every sum runs in an order that depends on
 // the block width alone, and the scan walks a sequence's tokens in order, so a position's bits do not depend on
 // how the tokens were cut into steps or on the batch.  NikolayBlagoev/garlic-inference has no recurrent mixer.
-#include "common.cuh"
-#include <math.h>
+#include "rglru.cuh"
 
 #define RG_KS 8              // lanes that share an output: lane s sums the inputs k = s, s + 8, s + 16, ...
 #define RG_TG 8              // tokens per thread
 #define RG_OG 4              // outputs per thread
 #define RG_WPAD 8            // padding of a row of weights in shared memory: rows start on 16 bytes and spread over the banks
 
-__device__ __forceinline__ float rg_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
-__device__ __forceinline__ float rg_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float rg_gelu_tanh(float z) {
     return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
@@ -305,14 +302,6 @@ __device__ __forceinline__ void rm_mma(float (&d)[4], const uint32_t (&a)[4], ui
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
-// One output's sum by float32 multiply-adds of the whole inputs: what the three parts of a finite input times an infinite
-// weight are not (a part that is zero makes a NaN of it).
-__device__ __noinline__ float rm_plain(const float* u, const bf16* w, int bw) {
-    float s = 0.f;
-    for (int k = 0; k < bw; ++k) s = fmaf(to_f32(w[(size_t)k * bw]), u[k], s);
-    return s;
-}
-
 // MW: warps along the rows, 16 rows each; the 8 / MW warps of the same rows share the 64 outputs, 8 MW each.
 template <int MW>
 __global__ void __launch_bounds__(256, 2)

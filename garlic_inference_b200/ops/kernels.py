@@ -862,11 +862,22 @@ def conv_state_update(x: torch.Tensor, n_taps: int, state: torch.Tensor, tok_slo
                                   _bias_pair(in_bias, None, x.shape[1]), _stream()), l)
 
 
+def _gates_on_tcgen05(n: int, bw: int) -> bool:
+    """Rows and widths from which the tcgen05 kernel of the gates is the faster one.  In us, mma.sync / tcgen05, rows x blocks x channels:
+    128 x 16 x 320 28 / 26, 150 x 16 x 320 45 / 28, 256 x 8 x 320 28 / 21, 2,494 x 16 x 320 213 / 136, 128 x 40 x 128 24 / 25, 1,024 x 53 x 96 71 / 54,
+    1,024 x 80 x 64 55 / 40, 256 x 64 x 64 23 / 26, 1,024 x 160 x 32 50 / 58."""
+    return n >= (GATES_TCGEN05_ROWS if bw >= 96 else 512) and bw >= 64
+
+
+GATES_TCGEN05_ROWS = 192
+
+
 def rglru_gates(u: torch.Tensor, wa_t: torch.Tensor, wi_t: torch.Tensor, ba: torch.Tensor, bi: torch.Tensor,
-                lam: torch.Tensor, decay_scale: float):
+                lam: torch.Tensor, decay_scale: float, wa: Optional[torch.Tensor] = None, wi: Optional[torch.Tensor] = None):
     """The decay and the gated input of a real-gated linear recurrent unit from its input u float32 [n, width]:
     per block of channels r = sigmoid(Wa u + ba), i = sigmoid(Wi u + bi) with the matrices given transposed
-    ([blocks, in, out]); a = exp(-decay_scale r softplus(lam)), b = sqrt(1 - a^2) i u.  Returns (a, b) float32."""
+    ([blocks, in, out]); a = exp(-decay_scale r softplus(lam)), b = sqrt(1 - a^2) i u.  With the matrices given as [blocks, out, in]
+    beside (`wa`, `wi`, bfloat16) many rows may take another kernel, as precise but with other bits.  Returns (a, b) float32."""
     l = require_gpu()
     _dense(u, "u", torch.float32), _dense(wa_t, "wa_t"), _dense(wi_t, "wi_t", wa_t.dtype)
     n, width = u.shape
@@ -879,6 +890,13 @@ def rglru_gates(u: torch.Tensor, wa_t: torch.Tensor, wi_t: torch.Tensor, ba: tor
             raise KernelError(f"{name} has {v.numel()} elements for {width} channels")
     a = torch.empty((n, width), dtype=torch.float32, device=u.device)
     b = torch.empty((n, width), dtype=torch.float32, device=u.device)
+    if wa is not None and _gates_on_tcgen05(n, bw) and bw % 8 == 0 and u.data_ptr() % 32 == 0 and wa.data_ptr() % 16 == 0 and wi.data_ptr() % 16 == 0:
+        _dense(wa, "wa", torch.bfloat16), _dense(wi, "wi", torch.bfloat16)
+        if wa.shape != wa_t.shape or wi.shape != wa_t.shape or wa_t.dtype != torch.bfloat16:
+            raise KernelError(f"gate matrices {tuple(wa.shape)} / {tuple(wi.shape)} beside {tuple(wa_t.shape)}")
+        check(l.gi_rglru_gates_tcgen05(_ptr(u), _ptr(wa), _ptr(wi), _ptr(wa_t), _ptr(wi_t), _ptr(ba), _ptr(bi), _ptr(lam), code(ba.dtype),
+                                       float(decay_scale), _ptr(a), _ptr(b), n, width, blocks, _ptr(tcgen05_error_flag(u.device)), _stream()), l)
+        return a, b
     check(l.gi_rglru_gates(_ptr(u), _ptr(wa_t), _ptr(wi_t), code(wa_t.dtype), _ptr(ba), _ptr(bi), _ptr(lam), code(ba.dtype),
                            float(decay_scale), _ptr(a), _ptr(b), n, width, blocks, _stream()), l)
     return a, b
@@ -1358,7 +1376,7 @@ def check_bounded_waits(device) -> None:
         raise WaitRanOut(f"a tcgen05 kernel gave up a bounded wait or what it was asked for (code {code}: 11-13 product, 21-23 "
                          "prompt attention, 24 unmapped page, 25 shared memory that does not start on 1,024 bytes and nothing "
                          "written, 31-33 stream-K product, 34 a partial sum that was never announced, 41-43 decode attention, "
-                         "44 unmapped page, 61-63 experts' product, 71-74 float32 product, 81 delta rule)")
+                         "44 unmapped page, 61-63 experts' product, 71-74 float32 product, 81 delta rule, 91-94 recurrent gates)")
 
 
 def streamk_test_unanswered_flags(limit: int) -> None:

@@ -59,6 +59,7 @@ _SIGNATURES = {
     "gi_causal_conv": ([P, L, I, I, P, I, I, P, L, P, P, I, I, I, P], I),
     "gi_causal_conv_biased": ([P, L, I, I, P, I, I, P, L, P, P, I, I, I, P, P, I, P], I),
     "gi_rglru_gates": ([P, P, P, I, P, P, P, I, F, P, P, I, I, I, P], I),
+    "gi_rglru_gates_tcgen05": ([P, P, P, P, P, P, P, P, I, F, P, P, I, I, I, P, P], I),
     "gi_rglru_scan": ([P, P, P, L, I, P, I, P, L, P, P, P, L, I, I, P], I),
     "gi_gate_norm_add": ([P, L, P, L, P, I, P, I, P, P, I, I, I, F, P], I),
     "gi_xielu": ([P, L, P, I, P, I, I, I, P], I),

@@ -54,8 +54,10 @@ class RGLRU(Mixer):
         self.y_bias, self.x_bias, self.conv_bias = f32("y.b"), f32("x.b"), f32("conv.b")
         self.taps = load("conv")
         # [blocks, out, in] as stored -> [blocks, in, out]: thread o of a block reads w[k][o], a whole line per warp
-        self.wa_t = load("ra").transpose(1, 2).contiguous()
-        self.wi_t = load("ri").transpose(1, 2).contiguous()
+        wa, wi = load("ra"), load("ri")
+        self.wa_t, self.wi_t = wa.transpose(1, 2).contiguous(), wi.transpose(1, 2).contiguous()
+        # as stored too, for many rows of the bfloat16 engine (its tensor cores read a row of an output's weights)
+        self.as_stored = {"wa": wa.contiguous(), "wi": wi.contiguous()} if wa.dtype == wi.dtype == torch.bfloat16 else {}
         self.ba, self.bi, self.lam = f32("ra.b"), f32("ri.b"), f32("lam")
         self.w_o = load("o")
         self.state_floats = -(-(self.K * self.W) // 4) * 4          # S, then the last K - 1 inputs
@@ -79,7 +81,7 @@ class RGLRU(Mixer):
                                      renew_state=ctx.all_single, in_bias=self.x_bias, out_bias=self.conv_bias)
         if not ctx.all_single and self.K > 1:
             kernels.conv_state_update(conv_in, self.K, conv_state, ctx.tok_slot, in_bias=self.x_bias)
-        a, b = kernels.rglru_gates(u, self.wa_t, self.wi_t, self.ba, self.bi, self.lam, self.decay_scale)
+        a, b = kernels.rglru_gates(u, self.wa_t, self.wi_t, self.ba, self.bi, self.lam, self.decay_scale, **self.as_stored)
         return kernels.rglru_scan(a, b, proj[:, self.y_off:self.y_off + self.W], self.y_bias, cache.state,
                                   ctx.seq_spans(), ctx.tok_slot, out=out)
 

@@ -164,6 +164,41 @@ def test_recurrent_gates_beyond_the_finite_are_those_of_multiply_adds(n):
     assert float(tensor[0][n - 1, 6]) == 1.0 or n == 1                     # a gate shut by minus infinity keeps the state
 
 
+@pytest.mark.parametrize("blocks, bw", [(3, 8), (2, 64), (3, 72), (2, 320), (1, 600)])
+@pytest.mark.parametrize("n", [1, 128, 300])
+def test_recurrent_gates_of_many_rows(blocks, bw, n, monkeypatch):
+    """The tcgen05 kernel: blocks narrower than a tile of outputs, part tiles of outputs, inputs and rows; gates wide open, shut and in
+    between, inputs, weights and biases beyond the finite: no further from 64 bits than mma.sync (one part in 50 for the sample), and
+    infinities and NaN where that has them."""
+    from garlic_inference_b200.ops import kernels
+    monkeypatch.setattr(kernels, "_gates_on_tcgen05", lambda n, bw: True)
+    W = blocks * bw
+    u = rnd(n, W, seed=1, scale=2.0)
+    wa, wi = (rnd(blocks, bw, bw, seed=s, scale=bw ** -0.5, dtype=torch.bfloat16) for s in (2, 3))
+    wa_t, wi_t = wa.transpose(1, 2).contiguous(), wi.transpose(1, 2).contiguous()
+    ba, bi, lam = rnd(W, seed=4), rnd(W, seed=5), rnd(W, seed=6, scale=2.0)
+    ba[1], ba[2], bi[1], bi[2], lam[3], lam[4] = 60.0, -120.0, -120.0, 60.0, -30.0, 30.0
+    old = kernels.rglru_gates(u, wa_t, wi_t, ba, bi, lam, 8.0)
+    new = kernels.rglru_gates(u, wa_t, wi_t, ba, bi, lam, 8.0, wa=wa, wi=wi)
+    z = [torch.einsum("nbi,boi->nbo", u.double().view(n, blocks, bw), w.double()).reshape(n, W) + v.double() for w, v in ((wa, ba), (wi, bi))]
+    log_a = -8.0 * torch.sigmoid(z[0]) * torch.nn.functional.softplus(lam.double())
+    want = torch.exp(log_a), torch.sqrt(-torch.expm1(2 * log_a)) * torch.sigmoid(z[1]) * u.double()
+    # one against the other: a = exp(log a) with -log a up to 70 above atol, which magnifies the error of its gate, bw sums that may each
+    # lose 2^-24 of it: 70 sqrt(bw) 2^-24 or less, 1e-4
+    tol = dict(rtol=70 * bw ** 0.5 * 2.0 ** -24, atol=1e-30)
+    for got, other, w in zip(new, old, want):
+        assert (got.double() - w).norm() <= 1.02 * (other.double() - w).norm() + 2.0 ** -25 * w.norm()
+        torch.testing.assert_close(got, other, **tol)
+    u[0, 0], u[n // 2, W - 1], ba[5], bi[6] = math.inf, math.nan, math.inf, -math.inf
+    wa[0, 2, 3], wi[blocks - 1, 4, 1] = math.inf, -math.inf
+    wa_t, wi_t = wa.transpose(1, 2).contiguous(), wi.transpose(1, 2).contiguous()
+    old = kernels.rglru_gates(u, wa_t, wi_t, ba, bi, lam, 8.0)
+    for got, other in zip(kernels.rglru_gates(u, wa_t, wi_t, ba, bi, lam, 8.0, wa=wa, wi=wi), old):
+        assert torch.equal(got.isnan(), other.isnan()) and torch.equal(got.isinf(), other.isinf())
+        torch.testing.assert_close(got[other.isfinite()], other[other.isfinite()], **tol)
+    kernels.check_bounded_waits(DEV)
+
+
 @pytest.mark.parametrize("blocks, bw", [(80, 72), (40, 136), (160, 8)])
 def test_recurrent_gates_have_the_same_bits_in_tiles_of_every_height(blocks, bw):
     """Steps whose tiles are 16, 32, 64 and 128 rows high (`blocks` of channels enough for each), whole and part tiles."""
