@@ -244,12 +244,88 @@ extern "C" int gi_latent_norms(const void* src, long long ld, int q_off, int c_o
 // Decode steps in bfloat16: one new token per sequence, all heads of a sequence read the same cached rows.  A
 // block takes one token, up to 8 * HPW heads and one slice of the keys; it stages 32 rows at a time in shared
 // memory, where every head's scores and weighted sums read them (the exact-order kernel fetches them once per
-// head).  Warp w owns heads w HPW .. w HPW + HPW - 1 of the block's group for all keys of the slice, so the
+// head).  The slices are of one length over all sequences (ld_slice): a step's sequences are of all lengths, and its longest
+// would otherwise keep a few blocks at work when the others have left.  Warp w owns heads w HPW .. w HPW + HPW - 1 of the block's group for all keys of the slice, so the
 // running maximum and sum stay inside the warp; lane j scores key j of the 32, then the lanes turn to pairs of
 // value columns.  Scores, softmax and sums are float32.  The slices' (max, sum, weighted rows) go to `part`
-// [tokens, slices, heads, 2 + rank] and gi_latent_decode_combine merges them with the sink.
+// [blocks, heads, 2 + rank] and latent_decode_combine_kernel merges them with the sink.
 #define LD_WARPS 8
 #define LD_KEYS 32
+
+// chunks of 32 keys that token t sees, 0 for a row that is none (a recorded step's padding)
+__device__ __forceinline__ int ld_chunks(int t, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, int page_size,
+                                         int max_pages, int window, int* status) {
+    const int slot = tok_slot[t], pos = tok_pos[t];
+    if (slot < 0 || pos < 0 || pos / page_size >= max_pages) {
+        if (slot >= 0 && status) atomicExch(status, 4);
+        return 0;
+    }
+    return pos / LD_KEYS - (window > 0 ? max(0, pos - window + 1) : 0) / LD_KEYS + 1;
+}
+
+// Which token's slice, of how many, block b of `n_blocks` takes: every token's chunks are cut into the fewest slices of at most `per`
+// chunks, `per` the least that all tokens' slices are no more than the blocks.  t = -1: none.  By a whole block; warp 0 finds it.
+// With `table`, {first block, slices} of every token is written there.
+struct LdSlice { int t, split, n_splits; };
+__host__ __device__ __forceinline__ int2* ld_table(float* part, size_t floats) { return reinterpret_cast<int2*>(part + (floats + 1) / 2 * 2); }
+__device__ __forceinline__ LdSlice ld_slice(int b, int n_blocks, int n_tokens, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot,
+                                            int page_size, int max_pages, int window, int2* table, int* status, LdSlice* shared) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int total = 0, live = 0;
+        for (int t = lane; t < n_tokens; t += 32) {
+            const int c = ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, table ? status : nullptr);
+            total += c;
+            live += c > 0;
+        }
+        total = __reduce_add_sync(0xffffffffu, total);
+        live = __reduce_add_sync(0xffffffffu, live);
+        int per = max(1, (total + n_blocks - 1) / n_blocks), enough = n_blocks > live ? max(1, (total + n_blocks - live - 1) / (n_blocks - live)) : max(1, total);
+        while (per < enough) {
+            const int tried = (per + enough) / 2;
+            int n = 0;
+            for (int t = lane; t < n_tokens; t += 32) n += (ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, nullptr) + tried - 1) / tried;
+            if (__reduce_add_sync(0xffffffffu, n) <= n_blocks) enough = tried;
+            else per = tried + 1;
+        }
+        int base = 0;
+        if (lane == 0) shared->t = -1;
+        __syncwarp();
+        for (int t0 = 0; t0 < n_tokens; t0 += 32) {
+            const int t = t0 + lane;
+            const int n = t < n_tokens ? (ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, nullptr) + per - 1) / per : 0;
+            int end = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += x;
+            }
+            const int first = base + end - n;
+            if (b >= first && b < first + n) *shared = {t, b - first, n};
+            if (table && t < n_tokens) table[t] = make_int2(first, n);
+            base += __shfl_sync(0xffffffffu, end, 31);
+        }
+    }
+    __syncthreads();
+    return *shared;
+}
+
+// A block's slice, found before the kernel ahead has finished (positions and slots are nobody's output); block 0 writes the table behind
+// the slices' results.  Then: t, slot, pos, its chunks c0 .. c1 - 1, first seen key lo, its results at `my`.
+#define LD_FIND_SLICE                                                                                                            \
+    __shared__ LdSlice ld_mine;                                                                                                  \
+    gi_pdl_launch_dependents();                                                                                                  \
+    const bool ld_writes = blockIdx.x == 0 && blockIdx.y == 0;                                                                   \
+    if (ld_writes) gi_pdl_wait();                                                                                                \
+    const LdSlice ld_s = ld_slice(blockIdx.x, n_blocks, n_tokens, tok_pos, tok_slot, page_size, max_pages, window,               \
+                                  ld_writes ? ld_table(part, (size_t)n_blocks * H * stride) : nullptr, status, &ld_mine); \
+    if (!ld_writes) gi_pdl_wait();                                                                                               \
+    if (ld_s.t < 0) return;                                                                                                      \
+    const int t = ld_s.t, slot = tok_slot[t], pos = tok_pos[t], lo = window > 0 ? max(0, pos - window + 1) : 0;                  \
+    const int ld_n = pos / LD_KEYS - lo / LD_KEYS + 1;                                                                           \
+    const int c0 = lo / LD_KEYS + (int)((long long)ld_n * ld_s.split / ld_s.n_splits);                                           \
+    const int c1 = lo / LD_KEYS + (int)((long long)ld_n * (ld_s.split + 1) / ld_s.n_splits);                                     \
+    float* my = part + (size_t)blockIdx.x * H * stride;
 
 __device__ __forceinline__ float2 bf2_to_f2(uint32_t w) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
@@ -259,28 +335,18 @@ template <int HPW, int DPL2>
 __global__ void __launch_bounds__(LD_WARPS * 32)
 latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
                      const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
-                     int H, int dk, int rank, int page_size, int max_pages, int n_pool_pages, int n_splits,
+                     int H, int dk, int rank, int page_size, int max_pages, int n_pool_pages, int n_blocks, int n_tokens,
                      float scale, int* __restrict__ status, int window) {
-    gi_pdl_start();
     extern __shared__ __align__(16) unsigned char ld_smem[];
     constexpr int HG = HPW * LD_WARPS;
     float* q_s = reinterpret_cast<float*>(ld_smem);                  // HG rows of dk
     uint32_t* k_s = reinterpret_cast<uint32_t*>(q_s + HG * dk);      // 32 rows of kw words (kw odd: no bank conflicts)
     const int kw = dk / 2 + 1;
-    const int t = blockIdx.x, split = blockIdx.y, h0 = blockIdx.z * HG;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int slot = tok_slot[t], pos = tok_pos[t];
     const size_t stride = (size_t)rank + 2;
-    float* my = part + ((size_t)t * n_splits + split) * H * stride;
-    const bool dead = slot < 0 || pos < 0 || pos / page_size >= max_pages;
-    // the chunks from the one that holds the first seen key to the query's own
-    const int lo = window > 0 ? max(0, pos - window + 1) : 0, first_chunk = lo / LD_KEYS;
-    const int n_chunks = dead ? 0 : pos / LD_KEYS - first_chunk + 1;
-    const int per = (n_chunks + n_splits - 1) / n_splits;
-    const int c0 = first_chunk + split * per, c1 = min(first_chunk + n_chunks, c0 + per);
-    if (dead && slot >= 0 && threadIdx.x == 0) atomicExch(status, 4);
+    LD_FIND_SLICE
+    const int h0 = blockIdx.y * HG;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    if (c0 < c1)
         for (int i = threadIdx.x; i < HG * dk; i += blockDim.x) {
             const int hh = i / dk, c = i - hh * dk;
             q_s[i] = h0 + hh < H ? to_f32(q[((size_t)t * H + h0 + hh) * dk + c]) * scale : 0.f;
@@ -292,7 +358,7 @@ latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, 
 #pragma unroll
         for (int r = 0; r < 2 * DPL2; ++r) acc[hh][r] = 0.f;
     }
-    const int* bt = block_table + (size_t)(dead ? 0 : slot) * max_pages;
+    const int* bt = block_table + (size_t)slot * max_pages;
     const int vec_per_row = dk / 8;
     for (int c = c0; c < c1; ++c) {
         __syncthreads();
@@ -391,8 +457,7 @@ __global__ void __launch_bounds__(LD_WARPS * 32, 2)
 latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
                          const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
                          int H, int dk, int rank, int row_words, int page_size, int max_pages, int n_pool_pages,
-                         int n_splits, float scale, int* __restrict__ status, int window) {
-    gi_pdl_start();
+                         int n_blocks, int n_tokens, float scale, int* __restrict__ status, int window) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     constexpr int HG = 32, PW = 20;                                  // heads per block; words per row of weights
     const int kw = row_words;                                        // words per staged row, kw % 32 == 4
@@ -401,25 +466,11 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
     float* s_s = reinterpret_cast<float*>(k_s + LD_KEYS * kw);       // HG x 33 scores
     uint32_t* p_s = reinterpret_cast<uint32_t*>(s_s + HG * 33);      // HG rows of PW words: the weights
     float* corr_s = reinterpret_cast<float*>(p_s + HG * PW);         // HG
-    const int t = blockIdx.x, split = blockIdx.y, h0 = blockIdx.z * HG;
+    const size_t stride = (size_t)rank + 2;
+    LD_FIND_SLICE
+    const int h0 = blockIdx.y * HG;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;                          // the fragments' row group and column pair
-    const int slot = tok_slot[t], pos = tok_pos[t];
-    const size_t stride = (size_t)rank + 2;
-    float* my = part + ((size_t)t * n_splits + split) * H * stride;
-    const bool dead = slot < 0 || pos < 0 || pos / page_size >= max_pages;
-    // the chunks from the one that holds the first seen key to the query's own
-    const int lo = window > 0 ? max(0, pos - window + 1) : 0, first_chunk = lo / LD_KEYS;
-    const int n_chunks = dead ? 0 : pos / LD_KEYS - first_chunk + 1;
-    const int per = (n_chunks + n_splits - 1) / n_splits;
-    const int c0 = first_chunk + split * per, c1 = min(first_chunk + n_chunks, c0 + per);
-    if (dead && slot >= 0 && threadIdx.x == 0) atomicExch(status, 4);
-    if (c0 >= c1) {
-        // No keys in this slice: the merge reads its maximum alone, so the heads' columns of zeros are not written.  A decode
-        // step of 19 sequences of up to 24 tokens, 32 heads, 11 of 12 slices empty: 234 -> 223 us.
-        if (threadIdx.x < HG && h0 + (int)threadIdx.x < H) my[(size_t)(h0 + threadIdx.x) * stride] = -INFINITY;
-        return;
-    }
     const int vec_per_row = dk / 8, words = dk / 2;
 
     for (int idx = threadIdx.x; idx < HG * (kw / 4); idx += blockDim.x) {
@@ -439,7 +490,7 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
         for (int j = 0; j < NTW; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[mt][j][e] = 0.f;
-    const int* bt = block_table + (size_t)(dead ? 0 : slot) * max_pages;
+    const int* bt = block_table + (size_t)slot * max_pages;
     const int k_steps = (words + 7) / 8;                              // steps of 16 values; the rows' padding is zero
     const int mt_s = warp & 1, nt_s = warp >> 1;                      // this warp's tile of the scores
     const int n_tiles = (rank + 7) / 8;
@@ -567,31 +618,285 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
         }
 }
 
-__global__ void latent_decode_combine_kernel(const float* __restrict__ part, bf16* __restrict__ out, int H, int rank,
-                                             int n_splits, const void* __restrict__ sinks, int sink_dtype) {
-    gi_pdl_start();
-    const int t = blockIdx.x, h = blockIdx.y;
+// The same for rows of up to 64 KQ values, a block to an SM.  The scores of a chunk are shared out by values: a warp has a quarter of a
+// row's, both halves of the heads and one of the keys, so that the queries stay in registers and a staged row is read twice instead of
+// four times; the quarters meet in the softmax.  Copies are two chunks ahead.
+// Bound by the legacy tensor pipe (136 products a warp and chunk at 8 cycles) and the three barriers of a chunk.
+// Measured, 32 heads over rows of 576 (the merge included), us with a slice of its own length for every sequence and the kernel above /
+// with slices of one length / so: 20 sequences of 200 to 4,000 tokens 79 / 54 / 41, 1 of 2,048 37 / 35 / 25, 8 of 2,048 39 / 37 / 27, 32 of
+// 2,048 74 / 66 / 53, 64 of 200 to 4,000 156 / 121 / 112.
+#define LW_STAGES 3
+#define LW_SLD 40            // floats of a row of scores: 8 banks from head to head
+template <int KQ, int NTW>
+__global__ void __launch_bounds__(LD_WARPS * 32, 1)
+latent_decode_quarters_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
+                              const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
+                              int H, int dk, int rank, int row_words, int page_size, int max_pages, int n_pool_pages,
+                              int n_blocks, int n_tokens, float scale, int* __restrict__ status, int window) {
+    extern __shared__ __align__(16) unsigned char ld_smem[];
+    constexpr int HG = 32, PW = 20;                                  // heads per block; words per row of weights
+    const int kw = row_words;                                        // words per staged row, kw % 32 == 4
+    uint32_t* k_s = reinterpret_cast<uint32_t*>(ld_smem);            // [stage][32 rows of kw words]
+    float* s_s = reinterpret_cast<float*>(k_s + LW_STAGES * LD_KEYS * kw);       // [quarter][HG][LW_SLD]
+    uint32_t* p_s = reinterpret_cast<uint32_t*>(s_s + 4 * HG * LW_SLD);          // HG rows of PW words: the weights
+    float* corr_s = reinterpret_cast<float*>(p_s + HG * PW);         // HG
     const size_t stride = (size_t)rank + 2;
-    const float* base = part + ((size_t)t * n_splits * H + h) * stride;
-    const size_t step = (size_t)H * stride;
-    const float sink = sinks ? load_w(sinks, sink_dtype, h) : -INFINITY;
-    float M = sink;
-    for (int s = 0; s < n_splits; ++s) M = fmaxf(M, base[s * step]);
-    float L = sinks ? expf(sink - M) : 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-        const float ms = base[s * step];
-        if (ms != -INFINITY) L += expf(ms - M) * base[s * step + 1];
-    }
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-        float v = 0.f;
-        for (int s = 0; s < n_splits; ++s) {
-            const float ms = base[s * step];
-            if (ms != -INFINITY) v += expf(ms - M) * base[s * step + 2 + c];
+    LD_FIND_SLICE
+    const int h0 = blockIdx.y * HG;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, tq = lane & 3;                          // the fragments' row group and column pair
+    const int* bt = block_table + (size_t)slot * max_pages;
+    const int vec_per_row = dk / 8, k_steps = (dk + 15) / 16, per_quarter = (k_steps + 3) / 4;
+    const int quarter = warp & 3, keys = warp >> 2;                  // this warp's share of the scores: values, half of the keys
+    const int n_tiles = (rank + 7) / 8;
+    const uint32_t k_s_addr = (uint32_t)__cvta_generic_to_shared(k_s);
+    // Asynchronous 16-byte copies of a chunk's rows, four rows to a warp; keys out of sight, unmapped pages and the rows' padding are
+    // filled with zeros.  Lane r < 4 looks up where the warp's row r of the chunk after this one lies.
+    auto where = [&](int c) -> long long {                            // first element of this lane's row, or -1: zeros
+        const int key = c * LD_KEYS + warp * 4 + lane;
+        if (lane >= 4 || c >= c1 || key < lo || key > pos) return -1;
+        const int lp = key / page_size, page = bt[lp];
+        if (page < 0 || page >= n_pool_pages) { atomicExch(status, 5); return -1; }
+        return ((long long)page * page_size + (key - lp * page_size)) * dk;
+    };
+    long long next = where(c0);
+    auto stage = [&](int c) {
+        if (c < c1) {
+            const uint32_t to = k_s_addr + (uint32_t)((c - c0) % LW_STAGES * LD_KEYS + warp * 4) * kw * 4;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const long long at = __shfl_sync(0xffffffffu, next, r);
+                for (int v = lane; v < kw / 4; v += 32) {
+                    const int bytes = at >= 0 && v < vec_per_row ? 16 : 0;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(to + r * kw * 4 + v * 16), "l"(pool + (bytes ? at + v * 8 : 0)), "r"(bytes) : "memory");
+                }
+            }
+            next = where(c + 1);
         }
-        out[((size_t)t * H + h) * rank + c] = __float2bfloat16_rn(L > 0.f ? v / L : 0.f);
+        asm volatile("cp.async.commit_group;" ::: "memory");          // an empty group at the end: the count stays uniform
+    };
+    for (int c = c0; c < c0 + LW_STAGES - 1; ++c) stage(c);
+    // the queries' fragments of this warp's values, both halves of the heads
+    uint32_t qa[KQ][2][4];
+#pragma unroll
+    for (int i = 0; i < KQ; ++i)
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int h = h0 + 16 * mt + g + (e & 1) * 8, d = (quarter * per_quarter + i) * 16 + 2 * tq + (e >> 1) * 8;
+                qa[i][mt][e] = i < per_quarter && h < H && d < dk ? *reinterpret_cast<const uint32_t*>(q + ((size_t)t * H + h) * dk + d) : 0u;
+            }
+    float m[4], l[4];
+#pragma unroll
+    for (int hh = 0; hh < 4; ++hh) { m[hh] = -INFINITY; l[hh] = 0.f; }
+    float acc[2][NTW][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int j = 0; j < NTW; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[mt][j][e] = 0.f;
+
+    for (int c = c0; c < c1; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LW_STAGES - 2) : "memory");
+        __syncthreads();                                              // this chunk is there, the one before it is done with
+        stage(c + LW_STAGES - 1);
+        const uint32_t rows = k_s_addr + (uint32_t)((c - c0) % LW_STAGES * LD_KEYS) * kw * 4;
+        {
+            float sc[2][2][4] = {};                                   // [half of the heads][8 keys]
+            // lanes 0..7, 8..15: 8 keys' first and second 16 bytes of a step of 16 values; 16..31: of the next 8 keys
+            const uint32_t from = rows + ((keys * 16 + (lane >> 4) * 8 + (lane & 7)) * kw + (quarter * per_quarter) * 8 + (lane >> 3 & 1) * 4) * 4;
+#pragma unroll
+            for (int i = 0; i < KQ; ++i) {
+                if (i >= per_quarter || quarter * per_quarter + i >= k_steps) break;      // uniform over the warp
+                uint32_t b[4];
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(from + i * 32));
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    mma_bf16_16816(sc[mt][0], qa[i][mt], b[0], b[1]);
+                    mma_bf16_16816(sc[mt][1], qa[i][mt], b[2], b[3]);
+                }
+            }
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    float* to = s_s + (quarter * HG + 16 * mt + g) * LW_SLD + keys * 16 + nt * 8 + 2 * tq;
+                    *reinterpret_cast<float2*>(to) = make_float2(sc[mt][nt][0], sc[mt][nt][1]);
+                    *reinterpret_cast<float2*>(to + 8 * LW_SLD) = make_float2(sc[mt][nt][2], sc[mt][nt][3]);
+                }
+        }
+        __syncthreads();
+        // softmax of the chunk: warp w owns heads 4 w .. 4 w + 3, lane j is key j
+        {
+            const bool valid = c * LD_KEYS + lane >= lo && c * LD_KEYS + lane <= pos;
+            float sv[4], mx[4], pr[4];
+#pragma unroll
+            for (int hh = 0; hh < 4; ++hh) {
+                const float* x = s_s + (4 * warp + hh) * LW_SLD + lane;
+                const float sum = ((x[0] + x[HG * LW_SLD]) + x[2 * HG * LW_SLD]) + x[3 * HG * LW_SLD];
+                sv[hh] = valid ? sum * scale : -INFINITY;
+                mx[hh] = sv[hh];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int hh = 0; hh < 4; ++hh) mx[hh] = fmaxf(mx[hh], __shfl_xor_sync(0xffffffffu, mx[hh], o));
+#pragma unroll
+            for (int hh = 0; hh < 4; ++hh) {
+                const float m_new = fmaxf(m[hh], mx[hh]);             // every chunk holds a seen key
+                const float corr = expf(m[hh] - m_new);
+                const bf16 w = __float2bfloat16_rn(valid ? expf(sv[hh] - m_new) : 0.f);
+                pr[hh] = __bfloat162float(w);
+                l[hh] *= corr;
+                m[hh] = m_new;
+                reinterpret_cast<bf16*>(p_s + (4 * warp + hh) * PW)[lane] = w;
+                if (lane == 0) corr_s[4 * warp + hh] = corr;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int hh = 0; hh < 4; ++hh) pr[hh] += __shfl_xor_sync(0xffffffffu, pr[hh], o);
+#pragma unroll
+            for (int hh = 0; hh < 4; ++hh) l[hh] += pr[hh];
+        }
+        __syncthreads();
+        // weighted rows: this warp's NTW column tiles for both halves of the heads
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const float ca = corr_s[16 * mt + g], cb = corr_s[16 * mt + g + 8];
+#pragma unroll
+            for (int j = 0; j < NTW; ++j) { acc[mt][j][0] *= ca; acc[mt][j][1] *= ca; acc[mt][j][2] *= cb; acc[mt][j][3] *= cb; }
+        }
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            uint32_t a[2][4];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                const uint32_t* pa = p_s + (16 * mt + g) * PW + 8 * ks + tq;
+                a[mt][0] = pa[0]; a[mt][1] = pa[8 * PW]; a[mt][2] = pa[4]; a[mt][3] = pa[8 * PW + 4];
+            }
+#pragma unroll
+            for (int j = 0; j < NTW; j += 2) {
+                const int nt = warp * NTW + j;
+                if (nt >= n_tiles) continue;                          // uniform over the warp
+                // (the second tile's columns lie inside the staged row where it is one of the rank's; else its sums are not stored)
+                const uint32_t addr = rows + ((16 * ks + (lane & 15)) * kw + 4 * min(nt + (lane >> 4), n_tiles - 1)) * 4;
+                uint32_t b[4];
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(addr));
+                mma_bf16_16816(acc[0][j], a[0], b[0], b[1]);
+                mma_bf16_16816(acc[1][j], a[1], b[0], b[1]);
+                if (NTW > 1) {
+                    mma_bf16_16816(acc[0][(j + 1) % NTW], a[0], b[2], b[3]);
+                    mma_bf16_16816(acc[1][(j + 1) % NTW], a[1], b[2], b[3]);
+                }
+            }
+        }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // this slice's (max, sum) of the heads this warp owned in the softmax, and its columns of every head
+#pragma unroll
+    for (int hh = 0; hh < 4; ++hh) {
+        const int h = h0 + 4 * warp + hh;
+        if (h < H && lane == 0) { my[(size_t)h * stride] = m[hh]; my[(size_t)h * stride + 1] = l[hh]; }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) {
+            const int col = 8 * (warp * NTW + j) + 2 * tq;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int h = h0 + 16 * mt + g + half * 8;
+                if (h >= H) continue;
+                float* to = my + (size_t)h * stride + 2 + col;
+                if (col + 1 < rank && rank % 2 == 0) *reinterpret_cast<float2*>(to) = make_float2(acc[mt][j][2 * half], acc[mt][j][2 * half + 1]);
+                else {
+                    if (col < rank) to[0] = acc[mt][j][2 * half];
+                    if (col + 1 < rank) to[1] = acc[mt][j][2 * half + 1];
+                }
+            }
+        }
 }
 
+// Merges a token's slices: a block takes a head's columns, 2 NP to a thread.  table: {first block, slices} of each token.
+#define LC_THREADS 128
+template <int NP>
+__global__ void __launch_bounds__(LC_THREADS)
+latent_decode_combine_kernel(const float* __restrict__ part, const int2* __restrict__ table, bf16* __restrict__ out, int H, int rank,
+                             const void* __restrict__ sinks, int sink_dtype) {
+    gi_pdl_start();
+    __shared__ float w_s[LC_THREADS];
+    __shared__ float red[2];
+    const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, c0 = 2 * (blockIdx.z * LC_THREADS * NP + threadIdx.x);
+    const size_t stride = (size_t)rank + 2, step = (size_t)H * stride;
+    const int2 mine = table[t];
+    const float* base = part + ((size_t)mine.x * H + h) * stride;
+    const float sink = sinks ? load_w(sinks, sink_dtype, h) : -INFINITY;
+    // the maximum and the sum, by a warp; then LC_THREADS slices' weights at a time
+    if (threadIdx.x < 32) {
+        float M = sink;
+        for (int s = lane; s < mine.y; s += 32) M = fmaxf(M, base[s * step]);
+        M = warp_max(M);
+        float L = 0.f;
+        for (int s = lane; s < mine.y; s += 32) L += expf(base[s * step] - M) * base[s * step + 1];
+        L = warp_sum(L);
+        if (lane == 0) { red[0] = M; red[1] = L + (sinks ? expf(sink - M) : 0.f); }
+    }
+    __syncthreads();
+    const float M = red[0], inv = red[1] > 0.f ? 1.f / red[1] : 0.f;
+    float v[2 * NP];
+#pragma unroll
+    for (int i = 0; i < 2 * NP; ++i) v[i] = 0.f;
+    for (int s0 = 0; s0 < mine.y; s0 += LC_THREADS) {
+        const int n = min(LC_THREADS, mine.y - s0);
+        __syncthreads();
+        if ((int)threadIdx.x < n) w_s[threadIdx.x] = expf(base[(s0 + threadIdx.x) * step] - M);
+        __syncthreads();
+        const float* x = base + s0 * step + 2 + c0;
+        if (rank % 2 == 0) {                                 // rows of an even number of floats: pairs lie on 8 bytes
+#pragma unroll (NP == 1 ? 16 : 4)
+            for (int s = 0; s < n; ++s)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const float2 y = c0 + 2 * LC_THREADS * p < rank ? *reinterpret_cast<const float2*>(x + s * step + 2 * LC_THREADS * p) : make_float2(0.f, 0.f);
+                    v[2 * p] = fmaf(w_s[s], y.x, v[2 * p]);
+                    v[2 * p + 1] = fmaf(w_s[s], y.y, v[2 * p + 1]);
+                }
+        } else {
+            for (int s = 0; s < n; ++s)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const int c = c0 + 2 * LC_THREADS * p;
+                    if (c < rank) v[2 * p] = fmaf(w_s[s], x[s * step + 2 * LC_THREADS * p], v[2 * p]);
+                    if (c + 1 < rank) v[2 * p + 1] = fmaf(w_s[s], x[s * step + 2 * LC_THREADS * p + 1], v[2 * p + 1]);
+                }
+        }
+    }
+    bf16* dst = out + ((size_t)t * H + h) * rank;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const int c = c0 + 2 * LC_THREADS * p;
+        if (c < rank) dst[c] = __float2bfloat16_rn(v[2 * p] * inv);
+        if (c + 1 < rank) dst[c + 1] = __float2bfloat16_rn(v[2 * p + 1] * inv);
+    }
+}
+// A head's columns to one block, or to four where the heads are few.
+static int launch_latent_combine(const float* part, const int2* table, void* out, int n_tokens, int H, int rank, const void* sinks,
+                                 int sink_dtype, cudaStream_t s) {
+    if ((long long)n_tokens * H < 512)
+        gi_launch(latent_decode_combine_kernel<1>, dim3(n_tokens, H, (rank + 2 * LC_THREADS - 1) / (2 * LC_THREADS)), dim3(LC_THREADS), 0, s, part,
+                  table, (bf16*)out, H, rank, sinks, sink_dtype);
+    else
+        gi_launch(latent_decode_combine_kernel<2>, dim3(n_tokens, H, (rank + 4 * LC_THREADS - 1) / (4 * LC_THREADS)), dim3(LC_THREADS), 0, s, part,
+                  table, (bf16*)out, H, rank, sinks, sink_dtype);
+    return gi_check_launch("gi_latent_decode_combine");
+}
+
+// part: n_tokens n_splits H (2 + rank) floats (an even number of them), then two ints a token; n_tokens n_splits is the number of blocks (for every 32 heads).
 extern "C" int gi_latent_decode(const void* q, const void* pool, const int* block_table, const int* tok_pos,
                                 const int* tok_slot, float* part, void* out, int n_tokens, int H, int dk, int rank,
                                 int page_size, int max_pages, int n_pool_pages, int n_splits, float scale,
@@ -601,6 +906,9 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
                "gi_latent_decode: rows of %d (a multiple of 8) with %d value columns (at most 512)", dk, rank);
     GI_REQUIRE(n_splits >= 1 && n_splits <= 64 && H <= 65535 && n_tokens <= 65535, "gi_latent_decode: slices, heads, tokens");
     if (n_tokens == 0) return 0;
+    int n_blocks = n_tokens * n_splits;
+    const int2* table = ld_table(part, (size_t)n_blocks * H * (rank + 2));
+    GI_REQUIRE((uintptr_t)part % 8 == 0, "gi_latent_decode: the work space must start on 8 bytes");
     cudaStream_t s = (cudaStream_t)stream;
     {   // tensor cores: rows staged with 4 words of padding past a multiple of 32 words
         const int words16 = ((dk + 15) / 16) * 8;
@@ -608,23 +916,42 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
         const size_t smem_mma = ((size_t)(32 + LD_KEYS) * kw + 32 * 33 + 32 * 20 + 32) * 4;
         const int n_tiles = (rank + 7) / 8;
         const int NTW = n_tiles > 32 ? 8 : (n_tiles > 16 ? 4 : (n_tiles > 8 ? 2 : 1));
+        const size_t smem_q = ((size_t)LW_STAGES * LD_KEYS * kw + 4 * 32 * LW_SLD + 32 * 20 + 32) * 4;
+        if (dk <= 576) {
+            // a block to an SM, or two blocks a token where those are more
+            int n_sm = 148, dev = 0;
+            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+            const int groups = (H + 31) / 32, most = n_sm / groups > 2 * n_tokens ? n_sm / groups : 2 * n_tokens;
+            if (n_blocks > most) n_blocks = most;
+            table = ld_table(part, (size_t)n_blocks * H * (rank + 2));
+#define LDQ_CASE(Q, N)                                                                                                 \
+            if ((dk <= 192 ? 3 : 9) == Q && NTW == N) {                                                                \
+                if (int rc = gi_reserve_smem((const void*)latent_decode_quarters_kernel<Q, N>, smem_q, "gi_latent_decode")) return rc; \
+                gi_launch(latent_decode_quarters_kernel<Q, N>, dim3(n_blocks, groups), dim3(LD_WARPS * 32), smem_q, s, (const bf16*)q, \
+                          (const bf16*)pool, block_table, tok_pos, tok_slot, part, H, dk, rank, kw, page_size, max_pages, \
+                          n_pool_pages, n_blocks, n_tokens, scale, status, window);                                    \
+            }
+            LDQ_CASE(3, 1) LDQ_CASE(3, 2) LDQ_CASE(3, 4) LDQ_CASE(9, 1) LDQ_CASE(9, 2) LDQ_CASE(9, 4) LDQ_CASE(9, 8)
+#undef LDQ_CASE
+            int rc = gi_check_launch("gi_latent_decode");
+            if (rc) return rc;
+            return launch_latent_combine(part, table, out, n_tokens, H, rank, sinks, sink_dtype, s);
+        }
         if (smem_mma <= 200 * 1024) {
-            dim3 grid_mma(n_tokens, n_splits, (H + 31) / 32);
+            dim3 grid_mma(n_blocks, (H + 31) / 32);
 #define LDM_CASE(N)                                                                                                    \
             if (NTW == N) {                                                                                            \
                 int rc = gi_reserve_smem((const void*)latent_decode_mma_kernel<N>, smem_mma, "gi_latent_decode");      \
                 if (rc) return rc;                                                                                     \
                 gi_launch(latent_decode_mma_kernel<N>, grid_mma, dim3(LD_WARPS * 32), smem_mma, s, (const bf16*)q,     \
                           (const bf16*)pool, block_table, tok_pos, tok_slot, part, H, dk, rank, kw, page_size, max_pages, \
-                          n_pool_pages, n_splits, scale, status, window);                                                      \
+                          n_pool_pages, n_blocks, n_tokens, scale, status, window);                                                      \
             }
             LDM_CASE(1) LDM_CASE(2) LDM_CASE(4) LDM_CASE(8)
 #undef LDM_CASE
             int rc = gi_check_launch("gi_latent_decode");
             if (rc) return rc;
-            gi_launch(latent_decode_combine_kernel, dim3(n_tokens, H), dim3(128), 0, s, (const float*)part, (bf16*)out, H, rank,
-                      n_splits, sinks, sink_dtype);
-            return gi_check_launch("gi_latent_decode_combine");
+            return launch_latent_combine(part, table, out, n_tokens, H, rank, sinks, sink_dtype, s);
         }
     }
     const int HPW = H > 16 ? 4 : (H > 8 ? 2 : 1);
@@ -632,14 +959,14 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
     const int DPL2 = rank > 256 ? 8 : (rank > 128 ? 4 : (rank > 64 ? 2 : 1));
     const size_t smem = (size_t)HG * dk * 4 + (size_t)LD_KEYS * (dk / 2 + 1) * 4;
     GI_REQUIRE(smem <= 220 * 1024, "gi_latent_decode: rows of %d need %zu bytes of shared memory", dk, smem);
-    dim3 grid(n_tokens, n_splits, (H + HG - 1) / HG);
+    dim3 grid(n_blocks, (H + HG - 1) / HG);
 #define LD_CASE(A, B)                                                                                             \
     if (HPW == A && DPL2 == B) {                                                                                  \
         int rc = gi_reserve_smem((const void*)latent_decode_kernel<A, B>, smem, "gi_latent_decode");              \
         if (rc) return rc;                                                                                        \
         gi_launch(latent_decode_kernel<A, B>, grid, dim3(LD_WARPS * 32), smem, s, (const bf16*)q, (const bf16*)pool, \
-                  block_table, tok_pos, tok_slot, part, H, dk, rank, page_size, max_pages, n_pool_pages, n_splits, \
-                  scale, status, window);                                                                                 \
+                  block_table, tok_pos, tok_slot, part, H, dk, rank, page_size, max_pages, n_pool_pages, n_blocks, \
+                  n_tokens, scale, status, window);                                                                                 \
     }
     LD_CASE(1, 1) LD_CASE(1, 2) LD_CASE(1, 4) LD_CASE(1, 8)
     LD_CASE(2, 1) LD_CASE(2, 2) LD_CASE(2, 4) LD_CASE(2, 8)
@@ -647,7 +974,5 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
 #undef LD_CASE
     int rc = gi_check_launch("gi_latent_decode");
     if (rc) return rc;
-    gi_launch(latent_decode_combine_kernel, dim3(n_tokens, H), dim3(128), 0, s, (const float*)part, (bf16*)out, H, rank,
-              n_splits, sinks, sink_dtype);
-    return gi_check_launch("gi_latent_decode_combine");
+    return launch_latent_combine(part, table, out, n_tokens, H, rank, sinks, sink_dtype, s);
 }

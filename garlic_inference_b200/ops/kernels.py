@@ -1111,14 +1111,21 @@ def latent_decode_takes(dtype: torch.dtype, row: int, rank: int, heads: int) -> 
 
 
 def latent_decode_slices(n: int, heads: int) -> int:
-    """Slices of the keys for a step of n rows: about 320 blocks in all (two to an SM and some to even out sequences of
+    """Slices of the keys for a step of n rows over rows of more than 576 values: about 320 blocks in all (two to an SM and some to even out sequences of
     different lengths), 256 from 33 blocks of queries on, at most 16 slices.  A recorded step's rows are a power of two, so at up
     to 32 heads the first number matters at 32 rows, where sequences number 17 to 32.  Measured there at 32 heads over rows of
-    576, us at 8 / 10 / 12 slices: 17 sequences of 2,048 tokens 68 / 61 / 57, 24 69 / 62 / 58, 28 69 / 63 / 79, 32 72 / 74 / 86,
+    576 with slices of a length of their own for every sequence, us at 8 / 10 / 12 slices: 17 sequences of 2,048 tokens 68 / 61 / 57, 24 69 / 62 / 58, 28 69 / 63 / 79, 32 72 / 74 / 86,
     32 of 500 33 / 36 / 36; of 200 to 4,000 tokens 17 93 / 79 / 76, 20 93 / 79 / 76, 32 98 / 89 / 97.  1 sequence of 2,048 tokens
     at 4 / 8 / 16 slices 70 / 46 / 37, 8 sequences 71 / 47 / 39; 64 115 / 135 / 143, of 200 to 4,000 174 / 156 / 163."""
     blocks = n * -(-heads // 32)
     return max(1, min(16, (320 if blocks <= 32 else 256) // max(1, blocks)))
+
+
+def latent_decode_slices_short(n: int, heads: int) -> int:
+    """The same for rows of up to 576, whose kernel has an SM to itself and cuts all sequences' keys into slices of one length:
+    a block of up to 32 heads to an SM.  In us at 32 heads over rows of 576 and 3 / 4 / 5 slices: 20 sequences of 200 to 4,000 tokens in a
+    step of 32 rows 54 / 45 / 41; 1 sequence of 2,048 at 16 / 32 / 64 21 / 19 / 20."""
+    return max(2, min(32, -(-148 // max(1, n * -(-heads // 32)))))
 
 
 def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor, tok_pos: torch.Tensor,
@@ -1136,8 +1143,8 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor
     if one != 1 or pool_row != row:
         raise KernelError(f"a pool {tuple(pool.shape)} does not hold rows of {row} shared by all heads")
     if n_splits is None:
-        n_splits = latent_decode_slices(n, heads)
-    part = torch.empty((n, n_splits, heads, rank + 2), dtype=torch.float32, device=q.device)
+        n_splits = (latent_decode_slices_short if row <= 576 else latent_decode_slices)(n, heads)
+    part = torch.empty(-(-n * n_splits * heads * (rank + 2) // 2) * 2 + 2 * n, dtype=torch.float32, device=q.device)
     out = torch.empty((n, heads * rank), dtype=torch.bfloat16, device=q.device)
     check(l.gi_latent_decode(_ptr(q), _ptr(pool), _ptr(block_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(part),
                              _ptr(out), n, heads, row, rank, page_size, block_table.shape[1], n_pages, n_splits,

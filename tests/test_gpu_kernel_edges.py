@@ -974,6 +974,34 @@ def test_queries_keys_and_values_of_long_steps_have_the_bits_of_short_ones(dtype
 
 
 # ---- one token per sequence over latent rows ---------------------------------------------------------------------------
+@pytest.mark.parametrize("row, rank, heads", [(576, 512, 32), (200, 192, 17), (72, 65, 40), (64, 33, 1), (584, 512, 20)])
+@pytest.mark.parametrize("pos, n_splits", [([0], None), ([31, 32, 700, -1, 5, 63], None), ([300] * 40 + [-1], 2), ([2000, 3], 1)])
+def test_latent_decode_with_slices_of_one_length(row, rank, heads, pos, n_splits):
+    """Rows on both sides of the limits between the kernels, odd ranks, rows without a sequence between others, more slices than chunks and
+    as many blocks as sequences, with a sink and with a window: against 64 bits."""
+    from garlic_inference_b200.ops import kernels
+    page, n, scale = 32, len(pos), 0.1
+    per = max(pos) // page + 1
+    table = torch.arange(n * per, dtype=torch.int32, device=DEV).view(n, per).flip(0).contiguous()
+    q, pool = rnd(n, heads, row, seed=1, dtype=torch.bfloat16), rnd(n * per, 1, page, row, seed=2, dtype=torch.bfloat16)
+    slot = torch.tensor([i if p >= 0 else -1 for i, p in enumerate(pos)], dtype=torch.int32, device=DEV)
+    at = torch.tensor([max(p, 0) for p in pos], dtype=torch.int32, device=DEV)
+    status, sinks = torch.zeros(1, dtype=torch.int32, device=DEV), rnd(heads, seed=3)
+    for sink, window in ((None, 0), (sinks, 0), (None, 33)):
+        got = kernels.latent_decode(q, pool, table, at, slot, scale, sink, rank, status, n_splits=n_splits, window=window).view(n, heads, rank).double()
+        assert status.item() == 0
+        for t, p in list(enumerate(pos))[::7] + [(n - 1, pos[-1])]:
+            if p < 0:
+                assert not got[t].any()
+                continue
+            keys = pool[table[t].long()].reshape(per * page, row)[max(0, p - window + 1) if window else 0:p + 1].double()
+            s = q[t].double() @ keys.T * scale
+            w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), -1)[:, :-1] if sink is not None else torch.softmax(s, -1)
+            # the weights, their sum with them and the result are rounded to bfloat16, 2^-9 of each; the rest is float32
+            bound = 1.05 * 3 * 2 ** -9 * (w @ keys[:, :rank].abs()) + 1e-5
+            assert ((got[t] - w @ keys[:, :rank]).abs() <= bound).all(), (t, p)
+
+
 @pytest.mark.parametrize("heads", [17, 33])
 @pytest.mark.parametrize("n_splits, window", [(1, 0), (2, 0), (16, 0), (16, 40)])
 def test_latent_decode_with_slices_that_hold_no_keys(heads, n_splits, window):
