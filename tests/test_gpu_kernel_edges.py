@@ -973,6 +973,44 @@ def test_queries_keys_and_values_of_long_steps_have_the_bits_of_short_ones(dtype
     assert int(status.item()) == 0
 
 
+# ---- float32 attention of many tokens --------------------------------------------------------------------------------------
+@pytest.mark.parametrize("H, G, d, dv", [(8, 2, 128, 128), (6, 3, 64, 64), (3, 3, 72, 40), (16, 2, 100, 100), (4, 2, 128, 65)])
+@pytest.mark.parametrize("page, lens", [(16, [301]), (64, [133, 1, 170, 2, 3]), (32, [5, 228, 61])])
+@pytest.mark.parametrize("sink", [False, True])
+def test_float32_attention_of_rows_that_share_their_fetches(H, G, d, dv, page, lens, sink):
+    """Several heads and tokens to a block, sequences that end inside one, some behind cached tokens, rows without a sequence, a page that is
+    not mapped: the bits of fewer tokens at a time, which a block a row takes; and 64 bits."""
+    from garlic_inference_b200.ops import kernels
+    past = [0, 100, 3, 40, 0][:len(lens)]
+    per = max(p + n for p, n in zip(past, lens)) // page + 1
+    table = torch.arange(len(lens) * per, dtype=torch.int32, device=DEV).view(len(lens), per).flip(0).contiguous()
+    kp, vp = rnd(len(lens) * per, G, page, d, seed=1), rnd(len(lens) * per, G, page, d, seed=2)
+    kp[table[0, 0].item(), 0, 1, 0] = 1e30                       # a row far above the others
+    pos = torch.cat([torch.arange(p, p + n) for p, n in zip(past, lens)] + [torch.zeros(3)]).to(torch.int32).to(DEV)
+    slot = torch.cat([torch.full((n,), i) for i, n in enumerate(lens)] + [torch.full((3,), -1)]).to(torch.int32).to(DEV)
+    n = pos.numel()
+    q, sinks = rnd(n, H, d, seed=3), rnd(H, seed=4) if sink else None
+    run = lambda a, b, t, status: kernels.attention_generic(q[a:b].contiguous(), kp, vp, t, pos[a:b].contiguous(), slot[a:b].contiguous(),
+                                                            d ** -0.5, 0, status, sinks=sinks, value_dim=dv)
+    for t in (table, table.clone()):
+        if t is not table:
+            t[0, (past[0] + lens[0] - 1) // page] = -1           # the last page of the first sequence
+        status = torch.zeros(2, dtype=torch.int32, device=DEV)
+        got = run(0, n, t, status[:1])
+        want = torch.cat([run(a, min(n, a + 18), t, status[1:]) for a in range(0, n, 18)])
+        assert torch.equal(got, want) and int(status[0]) == int(status[1]) == (0 if t is table else 5)
+    got = run(0, n, table, torch.zeros(1, dtype=torch.int32, device=DEV)).view(n, H, dv)
+    assert not got[n - 3:].any()
+    for i in range(1, len(lens)):
+        for at in {sum(lens[:i]), sum(lens[:i + 1]) - 1}:
+            keys, vals = (x[table[i].long()].permute(1, 0, 2, 3).reshape(G, per * page, d)[:, :int(pos[at]) + 1].double() for x in (kp, vp))
+            s = torch.einsum("ghd,gkd->ghk", q[at].view(G, H // G, d).double(), keys) * d ** -0.5
+            if sink:
+                s = torch.cat([s, sinks.double().view(G, H // G, 1)], -1)
+            w = torch.softmax(s, -1)[..., :keys.shape[1]]
+            torch.testing.assert_close(got[at].view(G, H // G, dv).double(), torch.einsum("ghk,gkd->ghd", w, vals[..., :dv]), rtol=1e-5, atol=1e-5)
+
+
 # ---- one token per sequence over latent rows ---------------------------------------------------------------------------
 @pytest.mark.parametrize("row, rank, heads", [(576, 512, 32), (200, 192, 17), (72, 65, 40), (64, 33, 1), (584, 512, 20)])
 @pytest.mark.parametrize("pos, n_splits", [([0], None), ([31, 32, 700, -1, 5, 63], None), ([300] * 40 + [-1], 2), ([2000, 3], 1)])
