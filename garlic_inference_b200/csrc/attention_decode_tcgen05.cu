@@ -1,7 +1,7 @@
 // bfloat16 attention for decode steps on the fifth-generation tensor cores: head_dim 128, cache pages that
 // are a multiple of 64 tokens, at most 16 query heads per key/value head.
 //
-// One CTA takes one sequence, one key/value head and one slice of that sequence's keys.  The query heads
+// One CTA takes one sequence, one key/value head and one slice of that sequence's keys (the slices: fd_find_slice).  The query heads
 // that share the key/value head are the rows of one 128-row operand (rows beyond the group hold whatever
 // shared memory held: every output row depends on its own row alone, and those rows are never stored):
 //   warp 0, one lane:  TMA.  The group's queries once (16 rows); per 64 keys the keys and the values of the
@@ -40,6 +40,8 @@
 #define FD_COL_S 0
 #define FD_COL_O 128
 #define FD_LAZY 8.f
+#define FD_SLICED 64                           // sequences whose slices are of one length: two a lane
+#define FD_AT_ONCE 296                         // CTAs that the chip holds
 #define FD_SPIN_LIMIT (1 << 22)
 
 #define FD_ERR_PRODUCER 41
@@ -137,13 +139,97 @@ __device__ __forceinline__ void fd_st32(uint32_t taddr, const uint32_t (&u)[32])
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// grid (slices, key/value heads, sequences)
+__device__ __forceinline__ int fd_ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// Which sequence's slice, of how many, place `place` of `n_places` takes, by warp 0.  A step's sequences are of all lengths, and a
+// recorded step has rows that are none: with as many slices for each the longest sequence keeps a few CTAs at work when the others have
+// left.  Every sequence's tiles are cut into the fewest slices of at most `per` tiles, `per` the least with which all slices have a place
+// (n_seqs <= n_places).  Sequences of one length get what an even division gives them.  Without `cut` every sequence, rows that are none too,
+// has one place.  With `sorted` the longest slices come first: CTAs start in grid order, and a long one that starts last leaves the other
+// SMs idle.  A microsecond before the wait for the step's other kernels, beside the tensor memory's allocation.
+// Measured on a B200 (standalone, 8 key/value heads, lengths spread over 5 to 100 %; as many slices of each, in the order given -> here):
+// 5 sequences up to 6,000 in a step of 8 rows 30 -> 22 us, 10 in 16 52 -> 34; 20 up to 4,000 in 32 63 -> 41, 48 in 64 (sorted) 89 -> 76;
+// 64 up to 2,900 87 -> 67.  Even lengths: 64 of 2,048 85 -> 87, 32 of 3,000 64 -> 66, 8 of 3,000 22 -> 24 (in a recorded step of 8 the same).
+// first[i], count[i]: first place and slices (0: a row that is none) of
+// sequence seq[i], for i = 0, 1.
+struct FdSlice { int b, split, n_splits; };
+__device__ __forceinline__ void fd_find_slice(int place, int n_places, bool cut, bool sorted, int n_seqs, const int* __restrict__ tok_pos,
+                                              const int* __restrict__ tok_slot, int window, int2* order, FdSlice* found, int (&seq)[2],
+                                              int (&first)[2], int (&count)[2]) {
+    const int lane = threadIdx.x;
+    int tiles[2], n[2], key[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int b = min(i * 32 + lane, n_seqs - 1), pos = tok_pos[b];
+        const bool none = i * 32 + lane >= n_seqs || tok_slot[b] < 0 || pos < 0;
+        tiles[i] = none ? 0 : pos / FD_BN - (window > 0 ? max(0, pos + 1 - window) : 0) / FD_BN + 1;
+        n[i] = i * 32 + lane < n_seqs;
+        key[i] = tiles[i];
+    }
+    const int most = max(1, __reduce_max_sync(0xffffffffu, max(tiles[0], tiles[1])));
+    if (cut) {
+        const int total = __reduce_add_sync(0xffffffffu, tiles[0] + tiles[1]);
+        const int live = __popc(__ballot_sync(0xffffffffu, tiles[0] > 0)) + __popc(__ballot_sync(0xffffffffu, tiles[1] > 0));
+        // between the places' average and what does for as many slices of each as there are places for
+        const int each = n_places / max(1, live);
+        int enough = (most + each - 1) / each, per = min(enough, max(1, (total + n_places - 1) / n_places));
+        while (per < enough) {
+            const int tried = (per + enough) / 2;
+            if (__reduce_add_sync(0xffffffffu, fd_ceil_div(tiles[0], tried) + fd_ceil_div(tiles[1], tried)) <= n_places) enough = tried;
+            else per = tried + 1;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            n[i] = per >= most ? tiles[i] > 0 : fd_ceil_div(tiles[i], per);
+            key[i] = n[i] > 1 ? fd_ceil_div(tiles[i], n[i]) : tiles[i];
+        }
+    }
+    int rank[2] = {lane, 32 + lane};
+    if (sorted) {
+        // distinct keys: equal lengths by number, ranks of those beyond n_seqs last
+#pragma unroll
+        for (int i = 0; i < 2; ++i) key[i] = min(key[i], 1 << 24) * 64 + 63 - (i * 32 + lane);
+        int* keys = reinterpret_cast<int*>(order);
+        keys[lane] = key[0];
+        keys[32 + lane] = key[1];
+        __syncwarp();
+        rank[0] = rank[1] = 0;
+#pragma unroll
+        for (int j = 0; j < FD_SLICED; j += 4) {
+            const int4 k = *reinterpret_cast<const int4*>(keys + j);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) rank[i] += (k.x > key[i]) + (k.y > key[i]) + (k.z > key[i]) + (k.w > key[i]);
+        }
+        __syncwarp();
+    }
+    order[rank[0]] = make_int2(lane, n[0]);
+    order[rank[1]] = make_int2(32 + lane, n[1]);
+    if (lane == 0) found->b = -1;
+    __syncwarp();
+    const int4 o = reinterpret_cast<const int4*>(order)[lane];
+    int end = o.y + o.w;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += x;
+    }
+    seq[0] = o.x; seq[1] = o.z;
+    count[0] = o.y; count[1] = o.w;
+    first[0] = end - o.y - o.w; first[1] = end - o.w;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        if (place >= first[i] && place < first[i] + count[i]) *found = {seq[i], place - first[i], count[i]};
+}
+
+// grid (slices, key/value heads, sequences); with `sorted` or `table` (n_seqs <= FD_SLICED) one slice in x and places in z.  sorted: the longest
+// first.  table: slices of one length over all sequences; the partial results lie by place, and {first place, slices} of every sequence is
+// written to the table.
 __global__ void __launch_bounds__(FD_THREADS, 2)
 decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                       const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part_o,
                       float* __restrict__ part_ml, bf16* __restrict__ out, int n_q, int n_kv, int page_size, int max_pages, int n_pool_pages,
-                      int window, float scale_log2, int n_splits, int* __restrict__ error_flag) {
+                      int window, float scale_log2, int n_splits, int n_seqs, int sorted, int2* __restrict__ table, int* __restrict__ error_flag) {
     gi_pdl_launch_dependents();
     extern __shared__ unsigned char fd_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)fd_raw + 1023) & ~(uintptr_t)1023);
@@ -152,32 +238,10 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     unsigned char* v_tiles = k_tiles + FD_STAGES * FD_KV_BYTES;
     FdControl* ctl = reinterpret_cast<FdControl*>(v_tiles + FD_STAGES * FD_KV_BYTES);
 
-    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    const int kvh = blockIdx.y;
     const int grp = n_q / n_kv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // positions and slots are set before the step's first kernel: read before the wait below
-    const int slot = tok_slot[b], pos = tok_pos[b];
-    const int kv_len = pos + 1;
-    const int lo = window > 0 ? max(0, kv_len - window) : 0;
-    const int kt_lo = lo / FD_BN;
-    const int nt_all = slot < 0 ? 0 : (kv_len - kt_lo * FD_BN + FD_BN - 1) / FD_BN;
-    const int per = (nt_all + n_splits - 1) / n_splits;
-    const int t0 = split * per, n_tiles = max(0, min(nt_all, t0 + per) - t0);
-    const size_t row_base = (size_t)b * n_q + (size_t)kvh * grp;         // the group's first row of q and of the partials
-    volatile int* abort = &ctl->abort;
-
-    if (n_tiles == 0) {                                                  // nothing for this slice: an empty partial
-        gi_pdl_wait();
-        if (n_splits == 1) {                                             // no slices: the output itself, zeros
-            for (int i = threadIdx.x; i < grp * FD_D; i += FD_THREADS) out[row_base * FD_D + i] = __float2bfloat16_rn(0.f);
-        } else if (threadIdx.x < grp) {
-            float* ml = part_ml + ((row_base + threadIdx.x) * n_splits + split) * 2;
-            ml[0] = -INFINITY;
-            ml[1] = 0.f;
-        }
-        return;
-    }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 128) {
         fd_mbar_init(&ctl->q_full, 1);
         for (int s = 0; s < FD_STAGES; ++s) {
             fd_mbar_init(&ctl->k_full[s], 1); fd_mbar_init(&ctl->k_empty[s], 1);
@@ -193,11 +257,64 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                      ::"r"(fd_smem(&ctl->tmem_base)), "r"(FD_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // positions and slots are set before the step's first kernel: read before the wait below
+    int split = blockIdx.x, b = blockIdx.z;
+    const bool writes_table = table && blockIdx.z == 0 && kvh == 0 && warp == 0;
+    int seq[2], first[2], count[2];
+    __shared__ alignas(16) int2 order[FD_SLICED];
+    __shared__ FdSlice found;
+    if ((sorted || table) && warp == 0)
+        fd_find_slice(blockIdx.z, gridDim.z, table != nullptr, sorted, n_seqs, tok_pos, tok_slot, window, order, &found, seq, first, count);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctl->tmem_base;
+    if (sorted || table) {
+        b = found.b;
+        split = found.split;
+        n_splits = found.n_splits;
+    }
+    auto free_tmem = [&] {
+        if (warp == 1)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FD_TMEM_COLS) : "memory");
+    };
+    auto write_table = [&] {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (seq[i] < n_seqs) table[seq[i]] = make_int2(first[i], count[i]);
+    };
+    if (b < 0) {                                 // a place that no slice needs
+        gi_pdl_wait();
+        if (writes_table) write_table();
+        free_tmem();
+        return;
+    }
+    const int slot = tok_slot[b], pos = tok_pos[b];
+    const int kv_len = pos + 1;
+    const int lo = window > 0 ? max(0, kv_len - window) : 0;
+    const int kt_lo = lo / FD_BN;
+    const int nt_all = slot < 0 ? 0 : (kv_len - kt_lo * FD_BN + FD_BN - 1) / FD_BN;
+    const int per = (nt_all + n_splits - 1) / n_splits;
+    const int t0 = split * per, n_tiles = max(0, min(nt_all, t0 + per) - t0);
+    const size_t row_base = (size_t)b * n_q + (size_t)kvh * grp;         // the group's first row of q
+    // the partial result of the group's head r: part_base + r * part_step
+    const size_t part_base = table ? (size_t)blockIdx.z * n_q + (size_t)kvh * grp : row_base * n_splits + split;
+    const size_t part_step = table ? 1 : n_splits;
+    volatile int* abort = &ctl->abort;
 
+    if (n_tiles == 0) {                                                  // nothing for this slice: an empty partial
+        gi_pdl_wait();
+        if (n_splits == 1) {                                             // no slices: the output itself, zeros
+            for (int i = threadIdx.x; i < grp * FD_D; i += FD_THREADS) out[row_base * FD_D + i] = __float2bfloat16_rn(0.f);
+        } else if (threadIdx.x < grp) {
+            float* ml = part_ml + (part_base + threadIdx.x * part_step) * 2;
+            ml[0] = -INFINITY;
+            ml[1] = 0.f;
+        }
+        if (writes_table) write_table();
+        free_tmem();
+        return;
+    }
     // the lane that issues the copies
     const int* bt_row = block_table + (size_t)slot * max_pages;
     auto tile_row = [&](int it) {
@@ -232,6 +349,7 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         while (copies_ok && next_v < min(n_tiles, FD_STAGES) && settled(next_v)) copies_ok = load(next_v++, false);
     }
     gi_pdl_wait();                               // q and the newest key come from the kernel before this one
+    if (writes_table) write_table();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -367,7 +485,7 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (!ok && !*abort) { *abort = 1; atomicExch(error_flag, FD_ERR_SOFTMAX); }
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float* dst = part_o + ((row_base + r) * n_splits + split) * FD_D;
+            float* dst = part_o + (part_base + r * part_step) * FD_D;
             bf16* whole = out + (row_base + r) * FD_D;                   // without slices the output is written here
             const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
@@ -393,7 +511,7 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
             }
             if (mine && n_splits > 1) {
-                float* ml = part_ml + ((row_base + r) * n_splits + split) * 2;
+                float* ml = part_ml + (part_base + r * part_step) * 2;
                 ml[0] = l > 0.f ? ref : -INFINITY;       // a slice in which this row saw no key counts as empty
                 ml[1] = l;
             }
@@ -401,10 +519,53 @@ decode_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FD_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    free_tmem();
+}
+
+// Merges slices of one length: a warp to a (sequence, query head), four columns a lane.  A sequence in one slice has its result already; a
+// row that is none gets zeros.
+#define FC_WARPS 4
+__global__ void __launch_bounds__(FC_WARPS * 32)
+decode_combine_slices_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int2* __restrict__ table,
+                             bf16* __restrict__ out, int n_q) {
+    gi_pdl_start();
+    const int lane = threadIdx.x & 31, head = blockIdx.x * FC_WARPS + (threadIdx.x >> 5), b = blockIdx.y;
+    const int2 places = table[b];
+    if (head >= n_q || places.y == 1) return;
+    const size_t row0 = (size_t)places.x * n_q + head;
+    const float2* ml = reinterpret_cast<const float2*>(part_ml);
+    float M = -INFINITY, L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = 0; s0 < places.y; s0 += 4) {
+        float2 v[4];
+        float4 o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {            // all fetches before the first use
+            const size_t row = row0 + (size_t)min(s0 + i, places.y - 1) * n_q;
+            v[i] = ml[row];
+            o[i] = *reinterpret_cast<const float4*>(part_o + row * FD_D + lane * 4);
+        }
+        float m = M;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (s0 + i < places.y) m = fmaxf(m, v[i].x);
+        const float turn = M == -INFINITY ? 0.f : exp2f(M - m);
+        M = m;
+        L *= turn;
+        for (int c = 0; c < 4; ++c) acc[c] *= turn;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (s0 + i >= places.y || v[i].x == -INFINITY) continue;     // a slice in which this row saw no key
+            const float f = exp2f(v[i].x - M);
+            L += f * v[i].y;
+            acc[0] += f * o[i].x; acc[1] += f * o[i].y; acc[2] += f * o[i].z; acc[3] += f * o[i].w;
+        }
     }
+    uint2 v;
+    __nv_bfloat162 p0 = __floats2bfloat162_rn(L > 0.f ? acc[0] / L : 0.f, L > 0.f ? acc[1] / L : 0.f);
+    __nv_bfloat162 p1 = __floats2bfloat162_rn(L > 0.f ? acc[2] / L : 0.f, L > 0.f ? acc[3] / L : 0.f);
+    v.x = *reinterpret_cast<uint32_t*>(&p0); v.y = *reinterpret_cast<uint32_t*>(&p1);
+    *reinterpret_cast<uint2*>(out + ((size_t)b * n_q + head) * FD_D + lane * 4) = v;
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -441,11 +602,13 @@ static int fd_make_map(CUtensorMap* map, const void* base, long long rows, long 
 // The slices' partial results: part_o float32 [n_seqs * n_q * n_splits * 128] (unnormalised), part_ml float32
 // [n_seqs * n_q * n_splits * 2] (reference in powers of two, sum); gi_attention_decode_combine merges them.
 // With n_splits == 1 the kernel writes out [n_seqs, n_q * 128] bfloat16 itself and the scratch is not touched.
+// With n_places > 0 (at most FD_SLICED sequences, n_places >= n_seqs) the sequences are cut into slices of one length, at most n_places in all,
+// and merged here: part_o is [n_places * n_q * 128], part_ml [n_places * n_q * 2] with two ints for every sequence behind it; n_splits is 1.
 // Takes head_dim 128, page sizes that are a multiple of 64 and groups of at most 16 query heads.
 extern "C" int gi_attention_decode_tcgen05(const void* q, const void* k_pool, const void* v_pool, const int* block_table,
                                            const int* tok_pos, const int* tok_slot, float* part_o, float* part_ml,
                                            void* out, int n_seqs, int n_q, int n_kv, int d, int page_size, int max_pages,
-                                           int n_pool_pages, int window, float scale, int n_splits, int* error_flag,
+                                           int n_pool_pages, int window, float scale, int n_splits, int n_places, int* error_flag,
                                            void* stream) {
     GI_REQUIRE(d == FD_D, "gi_attention_decode_tcgen05: head_dim %d; this kernel takes 128", d);
     GI_REQUIRE(page_size > 0 && page_size % FD_BN == 0, "gi_attention_decode_tcgen05: page size %d is no multiple of 64", page_size);
@@ -456,7 +619,9 @@ extern "C" int gi_attention_decode_tcgen05(const void* q, const void* k_pool, co
     GI_REQUIRE(error_flag != nullptr, "gi_attention_decode_tcgen05: an error flag on the device is required");
     GI_REQUIRE(((uintptr_t)q % 16 == 0) && ((uintptr_t)k_pool % 16 == 0) && ((uintptr_t)v_pool % 16 == 0) &&
                ((uintptr_t)part_o % 16 == 0) && ((uintptr_t)out % 16 == 0), "gi_attention_decode_tcgen05: operands must start on 16 bytes");
-    GI_REQUIRE(out != nullptr && (n_splits == 1 || (part_o != nullptr && part_ml != nullptr)), "gi_attention_decode_tcgen05: buffers");
+    GI_REQUIRE(n_places == 0 || (n_places >= n_seqs && n_places <= 65535 && n_seqs <= FD_SLICED && n_splits == 1 && (uintptr_t)part_ml % 8 == 0),
+               "gi_attention_decode_tcgen05: %d places for %d sequences", n_places, n_seqs);
+    GI_REQUIRE(out != nullptr && ((n_splits == 1 && n_places == 0) || (part_o != nullptr && part_ml != nullptr)), "gi_attention_decode_tcgen05: buffers");
     if (n_seqs == 0) return 0;
     CUtensorMap map_q, map_k, map_v;
     if (int rc = fd_make_map(&map_q, q, (long long)n_seqs * n_q, d, FD_QROWS)) return rc;
@@ -465,8 +630,15 @@ extern "C" int gi_attention_decode_tcgen05(const void* q, const void* k_pool, co
     if (int rc = fd_make_map(&map_v, v_pool, pool_rows, d, FD_BN)) return rc;
     const size_t smem = (size_t)FD_Q_BYTES + 2 * FD_STAGES * FD_KV_BYTES + sizeof(FdControl) + 1024;
     if (int rc = gi_reserve_smem((const void*)decode_tcgen05_kernel, smem, "gi_attention_decode_tcgen05")) return rc;
-    gi_launch(decode_tcgen05_kernel, dim3(n_splits, n_kv, n_seqs), dim3(FD_THREADS), smem, (cudaStream_t)stream, map_q, map_k,
+    // The longest first, where the chip does not hold all CTAs at once
+    const int sorted = n_seqs >= 2 && n_seqs <= FD_SLICED && n_splits == 1 && (n_places ? n_places : n_seqs) * n_kv > FD_AT_ONCE;
+    int2* table = n_places ? reinterpret_cast<int2*>(part_ml + (size_t)n_places * n_q * 2) : nullptr;
+    gi_launch(decode_tcgen05_kernel, dim3(n_splits, n_kv, n_places ? n_places : n_seqs), dim3(FD_THREADS), smem, (cudaStream_t)stream, map_q, map_k,
               map_v, block_table, tok_pos, tok_slot, part_o, part_ml, (bf16*)out, n_q, n_kv, page_size, max_pages, n_pool_pages, window,
-              scale * 1.4426950408889634f, n_splits, error_flag);
+              scale * 1.4426950408889634f, n_splits, n_seqs, sorted, table, error_flag);
+    if (int rc = gi_check_launch("gi_attention_decode_tcgen05")) return rc;
+    if (n_places)
+        gi_launch(decode_combine_slices_kernel, dim3((n_q + FC_WARPS - 1) / FC_WARPS, n_seqs), dim3(FC_WARPS * 32), 0, (cudaStream_t)stream,
+                  part_o, part_ml, table, (bf16*)out, n_q);
     return gi_check_launch("gi_attention_decode_tcgen05");
 }

@@ -1668,8 +1668,17 @@ def decode_splits_tcgen05(n_seqs: int, n_kv: int) -> int:
     """Slices of the keys per (sequence, key/value head) in the tcgen05 decode kernel.  Measured on a B200 at
     2,048 and 4,096 cached tokens (8 key/value heads): about 256 CTAs at small batches (16 slices at batch 1,
     4 at batch 8, 2 at batch 16) and no slicing from 256 (sequence, head) pairs on (batch 64: 86 us whole
-    against 93 us in two slices).  Fixed per batch size: a recorded step is replayed while the sequences grow."""
+    against 93 us in two slices).  For steps that `decode_places_tcgen05` leaves to it.  Fixed per batch size: a recorded step is replayed while the sequences grow."""
     return max(1, min(16, -(-256 // max(1, n_seqs * n_kv))))
+
+
+def decode_places_tcgen05(n_seqs: int, n_kv: int) -> int:
+    """Places for slices of one length over all sequences of a step in the tcgen05 decode kernel, 0: as many slices of each
+    (`decode_splits_tcgen05`).  The lengths are known on the device alone, the places are fixed per batch size.  As many CTAs as a B200
+    holds at once (296): 20 sequences of up to 4,000 tokens in a step of 32 rows, 8 heads: 45 / 41 / 49 us at 256 / 296 / 444 CTAs.
+    Beyond 256 (sequence, head) pairs a cut does not pay for the merge (48 sequences in 64 rows: 81 us in two slices of each, 76 whole and the
+    longest first); a single sequence divides evenly anyway; the kernel orders 64 sequences at most."""
+    return max(n_seqs, min(16 * n_seqs, 296 // n_kv)) if 2 <= n_seqs <= 64 and n_seqs * n_kv <= 256 else 0
 
 
 def tcgen05_decode_takes(dtype: torch.dtype, head_dim: int, page_size: int, group: int) -> bool:
@@ -1691,15 +1700,19 @@ def attention_decode_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
         raise KernelError(f"cache pools {tuple(k_pool.shape)} do not fit head_dim {d}")
     if tok_pos.numel() < n or tok_slot.numel() < n:
         raise KernelError("tok_pos / tok_slot are shorter than the token rows")
-    n_splits = n_splits or decode_splits_tcgen05(n, n_kv)
+    n_places = 0 if n_splits else decode_places_tcgen05(n, n_kv)
+    n_splits = 1 if n_places else n_splits or decode_splits_tcgen05(n, n_kv)
     out = torch.empty((n, n_q * d), dtype=q.dtype, device=q.device)
     part_o = part_ml = None
-    if n_splits > 1:
+    if n_places:
+        part_o = torch.empty((n_places * n_q * d,), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((n_places * n_q * 2 + 2 * n,), dtype=torch.float32, device=q.device)
+    elif n_splits > 1:
         part_o = torch.empty((n * n_q * n_splits * d,), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n * n_q * n_splits * 2,), dtype=torch.float32, device=q.device)
     check(l.gi_attention_decode_tcgen05(_ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(block_table), _ptr(tok_pos),
                                         _ptr(tok_slot), _ptr(part_o), _ptr(part_ml), _ptr(out), n, n_q, n_kv, d, page_size,
-                                        block_table.shape[1], n_pages, int(window or 0), float(scale), n_splits,
+                                        block_table.shape[1], n_pages, int(window or 0), float(scale), n_splits, n_places,
                                         _ptr(tcgen05_error_flag(q.device)), _stream()), l)
     if n_splits > 1:                                 # one slice: the kernel wrote the output itself
         check(l.gi_attention_decode_combine(_ptr(part_o), _ptr(part_ml), _ptr(out), n * n_q, d, n_splits, _stream()), l)

@@ -706,6 +706,35 @@ def test_attention_decode_tcgen05(n_q, n_kv, page, window, splits):
         torch.testing.assert_close(out[i], ref, rtol=2e-2, atol=2e-2, msg=lambda msg: f"seq {s}: {msg}")
 
 
+@pytest.mark.parametrize("n,n_kv,group,window", [
+    (2, 1, 2, 0), (3, 2, 16, 0), (20, 8, 1, 0), (32, 8, 2, 300), (64, 4, 1, 0),      # slices of one length, merged
+    (33, 8, 1, 0), (64, 5, 3, 0), (64, 8, 1, 130), (65, 5, 1, 0)])                   # whole: the longest first; in the order given
+def test_attention_decode_tcgen05_of_uneven_sequences(n, n_kv, group, window):
+    """Lengths from 1 to 2,000 with equal ones among them, rows that are none at both ends and between, and a step that is nothing but such
+    rows: every sequence once, whole."""
+    d, page, n_q = 128, 64, n_kv * group
+    lens = [2000, 1, 64, 65, 700, 700][:n] + [1 + (i * 397) % 900 for i in range(6, n)]
+    k_pool, v_pool, bt, kd, vd = make_cache(n, lens, n_kv, d, page, torch.bfloat16, seed=n + n_kv)
+    slots = [s if s == 0 or s % 7 else -1 for s in range(n)][::-1] if n > 3 else list(range(n))
+    if n > 3:
+        slots[0] = -1
+    pos = [lens[s] - 1 if s >= 0 else 0 for s in slots]
+    g = torch.Generator(device=DEV).manual_seed(22)
+    q = torch.randn(n, n_q, d, generator=g, device=DEV).to(torch.bfloat16)
+    flag = K().tcgen05_error_flag(q.device)
+    flag.zero_()
+    on_device = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    out = K().attention_decode_tcgen05(q, k_pool, v_pool, bt, on_device(pos), on_device(slots), d ** -0.5, window).float().view(n, n_q, d)
+    none = K().attention_decode_tcgen05(q, k_pool, v_pool, bt, on_device(pos), on_device([-1] * n), d ** -0.5, window)
+    assert int(flag.item()) == 0 and float(none.float().abs().sum()) == 0
+    for i, s in enumerate(slots):
+        if s < 0:
+            assert float(out[i].abs().sum()) == 0, "a padding row gives zeros"
+            continue
+        ref = ref_attention(q[i].float(), kd[s], vd[s], pos[i], d ** -0.5, window).float()
+        torch.testing.assert_close(out[i], ref, rtol=2e-2, atol=2e-2, msg=lambda msg: f"seq {s}: {msg}")
+
+
 def test_attention_decode_tcgen05_finds_one_far_key():
     """One key among 700 carries all the weight, wherever it lies (a page's edge, the first and the last
     position, another slice): the value of that key comes out; a window that ends just short of it loses it."""
