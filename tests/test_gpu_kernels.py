@@ -886,3 +886,17 @@ def test_tensor_core_attention_refuses_other_sizes():
         K().attention_decode_bf16(q2, pool2, pool2, bt, z, z, 1.0, 0)
     assert not K().mma_attention_takes(torch.bfloat16, 256) and not K().mma_attention_takes(torch.float32, 64)
     assert K().mma_attention_takes(torch.bfloat16, 48)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,experts,hidden,ld", [(1, 1, 4, 4), (3, 9, 130, 131), (5, 8, 2052, 2056), (64, 16, 4096, 4096), (300, 17, 2044, 2047),
+                                                 (593, 8, 516, 520)])
+def test_router_logits_at_the_edges(n, experts, hidden, ld, dtype):
+    """Rows that end inside a lane's words, rows off the 16-byte boundary, few blocks and many: within the bound of a float32 sum of
+    `hidden` products (each rounded sum adds at most 2^-24 of the products' magnitudes)."""
+    g = torch.Generator(device=DEV).manual_seed(hidden)
+    x = torch.randn(n, ld, generator=g, device=DEV).to(dtype)[:, :hidden]
+    w = torch.randn(experts, hidden, generator=g, device=DEV)
+    z = K().router_logits(x, w).double()
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((z - exact).abs() <= hidden * 2.0 ** -24 * size).all())
