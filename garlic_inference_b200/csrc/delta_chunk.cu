@@ -110,7 +110,10 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
         float sq = 0.f, sk = 0.f;
         sq = fmaf(q.x, q.x, sq); sq = fmaf(q.y, q.y, sq); sq = fmaf(q.z, q.z, sq); sq = fmaf(q.w, q.w, sq);
         sk = fmaf(k.x, k.x, sk); sk = fmaf(k.y, k.y, sk); sk = fmaf(k.z, k.z, sk); sk = fmaf(k.w, k.w, sk);
-        const float iq = q_scale / sqrtf(warp_sum(sq) + unit_eps), ik = 1.f / sqrtf(warp_sum(sk) + unit_eps);
+        sq = warp_sum(sq);
+        sk = warp_sum(sk);
+        // (a token beyond the end is zeros also where unit_eps is zero)
+        const float iq = in ? q_scale / sqrtf(sq + unit_eps) : 0.f, ik = in ? 1.f / sqrtf(sk + unit_eps) : 0.f;
         if (ch < D) {
             *reinterpret_cast<float4*>(q_s + t * DC_LD + ch) = make_float4(q.x * iq, q.y * iq, q.z * iq, q.w * iq);
             *reinterpret_cast<float4*>(k_s + t * DC_LD + ch) = make_float4(k.x * ik, k.y * ik, k.z * ik, k.w * ik);

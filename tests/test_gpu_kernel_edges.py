@@ -793,6 +793,37 @@ def test_delta_rule_in_chunks(channel, d, dv, H, Hk, lens, at_a_time, monkeypatc
     kernels.check_bounded_waits(DEV)
 
 
+def _delta_case(n, H, d, dv, channel, seed=1, center=-2.0, spread=2.0):
+    """One sequence: (rows, logits of beta, logits of the decay, A_log, dt_bias, first state), one key head a head."""
+    n_dec = H * d if channel else H
+    return (rnd(n, 2 * H * d + H * dv, seed=seed), rnd(n, H, seed=seed + 1), rnd(n, n_dec, seed=seed + 2, scale=spread),
+            rnd(H, seed=seed + 3, scale=0.3), rnd(n_dec, seed=seed + 4) + center, rnd(1, H * dv * d, seed=seed + 5, scale=0.1))
+
+
+def _delta_run(case, H, d, dv, channel, chunks, eps=1e-6):
+    from garlic_inference_b200.ops import kernels
+    qkv, beta, al, A_log, dt, first = case
+    n, state = qkv.shape[0], first.clone()
+    spans = torch.tensor([[0, 0, n]], dtype=torch.int32, device=DEV)
+    out = kernels.delta_scan(qkv, (0, H * d, 2 * H * d), beta, (0, 0), A_log, dt, state, spans, torch.zeros(n, dtype=torch.int32, device=DEV),
+                             H, H, d, dv, eps, channel_decay=channel, decay_logits=al, chunks=chunks)
+    kernels.check_bounded_waits(DEV)
+    return out.view(n, H, dv), state.view(H, dv, d)
+
+
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n", [17, 31, 32])
+def test_delta_rule_in_chunks_without_an_addend_under_the_roots(channel, d, n, monkeypatch):
+    """unit_eps of zero: the tokens that fill a part chunk up are zeros all the same."""
+    from garlic_inference_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNK_TOKENS", 0)
+    case = _delta_case(n, 2, d, 32, channel)
+    for got, one in zip(_delta_run(case, 2, d, 32, channel, True, 0.0), _delta_run(case, 2, d, 32, channel, False, 0.0)):
+        # each within eight roundings to 2^-24 of the result (test_delta_rule_in_chunks)
+        assert bool(got.isfinite().all()) and float((got - one).norm() / one.norm()) < 16 * 2.0 ** -24
+
+
 def test_delta_rule_over_many_tokens_keeps_a_bounded_scratch(monkeypatch):
     """40,000 tokens of 16 heads of 128 would keep 680 MB: the room taken is the bound's, and the launches are counted."""
     from garlic_inference_b200.ops import counters, kernels
