@@ -285,6 +285,33 @@ __device__ __forceinline__ void dc_bulk(void* dst, const void* src, int bytes, v
                  ::"r"(t5_smem(dst)), "l"(src), "r"(bytes), "r"(t5_smem(bar)) : "memory");
 }
 
+// B u of a chunk by multiply-adds over the tokens up to an output's own, where an update is not finite: the tensor core multiplies it
+// with the zeros that B has for the tokens in front of it, and would make NaN of their outputs.  w: a lane's updates as the walk has them;
+// fb: B's fragments (three parts of 32 lanes' four words).  By a whole warp.
+__device__ __noinline__ void dc_outputs_in_order(const float (&w)[8], const uint32_t* fb, int g, int t, float (&acc)[2][4]) {
+#pragma unroll
+    for (int s = 0; s < DC_T; ++s) {
+        const int from = s % 8 / 2;                          // the lane of column g that has token s, and B's of token s in a row
+        const float lo = __shfl_sync(0xffffffffu, w[s / 8 * 4 + s % 2], g * 4 + from), hi = __shfl_sync(0xffffffffu, w[s / 8 * 4 + 2 + s % 2], g * 4 + from);
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int row = 2 * t + e;
+                float b = 0.f;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const uint32_t pair = fb[(j * 32 + row * 4 + from) * 4 + 2 * tile + s / 8];
+                    b += __uint_as_float(s % 2 ? pair & 0xffff0000u : pair << 16);
+                }
+                if (s <= tile * 8 + row) {
+                    acc[tile][e] = fmaf(lo, b, acc[tile][e]);
+                    acc[tile][2 + e] = fmaf(hi, b, acc[tile][2 + e]);
+                }
+            }
+    }
+}
+
 // 16 value columns to a block; four warps share the channels, a fifth makes the outputs while they are at the next chunk, and
 // waits for the copies so that they need not.  A thread's part of the state: columns g and g + 8 (rows of the tensor core's
 // tiles), of each of TN tiles the channels 2 t and 2 t + 1, where g and t are the lane's quotient and rest by 4.
@@ -318,12 +345,14 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
         return make_float4(((a.x + b.x) + d.x) + e.x, ((a.y + b.y) + d.y) + e.y, ((a.z + b.z) + d.z) + e.z, ((a.w + b.w) + d.w) + e.w);
     };
     // u of columns g, g + 8 and tokens 2 t, 2 t + 1 (first tile of rows) and 8 later: the tensor core's first operand
-    auto updates = [&](int c, const float4& lo, const float4& hi, uint32_t (&u)[3][4]) {
+    auto updates = [&](int c, const float4& lo, const float4& hi, float (&w)[8]) {
         const float4 s0 = total(c, 0), s1 = total(c, 1);
-        t5_split3(lo.x - s0.x, lo.y - s0.y, u[0][0], u[1][0], u[2][0]);
-        t5_split3(hi.x - s0.z, hi.y - s0.w, u[0][1], u[1][1], u[2][1]);
-        t5_split3(lo.z - s1.x, lo.w - s1.y, u[0][2], u[1][2], u[2][2]);
-        t5_split3(hi.z - s1.z, hi.w - s1.w, u[0][3], u[1][3], u[2][3]);
+        w[0] = lo.x - s0.x; w[1] = lo.y - s0.y; w[2] = hi.x - s0.z; w[3] = hi.y - s0.w;
+        w[4] = lo.z - s1.x; w[5] = lo.w - s1.y; w[6] = hi.z - s1.z; w[7] = hi.w - s1.w;
+    };
+    auto parts = [](const float (&w)[8], uint32_t (&u)[3][4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t5_split3(w[2 * i], w[2 * i + 1], u[0][i], u[1][i], u[2][i]);
     };
     constexpr int OF_A[6] = {2, 0, 1, 1, 0, 0}, OF_B[6] = {0, 2, 1, 0, 1, 0};      // small products first, the last one large
 
@@ -360,16 +389,23 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
             if (lane == 0 && c > 0 && c - 1 + DC_STAGES < n) fetch(c - 1 + DC_STAGES);
             const unsigned char* stage = dw_smem + c % DC_STAGES * STAGE;
             const float4* tv = reinterpret_cast<const float4*>(stage + C::HEAD) + lane * 2;
-            uint32_t u[3][4];
-            updates(c, tv[0], tv[1], u);
+            float w[8];
+            updates(c, tv[0], tv[1], w);
             const uint4* fb = reinterpret_cast<const uint4*>(stage + C::FA + C::FU) + lane;
-            const uint4 b[3] = {fb[0], fb[32], fb[64]};
             float acc[2][4] = {};
+            bool finite = true;
 #pragma unroll
-            for (int m = 0; m < 6; ++m) {
-                dc_mma(acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
-                dc_mma(acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
-            }
+            for (int i = 0; i < 8; ++i) finite = finite && fabsf(w[i]) <= 3.402823466e38f;
+            if (__all_sync(0xffffffffu, finite)) {
+                const uint4 b[3] = {fb[0], fb[32], fb[64]};
+                uint32_t u[3][4];
+                parts(w, u);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) {
+                    dc_mma(acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
+                    dc_mma(acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
+                }
+            } else dc_outputs_in_order(w, reinterpret_cast<const uint32_t*>(fb - lane), g, t, acc);
 #pragma unroll
             for (int tile = 0; tile < 2; ++tile) {
                 const float4 s = total(c, 2 + tile);
@@ -460,7 +496,11 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
         __syncthreads();
         if (gave_up[(c + 1) & 1]) return;
         uint32_t u[3][4];
-        updates(c, lo, hi, u);
+        {
+            float w[8];
+            updates(c, lo, hi, w);
+            parts(w, u);
+        }
         float small[TN][4], large[TN][4];
 #pragma unroll
         for (int i = 0; i < TN; ++i)

@@ -824,6 +824,28 @@ def test_delta_rule_in_chunks_without_an_addend_under_the_roots(channel, d, n, m
         assert bool(got.isfinite().all()) and float((got - one).norm() / one.norm()) < 16 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("d, n", [(64, 40), (128, 47)])
+@pytest.mark.parametrize("what, at", [("v", 20), ("v", 16), ("v", 31), ("k", 25), ("q", 30), ("beta", 9), ("decay", 37)])
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
+def test_delta_rule_in_chunks_keeps_later_tokens_out_of_earlier_outputs(channel, d, n, what, at, value, monkeypatch):
+    """One number beyond the finite inside a chunk: the outputs that are finite token by token are so in chunks, with the same values, and
+    no others."""
+    from garlic_inference_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNK_TOKENS", 0)
+    H, dv = 2, 32
+    case = _delta_case(n, H, d, dv, channel)
+    qkv, beta, al = case[:3]
+    {"q": qkv[:, 5:], "k": qkv[:, H * d + 5:], "v": qkv[:, 2 * H * d + 5:], "beta": beta, "decay": al}[what][at, 0] = value
+    (got, state), (one, state1) = _delta_run(case, H, d, dv, channel, True), _delta_run(case, H, d, dv, channel, False)
+    assert bool(one[:at].isfinite().all()) and bool(one[:, 1].isfinite().all())
+    for x, y in ((got, one), (state, state1)):
+        fine = y.isfinite()
+        assert torch.equal(x.isfinite(), fine)
+        # each within eight roundings to 2^-24 of the result (test_delta_rule_in_chunks)
+        assert float((x - y)[fine].norm() / y[fine].norm()) < 16 * 2.0 ** -24
+
+
 def test_delta_rule_over_many_tokens_keeps_a_bounded_scratch(monkeypatch):
     """40,000 tokens of 16 heads of 128 would keep 680 MB: the room taken is the bound's, and the launches are counted."""
     from garlic_inference_b200.ops import counters, kernels
