@@ -288,7 +288,9 @@ __device__ __forceinline__ void dc_bulk(void* dst, const void* src, int bytes, v
 // B u of a chunk by multiply-adds over the tokens up to an output's own, where an update is not finite: the tensor core multiplies it
 // with the zeros that B has for the tokens in front of it, and would make NaN of their outputs.  w: a lane's updates as the walk has them;
 // fb: B's fragments (three parts of 32 lanes' four words).  By a whole warp.
-__device__ __noinline__ void dc_outputs_in_order(const float (&w)[8], const uint32_t* fb, int g, int t, float (&acc)[2][4]) {
+__device__ __forceinline__ void dc_outputs_in_order(const float (&w)[8], const uint32_t* fb, int g, int t, float (&acc)[2][4]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e / 4][e % 4] = 0.f;
 #pragma unroll
     for (int s = 0; s < DC_T; ++s) {
         const int from = s % 8 / 2;                          // the lane of column g that has token s, and B's of token s in a row
@@ -392,20 +394,19 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
             float w[8];
             updates(c, tv[0], tv[1], w);
             const uint4* fb = reinterpret_cast<const uint4*>(stage + C::FA + C::FU) + lane;
+            const uint4 b[3] = {fb[0], fb[32], fb[64]};
+            uint32_t u[3][4];
+            parts(w, u);
             float acc[2][4] = {};
-            bool finite = true;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) finite = finite && fabsf(w[i]) <= 3.402823466e38f;
-            if (__all_sync(0xffffffffu, finite)) {
-                const uint4 b[3] = {fb[0], fb[32], fb[64]};
-                uint32_t u[3][4];
-                parts(w, u);
+            for (int m = 0; m < 6; ++m) {
+                dc_mma(acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
+                dc_mma(acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
+            }
+            float zero[2] = {0.f, 0.f};                      // NaN where a sum is not finite
 #pragma unroll
-                for (int m = 0; m < 6; ++m) {
-                    dc_mma(acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
-                    dc_mma(acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
-                }
-            } else dc_outputs_in_order(w, reinterpret_cast<const uint32_t*>(fb - lane), g, t, acc);
+            for (int e = 0; e < 4; ++e) { zero[0] = fmaf(acc[0][e], 0.f, zero[0]); zero[1] = fmaf(acc[1][e], 0.f, zero[1]); }
+            if (__builtin_expect(__any_sync(0xffffffffu, zero[0] + zero[1] != 0.f), 0)) dc_outputs_in_order(w, reinterpret_cast<const uint32_t*>(fb - lane), g, t, acc);
 #pragma unroll
             for (int tile = 0; tile < 2; ++tile) {
                 const float4 s = total(c, 2 + tile);
