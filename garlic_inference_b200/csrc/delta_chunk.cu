@@ -7,17 +7,20 @@
 //   u = T V - (T KG) S,   T = (1 + beta A)^-1 beta by forward substitution, KG_t = k_t G_t
 //   o = QG S + B u,       QG_t = q_t G_t
 //   S <- G_16 S + sum over s of u_s KE_s,  KE_s = k_s (decays s+1 .. 16)
-// Products of decays are made as products (never as quotients), so that none is beyond 1 and a decay of zero is exact.
+// Products of decays are made as products or as exponentials of sums (never as quotients), so that none is beyond 1 and a decay of zero
+// is exact.
 // delta_chunk_prepare_kernel makes everything that does not depend on S, for all chunks and heads at once; delta_chunk_walk_kernel
 // goes from chunk to chunk with S in registers.
 //
-// The products with S and u keep float32: every factor is cut into three bfloat16 parts that sum to it exactly, the six largest
-// products run on `mma.sync` from zero, small ones first (the error of a product is below 2^-25), and what they give meets S by
-// float32 multiply-adds.  The operands lie in memory as the tensor core's fragments, so that a lane reads its own 16 bytes.
-// Measured, 2,048 tokens, 16 heads of 128 x 128, a decay per channel: 382 us token by token (a chain of 174 ns a token), 170 us so (the
-// preparation 61, the walk 105).  Relative error (2-norm) of outputs / states against 64 bits in units of 1e-7, token by token and so,
-// 600 tokens: decays near 1 (softplus of values around -9) 17 / 22 and 16 / 21, around -4 2.8 / 2.3 and 2.7 / 2.1; around 0, where a
-// state is forgotten within a token and a result is one or two products, 1.2 / 0.33 and 1.45 / 0.47.
+// The products with S and u keep float32: every factor is cut into three bfloat16 parts that sum to it exactly (t5_split3 says where not),
+// the six largest products run on `mma.sync` from zero, small ones first (the error of a product is below 2^-25), and what they give
+// meets S by float32 multiply-adds.  The operands lie in memory as the tensor core's fragments, so that a lane reads its own 16 bytes.
+// Measured, 2,048 tokens, 16 heads of 128 x 128, a decay per channel: 382 us token by token (a chain of 174 ns a token), 188 us so (the
+// preparation 71, the walk 121).  Relative error (2-norm) of outputs / states against 64 bits in units of 1e-7, 600 tokens, token by token and
+// so, by what softplus is taken of: around -9 (decays near 1, a memory of thousands of tokens) 22 / 29 and 2.1 / 2.2, -4 2.3 / 2.1 and 1.6 / 1.2,
+// -2 1.50 / 1.21 and 1.45 / 1.02, 0 (a state is halved by a token) 1.25 / 0.85 and 1.30 / 0.88, 3 1.19 / 0.72 and 1.19 / 0.71.  With decays as products of
+// rounded decays, what a token takes off straight from its value, and a token's own part among the tensor core's sums it was 170 us and
+// 20 / 26, 2.2 / 2.0, 1.65 / 1.34, 1.52 / 1.08, 1.38 / 0.96.
 #include "scan.cuh"
 #include "tcgen05.cuh"
 
@@ -27,9 +30,13 @@
 #define DC_LD 136                    // floats of a row in the preparation's shared memory: 8 banks from row to row
 #define DC_ERR_WAIT 81
 
-// bytes of a chunk of one head: fragments of [T KG; QG] (32 rows), of KE, of B, and G_16; then T V in slices of 16 columns
+// bytes of a chunk of one head: fragments of [T KG; QG] (32 rows), of KE without its last token's row, of B without its diagonal, G_16, the
+// last token's key and B's diagonal as floats; then T V in slices of 16 columns.  (What a token has of itself, in an output and in
+// the state behind it, joins the other sums last by a float32 multiply-add: where little is left of the state it is all but the result,
+// and the tensor core, which cuts its sums off, would cut it.)
 template <int D> struct DcChunk {
-    static constexpr int FA = 32 * D * 6, FU = DC_T * D * 6, FB = DC_T * DC_T * 6, G = D * 4, HEAD = FA + FU + FB + G;
+    static constexpr int FA = 32 * D * 6, FU = DC_T * D * 6, FB = DC_T * DC_T * 6, G = D * 4, KL = D * 4, BD = DC_T * 4;
+    static constexpr int AT_G = FA + FU + FB, AT_KL = AT_G + G, AT_BD = AT_KL + KL, HEAD = AT_BD + BD;
 };
 
 // rows of sequence i in this launch's window, and its first chunk
@@ -55,7 +62,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
     extern __shared__ __align__(16) float dc_smem[];
     float *q_s = dc_smem, *k_s = q_s + DC_T * DC_LD, *g_s = k_s + DC_T * DC_LD, *kg_s = g_s + DC_T * DC_LD, *ke_s = kg_s + DC_T * DC_LD;
     __shared__ __align__(16) float A_s[DC_T][DC_T], B_s[DC_T][DC_T];
-    __shared__ float beta_s[DC_T];
+    __shared__ float beta_s[DC_T], diag_s[DC_T];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, kh = h / (H / Hk);
     // which sequence this chunk is of
     int seq = 0, c = blockIdx.x;
@@ -99,13 +106,21 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
         const bool in = t < len;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q, g = make_float4(1.f, 1.f, 1.f, 1.f);
         if (in && ch < D) { q = q4[i]; k = k4[i]; }
+        float4 log_g = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in) {
-            g.x = expf(-rate * rc_softplus(a4[i].x + d4.x));
+            log_g.x = -rate * rc_softplus(a4[i].x + d4.x);
+            g.x = expf(log_g.x);
             if (CH) {
-                g.y = expf(-rate * rc_softplus(a4[i].y + d4.y));
-                g.z = expf(-rate * rc_softplus(a4[i].z + d4.z));
-                g.w = expf(-rate * rc_softplus(a4[i].w + d4.w));
-            } else g.y = g.z = g.w = g.x;
+                log_g.y = -rate * rc_softplus(a4[i].y + d4.y);
+                log_g.z = -rate * rc_softplus(a4[i].z + d4.z);
+                log_g.w = -rate * rc_softplus(a4[i].w + d4.w);
+                g.y = expf(log_g.y);
+                g.z = expf(log_g.z);
+                g.w = expf(log_g.w);
+            } else {
+                log_g.y = log_g.z = log_g.w = log_g.x;
+                g.y = g.z = g.w = g.x;
+            }
         }
         float sq = 0.f, sk = 0.f;
         sq = fmaf(q.x, q.x, sq); sq = fmaf(q.y, q.y, sq); sq = fmaf(q.z, q.z, sq); sq = fmaf(q.w, q.w, sq);
@@ -118,6 +133,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
             *reinterpret_cast<float4*>(q_s + t * DC_LD + ch) = make_float4(q.x * iq, q.y * iq, q.z * iq, q.w * iq);
             *reinterpret_cast<float4*>(k_s + t * DC_LD + ch) = make_float4(k.x * ik, k.y * ik, k.z * ik, k.w * ik);
             *reinterpret_cast<float4*>(g_s + t * DC_LD + ch) = g;
+            *reinterpret_cast<float4*>(kg_s + t * DC_LD + ch) = log_g;
         }
         if (lane == 0) beta_s[t] = in ? rc_sigmoid(b1[i]) : 0.f;
     }
@@ -167,24 +183,27 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
             const float a = part_sum_tokens<P>(*reinterpret_cast<float (*)[P]>(ka + half * 8), part);
             const float b = part_sum_tokens<P>(*reinterpret_cast<float (*)[P]>(qa + half * 8), part);
             A_s[t][s] = t > s ? a : 0.f;
-            B_s[t][s] = t >= s ? b : 0.f;
+            B_s[t][s] = t > s ? b : 0.f;
+            if (t == s) diag_s[t] = b;
         }
     }
     __syncthreads();
 
-    // x <- (1 + beta A)^-1 beta x by forward substitution
+    // x <- (1 + beta A)^-1 beta x by forward substitution.  What is taken off a number is summed up first: keys are unit vectors, so it is
+    // a fraction of the number, and so are its roundings.
     auto substitute = [&](float (&x)[DC_T]) {
 #pragma unroll
         for (int t = 0; t < DC_T; ++t) {
+            float off = 0.f;
 #pragma unroll
             for (int s = 0; s < t; s += 4) {
                 const float4 a = *reinterpret_cast<const float4*>(&A_s[t][s]);       // zero from t on
-                x[t] = fmaf(-a.x, x[s], x[t]);
-                if (s + 1 < t) x[t] = fmaf(-a.y, x[s + 1], x[t]);
-                if (s + 2 < t) x[t] = fmaf(-a.z, x[s + 2], x[t]);
-                if (s + 3 < t) x[t] = fmaf(-a.w, x[s + 3], x[t]);
+                off = fmaf(a.x, x[s], off);
+                if (s + 1 < t) off = fmaf(a.y, x[s + 1], off);
+                if (s + 2 < t) off = fmaf(a.z, x[s + 2], off);
+                if (s + 3 < t) off = fmaf(a.w, x[s + 3], off);
             }
-            x[t] *= beta_s[t];
+            x[t] = (x[t] - off) * beta_s[t];
         }
     };
     // T V: a thread takes a value column; a lane of the walk finds its eight tokens and columns side by side
@@ -205,22 +224,25 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
         for (int i = tid; i < min(dv - col0, 128) * DC_T / 4; i += 128) tv[col0 * DC_T / 4 + i] = reinterpret_cast<const float4*>(ke_s)[i];
     }
     __syncthreads();
-    // a thread takes a channel: its products of decays, and T KG
+    // a thread takes a channel: its products of decays as exponentials of sums (a product of decays near 1 would keep the rounding of
+    // every one of them, the same way for all tokens of a long memory), and T KG
     if (tid < D) {
-        float g[DC_T], x[DC_T], run = 1.f;
+        float l[DC_T], x[DC_T], sum = 0.f, run = 1.f;
 #pragma unroll
         for (int t = 0; t < DC_T; ++t) {
-            g[t] = g_s[t * DC_LD + tid];
-            run *= g[t];
+            l[t] = kg_s[t * DC_LD + tid];
+            sum += l[t];
+            run = expf(sum);
             x[t] = k_s[t * DC_LD + tid] * run;
             q_s[t * DC_LD + tid] *= run;
         }
-        reinterpret_cast<float*>(chunk + DcChunk<D>::FA + DcChunk<D>::FU + DcChunk<D>::FB)[tid] = run;
-        run = 1.f;
+        reinterpret_cast<float*>(chunk + DcChunk<D>::AT_G)[tid] = run;
+        reinterpret_cast<float*>(chunk + DcChunk<D>::AT_KL)[tid] = k_s[(len - 1) * DC_LD + tid];
+        sum = 0.f;
 #pragma unroll
         for (int t = DC_T - 1; t >= 0; --t) {
-            ke_s[t * DC_LD + tid] = k_s[t * DC_LD + tid] * run;
-            run *= g[t];
+            ke_s[t * DC_LD + tid] = t == len - 1 ? 0.f : k_s[t * DC_LD + tid] * expf(sum);
+            sum += l[t];
         }
         substitute(x);
 #pragma unroll
@@ -262,6 +284,7 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, long long ldq, int q_o
         for (int j = 0; j < 3; ++j) fu[((i >> 5) * 3 + j) * 32 + ln] = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
     }
     // of B
+    if (tid >= 32 && tid < 32 + DC_T) reinterpret_cast<float*>(chunk + DcChunk<D>::AT_BD)[tid - 32] = diag_s[tid - 32];
     if (tid < 32) {
         uint4* fb = reinterpret_cast<uint4*>(chunk + DcChunk<D>::FA + DcChunk<D>::FU);
         const int g = lane >> 2, t = lane & 3;
@@ -285,7 +308,7 @@ __device__ __forceinline__ void dc_bulk(void* dst, const void* src, int bytes, v
                  ::"r"(t5_smem(dst)), "l"(src), "r"(bytes), "r"(t5_smem(bar)) : "memory");
 }
 
-// B u of a chunk by multiply-adds over the tokens up to an output's own, where an update is not finite: the tensor core multiplies it
+// B u of a chunk by multiply-adds over the tokens in front of an output's own, where an update is not finite: the tensor core multiplies it
 // with the zeros that B has for the tokens in front of it, and would make NaN of their outputs.  w: a lane's updates as the walk has them;
 // fb: B's fragments (three parts of 32 lanes' four words).  By a whole warp.
 __device__ __forceinline__ void dc_outputs_in_order(const float (&w)[8], const uint32_t* fb, int g, int t, float (&acc)[2][4]) {
@@ -306,7 +329,7 @@ __device__ __forceinline__ void dc_outputs_in_order(const float (&w)[8], const u
                     const uint32_t pair = fb[(j * 32 + row * 4 + from) * 4 + 2 * tile + s / 8];
                     b += __uint_as_float(s % 2 ? pair & 0xffff0000u : pair << 16);
                 }
-                if (s <= tile * 8 + row) {
+                if (s < tile * 8 + row) {
                     acc[tile][e] = fmaf(lo, b, acc[tile][e]);
                     acc[tile][2 + e] = fmaf(hi, b, acc[tile][2 + e]);
                 }
@@ -395,25 +418,38 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
             updates(c, tv[0], tv[1], w);
             const uint4* fb = reinterpret_cast<const uint4*>(stage + C::FA + C::FU) + lane;
             const uint4 b[3] = {fb[0], fb[32], fb[64]};
+            const float2* diag = reinterpret_cast<const float2*>(stage + C::AT_BD) + t;
+            const float2 own[2] = {diag[0], diag[4]};
+            const float4 of_state[2] = {total(c, 2), total(c, 3)};
             uint32_t u[3][4];
             parts(w, u);
-            float acc[2][4] = {};
+            float acc[2][4] = {}, large[2][4] = {};
 #pragma unroll
             for (int m = 0; m < 6; ++m) {
-                dc_mma(acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
-                dc_mma(acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
+                dc_mma(m == 5 ? large[0] : acc[0], u[OF_A[m]], b[OF_B[m]].x, b[OF_B[m]].y);
+                dc_mma(m == 5 ? large[1] : acc[1], u[OF_A[m]], b[OF_B[m]].z, b[OF_B[m]].w);
             }
             float zero[2] = {0.f, 0.f};                      // NaN where a sum is not finite
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { zero[0] = fmaf(acc[0][e], 0.f, zero[0]); zero[1] = fmaf(acc[1][e], 0.f, zero[1]); }
-            if (__builtin_expect(__any_sync(0xffffffffu, zero[0] + zero[1] != 0.f), 0)) dc_outputs_in_order(w, reinterpret_cast<const uint32_t*>(fb - lane), g, t, acc);
+            for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    acc[tile][e] += large[tile][e];
+                    zero[tile] = fmaf(acc[tile][e], 0.f, zero[tile]);
+                }
+            if (__builtin_expect(__any_sync(0xffffffffu, zero[0] + zero[1] != 0.f), 0))
+                dc_outputs_in_order(w, reinterpret_cast<const uint32_t*>(fb - lane), g, t, acc);
 #pragma unroll
             for (int tile = 0; tile < 2; ++tile) {
-                const float4 s = total(c, 2 + tile);
+                const float4 s = of_state[tile];
+                const float2 b1 = own[tile];
                 const int at = c * DC_T + tile * 8 + 2 * t;
                 float* dst = out + (size_t)(sp.start + at) * H * dv + h * dv + v0 + g;
-                if (at < sp.len) { dst[0] = acc[tile][0] + s.x; dst[8] = acc[tile][2] + s.z; }
-                if (at + 1 < sp.len) { dst[(size_t)H * dv] = acc[tile][1] + s.y; dst[(size_t)H * dv + 8] = acc[tile][3] + s.w; }
+                if (at < sp.len) { dst[0] = fmaf(b1.x, w[tile * 4], acc[tile][0] + s.x); dst[8] = fmaf(b1.x, w[tile * 4 + 2], acc[tile][2] + s.z); }
+                if (at + 1 < sp.len) {
+                    dst[(size_t)H * dv] = fmaf(b1.y, w[tile * 4 + 1], acc[tile][1] + s.y);
+                    dst[(size_t)H * dv + 8] = fmaf(b1.y, w[tile * 4 + 3], acc[tile][3] + s.w);
+                }
             }
         }
         if (!ok && lane == 0) {                     // the copies still in flight land before the block leaves
@@ -478,7 +514,7 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
             // (what the other half of the step reads of the chunk is on its way before the barrier)
             const uint4* fu = reinterpret_cast<const uint4*>(stage + C::FA) + (size_t)cg * KS * 3 * 32 + lane;
             const float4* tv = reinterpret_cast<const float4*>(stage + C::HEAD) + lane * 2;
-            const float* G = reinterpret_cast<const float*>(stage + C::FA + C::FU + C::FB) + cg * (D / 4) + 2 * t;
+            const float* G = reinterpret_cast<const float*>(stage + C::AT_G) + cg * (D / 4) + 2 * t;
             lo = tv[0];
             hi = tv[1];
 #pragma unroll
@@ -497,10 +533,19 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
         __syncthreads();
         if (gave_up[(c + 1) & 1]) return;
         uint32_t u[3][4];
+        float last[2];                                       // the last token's updates of columns g and g + 8, and its key
+        float2 key[TN];
         {
             float w[8];
             updates(c, lo, hi, w);
             parts(w, u);
+            const float* K = reinterpret_cast<const float*>(stage + C::AT_KL) + cg * (D / 4) + 2 * t;
+#pragma unroll
+            for (int i = 0; i < TN; ++i) key[i] = *reinterpret_cast<const float2*>(K + i * 8);
+            const int at = min(DC_T, sp.len - c * DC_T) - 1, from = g * 4 + at % 8 / 2;
+            const float even[2] = {at < 8 ? w[0] : w[4], at < 8 ? w[2] : w[6]}, odd[2] = {at < 8 ? w[1] : w[5], at < 8 ? w[3] : w[7]};
+#pragma unroll
+            for (int i = 0; i < 2; ++i) last[i] = __shfl_sync(0xffffffffu, at % 2 ? odd[i] : even[i], from);
         }
         float small[TN][4], large[TN][4];
 #pragma unroll
@@ -518,7 +563,8 @@ delta_chunk_walk_kernel(const unsigned char* __restrict__ chunks, float* __restr
 #pragma unroll
         for (int i = 0; i < TN; ++i) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) S[i][e] = fmaf(S[i][e], e & 1 ? decay[i].y : decay[i].x, large[i][e] + small[i][e]);
+            for (int e = 0; e < 4; ++e)
+                S[i][e] = fmaf(last[e >> 1], e & 1 ? key[i].y : key[i].x, fmaf(S[i][e], e & 1 ? decay[i].y : decay[i].x, small[i][e] + large[i][e]));
         }
         if (c + 1 < n) rows_of(c + 1);
     }

@@ -846,6 +846,35 @@ def test_delta_rule_in_chunks_keeps_later_tokens_out_of_earlier_outputs(channel,
         assert float((x - y)[fine].norm() / y[fine].norm()) < 16 * 2.0 ** -24
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("center, share", [(-9.0, 0.25), (-4.0, 0.8), (-2.0, 1.0), (0.0, 1.1), (3.0, 1.1)])
+def test_delta_rule_in_chunks_is_as_close_to_64_bits_as_token_by_token(channel, d, center, share, monkeypatch):
+    """From decays near 1 (long memories: token by token every rounded decay adds its error, in chunks one rounded product of 16) to states
+    that are forgotten within a token, where both round a result a few times (a tenth for what is not the same number of times)."""
+    from garlic_inference_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNK_TOKENS", 0)
+    n, H, dv = 600, 4, 64
+    case = _delta_case(n, H, d, dv, channel, spread=1.0)
+    case[4].fill_(center)
+    case[5].zero_()
+    qkv, beta, al, A_log, dt, _ = (x.double() for x in case)
+    q, k, v = (qkv[:, a:a + m].reshape(n, H, -1) for a, m in ((0, H * d), (H * d, H * d), (2 * H * d, H * dv)))
+    unit = lambda x: x / torch.sqrt((x ** 2).sum(-1, keepdim=True) + 1e-6)
+    q, k, beta = unit(q) * d ** -0.5, unit(k), torch.sigmoid(beta)
+    g = torch.exp(-torch.exp(A_log)[:, None] * torch.nn.functional.softplus(al + dt).view(n, H, -1))
+    S, want = torch.zeros(H, dv, d, dtype=torch.float64, device=DEV), torch.zeros(n, H, dv, dtype=torch.float64, device=DEV)
+    for t in range(n):
+        S = S * g[t][:, None, :]
+        S = S + (beta[t][:, None] * (v[t] - (S @ k[t][:, :, None])[..., 0]))[:, :, None] * k[t][:, None, :]
+        want[t] = (S @ q[t][:, :, None])[..., 0]
+    (got, state), (one, state1) = _delta_run(case, H, d, dv, channel, True), _delta_run(case, H, d, dv, channel, False)
+    far = lambda x, y: float((x.double() - y).norm() / y.norm())
+    assert far(got, want) < share * far(one, want)
+    # (a state is the work of a few tokens where it forgets: fewer roundings to compare)
+    assert far(state, S) < (share if center < -2.0 else 1.3) * far(state1, S)
+
+
 def test_delta_rule_over_many_tokens_keeps_a_bounded_scratch(monkeypatch):
     """40,000 tokens of 16 heads of 128 would keep 680 MB: the room taken is the bound's, and the launches are counted."""
     from garlic_inference_b200.ops import counters, kernels
