@@ -955,11 +955,19 @@ DELTA_PAIR_TOKENS = 8
 DELTA_SCRATCH_BYTES = 256 << 20    # what the pair keeps of a step's tokens at a time (15,000 of 16 heads of 128 on 8 key heads)
 # Tokens a sequence from which on a prompt is taken in chunks, where the caller lets it: a chunk's preparation costs the same however few
 # blocks (16 value columns of a head of a sequence) there are, and token by token is a chain that many blocks hide.  In us, token by token /
-# so, heads of 128 x 128: 1 x 64 tokens of 8 heads 15.9 / 15.5, 1 x 128 27.5 / 18.8, 1 x 2,048 373 / 140; 16 heads: 2 x 100 28.3 / 28.5,
-# 4 x 128 54.5 / 51.9, 8 x 100 82 / 86, 8 x 256 193 / 174, 16 x 128 177 / 192, 64 x 32 182 / 325.
+# so, heads of 128 x 128, a decay per channel: 1 x 64 tokens of 8 heads 22 / 19, 1 x 128 40 / 26, 1 x 2,048 562 / 153; of 16 heads: 1 x 64 22.8 / 23.0,
+# 2 x 100 42 / 36, 3 x 100 44 / 45, 4 x 128 55 / 57, 5 x 300 177 / 151, 8 x 100 82 / 96, 8 x 256 194 / 190, 8 x 500 370 / 350, 16 x 128 177 / 208, 16 x 500
+# 652 / 742.  A decay per head: 2 x 100 36 / 34, 3 x 600 190 / 163, 4 x 1,000 317 / 337, 6 x 600 295 / 313, 16 x 500 545 / 698; 16 x 300 of 8 heads of 64 x 64
+# 77 / 95 (per channel 91 / 107).
 DELTA_CHUNK_TOKENS = 64
 DELTA_CHUNK_BLOCKS = 512           # as many more tokens for every so many blocks
 DELTA_CHUNK_ROWS = 1024            # and room for so many rows at a time
+
+
+def _delta_in_chunks(n: int, n_seq: int, n_heads: int, key_dim: int, value_dim: int, channel_decay: bool) -> bool:
+    blocks = n_seq * n_heads * value_dim // 16
+    return blocks <= (1024 if channel_decay and key_dim == 128 else 448) and \
+        n * DELTA_CHUNK_BLOCKS >= DELTA_CHUNK_TOKENS * n_seq * (DELTA_CHUNK_BLOCKS + blocks)
 
 
 def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: tuple, A_log: torch.Tensor,
@@ -970,8 +978,8 @@ def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: 
     head) and v (per head) at `offsets`; `ab` float32 holds the logits of beta and of the decay at `ab_offsets`
     (one column per head; with `channel_decay` the decay has one column per head and key channel, and dt_bias as
     many elements).  `decay_logits`: the decay's logits as a float32 matrix of their own (its column
-    ab_offsets[1] is the first).  `chunks`: prompts may be taken 16 tokens at a time, as precise but with sums in another
-    order, so that a token's bits depend on where its portion begins.  Returns float32 [n, n_heads * value_dim]."""
+    ab_offsets[1] is the first).  `chunks`: prompts may be taken 16 tokens at a time, as close to 64 bits or closer but with sums
+    in another order, so that a token's bits depend on where its portion begins and on what else is in the step.  Returns float32 [n, n_heads * value_dim]."""
     l = require_gpu()
     _rows(qkv, "qkv", torch.float32), _rows(ab, "ab", torch.float32), _rows(state, "state", torch.float32)
     _dense(A_log, "A_log"), _dense(dt_bias, "dt_bias", A_log.dtype)
@@ -987,8 +995,7 @@ def delta_scan(qkv: torch.Tensor, offsets: tuple, ab: torch.Tensor, ab_offsets: 
             qkv.data_ptr() % 16 == 0 and state.data_ptr() % 16 == 0:
         each = l.gi_delta_chunk_bytes(n_heads, key_dim, value_dim)
         at_a_time = min(n, (DELTA_SCRATCH_BYTES // each - n_seq) * 16)
-        blocks = n_seq * n_heads * value_dim // 16
-        if chunks and n * DELTA_CHUNK_BLOCKS >= DELTA_CHUNK_TOKENS * n_seq * (DELTA_CHUNK_BLOCKS + blocks) and at_a_time >= min(n, DELTA_CHUNK_ROWS):
+        if chunks and _delta_in_chunks(n, n_seq, n_heads, key_dim, value_dim, channel_decay) and at_a_time >= min(n, DELTA_CHUNK_ROWS):
             space = torch.empty((at_a_time // 16 + n_seq) * each, dtype=torch.uint8, device=qkv.device)
             check(l.gi_delta_chunk_scan(_ptr(qkv), qkv.stride(0), *map(int, offsets), _ptr(ab), ab.stride(0), *map(int, ab_offsets),
                                         _ptr(decay_logits), decay_logits.stride(0) if decay_logits is not None else 0, _ptr(A_log),
