@@ -327,6 +327,10 @@ __device__ __forceinline__ LdSlice ld_slice(int b, int n_blocks, int n_tokens, c
     const int c1 = lo / LD_KEYS + (int)((long long)ld_n * (ld_s.split + 1) / ld_s.n_splits);                                     \
     float* my = part + (size_t)blockIdx.x * H * stride;
 
+// What a chunk's exponents are taken from: the maximum, which is minus infinity while all scores are (every chunk holds a seen key, but its
+// score may be beyond the finite): their weights are zero then.
+__device__ __forceinline__ float ld_from(float maximum) { return maximum == -INFINITY ? 0.f : maximum; }
+
 __device__ __forceinline__ float2 bf2_to_f2(uint32_t w) {
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
 }
@@ -393,9 +397,9 @@ latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, 
 #pragma unroll
         for (int hh = 0; hh < HPW; ++hh) {
             const float sv = valid ? s[hh] : -INFINITY;
-            const float m_new = fmaxf(m[hh], warp_max(sv));          // every chunk holds a seen key
-            const float corr = expf(m[hh] - m_new);
-            p[hh] = valid ? expf(sv - m_new) : 0.f;
+            const float m_new = fmaxf(m[hh], warp_max(sv)), from = ld_from(m_new);
+            const float corr = expf(m[hh] - from);
+            p[hh] = valid ? expf(sv - from) : 0.f;
             l[hh] = l[hh] * corr + warp_sum(p[hh]);
             m[hh] = m_new;
 #pragma unroll
@@ -562,9 +566,9 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
             for (int hh = 0; hh < 4; ++hh) {
                 const int h = 4 * warp + hh;
                 const float sv = valid ? s_s[h * 33 + lane] : -INFINITY;
-                const float m_new = fmaxf(m[hh], warp_max(sv));       // every chunk holds a seen key
-                const float corr = expf(m[hh] - m_new);
-                const bf16 pr = __float2bfloat16_rn(valid ? expf(sv - m_new) : 0.f);
+                const float m_new = fmaxf(m[hh], warp_max(sv)), from = ld_from(m_new);
+                const float corr = expf(m[hh] - from);
+                const bf16 pr = __float2bfloat16_rn(valid ? expf(sv - from) : 0.f);
                 l[hh] = l[hh] * corr + warp_sum(__bfloat162float(pr));
                 m[hh] = m_new;
                 reinterpret_cast<bf16*>(p_s + h * PW)[lane] = pr;
@@ -746,9 +750,9 @@ latent_decode_quarters_kernel(const bf16* __restrict__ q, const bf16* __restrict
                 for (int hh = 0; hh < 4; ++hh) mx[hh] = fmaxf(mx[hh], __shfl_xor_sync(0xffffffffu, mx[hh], o));
 #pragma unroll
             for (int hh = 0; hh < 4; ++hh) {
-                const float m_new = fmaxf(m[hh], mx[hh]);             // every chunk holds a seen key
-                const float corr = expf(m[hh] - m_new);
-                const bf16 w = __float2bfloat16_rn(valid ? expf(sv[hh] - m_new) : 0.f);
+                const float m_new = fmaxf(m[hh], mx[hh]), from = ld_from(m_new);
+                const float corr = expf(m[hh] - from);
+                const bf16 w = __float2bfloat16_rn(valid ? expf(sv[hh] - from) : 0.f);
                 pr[hh] = __bfloat162float(w);
                 l[hh] *= corr;
                 m[hh] = m_new;
@@ -842,7 +846,8 @@ latent_decode_combine_kernel(const float* __restrict__ part, const int2* __restr
         for (int s = lane; s < mine.y; s += 32) M = fmaxf(M, base[s * step]);
         M = warp_max(M);
         float L = 0.f;
-        for (int s = lane; s < mine.y; s += 32) L += expf(base[s * step] - M) * base[s * step + 1];
+        for (int s = lane; s < mine.y; s += 32)
+            if (base[s * step] != -INFINITY) L += expf(base[s * step] - M) * base[s * step + 1];
         L = warp_sum(L);
         if (lane == 0) { red[0] = M; red[1] = L + (sinks ? expf(sink - M) : 0.f); }
     }
@@ -854,7 +859,10 @@ latent_decode_combine_kernel(const float* __restrict__ part, const int2* __restr
     for (int s0 = 0; s0 < mine.y; s0 += LC_THREADS) {
         const int n = min(LC_THREADS, mine.y - s0);
         __syncthreads();
-        if ((int)threadIdx.x < n) w_s[threadIdx.x] = expf(base[(s0 + threadIdx.x) * step] - M);
+        if ((int)threadIdx.x < n) {
+            const float m = base[(s0 + threadIdx.x) * step];
+            w_s[threadIdx.x] = m == -INFINITY ? -1.f : expf(m - M);      // -1: a slice in which no score was above minus infinity is left out
+        }
         __syncthreads();
         const float* x = base + s0 * step + 2 + c0;
         if (rank % 2 == 0) {                                 // rows of an even number of floats: pairs lie on 8 bytes
@@ -863,14 +871,17 @@ latent_decode_combine_kernel(const float* __restrict__ part, const int2* __restr
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
                     const float2 y = c0 + 2 * LC_THREADS * p < rank ? *reinterpret_cast<const float2*>(x + s * step + 2 * LC_THREADS * p) : make_float2(0.f, 0.f);
-                    v[2 * p] = fmaf(w_s[s], y.x, v[2 * p]);
-                    v[2 * p + 1] = fmaf(w_s[s], y.y, v[2 * p + 1]);
+                    if (!(w_s[s] < 0.f)) {
+                        v[2 * p] = fmaf(w_s[s], y.x, v[2 * p]);
+                        v[2 * p + 1] = fmaf(w_s[s], y.y, v[2 * p + 1]);
+                    }
                 }
         } else {
             for (int s = 0; s < n; ++s)
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
                     const int c = c0 + 2 * LC_THREADS * p;
+                    if (w_s[s] < 0.f) continue;
                     if (c < rank) v[2 * p] = fmaf(w_s[s], x[s * step + 2 * LC_THREADS * p], v[2 * p]);
                     if (c + 1 < rank) v[2 * p + 1] = fmaf(w_s[s], x[s * step + 2 * LC_THREADS * p + 1], v[2 * p + 1]);
                 }

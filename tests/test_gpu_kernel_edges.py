@@ -1146,3 +1146,26 @@ def test_latent_decode_with_slices_that_hold_no_keys(heads, n_splits, window):
         # the weights and the result are rounded to bfloat16, 2^-9 of each; the rest is float32
         bound = 1.1 * 2 ** -8 * (w @ keys[:, :rank].abs()) + 1e-5
         assert ((got[t] - w @ keys[:, :rank]).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("row, rank, heads", [(576, 512, 32), (192, 128, 16), (200, 33, 5), (584, 512, 20), (1600, 512, 4)])
+@pytest.mark.parametrize("below", [(0, 1024), (1024, 2048), (0, 32), (64, 96), (0, 2048)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_latent_decode_over_scores_of_minus_infinity(row, rank, heads, below, sink):
+    """Whole chunks and whole slices of keys whose scores are below the finite weigh nothing, and leave the others' sums alone."""
+    from garlic_inference_b200.ops import kernels
+    page, n = 64, 2048
+    pool, q = rnd(n // page, 1, page, row, seed=1, dtype=torch.bfloat16), rnd(1, heads, row, seed=2, dtype=torch.bfloat16)
+    q[..., -1] = 100.0
+    pool.view(n, row)[below[0]:below[1], -1] = -3e38
+    table = torch.arange(n // page, dtype=torch.int32, device=DEV).view(1, -1)
+    pos, slot, status = (torch.tensor([v], dtype=torch.int32, device=DEV) for v in (n - 1, 0, 0))
+    sinks = rnd(heads, seed=3) if sink else None
+    keys = pool.view(n, row).double()
+    s = q[0].double() @ keys.T * 0.05
+    s[:, below[0]:below[1]] = -math.inf
+    w = torch.softmax(torch.cat([s, sinks.double()[:, None]], 1), -1)[:, :-1] if sink else torch.softmax(s, -1).nan_to_num(0.0)
+    for splits in (1, 2, None):
+        got = kernels.latent_decode(q, pool, table, pos, slot, 0.05, sinks, rank, status, n_splits=splits).view(heads, rank).double()
+        # as in test_latent_decode_with_slices_that_hold_no_keys
+        assert ((got - w @ keys[:, :rank]).abs() <= 1.1 * 2 ** -8 * (w @ keys[:, :rank].abs()) + 1e-5).all()
