@@ -254,72 +254,124 @@ extern "C" int gi_latent_norms(const void* src, long long ld, int q_off, int c_o
 
 // chunks of 32 keys that token t sees, 0 for a row that is none (a recorded step's padding)
 __device__ __forceinline__ int ld_chunks(int t, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, int page_size,
-                                         int max_pages, int window, int* status) {
+                                         int max_pages, int window, bool& bad) {
     const int slot = tok_slot[t], pos = tok_pos[t];
     if (slot < 0 || pos < 0 || pos / page_size >= max_pages) {
-        if (slot >= 0 && status) atomicExch(status, 4);
+        bad = bad || slot >= 0;
         return 0;
     }
     return pos / LD_KEYS - (window > 0 ? max(0, pos - window + 1) : 0) / LD_KEYS + 1;
 }
 
-// Which token's slice, of how many, block b of `n_blocks` takes: every token's chunks are cut into the fewest slices of at most `per`
-// chunks, `per` the least that all tokens' slices are no more than the blocks.  t = -1: none.  By a whole block; warp 0 finds it.
-// With `table`, {first block, slices} of every token is written there.
+// Which token's slice, of how many, block b of `n_blocks` takes (n_blocks >= n_tokens).  Up to LD_SLICED tokens: every token's chunks are cut into the
+// fewest slices of at most `per` chunks, `per` the least (from `least` on) with which all tokens' slices are no more than the blocks.  Beyond, where
+// every one of so many blocks would search for longer than that evens out: as many slices of each, n_blocks / n_tokens.  t = -1: none.  From
+// positions and slots alone, before the kernel ahead has finished: a thread looks a token up, warp 0 searches with them in registers.
+// Measured in a recorded step, 32 heads over rows of 576, us with the tokens looked up in every pass of the search and no limit / so: 1 sequence
+// of 20 tokens 15.5 / 13.9, 64 of 200 to 4,000 112 / 109, 128 of 100 41.6 / 36.9, 256 of 100 93 / 50, 1,000 of 50 to 600 833 / 294; a slice or
+// more of its own length for every sequence 20.5, 186, 39.7, 56, 343.
+#define LD_SLICED (LD_WARPS * 32)
 struct LdSlice { int t, split, n_splits; };
+struct LdFind { LdSlice mine; int chunks[LD_SLICED]; };
 __host__ __device__ __forceinline__ int2* ld_table(float* part, size_t floats) { return reinterpret_cast<int2*>(part + (floats + 1) / 2 * 2); }
-__device__ __forceinline__ LdSlice ld_slice(int b, int n_blocks, int n_tokens, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot,
-                                            int page_size, int max_pages, int window, int2* table, int* status, LdSlice* shared) {
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int total = 0, live = 0;
-        for (int t = lane; t < n_tokens; t += 32) {
-            const int c = ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, table ? status : nullptr);
-            total += c;
-            live += c > 0;
-        }
-        total = __reduce_add_sync(0xffffffffu, total);
-        live = __reduce_add_sync(0xffffffffu, live);
-        int per = max(1, (total + n_blocks - 1) / n_blocks), enough = n_blocks > live ? max(1, (total + n_blocks - live - 1) / (n_blocks - live)) : max(1, total);
-        while (per < enough) {
-            const int tried = (per + enough) / 2;
-            int n = 0;
-            for (int t = lane; t < n_tokens; t += 32) n += (ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, nullptr) + tried - 1) / tried;
-            if (__reduce_add_sync(0xffffffffu, n) <= n_blocks) enough = tried;
-            else per = tried + 1;
-        }
-        int base = 0;
-        if (lane == 0) shared->t = -1;
-        __syncwarp();
-        for (int t0 = 0; t0 < n_tokens; t0 += 32) {
-            const int t = t0 + lane;
-            const int n = t < n_tokens ? (ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, nullptr) + per - 1) / per : 0;
-            int end = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_up_sync(0xffffffffu, end, o);
-                if (lane >= o) end += x;
-            }
-            const int first = base + end - n;
-            if (b >= first && b < first + n) *shared = {t, b - first, n};
-            if (table && t < n_tokens) table[t] = make_int2(first, n);
-            base += __shfl_sync(0xffffffffu, end, 31);
-        }
+// ceil(a / b) for many a: by a multiplication where that is exact (a + b below 2^16, two million positions)
+struct LdCeil {
+    int b;
+    unsigned scale;
+    __device__ __forceinline__ LdCeil(int b_, int most) : b(b_), scale(most + b_ < 65536 ? 0xffffffffu / b_ + 1 : 0u) {}
+    __device__ __forceinline__ int operator()(int a) const {
+        return b == 1 ? a : scale ? (int)__umulhi(a + b - 1, scale) : (int)(((long long)a + b - 1) / b);
     }
-    __syncthreads();
-    return *shared;
+};
+// first[i], count[i]: first block and slices of token 32 i + lane, for the table
+__device__ __forceinline__ void ld_find_slice(int b, int n_blocks, int n_tokens, int least, LdFind* find, int (&first)[LD_SLICED / 32],
+                                              int (&count)[LD_SLICED / 32]) {
+    const int lane = threadIdx.x;
+    int total = 0, live = 0, most = 0;
+#pragma unroll
+    for (int i = 0; i < LD_SLICED / 32; ++i) {
+        if (i * 32 >= n_tokens) break;
+        count[i] = i * 32 + lane < n_tokens ? find->chunks[i * 32 + lane] : 0;
+        total += count[i];
+        live += count[i] > 0;
+        most = max(most, count[i]);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    live = __reduce_add_sync(0xffffffffu, live);
+    most = __reduce_max_sync(0xffffffffu, most);
+    int per = max(least, (total + n_blocks - 1) / n_blocks);
+    int enough = min(max(1, most), max(per, n_blocks > live ? (total + n_blocks - live - 1) / (n_blocks - live) : most));
+    per = min(per, enough);
+    while (per < enough) {
+        const LdCeil slices((per + enough) / 2, most);
+        int n = 0;
+#pragma unroll
+        for (int i = 0; i < LD_SLICED / 32; ++i) {
+            if (i * 32 >= n_tokens) break;
+            n += slices(count[i]);
+        }
+        if (__reduce_add_sync(0xffffffffu, n) <= n_blocks) enough = slices.b;
+        else per = slices.b + 1;
+    }
+    if (lane == 0) find->mine.t = -1;
+    __syncwarp();
+    const LdCeil slices(per, most);
+    int base = 0;
+#pragma unroll
+    for (int i = 0; i < LD_SLICED / 32; ++i) {
+        if (i * 32 >= n_tokens) break;
+        count[i] = slices(count[i]);
+        int end = count[i];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+        }
+        first[i] = base + end - count[i];
+        if (b >= first[i] && b < first[i] + count[i]) find->mine = {i * 32 + lane, b - first[i], count[i]};
+        base += __shfl_sync(0xffffffffu, end, 31);
+    }
 }
 
-// A block's slice, found before the kernel ahead has finished (positions and slots are nobody's output); block 0 writes the table behind
-// the slices' results.  Then: t, slot, pos, its chunks c0 .. c1 - 1, first seen key lo, its results at `my`.
+// By a whole block; waits for the kernel ahead, and writes {first block, slices} of every token to the table.
+__device__ __forceinline__ LdSlice ld_slice(int n_blocks, int n_tokens, int least, const int* __restrict__ tok_pos, const int* __restrict__ tok_slot,
+                                            int page_size, int max_pages, int window, int2* table, int* status, LdFind* find) {
+    gi_pdl_launch_dependents();
+    const int b = blockIdx.x, tid = threadIdx.x;
+    bool bad = false;                            // a row beyond its page table
+    if (n_tokens > LD_SLICED) {
+        const int each = n_blocks / n_tokens, t = b / each;
+        const int chunks = t < n_tokens ? ld_chunks(t, tok_pos, tok_slot, page_size, max_pages, window, bad) : 0;
+        const LdSlice s = {b % each < chunks ? t : -1, b % each, min(each, chunks)};
+        gi_pdl_wait();
+        if (t < n_tokens && s.split == 0 && blockIdx.y == 0 && tid == 0) {
+            table[t] = make_int2(b, s.n_splits);
+            if (bad) atomicExch(status, 4);
+        }
+        return s;
+    }
+    if (tid < n_tokens) find->chunks[tid] = ld_chunks(tid, tok_pos, tok_slot, page_size, max_pages, window, bad);
+    __syncthreads();
+    int first[LD_SLICED / 32], count[LD_SLICED / 32];
+    if (tid < 32) ld_find_slice(b, n_blocks, n_tokens, least, find, first, count);
+    gi_pdl_wait();
+    if (b == 0 && blockIdx.y == 0) {
+        if (tid < 32) {
+#pragma unroll
+            for (int i = 0; i < LD_SLICED / 32; ++i)
+                if (i * 32 + tid < n_tokens) table[i * 32 + tid] = make_int2(first[i], count[i]);
+        }
+        if (bad) atomicExch(status, 4);
+    }
+    __syncthreads();
+    return find->mine;
+}
+
+// A block's slice: t, slot, pos, its chunks c0 .. c1 - 1, first seen key lo, its results at `my`.
 #define LD_FIND_SLICE                                                                                                            \
-    __shared__ LdSlice ld_mine;                                                                                                  \
-    gi_pdl_launch_dependents();                                                                                                  \
-    const bool ld_writes = blockIdx.x == 0 && blockIdx.y == 0;                                                                   \
-    if (ld_writes) gi_pdl_wait();                                                                                                \
-    const LdSlice ld_s = ld_slice(blockIdx.x, n_blocks, n_tokens, tok_pos, tok_slot, page_size, max_pages, window,               \
-                                  ld_writes ? ld_table(part, (size_t)n_blocks * H * stride) : nullptr, status, &ld_mine); \
-    if (!ld_writes) gi_pdl_wait();                                                                                               \
+    __shared__ LdFind ld_mine;                                                                                                   \
+    const LdSlice ld_s = ld_slice(n_blocks, n_tokens, least, tok_pos, tok_slot, page_size, max_pages, window,                    \
+                                  ld_table(part, (size_t)n_blocks * H * stride), status, &ld_mine);                             \
     if (ld_s.t < 0) return;                                                                                                      \
     const int t = ld_s.t, slot = tok_slot[t], pos = tok_pos[t], lo = window > 0 ? max(0, pos - window + 1) : 0;                  \
     const int ld_n = pos / LD_KEYS - lo / LD_KEYS + 1;                                                                           \
@@ -339,7 +391,7 @@ template <int HPW, int DPL2>
 __global__ void __launch_bounds__(LD_WARPS * 32)
 latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
                      const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
-                     int H, int dk, int rank, int page_size, int max_pages, int n_pool_pages, int n_blocks, int n_tokens,
+                     int H, int dk, int rank, int page_size, int max_pages, int n_pool_pages, int n_blocks, int n_tokens, int least,
                      float scale, int* __restrict__ status, int window) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     constexpr int HG = HPW * LD_WARPS;
@@ -461,7 +513,7 @@ __global__ void __launch_bounds__(LD_WARPS * 32, 2)
 latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
                          const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
                          int H, int dk, int rank, int row_words, int page_size, int max_pages, int n_pool_pages,
-                         int n_blocks, int n_tokens, float scale, int* __restrict__ status, int window) {
+                         int n_blocks, int n_tokens, int least, float scale, int* __restrict__ status, int window) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     constexpr int HG = 32, PW = 20;                                  // heads per block; words per row of weights
     const int kw = row_words;                                        // words per staged row, kw % 32 == 4
@@ -630,13 +682,14 @@ latent_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ po
 // with slices of one length / so: 20 sequences of 200 to 4,000 tokens 79 / 54 / 41, 1 of 2,048 37 / 35 / 25, 8 of 2,048 39 / 37 / 27, 32 of
 // 2,048 74 / 66 / 53, 64 of 200 to 4,000 156 / 121 / 112.
 #define LW_STAGES 3
+#define LW_PER_SM(KQ) ((KQ) == 3 ? 2 : 1)        // blocks to an SM
 #define LW_SLD 40            // floats of a row of scores: 8 banks from head to head
 template <int KQ, int NTW>
-__global__ void __launch_bounds__(LD_WARPS * 32, 1)
+__global__ void __launch_bounds__(LD_WARPS * 32, LW_PER_SM(KQ))
 latent_decode_quarters_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, const int* __restrict__ block_table,
                               const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, float* __restrict__ part,
                               int H, int dk, int rank, int row_words, int page_size, int max_pages, int n_pool_pages,
-                              int n_blocks, int n_tokens, float scale, int* __restrict__ status, int window) {
+                              int n_blocks, int n_tokens, int least, float scale, int* __restrict__ status, int window) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     constexpr int HG = 32, PW = 20;                                  // heads per block; words per row of weights
     const int kw = row_words;                                        // words per staged row, kw % 32 == 4
@@ -917,7 +970,7 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
                "gi_latent_decode: rows of %d (a multiple of 8) with %d value columns (at most 512)", dk, rank);
     GI_REQUIRE(n_splits >= 1 && n_splits <= 64 && H <= 65535 && n_tokens <= 65535, "gi_latent_decode: slices, heads, tokens");
     if (n_tokens == 0) return 0;
-    int n_blocks = n_tokens * n_splits;
+    int n_blocks = n_tokens * n_splits, least = 1;
     const int2* table = ld_table(part, (size_t)n_blocks * H * (rank + 2));
     GI_REQUIRE((uintptr_t)part % 8 == 0, "gi_latent_decode: the work space must start on 8 bytes");
     cudaStream_t s = (cudaStream_t)stream;
@@ -929,18 +982,20 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
         const int NTW = n_tiles > 32 ? 8 : (n_tiles > 16 ? 4 : (n_tiles > 8 ? 2 : 1));
         const size_t smem_q = ((size_t)LW_STAGES * LD_KEYS * kw + 4 * 32 * LW_SLD + 32 * 20 + 32) * 4;
         if (dk <= 576) {
-            // a block to an SM, or two blocks a token where those are more
+            // as many blocks as the chip holds at once, or two a token where those are more.  Tokens that fill it by themselves are cut
+            // into slices of 16 chunks at least: shorter ones cost more blocks than they even out.
             int n_sm = 148, dev = 0;
             if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-            const int groups = (H + 31) / 32, most = n_sm / groups > 2 * n_tokens ? n_sm / groups : 2 * n_tokens;
+            const int groups = (H + 31) / 32, at_once = n_sm * LW_PER_SM(dk <= 192 ? 3 : 9) / groups, most = at_once > 2 * n_tokens ? at_once : 2 * n_tokens;
             if (n_blocks > most) n_blocks = most;
+            if (n_tokens >= at_once) least = 16;
             table = ld_table(part, (size_t)n_blocks * H * (rank + 2));
 #define LDQ_CASE(Q, N)                                                                                                 \
             if ((dk <= 192 ? 3 : 9) == Q && NTW == N) {                                                                \
                 if (int rc = gi_reserve_smem((const void*)latent_decode_quarters_kernel<Q, N>, smem_q, "gi_latent_decode")) return rc; \
                 gi_launch(latent_decode_quarters_kernel<Q, N>, dim3(n_blocks, groups), dim3(LD_WARPS * 32), smem_q, s, (const bf16*)q, \
                           (const bf16*)pool, block_table, tok_pos, tok_slot, part, H, dk, rank, kw, page_size, max_pages, \
-                          n_pool_pages, n_blocks, n_tokens, scale, status, window);                                    \
+                          n_pool_pages, n_blocks, n_tokens, least, scale, status, window);                                    \
             }
             LDQ_CASE(3, 1) LDQ_CASE(3, 2) LDQ_CASE(3, 4) LDQ_CASE(9, 1) LDQ_CASE(9, 2) LDQ_CASE(9, 4) LDQ_CASE(9, 8)
 #undef LDQ_CASE
@@ -956,7 +1011,7 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
                 if (rc) return rc;                                                                                     \
                 gi_launch(latent_decode_mma_kernel<N>, grid_mma, dim3(LD_WARPS * 32), smem_mma, s, (const bf16*)q,     \
                           (const bf16*)pool, block_table, tok_pos, tok_slot, part, H, dk, rank, kw, page_size, max_pages, \
-                          n_pool_pages, n_blocks, n_tokens, scale, status, window);                                                      \
+                          n_pool_pages, n_blocks, n_tokens, least, scale, status, window);                                                      \
             }
             LDM_CASE(1) LDM_CASE(2) LDM_CASE(4) LDM_CASE(8)
 #undef LDM_CASE
@@ -977,7 +1032,7 @@ extern "C" int gi_latent_decode(const void* q, const void* pool, const int* bloc
         if (rc) return rc;                                                                                        \
         gi_launch(latent_decode_kernel<A, B>, grid, dim3(LD_WARPS * 32), smem, s, (const bf16*)q, (const bf16*)pool, \
                   block_table, tok_pos, tok_slot, part, H, dk, rank, page_size, max_pages, n_pool_pages, n_blocks, \
-                  n_tokens, scale, status, window);                                                                                 \
+                  n_tokens, least, scale, status, window);                                                                                 \
     }
     LD_CASE(1, 1) LD_CASE(1, 2) LD_CASE(1, 4) LD_CASE(1, 8)
     LD_CASE(2, 1) LD_CASE(2, 2) LD_CASE(2, 4) LD_CASE(2, 8)

@@ -1128,11 +1128,17 @@ def latent_decode_slices(n: int, heads: int) -> int:
     return max(1, min(16, (320 if blocks <= 32 else 256) // max(1, blocks)))
 
 
-def latent_decode_slices_short(n: int, heads: int) -> int:
-    """The same for rows of up to 576, whose kernel has an SM to itself and cuts all sequences' keys into slices of one length:
-    a block of up to 32 heads to an SM.  In us at 32 heads over rows of 576 and 3 / 4 / 5 slices: 20 sequences of 200 to 4,000 tokens in a
-    step of 32 rows 54 / 45 / 41; 1 sequence of 2,048 at 16 / 32 / 64 21 / 19 / 20."""
-    return max(2, min(32, -(-148 // max(1, n * -(-heads // 32)))))
+def latent_decode_slices_short(n: int, heads: int, row: int = 576) -> int:
+    """The same for rows of up to 576, whose kernel has an SM to itself (half of one for rows of up to 192) and cuts all sequences' keys into
+    slices of one length: a block of up to 32 heads to an SM.  In us at 32 heads over rows of 576 and 3 / 4 / 5 slices: 20 sequences of 200 to
+    4,000 tokens in a step of 32 rows 54 / 45 / 41; 1 sequence of 2,048 at 16 / 32 / 64 21 / 19 / 20.  Beyond LATENT_SLICED rows, where the kernel
+    does not look for a common length, as the other kernels."""
+    if n > LATENT_SLICED:
+        return latent_decode_slices(n, heads)
+    return max(2, min(32, -(-(296 if row <= 192 else 148) // max(1, n * -(-heads // 32)))))
+
+
+LATENT_SLICED = 256
 
 
 def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor, tok_pos: torch.Tensor,
@@ -1150,7 +1156,7 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor
     if one != 1 or pool_row != row:
         raise KernelError(f"a pool {tuple(pool.shape)} does not hold rows of {row} shared by all heads")
     if n_splits is None:
-        n_splits = (latent_decode_slices_short if row <= 576 else latent_decode_slices)(n, heads)
+        n_splits = latent_decode_slices_short(n, heads, row) if row <= 576 else latent_decode_slices(n, heads)
     part = torch.empty(-(-n * n_splits * heads * (rank + 2) // 2) * 2 + 2 * n, dtype=torch.float32, device=q.device)
     out = torch.empty((n, heads * rank), dtype=torch.bfloat16, device=q.device)
     check(l.gi_latent_decode(_ptr(q), _ptr(pool), _ptr(block_table), _ptr(tok_pos), _ptr(tok_slot), _ptr(part),

@@ -1169,3 +1169,30 @@ def test_latent_decode_over_scores_of_minus_infinity(row, rank, heads, below, si
         got = kernels.latent_decode(q, pool, table, pos, slot, 0.05, sinks, rank, status, n_splits=splits).view(heads, rank).double()
         # as in test_latent_decode_with_slices_that_hold_no_keys
         assert ((got - w @ keys[:, :rank]).abs() <= 1.1 * 2 ** -8 * (w @ keys[:, :rank].abs()) + 1e-5).all()
+
+
+@pytest.mark.parametrize("row, rank, heads", [(576, 512, 3), (192, 128, 40), (584, 512, 2), (1600, 512, 1)])
+@pytest.mark.parametrize("n, n_splits", [(64, None), (150, None), (256, None), (256, 1), (257, None), (257, 3), (600, None)])
+def test_latent_decode_of_hundreds_of_sequences(row, rank, heads, n, n_splits):
+    """Both sides of the count up to which slices are of one length: short sequences, one long one, rows that are none, and a row beyond its
+    table that is told and gets zeros."""
+    from garlic_inference_b200.ops import kernels
+    page, per, scale = 32, 30, 0.1
+    table = (torch.arange(n * per, dtype=torch.int32, device=DEV) % 997).view(n, per).flip(0).contiguous()
+    q, pool = rnd(n, heads, row, seed=1, dtype=torch.bfloat16), rnd(997, 1, page, row, seed=2, dtype=torch.bfloat16)
+    pos = torch.tensor([(i * 37) % 90 for i in range(n)], dtype=torch.int32)
+    pos[n // 2], pos[n // 3] = 900, per * page
+    slot = torch.arange(n, dtype=torch.int32)
+    slot[5::11] = -1
+    slot[n // 2], slot[n // 3] = n // 2, n // 3
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = kernels.latent_decode(q, pool, table, pos.to(DEV), slot.to(DEV), scale, None, rank, status, n_splits=n_splits).view(n, heads, rank).double()
+    assert status.item() == 4
+    for t in range(n):
+        if slot[t] < 0 or t == n // 3:
+            assert not got[t].any()
+            continue
+        keys = pool[table[t].long()].reshape(per * page, row)[:pos[t] + 1].double()
+        w = torch.softmax(q[t].double() @ keys.T * scale, -1)
+        # the weights, their sum with them and the result are rounded to bfloat16, 2^-9 of each at most: three times that of what is summed
+        assert ((got[t] - w @ keys[:, :rank]).abs() <= 3.1 * 2 ** -9 * (w @ keys[:, :rank].abs()) + 1e-5).all(), t
