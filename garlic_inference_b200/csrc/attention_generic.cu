@@ -39,6 +39,7 @@
 // aligned to the last key, float32 intermediates).
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 #define AG_WARPS 4
 #define AR_BLOCKS 148        // blocks from which on rows share their fetches
@@ -224,8 +225,10 @@ static int launch_generic(const void* q, const void* k_pool, const void* v_pool,
 }
 
 // The same for prompts of the float32 engine (no window, no chunks, one map): a block takes HR query heads of one key head and TQ
-// neighbouring tokens, whose rows share every key and value that is fetched.  Chunks, warps, sums and their order are the kernel's above for every row, and so
-// are the bits.
+// neighbouring tokens of a sequence, whose rows share every key and value that is fetched.  Where neighbouring tokens are of several sequences
+// (a decode step, short portions) each of these has a block of its own: TQ blocks stand by, one for every token that may be a sequence's first,
+// the first tokens' in front.  Chunks, warps, sums and their order are
+// the kernel's above for every row, and so are the bits.
 // Bound above by the fetches (a block read every key and value of its token for one head, a key's row to a lane); here by the
 // multiply-adds and the operands' reads from shared memory.  Measured, two sequences of up to 300 tokens, 16 heads of 128 on 4 key heads: 213 us a
 // row to a block, 98 us so.
@@ -246,24 +249,28 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
     float* l_s = m_s + AG_WARPS * R;                         // [AG_WARPS][R]
     long long* v_s = reinterpret_cast<long long*>(l_s + AG_WARPS * R);       // [AG_WARPS][32]
     // (a prompt's last tokens first: they see most)
-    const int t0 = (gridDim.x - 1 - blockIdx.x) * TQ, h0 = blockIdx.y * HR, kvh = h0 / (n_q / n_kv);
+    const int t0 = (gridDim.x - 1 - blockIdx.x) * TQ, first = t0 + blockIdx.z, h0 = blockIdx.y * HR, kvh = h0 / (n_q / n_kv);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int pos[TQ], slot[TQ];
+    if (first >= n_tokens) return;
+    auto known = [&](int t) { return tok_slot[t] >= 0 && tok_pos[t] >= 0 && tok_pos[t] / page_size < max_pages; };
+    const int at = tok_slot[first];                          // the block's sequence
+    if (!known(first)) {
+        for (int j = threadIdx.x; j < HR * d_v; j += AG_WARPS * 32) out[((size_t)first * n_q + h0) * d_v + j] = 0.f;
+        if (at >= 0 && threadIdx.x == 0) atomicExch(status, 4);
+        return;
+    }
+    if (first > t0 && tok_slot[first - 1] == at && known(first - 1)) return;        // a block before this one has it
+    // its tokens, and the last position that they see
+    int pos[TQ], n_mine = 0, last = -1;
 #pragma unroll
     for (int i = 0; i < TQ; ++i) {
-        const bool in = t0 + i < n_tokens;
-        slot[i] = in ? tok_slot[t0 + i] : -1;
-        pos[i] = in ? tok_pos[t0 + i] : -1;
-        if (slot[i] < 0 || pos[i] < 0 || pos[i] / page_size >= max_pages) {
-            if (in)
-                for (int j = threadIdx.x; j < HR * d_v; j += AG_WARPS * 32) out[((size_t)(t0 + i) * n_q + h0) * d_v + j] = 0.f;
-            if (slot[i] >= 0 && threadIdx.x == 0) atomicExch(status, 4);
-            slot[i] = -1;
-            pos[i] = -1;
-        }
+        const int t = first + i;
+        if (n_mine == i && t < min(t0 + TQ, n_tokens) && tok_slot[t] == at && known(t)) ++n_mine;
+        pos[i] = i < n_mine ? tok_pos[t] : -1;
+        last = max(last, pos[i]);
     }
-    for (int i = threadIdx.x; i < R * d; i += AG_WARPS * 32) {
-        const int r = i / d, t = t0 + r / HR;
+    for (int i = threadIdx.x; i < n_mine * HR * d; i += AG_WARPS * 32) {
+        const int r = i / d, t = first + r / HR;
         q_s[i] = t < n_tokens ? q[((size_t)t * n_q + h0 + r % HR) * d + i % d] * scale : 0.f;
     }
     __syncthreads();
@@ -274,20 +281,10 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
 #pragma unroll
         for (int e = 0; e < DPL; ++e) acc[r][e] = 0.f;
     }
-    // tokens of one sequence at a time: mostly all of them
-    for (int first = 0; first < TQ; ++first) {
-        int at = -1, last = -1;                              // (over a run of tokens with the slot of the first that is left)
-        bool begins = true;
-#pragma unroll
-        for (int i = 0; i < TQ; ++i) {
-            if (i == first) at = slot[i];
-            if (i < first && slot[i] == (first < TQ ? tok_slot[min(t0 + first, n_tokens - 1)] : -1) && slot[i] >= 0) begins = false;
-        }
-        if (at < 0 || !begins) continue;
-#pragma unroll
-        for (int i = 0; i < TQ; ++i)
-            if (slot[i] == at) last = max(last, pos[i]);
-        const int* bt = block_table + (size_t)at * max_pages;
+    // the rows 0 .. ROWS - 1
+    const int* bt = block_table + (size_t)at * max_pages;
+    auto walk = [&](auto rows) {
+        constexpr int ROWS = decltype(rows)::value;
         for (int c = warp; c <= last / 32; c += AG_WARPS) {
             const int j = c * 32 + lane;
             long long row = -1, vrow = -1;                   // element offsets of this lane's key and value rows
@@ -299,16 +296,16 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
                     vrow = (((long long)page * n_kv + kvh) * page_size + (j - lp * page_size)) * v_row;
                 }
             }
-            float a[R];
+            float a[ROWS];
 #pragma unroll
-            for (int r = 0; r < R; ++r) a[r] = 0.f;
+            for (int r = 0; r < ROWS; ++r) a[r] = 0.f;
             if (row >= 0) {
                 const float4* kr = reinterpret_cast<const float4*>(k_pool + row);
 #pragma unroll 8
                 for (int i = 0; i < d / 4; ++i) {
                     const float4 k = kr[i];
 #pragma unroll
-                    for (int r = 0; r < R; ++r) {
+                    for (int r = 0; r < ROWS; ++r) {
                         const float4 x = *reinterpret_cast<const float4*>(q_s + r * d + 4 * i);
                         const float y[4] = {x.x, x.y, x.z, x.w};
                         a[r] += dot_vec(k, y);
@@ -317,10 +314,10 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
             }
             __syncwarp();                                    // the chunk before is done with
             v_s[warp * 32 + lane] = vrow;
-            bool any[R];
+            bool any[ROWS];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const bool sees = slot[r / HR] == at && row >= 0 && j <= pos[r / HR];
+            for (int r = 0; r < ROWS; ++r) {
+                const bool sees = row >= 0 && j <= pos[r / HR];
                 const float s = sees ? a[r] : -INFINITY, cmax = warp_max(s);
                 any[r] = cmax != -INFINITY;
                 float p = 0.f;
@@ -347,7 +344,7 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
                     for (int e = 0; e < DPL; ++e) v[jj][e] = there[jj] && lane + 32 * e < d_v ? v_pool[vj + lane + 32 * e] : 0.f;
                 }
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
+                for (int r = 0; r < ROWS; ++r) {
                     const float4 p4 = *reinterpret_cast<const float4*>(p_s + (warp * R + r) * 32 + j4);
                     const float p[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
@@ -359,7 +356,10 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
                 }
             }
         }
-    }
+    };
+    if (n_mine == 1) walk(std::integral_constant<int, HR>{});
+    else if (TQ > 2 && n_mine == 2) walk(std::integral_constant<int, 2 * HR>{});
+    else walk(std::integral_constant<int, R>{});
     if (lane == 0)
 #pragma unroll
         for (int r = 0; r < R; ++r) { m_s[warp * R + r] = m[r]; l_s[warp * R + r] = l[r]; }
@@ -369,9 +369,8 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
         for (int e = 0; e < DPL; ++e)
             if (lane + 32 * e < dw) acc_s[(warp * R + r) * dw + lane + 32 * e] = acc[r][e];
     __syncthreads();
-    for (int i = threadIdx.x; i < R * d_v; i += AG_WARPS * 32) {
+    for (int i = threadIdx.x; i < n_mine * HR * d_v; i += AG_WARPS * 32) {
         const int r = i / d_v, c = i % d_v, t = r / HR;
-        if (tok_slot[min(t0 + t, n_tokens - 1)] < 0 || t0 + t >= n_tokens || tok_pos[t0 + t] < 0 || tok_pos[t0 + t] / page_size >= max_pages) continue;
         float M = -INFINITY;
         for (int w = 0; w < AG_WARPS; ++w) M = fmaxf(M, m_s[w * R + r]);
         const float sink = sinks ? load_w(sinks, sink_dtype, h0 + r % HR) : -INFINITY;
@@ -381,7 +380,7 @@ attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k
         if (sinks) L += expf(sink - M);
         for (int w = 0; w < AG_WARPS; ++w)
             if (m_s[w * R + r] != -INFINITY) v += expf(m_s[w * R + r] - M) * acc_s[(w * R + r) * dw + c];
-        out[((size_t)(t0 + t) * n_q + h0 + r % HR) * d_v + c] = L > 0.f ? v / L : 0.f;
+        out[((size_t)(first + t) * n_q + h0 + r % HR) * d_v + c] = L > 0.f ? v / L : 0.f;
     }
 }
 
@@ -394,13 +393,13 @@ static int launch_shared_rows(const float* q, const float* k_pool, const float* 
     const size_t smem = ((size_t)R * d + (size_t)AG_WARPS * R * dw + (size_t)AG_WARPS * R * 34) * sizeof(float) + AG_WARPS * 32 * sizeof(long long);
     const auto kernel = attn_shared_rows_kernel<DPL, HR, TQ>;
     if (int rc = gi_reserve_smem((const void*)kernel, smem, "gi_attention_generic")) return rc;
-    gi_launch(kernel, dim3((n_tokens + TQ - 1) / TQ, n_q / HR), dim3(AG_WARPS * 32), smem, s, q, k_pool, v_pool, block_table, tok_pos, tok_slot, out,
+    gi_launch(kernel, dim3((n_tokens + TQ - 1) / TQ, n_q / HR, TQ), dim3(AG_WARPS * 32), smem, s, q, k_pool, v_pool, block_table, tok_pos, tok_slot, out,
               n_tokens, n_q, n_kv, d, page_size, max_pages, n_pool_pages, scale, sinks, sink_dtype, d_v, status, v_row);
     return gi_check_launch("gi_attention_generic");
 }
 
 // The general entry point: everything the file's head lists.  `out` is written in the activation type unless
-// `out_f32` is given.  Key rows whose width is a multiple of 16 bytes are read with vector loads, others
+// `out_f32` is given.  single: every token is of a sequence of its own (a decode step), which only the choice of kernel heeds.  Key rows whose width is a multiple of 16 bytes are read with vector loads, others
 // element by element; value rows may have any width.
 extern "C" int gi_attention_masked(const void* q, const void* k_pool, const void* v_pool, int act_dtype,
                                    const int* block_table, const int* tok_pos, const int* tok_slot,
@@ -409,7 +408,7 @@ extern "C" int gi_attention_masked(const void* q, const void* k_pool, const void
                                    int sink_dtype, int d_v, int* status, int chunk, int n_vh, int v_row, int maps,
                                    float* out_f32, const float* dist_bias, int n_dist, const void* mean_k,
                                    const void* mean_v, const int* mean_table, int mean_block, int mean_rows,
-                                   int mean_max_pages, int mean_pages, int keep_first, void* stream) {
+                                   int mean_max_pages, int mean_pages, int keep_first, int single, void* stream) {
     GI_REQUIRE(keep_first >= 0 && (keep_first == 0 || (window > 0 && chunk == 0 && mean_block == 0)), "gi_attention_generic: "
                "kept first tokens come with a window, without chunks and rows for blocks");
     GI_REQUIRE(n_tokens >= 0 && n_q > 0 && n_kv > 0 && d > 0, "gi_attention_generic: sizes must be positive");
@@ -430,9 +429,12 @@ extern "C" int gi_attention_masked(const void* q, const void* k_pool, const void
     cudaStream_t s = (cudaStream_t)stream;
     // Many tokens of plain heads in float32: rows that share their fetches, where that leaves a block for every SM.  In us, a block a row / so,
     // 16 heads of 128 on 4 key heads, new tokens behind cached ones: 32 behind none 15 / 21, 64 behind none 17 / 22, 64 behind 2,000 357 / 220, 128
-    // behind none 42 / 26, 400 behind none 260 / 103; on 8 key heads 128 behind none 42 / 24; 32 heads of 64 100 behind none 39 / 19.
+    // behind none 44 / 28, 400 behind none 261 / 100; on 8 key heads 128 behind none 46 / 28; 32 heads of 64 on 8 100 behind none 39 / 19; 64 single
+    // tokens of 32 heads of 128 on 8 behind 2,000 846 / 472, 60 and a portion of 300 behind 500 1,240 / 353.  Not where every token is of a
+    // sequence of its own and so is every head (`single`, one query head a key head): nothing is shared then, and the registers leave fewer
+    // warps to wait: 64 of 16 heads of 128 behind 300 104 / 123.
     const int group = n_q / n_kv, hr = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1, tq = hr == 4 ? 2 : 4;
-    if (act_dtype == GI_DTYPE_F32 && (long long)((n_tokens + tq - 1) / tq) * (n_q / hr) >= AR_BLOCKS && window == 0 && chunk == 0 && maps == 1 && out && !out_f32 && !dist_bias && mean_block == 0 &&
+    if (act_dtype == GI_DTYPE_F32 && !(single && hr == 1) && (long long)((n_tokens + tq - 1) / tq) * (n_q / hr) >= AR_BLOCKS && window == 0 && chunk == 0 && maps == 1 && out && !out_f32 && !dist_bias && mean_block == 0 &&
         n_vh == n_kv && d % 4 == 0 && d <= 128 && d_v <= 128 && (uintptr_t)q % 16 == 0) {
 #define AR_LAUNCH(DPL, HR, TQ) return launch_shared_rows<DPL, HR, TQ>((const float*)q, (const float*)k_pool, (const float*)v_pool, block_table, tok_pos, \
             tok_slot, (float*)out, n_tokens, n_q, n_kv, d, page_size, max_pages, n_pool_pages, scale, sinks, sink_dtype, d_v, status, v_row, s)
@@ -462,9 +464,9 @@ extern "C" int gi_attention_generic(const void* q, const void* k_pool, const voi
                                     const int* block_table, const int* tok_pos, const int* tok_slot,
                                     void* out, int n_tokens, int n_q, int n_kv, int d, int page_size,
                                     int max_pages, int n_pool_pages, int window, float scale, const void* sinks,
-                                    int sink_dtype, int d_v, int* status, void* stream) {
+                                    int sink_dtype, int d_v, int* status, int single, void* stream) {
     GI_REQUIRE(d_v > 0 && d_v <= d, "gi_attention_generic: %d value columns of rows of %d", d_v, d);
     return gi_attention_masked(q, k_pool, v_pool, act_dtype, block_table, tok_pos, tok_slot, out, n_tokens, n_q, n_kv, d,
                                page_size, max_pages, n_pool_pages, window, scale, sinks, sink_dtype, d_v, status, 0, n_kv, d,
-                               1, nullptr, nullptr, 0, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, stream);
+                               1, nullptr, nullptr, 0, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, single, stream);
 }

@@ -269,10 +269,11 @@ def qk_norm_rope_append(qkv: torch.Tensor, n_q: int, n_kv: int, head_dim: int,
 def attention_generic(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor,
                       tok_pos: torch.Tensor, tok_slot: torch.Tensor, scale: float, window: int,
                       status: torch.Tensor, sinks: Optional[torch.Tensor] = None,
-                      value_dim: Optional[int] = None) -> torch.Tensor:
+                      value_dim: Optional[int] = None, single: bool = False) -> torch.Tensor:
     """Exact-order attention of q [n, n_q, d] over the paged cache; returns [n, n_q * value_dim] (value_dim = d
     unless given: the first columns of the value rows).  `sinks` [n_q]: a number per head that joins the
-    softmax's denominator as exp(sink), without a value."""
+    softmax's denominator as exp(sink), without a value.  `single`: every token is of a sequence of its own (a decode step):
+    the same bits, perhaps by another kernel."""
     l = require_gpu()
     _dense(q, "q")
     n, n_q, d = q.shape
@@ -291,7 +292,7 @@ def attention_generic(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
     check(l.gi_attention_generic(_ptr(q), _ptr(k_pool), _ptr(v_pool), code(q.dtype), _ptr(block_table),
                                  _ptr(tok_pos), _ptr(tok_slot), _ptr(out), n, n_q, n_kv, d, page_size,
                                  block_table.shape[1], n_pages, int(window or 0), float(scale), _ptr(sinks),
-                                 code(sinks.dtype) if sinks is not None else F32, d_v, _ptr(status), _stream()), l)
+                                 code(sinks.dtype) if sinks is not None else F32, d_v, _ptr(status), int(single), _stream()), l)
     return out
 
 
@@ -323,7 +324,7 @@ def attention_masked(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor
                                 _ptr(tok_slot), None if out_float32 else _ptr(out), n, n_q, n_kv, d, page_size,
                                 block_table.shape[1], n_pages, int(window or 0), float(scale), _ptr(sinks), F32, dv,
                                 _ptr(status), int(chunk or 0), n_vh, dv, int(maps), _ptr(out) if out_float32 else None,
-                                _ptr(dist_bias), n_dist, *_means_args(means, k_pool, v_pool), int(keep_first), _stream()), l)
+                                _ptr(dist_bias), n_dist, *_means_args(means, k_pool, v_pool), int(keep_first), 0, _stream()), l)
     return out
 
 

@@ -33,8 +33,8 @@ _SIGNATURES = {
     "gi_cast": ([P, I, P, I, L, P], I),
     "gi_qk_norm_rope_append": ([P, P, P, P, I, P, P, I, F, P, P, I, P, P, P,
                                 I, I, I, I, I, I, I, I, I, P, P], I),
-    "gi_attention_generic": ([P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P, I, I, P, P], I),
-    "gi_attention_masked": ([P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P, I, I, P, I, I, I, I, P, P, I, P, P, P, I, I, I, I, I, P], I),
+    "gi_attention_generic": ([P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P, I, I, P, I, P], I),
+    "gi_attention_masked": ([P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, F, P, I, I, P, I, I, I, I, P, P, I, P, P, P, I, I, I, I, I, I, P], I),
     "gi_attn_prepare": ([P, I, L, I, I, I, P, I, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P, I, P, I, F, F, I,
                          P, P, P, I, I, I, I, F, F, P], I),
     "gi_pool_blocks": ([P, P, I, P, P, P, I, I, I, I, I, I, I, I, P, P, P, P, I, I, I, I, P], I),

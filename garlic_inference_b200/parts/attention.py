@@ -159,7 +159,7 @@ class GQAAttention(Mixer):
                 return kernels.attention_prefill_bf16(q, kv.k_pool, kv.v_pool, kv.block_table, self._runs(ctx, 64),
                                                       self.scale, self.window or 0, rows_covered=covered)
         return kernels.attention_generic(q, kv.k_pool, kv.v_pool, kv.block_table, ctx.tok_pos, ctx.tok_slot,
-                                         self.scale, self.window or 0, ctx.status)
+                                         self.scale, self.window or 0, ctx.status, single=ctx.all_single)
 
 
 register_part(GQAAttention.kind, GQAAttention)

@@ -1093,6 +1093,28 @@ def test_float32_attention_of_rows_that_share_their_fetches(H, G, d, dv, page, l
             torch.testing.assert_close(got[at].view(G, H // G, dv).double(), torch.einsum("ghk,gkd->ghd", w, vals[..., :dv]), rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("H, G, d", [(4, 4, 128), (6, 3, 64), (16, 4, 100), (3, 3, 40)])
+@pytest.mark.parametrize("lens", [[1] * 200, [3] * 67, [2, 5, 1, 7] * 13, [150] + [1] * 61])
+@pytest.mark.parametrize("single", [False, True])
+def test_float32_attention_of_neighbours_of_several_sequences(H, G, d, lens, single):
+    """Single tokens and short portions side by side, rows that are none and a row beyond its table between them: the bits of a token alone."""
+    from garlic_inference_b200.ops import kernels
+    page, per, n = 16, 12, sum(lens)
+    table = torch.arange(len(lens) * per, dtype=torch.int32, device=DEV).view(len(lens), per).flip(0).contiguous()
+    kp, vp = rnd(len(lens) * per, G, page, d, seed=1), rnd(len(lens) * per, G, page, d, seed=2)
+    past = [(i * 7) % 40 for i in range(len(lens))]
+    pos = torch.cat([torch.arange(p, p + m) for p, m in zip(past, lens)]).to(torch.int32)
+    slot = torch.cat([torch.full((m,), i) for i, m in enumerate(lens)]).to(torch.int32)
+    slot[9::23], slot[n - 1], pos[n // 2] = -1, -1, per * page
+    pos, slot, q = pos.to(DEV), slot.to(DEV), rnd(n, H, d, seed=3)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    got = kernels.attention_generic(q, kp, vp, table, pos, slot, d ** -0.5, 0, status, single=single)
+    assert status.item() == 4
+    want = torch.cat([kernels.attention_generic(q[i:i + 1].contiguous(), kp, vp, table, pos[i:i + 1].contiguous(), slot[i:i + 1].contiguous(),
+                                                d ** -0.5, 0, status) for i in range(n)])
+    assert torch.equal(got, want) and not got[n // 2].any() and not got[n - 1].any()
+
+
 # ---- one token per sequence over latent rows ---------------------------------------------------------------------------
 @pytest.mark.parametrize("row, rank, heads", [(576, 512, 32), (200, 192, 17), (72, 65, 40), (64, 33, 1), (584, 512, 20)])
 @pytest.mark.parametrize("pos, n_splits", [([0], None), ([31, 32, 700, -1, 5, 63], None), ([300] * 40 + [-1], 2), ([2000, 3], 1)])
