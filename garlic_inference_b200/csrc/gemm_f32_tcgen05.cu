@@ -47,7 +47,7 @@ struct GfControl {
 template <int NT> struct GfShape {
     static constexpr int PART = NT * GF_BK * 2;                                   // bytes of one part of A in a slice
     // slices of W and of A's parts in shared memory: W's are let go once they are split, A's after their products
-    static constexpr int WS = NT == 128 ? 2 : NT == 16 ? 5 : NT == 32 ? 4 : 3, AS = NT == 128 || NT == 96 ? 3 : NT == 64 ? 4 : NT == 32 ? 6 : 8;
+    static constexpr int WS = NT == 128 ? 2 : NT == 16 ? 5 : NT == 96 ? 3 : 4, AS = NT == 128 || NT == 96 ? 3 : NT == 64 ? 4 : NT == 32 ? 6 : 8;
     static constexpr int ACCS = NT <= 32 ? 4 : NT <= 96 ? 3 : 2, SPLITS = NT <= 32 ? 4 : NT == 64 ? 3 : 2;      // accumulators and split slices in tensor memory
     static_assert(WS <= GF_RING && AS <= GF_RING && SPLITS <= GF_RING, "rings");
     static_assert(ACCS * NT + SPLITS * GF_A_COLS <= GF_TMEM_COLS, "tensor memory");
@@ -106,6 +106,9 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int it = warp >> 2; it < own; it += 2) {
             const int s = it % S::WS, last = it - S::SPLITS;                    // the slice that had these columns before
             const uint32_t at = split0 + it % S::SPLITS * GF_A_COLS + ((uint32_t)(q * 32) << 16);
+            // In a ring of odd length the slice before this one in its place is the other group's, and may not even have landed: the barrier
+            // would then be a phase behind, and its parity say that this slice is there.  So first wait until that one has been let go.
+            if (S::WS % 2 && it >= S::WS && !t5_warp_wait(&ctl->w_empty[s], (it / S::WS & 1) ^ 1, abort, error_flag, GF_ERR_SPLIT)) break;
             if (!t5_warp_wait(&ctl->w_full[s], it / S::WS & 1, abort, error_flag, GF_ERR_SPLIT)) break;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {

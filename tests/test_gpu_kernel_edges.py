@@ -341,6 +341,31 @@ def test_every_form_of_the_float32_product_gives_the_same_bits(M, N, K):
     kernels.check_bounded_waits(DEV)
 
 
+@pytest.mark.parametrize("M, N", [(5, 1000), (64, 512), (130, 260)])
+def test_float32_product_of_long_rows(M, N):
+    """Rings that go round many times in every form, with the sums kept and left in memory, W not in the L2 cache: the same bits time after
+    time, within the error of float32 sums."""
+    from garlic_inference_b200.ops import kernels
+    from garlic_inference_b200.ops.library import check, require_gpu
+    l, flag, K = require_gpu(), kernels.tcgen05_error_flag(torch.device(DEV, 0)), 17408
+    a, w, other = rnd(M, K, seed=1), rnd(N, K, seed=2), torch.empty(256 << 20, dtype=torch.uint8, device=DEV)
+    want = a.double() @ w.double().T
+    tol = (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)               # a rounding an addition
+    space = torch.empty(6 * M * K + 4 * M * N * (K // 64) + 512, dtype=torch.uint8, device=DEV)
+    first = None
+    for tile in (16, 32, 64, 96, 128):
+        for shares in (1, 4, 9):
+            for _ in range(4):
+                other.zero_()
+                out = torch.full((M, N), 7.0, device=DEV)
+                check(l.gi_sgemm_split_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), space.data_ptr(), space.numel(), M, N, K, K, N, tile, shares,
+                                          flag.data_ptr(), 0), l)
+                first = out if first is None else first
+                assert torch.equal(out, first), (tile, shares)
+    assert ((first.double() - want).abs() <= tol).all()
+    kernels.check_bounded_waits(DEV)
+
+
 @pytest.mark.parametrize("M", [2097120, 2097121, 4194240])
 @pytest.mark.parametrize("N", [3, 16])
 def test_float32_product_of_millions_of_rows(M, N):
