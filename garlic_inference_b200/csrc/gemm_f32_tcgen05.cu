@@ -1,7 +1,7 @@
 // True float32 matrix product for the 32-bit engine on tensor cores: C[M,N] = A[M,K] . W[N,K]^T for weights of a million elements
 // and more (gemm_f32.cu has the others).  Upstream has no 32-bit path.
 //
-// A float32 number is the exact sum of three bfloat16 numbers, and products of those are exact in float32.  Of the nine
+// 2^24 times a float32 number is the exact sum of three bfloat16 numbers (gf_split), and products of those are exact in float32.  Of the nine
 // products of two such sums the six largest are made (what is left out is at most 2^-25 of a product, below its rounding to
 // float32).  The accumulator starts from zero for every 64 inputs, takes the five small products of all of them first and the
 // large one last, and these sums meet in registers by float32 adds that round to nearest, in ascending order: the tensor
@@ -56,14 +56,53 @@ template <int NT> struct GfShape {
     static_assert(SMEM <= 232448, "shared memory");
 };
 
-// A finite sum, or the output by float32 FMAs in order: the parts of an infinity (and of a number that rounds up to one) are none.
+// The parts of 2^24 x: of x itself the third would fall under bfloat16's smallest number from 2^-110 down (and the second from 2^-118 down), so
+// every float32 number, subnormal ones too, is the exact sum of its parts.  A sum is 2^48 times the output; one that passes the largest
+// number with that (an output of 2^80 and more, or an input of 2^104) is not finite and made by FMAs.
+#define GF_SCALE 16777216.f
+#define GF_UNSCALE (1.f / (GF_SCALE * GF_SCALE))
+__device__ __forceinline__ void gf_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    t5_apart(t5_mul2(t5_pair(x, y), t5_pair(GF_SCALE, GF_SCALE)), x, y);
+    t5_split3(x, y, hi, mid, lo);
+}
+
+__device__ __forceinline__ bool gf_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// An output whose sum is not finite (the parts of an infinity, and of a number that rounds up to one, are none), by float32 FMAs in order.  K
+// is a multiple of 4 and w starts on 16 bytes; 16 words of w are under way at a time.  In us, W of 2,048 x 2,048, one row of A with an
+// infinity / all: 300 rows 80 / 1,385 (a float at a time, in front of the stores, 212 / 9,121), 1 row 165 (569), 8 521 / 714 (1,381 / 2,059); finite
+// 34, 14 and 15.
 __device__ __noinline__ float gf_plain(const float* a, const float* w, int K) {
     float s = 0.f;
-    for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += 64) {
+        float4 x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = *reinterpret_cast<const float4*>(w + min(k0 + 4 * i, K - 4));
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float* y = a + k0 + 4 * i;
+            if (k0 + 4 * i < K) { s = fmaf(y[0], x[i].x, s); s = fmaf(y[1], x[i].y, s); s = fmaf(y[2], x[i].z, s); s = fmaf(y[3], x[i].w, s); }
+        }
+    }
     return s;
 }
-__device__ __forceinline__ float gf_finite(float v, const float* a, const float* w, int K) {
-    return fabsf(v) <= 3.402823466e38f ? v : gf_plain(a, w, K);
+// The same for eight rows of A, which a word of w is fetched once for: where many outputs are not finite.
+struct GfEight { float v[8]; };
+__device__ __noinline__ GfEight gf_eight(const float* a, long long lda, int rows, const float* w, int K) {
+    GfEight s;
+    const float* of[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { s.v[j] = 0.f; of[j] = a + (long long)min(j, rows - 1) * lda; }
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(w + k);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float* y = of[j] + k;
+            s.v[j] = fmaf(y[0], x.x, s.v[j]); s.v[j] = fmaf(y[1], x.y, s.v[j]); s.v[j] = fmaf(y[2], x.z, s.v[j]); s.v[j] = fmaf(y[3], x.w, s.v[j]);
+        }
+    }
+    return s;
 }
 
 // sums: nothing, or where the sums of 64 inputs go ([sum][M][N]) when `shares` blocks share the inputs of a tile.
@@ -117,8 +156,8 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const float4 v = *reinterpret_cast<const float4*>(src + ((c ^ swap) << 4));      // as the 128-byte swizzle put them
-                    t5_split3(v.x, v.y, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
-                    t5_split3(v.z, v.w, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
+                    gf_split(v.x, v.y, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
+                    gf_split(v.z, v.w, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
                 }
                 if (half == 0) {
                     if (last >= 0 && !t5_warp_wait(&ctl->done[last % GF_RING], last / GF_RING & 1, abort, error_flag, GF_ERR_SPLIT)) { it = own; break; }
@@ -174,14 +213,37 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                             sums[((size_t)u * M + m0 + c) * N + n] = pair[c % 2];
                         }
             }
-            if (ok && !sums && n < N)
+            if (!ok || sums) continue;
+            bool finite = true;
 #pragma unroll
-                for (int c = 0; c < COLS; ++c)
-                    if (m0 + c < M) {
-                        float pair[2];
-                        t5_apart(sum[c / 2], pair[0], pair[1]);
-                        C[(size_t)(m0 + c) * ldc + n] = gf_finite(pair[c % 2], A + (size_t)(m0 + c) * lda, W + (size_t)n * K, K);
+            for (int c = 0; c < COLS; ++c)
+                if (n < N && m0 + c < M) {
+                    float pair[2];
+                    t5_apart(sum[c / 2], pair[0], pair[1]);
+                    finite = finite && gf_finite(pair[c % 2]);
+                    C[(size_t)(m0 + c) * ldc + n] = pair[c % 2] * GF_UNSCALE;
+                }
+            if (!__all_sync(0xffffffffu, finite))            // (what is not finite is so in C too)
+                for (int c0 = 0; c0 < min(COLS, M - m0); c0 += 8) {
+                    const int rows = min(8, M - m0 - c0), of = min(n, N - 1);
+                    unsigned mine = 0;                       // this lane's outputs that are not finite
+                    int columns = 0;
+                    for (int c = 0; c < rows; ++c) {
+                        const bool odd = n < N && !gf_finite(C[(size_t)(m0 + c0 + c) * ldc + of]);
+                        mine |= (unsigned)odd << c;
+                        columns += __any_sync(0xffffffffu, odd);
                     }
+                    const float *a = A + (size_t)(m0 + c0) * lda, *w = W + (size_t)of * K;
+                    if (columns > 2) {
+                        const GfEight v = gf_eight(a, lda, rows, w, K);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            if (mine >> c & 1) C[(size_t)(m0 + c0 + c) * ldc + n] = v.v[c];
+                    } else {
+                        for (int c = 0; c < rows; ++c)
+                            if (mine >> c & 1) C[(size_t)(m0 + c0 + c) * ldc + n] = gf_plain(a + c * lda, w, K);
+                    }
+                }
         }
     } else if (NT == GF_FEW && warp == 17) {
         // few rows: this warp makes their parts itself, which saves a launch.  Two lanes to a row, 32 inputs each, a slice ahead.
@@ -213,8 +275,8 @@ sgemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             uint32_t part[3][16];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                t5_split3(v[c].x, v[c].y, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
-                t5_split3(v[c].z, v[c].w, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
+                gf_split(v[c].x, v[c].y, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
+                gf_split(v[c].z, v[c].w, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
             }
             if (it + 1 < own) fetch();
             if (last >= 0 && !t5_warp_wait(&ctl->done[last % GF_RING], last / GF_RING & 1, abort, error_flag, GF_ERR_COPY)) break;
@@ -305,7 +367,7 @@ add_sums_kernel(const float* __restrict__ sums, const float* __restrict__ A, con
 #pragma unroll 8
         for (int u = 0; u < n_sums; ++u) v += sums[u * total + i];
         const long long m = i / N, n = i - m * N;
-        C[m * ldc + n] = gf_finite(v, A + m * lda, W + n * K, K);
+        C[m * ldc + n] = gf_finite(v) ? v * GF_UNSCALE : gf_plain(A + m * lda, W + n * K, K);
     }
 }
 
@@ -320,7 +382,7 @@ split_rows_kernel(const float* __restrict__ A, uint32_t* __restrict__ parts, int
         const int k = (int)(i - m * pairs) * 2;
         const float* a = A + m * lda + k;
         uint32_t hi, mid, lo;
-        t5_split3(k < K ? a[0] : 0.f, k + 1 < K ? a[1] : 0.f, hi, mid, lo);
+        gf_split(k < K ? a[0] : 0.f, k + 1 < K ? a[1] : 0.f, hi, mid, lo);
         parts[i] = hi;
         parts[total + i] = mid;
         parts[2 * total + i] = lo;
@@ -330,10 +392,11 @@ split_rows_kernel(const float* __restrict__ A, uint32_t* __restrict__ parts, int
 // Which form takes the least time, by what was measured: microseconds a slice of 64 inputs by NT (16: the rows are split by one warp
 // a block, the others: a launch before), and what further launches cost.  Shares of the inputs where the tiles would leave half
 // of the SMs idle: the sums go through memory.
-// In us, this file's product / FMAs in order (gemm_f32.cu), rows x N x K: 1 x 1,024 x 1,024 9.6 / 9.0, 1 x 2,048 x 2,048 14 / 17, 1 x 2,048 x 5,632
-// 25 / 46, 8 x 11,264 x 2,048 27 / 54, 17 x 2,048 x 2,048 17 / 30, 100 x 6,144 x 1,024 22 / 62, 491 x 1,024 x 1,024 20 / 51,
-// 491 x 2,048 x 2,048 37 / 129, 491 x 11,264 x 2,048 135 / 500, 491 x 2,048 x 5,632 83 / 343.  64 rows of A take 0.82 us a slice where the
-// tensor core alone takes 0.41: the hand-overs between the four roles; 128 rows are bound by it, but leave more SMs idle.
+// In us, this file's product / FMAs in order (gemm_f32.cu), rows x N x K: 1 x 1,024 x 1,024 8.5 / 8.7, 1 x 2,048 x 2,048 14 / 18, 1 x 2,048 x 5,632
+// 25 / 46, 1 x 11,264 x 2,048 34 / 31, 8 x 11,264 x 2,048 33 / 57, 17 x 2,048 x 2,048 17 / 34, 100 x 6,144 x 1,024 22 / 77, 491 x 1,024 x 1,024 18 / 121,
+// 491 x 2,048 x 2,048 36 / 308, 491 x 11,264 x 2,048 124 / 503, 491 x 2,048 x 5,632 82 / 833, 2,048 x 11,264 x 2,048 517 / 1,722.  Rows of A take 0.82 us a
+// slice (64) and 1.55 (128) where the products alone, 24 of 128 x 64 or 128 x 16, take 0.39 and 0.78: the hand-overs between the
+// four roles bound both.
 struct GfPlan { int nt, shares; };
 static GfPlan gf_plan(int M, int N, int K, int n_sm) {
     const int all = (K + GF_BK - 1) / GF_BK, n_tiles = (N + GF_ROWS - 1) / GF_ROWS;

@@ -139,7 +139,8 @@ __device__ __forceinline__ void t5_st16(uint32_t at, const uint32_t (&r)[16]) {
 }
 
 // {x, y} as three pairs of bfloat16 that sum to them exactly: each part is what is left, rounded to nearest, so that a part is at most
-// 2^-9 of the one before it (24 bits of mantissa = 8 + 8 + 8).  Not for infinities, NaN and what rounds to an infinity.
+// 2^-9 of the one before it (24 bits of mantissa = 8 + 8 + 8).  Not for infinities, NaN and what rounds to an infinity, and below 2^-110 only to
+// 2^-134, half of bfloat16's smallest number.
 typedef unsigned long long t5_f2;             // two floats in a register pair
 __device__ __forceinline__ t5_f2 t5_pair(float x, float y) {
     t5_f2 d;

@@ -1232,24 +1232,27 @@ def latent_norms(src: torch.Tensor, q_off: int, c_off: int, q_norm: torch.Tensor
 # takes as long as by FMAs (9.6 us against 9.0 at 1,024 x 1,024, 14 against 17 at 2,048 x 2,048) and many rows a third
 SPLIT_MIN_ELEMENTS = 1 << 20
 SPLIT_MIN_INPUTS = 512
-SPLIT_SPACE = 1 << 27          # bytes of the parts of A at a time
+SPLIT_SPACE = 1 << 27          # bytes of the parts of A and of the sums at a time
+SPLIT_MAX_COLUMNS = 1 << 24    # (the kernel's limit)
 
 
 def _sgemm(l, a: torch.Tensor, lda: int, w: torch.Tensor, out: torch.Tensor, ldc: int) -> None:
     """Which of the two float32 products runs follows from the weight alone, so that a row's bits do not depend on the step."""
     (m, k), n = a.shape, w.shape[0]
-    if n * k < SPLIT_MIN_ELEMENTS or k < SPLIT_MIN_INPUTS or k % 4 or w.data_ptr() % 16 or m == 0:
+    if n * k < SPLIT_MIN_ELEMENTS or n > SPLIT_MAX_COLUMNS or k < SPLIT_MIN_INPUTS or k % 4 or w.data_ptr() % 16 or m == 0:
         check(l.gi_sgemm_nt(_ptr(a), _ptr(w), _ptr(out), m, n, k, lda, ldc, _stream()), l)
         return
-    row_bytes = 6 * ((k + 7) // 8 * 8)
-    rows = min(m, max(128, SPLIT_SPACE // row_bytes // 128 * 128))
-    flag = _ptr(tcgen05_error_flag(a.device))
-    for r in range(0, m, rows):
-        part = min(rows, m - r)
+    flag, r = _ptr(tcgen05_error_flag(a.device)), 0
+    while r < m:
+        part = min(m - r, max(128, SPLIT_SPACE // (6 * ((k + 7) // 8 * 8)) // 128 * 128))
         size = l.gi_sgemm_split_space(part, n, k)
+        while size > SPLIT_SPACE and part > 16:            # (the sums of inputs that blocks share)
+            part = -(-part // 2)
+            size = l.gi_sgemm_split_space(part, n, k)
         space = torch.empty(size, dtype=torch.uint8, device=a.device)
         check(l.gi_sgemm_split_nt(_ptr(a[r:]), _ptr(w), _ptr(out[r:]), _ptr(space), size, part, n, k, lda, ldc, 0, 0, flag, _stream()), l)
         counters.launches += l.gi_sgemm_split_launches(part, n, k) - 1
+        r += part
 
 
 def sgemm_nt(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

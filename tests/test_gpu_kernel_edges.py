@@ -341,6 +341,49 @@ def test_every_form_of_the_float32_product_gives_the_same_bits(M, N, K):
     kernels.check_bounded_waits(DEV)
 
 
+@pytest.mark.parametrize("a_scale, w_scale", [(1e-36, 1.0), (1e-40, 1e20), (1.0, 1e-36), (1e25, 1e-42), (1e-22, 1e-21), (1e13, 1e14), (1e30, 1e-3), (2e37, 1e-30)])
+def test_float32_product_of_small_and_large_numbers(a_scale, w_scale):
+    """Numbers from below the smallest normal one to near the largest, in every form: within the error of float32 sums, of results below the
+    normal ones too."""
+    from garlic_inference_b200.ops import kernels
+    from garlic_inference_b200.ops.library import check, require_gpu
+    l, flag, N, K = require_gpu(), kernels.tcgen05_error_flag(torch.device(DEV, 0)), 260, 640
+    for M in (3, 70):
+        a, w = rnd(M, K, seed=1, scale=a_scale), rnd(N, K, seed=2, scale=w_scale)
+        want, tol = a.double() @ w.double().T, (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + K * 2.0 ** -149
+        space = torch.empty(6 * M * K + 4 * M * N * (K // 64) + 512, dtype=torch.uint8, device=DEV)
+        for tile in (16, 32, 64, 96, 128):
+            for shares in (1, 3):
+                out = torch.full((M, N), 7.0, device=DEV)
+                check(l.gi_sgemm_split_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), space.data_ptr(), space.numel(), M, N, K, K, N, tile, shares,
+                                          flag.data_ptr(), 0), l)
+                assert ((out.double() - want).abs() <= tol).all(), (M, tile, shares)
+
+
+@pytest.mark.parametrize("space", [1 << 17, 1 << 20])
+def test_float32_product_some_rows_at_a_time(space, monkeypatch):
+    """Portions of 11 to 128 rows, as many as fit the work space or half and half again, rows that lie apart on both sides: every row's bits
+    alone, the columns beside left alone, the launches counted."""
+    from garlic_inference_b200.ops import kernels
+    M, N, K = 300, 1030, 1024
+    w, full = rnd(N, K, seed=1), rnd(M, K + 5, seed=2)
+    alone = torch.cat([kernels.sgemm_nt(full[r:r + 1, :K].contiguous(), w) for r in range(M)])
+    monkeypatch.setattr(kernels, "SPLIT_SPACE", space)
+    l, out = kernels.require_gpu(), torch.full((M, N + 3), 7.0, device=DEV)
+    before = kernels.counters.launches
+    kernels.sgemm_nt_strided(full[:, :K], w, out[:, :N])
+    want, r, parts = 0, 0, []
+    while r < M:
+        parts.append(min(M - r, 128))
+        while parts[-1] > 16 and l.gi_sgemm_split_space(parts[-1], N, K) > space:
+            parts[-1] = -(-parts[-1] // 2)
+        want, r = want + l.gi_sgemm_split_launches(parts[-1], N, K), r + parts[-1]
+    assert len(parts) > 2
+    assert kernels.counters.launches - before == want
+    assert torch.equal(out[:, :N], alone) and bool((out[:, N:] == 7.0).all())
+    kernels.check_bounded_waits(DEV)
+
+
 @pytest.mark.parametrize("M, N", [(5, 1000), (64, 512), (130, 260)])
 def test_float32_product_of_long_rows(M, N):
     """Rings that go round many times in every form, with the sums kept and left in memory, W not in the L2 cache: the same bits time after
