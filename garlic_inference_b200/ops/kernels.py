@@ -1731,7 +1731,9 @@ def attention_decode_tcgen05(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torc
                                         _ptr(tok_slot), _ptr(part_o), _ptr(part_ml), _ptr(out), n, n_q, n_kv, d, page_size,
                                         block_table.shape[1], n_pages, int(window or 0), float(scale), n_splits, n_places,
                                         _ptr(tcgen05_error_flag(q.device)), _stream()), l)
-    if n_splits > 1:                                 # one slice: the kernel wrote the output itself
+    if n_places:                                     # the merge, behind the same entry point
+        counters.launches += 1
+    elif n_splits > 1:                               # one slice: the kernel wrote the output itself
         check(l.gi_attention_decode_combine(_ptr(part_o), _ptr(part_ml), _ptr(out), n * n_q, d, n_splits, _stream()), l)
     return out
 

@@ -142,8 +142,14 @@ def time_attention() -> None:
                                                                             HEAD_DIM ** -0.5, 0)) for p in pools])
             print(f"attn_decode batch={batch:3d} ctx={ctx}  mma.sync {ms * 1e3:7.1f} us  {nbytes / ms / 1e6:5.0f} GB/s  "
                   f"tcgen05 {ms2 * 1e3:7.1f} us  {nbytes / ms2 / 1e6:5.0f} GB/s  "
-                  f"(slices {kernels.decode_splits(batch, N_KV)} / {kernels.decode_splits_tcgen05(batch, N_KV)})", flush=True)
+                  f"(slices {kernels.decode_splits(batch, N_KV)} / {_slices(batch)})", flush=True)
             del pools
+
+
+def _slices(batch: int) -> str:
+    """How the tcgen05 decode kernel cuts the keys of a batch."""
+    places = kernels.decode_places_tcgen05(batch, N_KV)
+    return f"{places} places over all sequences" if places else f"{kernels.decode_splits_tcgen05(batch, N_KV)} a sequence"
 
 
 def time_attention_long() -> None:
@@ -157,7 +163,7 @@ def time_attention_long() -> None:
             ms = graph_time([(lambda p=p: kernels.attention_decode_tcgen05(q, p[0], p[1], table, pos, slot,
                                                                            HEAD_DIM ** -0.5, 0)) for p in pools])
             print(f"attn_decode batch={batch:3d} ctx={ctx:6d}  tcgen05 {ms * 1e3:7.1f} us  {nbytes / ms / 1e6:5.0f} GB/s  "
-                  f"({kernels.decode_splits_tcgen05(batch, N_KV)} slices)", flush=True)
+                  f"({_slices(batch)})", flush=True)
             del pools
     for m in (8192, 16384):
         n_pages = m // PAGE

@@ -758,6 +758,29 @@ def test_attention_decode_tcgen05_finds_one_far_key():
     assert int(K().tcgen05_error_flag(q.device).item()) == 0
 
 
+@pytest.mark.parametrize("n, n_kv", [(8, 8), (20, 4), (32, 8), (64, 2), (40, 8)])
+def test_attention_decode_tcgen05_finds_a_far_key_of_every_sequence(n, n_kv):
+    """Uneven sequences in slices of one length (and the longest first, without): in each one key carries all the weight, at edges of tiles of
+    64, at both ends and between, and its value comes out; the kernels behind the call are counted."""
+    d, page, n_q = 128, 64, 2 * n_kv
+    lens = [1500, 1, 64, 65, 700, 128, 129, 321][:n] + [1 + (i * 397) % 1100 for i in range(8, n)]
+    k_pool, v_pool, bt, kd, vd = make_cache(n, lens, n_kv, d, page, torch.bfloat16, seed=n)
+    pos, slot = (torch.tensor(a, dtype=torch.int32, device=DEV) for a in ([m - 1 for m in lens], list(range(n))))
+    places = K().decode_places_tcgen05(n, n_kv)
+    assert (places > 0) == (n * n_kv <= 256)
+    for at in (0.0, 1.0, 0.5, 0.25, 0.8):
+        for edge in (-1, 0):
+            far = [min(m - 1, max(0, int(at * m) // 64 * 64 + edge if 0.0 < at < 1.0 else int(at * m) - (at == 1.0))) for m in lens]
+            q = torch.stack([torch.stack([kd[s][far[s], h // 2] * 2.0 for h in range(n_q)]) for s in range(n)]).to(torch.bfloat16)
+            before = K().counters.launches
+            out = K().attention_decode_tcgen05(q, k_pool, v_pool, bt, pos, slot, 1.0, 0).float().view(n, n_q, d)
+            assert K().counters.launches - before == (2 if places or K().decode_splits_tcgen05(n, n_kv) > 1 else 1)
+            for s in range(n):
+                want = torch.stack([vd[s][far[s], h // 2] for h in range(n_q)]).float()
+                torch.testing.assert_close(out[s], want, rtol=2e-2, atol=2e-2, msg=lambda msg: f"sequence {s} of {lens[s]}, key {far[s]}: {msg}")
+    assert int(K().tcgen05_error_flag(q.device).item()) == 0
+
+
 @pytest.mark.parametrize("kernel", ["decode", "prefill"])
 def test_tcgen05_attention_over_thousands_of_keys(kernel):
     """4,100 cached keys (65 tiles, 16 slices in the decode kernel): one far key that carries all the weight is
