@@ -1694,8 +1694,11 @@ def decode_places_tcgen05(n_seqs: int, n_kv: int) -> int:
     (`decode_splits_tcgen05`).  The lengths are known on the device alone, the places are fixed per batch size.  As many CTAs as a B200
     holds at once (296): 20 sequences of up to 4,000 tokens in a step of 32 rows, 8 heads: 45 / 41 / 49 us at 256 / 296 / 444 CTAs.
     Beyond 256 (sequence, head) pairs a cut does not pay for the merge (48 sequences in 64 rows: 81 us in two slices of each, 76 whole and the
-    longest first); a single sequence divides evenly anyway; the kernel orders 64 sequences at most."""
-    return max(n_seqs, min(16 * n_seqs, 296 // n_kv)) if 2 <= n_seqs <= 64 and n_seqs * n_kv <= 256 else 0
+    longest first); few sequences or pairs divide evenly enough, and finding a slice costs a microsecond or two, which even sequences pay for
+    uneven ones.  Recorded, as many slices of each / so: 2 of 50 and 4,000 tokens, 8 heads, 15.8 / 17.3, 3 of up to 4,000 17.0 / 18.6, 5 of
+    up to 6,000 with 4 heads 20.4 / 20.2, with 8 30.8 / 27.8, 10 of up to 6,000 52 / 41, 20 of up to 4,000 in 32 rows 65 / 49; 8 of 2,048
+    22.8 / 24.0, 16 of 500 16.3 / 16.6, 32 of 100 9.2 / 10.7, 32 of 2,000 59 / 62.  The kernel orders 64 sequences at most."""
+    return max(n_seqs, min(16 * n_seqs, 296 // n_kv)) if 8 <= n_seqs <= 64 and 64 <= n_seqs * n_kv <= 256 else 0
 
 
 def tcgen05_decode_takes(dtype: torch.dtype, head_dim: int, page_size: int, group: int) -> bool:

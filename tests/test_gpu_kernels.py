@@ -767,7 +767,7 @@ def test_attention_decode_tcgen05_finds_a_far_key_of_every_sequence(n, n_kv):
     k_pool, v_pool, bt, kd, vd = make_cache(n, lens, n_kv, d, page, torch.bfloat16, seed=n)
     pos, slot = (torch.tensor(a, dtype=torch.int32, device=DEV) for a in ([m - 1 for m in lens], list(range(n))))
     places = K().decode_places_tcgen05(n, n_kv)
-    assert (places > 0) == (n * n_kv <= 256)
+    assert (places > 0) == (64 <= n * n_kv <= 256)
     for at in (0.0, 1.0, 0.5, 0.25, 0.8):
         for edge in (-1, 0):
             far = [min(m - 1, max(0, int(at * m) // 64 * 64 + edge if 0.0 < at < 1.0 else int(at * m) - (at == 1.0))) for m in lens]

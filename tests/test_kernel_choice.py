@@ -12,3 +12,10 @@ from garlic_inference_b200.ops import kernels
     ([100] * 8, 16, 128, True, False), ([40], 16, 128, True, False)])
 def test_delta_rule_in_chunks_or_token_by_token(lens, heads, d, channel, chunks):
     assert kernels._delta_in_chunks(sum(lens), len(lens), heads, d, d, channel) == chunks
+
+
+@pytest.mark.parametrize("n, heads, cut", [(1, 8, False), (2, 8, False), (4, 16, False), (8, 4, False), (8, 8, True), (16, 4, True), (32, 8, True),
+                                           (64, 4, True), (33, 8, False), (65, 2, False), (64, 8, False)])
+def test_decode_attention_in_slices_of_one_length(n, heads, cut):
+    places = kernels.decode_places_tcgen05(n, heads)
+    assert (places > 0) == cut and (not cut or n <= places <= 16 * n)
