@@ -146,7 +146,8 @@ __device__ __forceinline__ int fd_ceil_div(int a, int b) { return (a + b - 1) / 
 // left.  Every sequence's tiles are cut into the fewest slices of at most `per` tiles, `per` the least with which all slices have a place
 // (n_seqs <= n_places).  Sequences of one length get what an even division gives them.  Without `cut` every sequence, rows that are none too,
 // has one place.  With `sorted` the longest slices come first: CTAs start in grid order, and a long one that starts last leaves the other
-// SMs idle.  A microsecond before the wait for the step's other kernels, beside the tensor memory's allocation.
+// SMs idle.  One to two microseconds in front of a CTA's first copy: what even sequences pay for uneven ones.  A sequence's sums are cut by
+// the lengths of its neighbours too, so its bits depend on them.
 // Measured on a B200 (standalone, 8 key/value heads, lengths spread over 5 to 100 %; as many slices of each, in the order given -> here):
 // 5 sequences up to 6,000 in a step of 8 rows 30 -> 22 us, 10 in 16 52 -> 34; 20 up to 4,000 in 32 63 -> 41, 48 in 64 (sorted) 89 -> 76;
 // 64 up to 2,900 87 -> 67.  Even lengths: 64 of 2,048 85 -> 87, 32 of 3,000 64 -> 66, 8 of 3,000 22 -> 24 (in a recorded step of 8 the same).

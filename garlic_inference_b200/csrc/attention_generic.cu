@@ -230,8 +230,8 @@ static int launch_generic(const void* q, const void* k_pool, const void* v_pool,
 // the first tokens' in front.  Chunks, warps, sums and their order are
 // the kernel's above for every row, and so are the bits.
 // Bound above by the fetches (a block read every key and value of its token for one head, a key's row to a lane); here by the
-// multiply-adds and the operands' reads from shared memory.  Measured, two sequences of up to 300 tokens, 16 heads of 128 on 4 key heads: 213 us a
-// row to a block, 98 us so.
+// multiply-adds and the operands' reads from shared memory.  Measured, sequences of 300 and 200 tokens, 16 heads of 128 on 4 key heads: 223 us a
+// row to a block, 92 us so (109 where a block took its tokens' sequences in turn).
 template <int DPL, int HR, int TQ>
 __global__ void __launch_bounds__(AG_WARPS * 32)
 attn_shared_rows_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,

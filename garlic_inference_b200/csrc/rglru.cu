@@ -11,9 +11,10 @@
 //                    with act the tanh form of gelu, rounded once into the activation type.
 //
 // The gate matrices arrive transposed, [blocks, in, out]; a block of threads keeps a slice of output channels of
-// both matrices in shared memory and streams tiles of tokens past them.  Every sum runs in an order that depends on
-// the block width alone, and the scan walks a sequence's tokens in order, so a position's bits do not depend on
-// how the tokens were cut into steps or on the batch.  NikolayBlagoev/garlic-inference has no recurrent mixer.
+// both matrices in shared memory and streams tiles of tokens past them.  In this file every sum runs in an order that depends on
+// the block width alone, and the scan walks a sequence's tokens in order: in the 32-bit engine a position's bits do not depend on
+// how the tokens were cut into steps or on the batch.  In bfloat16 steps of many rows have their gates from rglru_tcgen05.cu, as
+// precise but with other bits, so there they follow the step's row count.  NikolayBlagoev/garlic-inference has no recurrent mixer.
 #include "rglru.cuh"
 
 #define RG_KS 8              // lanes that share an output: lane s sums the inputs k = s, s + 8, s + 16, ...
