@@ -8,8 +8,8 @@
 //   warps 0..3     split u: TMA brings 128 rows x 64 inputs, a lane takes a row and puts its parts into tensor memory
 //   warps 4..19    add the sums up and make a and b from them: four groups of four, 16 outputs of both gates each
 //   warps 20..22   TMA of u, TMA of both matrices, products
-// Bound by what is done one after another for an item: of the 12.5 us that one takes at 16 blocks of 320 its products are about 2 and the
-// issue of what comes after the sums, some 100 instructions for an output, about 3.3; all adders wait for one item at a time.
+// Bound by what is done one after another for an item: products, sums and then some 100 instructions for an output, while all adders wait
+// for one item at a time.  At 16 blocks of 320 the tensor core is busy for 16 % of the time, the issue slots for 56 %.
 // Measured, 16 blocks of 320, 2,494 rows: 213 us by mma.sync (rglru.cu: three legacy products and four adds for every 16 inputs, and 250
 // instructions an output), 192 us so, 138 us with the divisions and roots below.  Relative errors of b (2-norm) against 64 bits in
 // units of 1e-8, mma.sync / so: blocks of 64 7.4 / 7.5, 72 7.6 / 7.6, 320 8.0 / 7.8, 1,280 9.6 / 8.3; inputs of three times the size 8.9 / 8.4;
